@@ -17,8 +17,8 @@
 //   dL/dp   = (dL/dn - n (n.dL/dn)) / |p|
 // with g = dL/drgb.  Gradients are summed over rays with atomics; lanes of a
 // warp that hit the same leaf are first reduced in registers (match_any +
-// a rank-ordered shuffle tree), so one lane per distinct leaf issues the six
-// atomicAdds.  Summation order across warps is not fixed, so gradients can
+// pointer jumping along each leaf's lanes), so one lane per distinct leaf
+// issues the atomics.  Summation order across warps is not fixed, so gradients can
 // differ in the last bits between runs.
 #include "svo_device.cuh"
 #include "svo_internal.h"
@@ -41,7 +41,6 @@ struct DiffArgs {
     float *rgb;
     const float *d_rgb;
     float *g_rgb, *g_n;
-    unsigned long long *queue;
     uint32_t *status;
     // fused L2 loss (svo_diff_backward_l2): dL/drgb = loss_scale (rgb - target)
     const float *target;
@@ -70,11 +69,36 @@ struct Shading {
     float nx, ny, nz, inv_len, ln, a, nd, s;
 };
 
-__device__ __forceinline__ Shading shade_terms(const float *p_n, uint32_t stride, uint32_t leaf, float dx, float dy,
-                                               float dz, float lx, float ly, float lz) {
+struct LeafParams {
+    float c[3], p[3];  // colour and (unnormalised) normal
+};
+
+// kRec: colour and normal share one 16-byte aligned record (the normal at
+// floats 3..5), read as a float4 and a float2 instead of six floats.
+template <bool kRec>
+__device__ __forceinline__ LeafParams load_leaf(const DiffArgs &a, uint32_t leaf) {
+    LeafParams l;
+    const float *c = a.p_rgb + (uint64_t)a.stride * leaf;
+    if constexpr (kRec) {
+        const float4 q = __ldg(reinterpret_cast<const float4 *>(c));
+        const float2 r = __ldg(reinterpret_cast<const float2 *>(c + 4));
+        l.c[0] = q.x; l.c[1] = q.y; l.c[2] = q.z;
+        l.p[0] = q.w; l.p[1] = r.x; l.p[2] = r.y;
+    } else {
+        const float *p = a.p_n + (uint64_t)a.stride * leaf;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            l.c[k] = __ldg(c + k);
+            l.p[k] = __ldg(p + k);
+        }
+    }
+    return l;
+}
+
+__device__ __forceinline__ Shading shade_terms(const LeafParams &l, float dx, float dy, float dz, float lx, float ly,
+                                               float lz) {
     Shading sh;
-    const float *pn = p_n + (uint64_t)stride * leaf;
-    float px = pn[0], py = pn[1], pz = pn[2];
+    const float px = l.p[0], py = l.p[1], pz = l.p[2];
     float len2 = px * px + py * py + pz * pz;
     sh.inv_len = len2 > 0.0f ? 1.0f / sqrtf(len2) : 0.0f;
     sh.nx = px * sh.inv_len;
@@ -89,67 +113,72 @@ __device__ __forceinline__ Shading shade_terms(const float *p_n, uint32_t stride
     return sh;
 }
 
-// Slots a warp takes from the queue at once (multiples of 32): a forward
-// warp traces one 8x4 tile at a time; the adjoint, without traversal, is
-// short per slot, so it takes several tiles per queue access.
-constexpr int kFwdChunk = 64;
-constexpr int kBwdChunk = 128;
+// Threads per CTA of the tracing kernels (forward, and the adjoint that traces
+// again).  A warp traces one 8x4 tile; the hardware starts the next CTA where
+// one has finished, so no work counter is read or reset, and a small image
+// has every tile in flight at once.  The persistent form before it gave a
+// warp 2 (forward) or 4 (adjoint) tiles per counter access, one after another:
+// a 3-view 333x251 image took 83 us forward and now takes 52, 12 views of
+// 512x512 took 164 and take 145 (256^3 scenes, 30-45 dependent steps a ray).
+// Whole steps with 32, 64, 128 and 256 threads: 240, 225, 222 and 224 us.
+constexpr int kTraceThreads = 128;
 
-template <bool kTab, bool kRecord>
-__global__ void k_diff_forward(DiffArgs a) {
-    const int lane = threadIdx.x & 31;
+template <bool kTab, bool kRecord, bool kRec>
+__global__ void __launch_bounds__(kTraceThreads) k_diff_forward(DiffArgs a) {
+    const uint64_t slot = (uint64_t)blockIdx.x * kTraceThreads + threadIdx.x;
     RayStackFor<kTab> stk;
-    unsigned long long base = 0, end = 0;
-    while (true) {
-        if (base >= end) {
-            if (lane == 0) base = atomicAdd(a.queue, (unsigned long long)kFwdChunk);
-            base = __shfl_sync(0xffffffffu, base, 0);
-            if (base >= a.total) break;
-            end = min(base + (unsigned long long)kFwdChunk, (unsigned long long)a.total);
-        }
-        const unsigned long long slot = base + lane;
-        base += 32;
-        uint32_t idx, view;
-        if (!tile_pixel(a, slot, idx, view)) continue;
-        const float2 *r2 = reinterpret_cast<const float2 *>(a.rays) + 3 * (uint64_t)idx;
-        float2 p0 = __ldg(r2), p1 = __ldg(r2 + 1), p2 = __ldg(r2 + 2);
-        RayState st;
-        ray_init_any<kTab>(st, a.oct, a.tab, p0.x, p0.y, p1.x, p1.y, p2.x, p2.y);
-        RayResult res;
-        while (!ray_step_any<kTab, false>(st, stk, a.oct, a.tab, a.n_words, 0.0f, res)) {
-        }
-        if (res.status == kFault) atomicOr(a.status, 1u);
-        bool hit = res.status == kLeafHit;
-        if (kRecord) a.hit_leaf[idx] = hit ? res.leaf : 0xFFFFFFFFu;
-        float c0 = 0.0f, c1 = 0.0f, c2 = 0.0f;
-        if (hit) {
-            float lx = a.lights[3 * view], ly = a.lights[3 * view + 1], lz = a.lights[3 * view + 2];
-            Shading sh = shade_terms(a.p_n, a.stride, res.leaf, p1.y, p2.x, p2.y, lx, ly, lz);
-            float spec = sh.s * sh.s * 0.2f;
-            const float *c = a.p_rgb + (uint64_t)a.stride * res.leaf;
-            c0 = c[0] * 0.9f * sh.a + spec;
-            c1 = c[1] * 0.9f * sh.a + spec;
-            c2 = c[2] * 0.9f * sh.a + spec;
-        }
-        a.rgb[3 * (uint64_t)idx] = c0;
-        a.rgb[3 * (uint64_t)idx + 1] = c1;
-        a.rgb[3 * (uint64_t)idx + 2] = c2;
+    uint32_t idx, view;
+    if (!tile_pixel(a, slot, idx, view)) return;
+    const float2 *r2 = reinterpret_cast<const float2 *>(a.rays) + 3 * (uint64_t)idx;
+    float2 p0 = __ldg(r2), p1 = __ldg(r2 + 1), p2 = __ldg(r2 + 2);
+    RayState st;
+    ray_init_any<kTab>(st, a.oct, a.tab, p0.x, p0.y, p1.x, p1.y, p2.x, p2.y);
+    RayResult res;
+    while (!ray_step_any<kTab, false>(st, stk, a.oct, a.tab, a.n_words, 0.0f, res)) {
     }
+    if (res.status == kFault) atomicOr(a.status, 1u);
+    bool hit = res.status == kLeafHit;
+    if (kRecord) a.hit_leaf[idx] = hit ? res.leaf : 0xFFFFFFFFu;
+    float c0 = 0.0f, c1 = 0.0f, c2 = 0.0f;
+    if (hit) {
+        float lx = a.lights[3 * view], ly = a.lights[3 * view + 1], lz = a.lights[3 * view + 2];
+        const LeafParams l = load_leaf<kRec>(a, res.leaf);
+        Shading sh = shade_terms(l, p1.y, p2.x, p2.y, lx, ly, lz);
+        float spec = sh.s * sh.s * 0.2f;
+        c0 = l.c[0] * 0.9f * sh.a + spec;
+        c1 = l.c[1] * 0.9f * sh.a + spec;
+        c2 = l.c[2] * 0.9f * sh.a + spec;
+    }
+    a.rgb[3 * (uint64_t)idx] = c0;
+    a.rgb[3 * (uint64_t)idx + 1] = c1;
+    a.rgb[3 * (uint64_t)idx + 2] = c2;
 }
 
-// Sum of v over the lanes in `peers` (the lanes holding the same key), left
-// in the group's lowest lane.  Lane ranks within the group form a binary
-// tree: at distance k a lane whose rank is a multiple of 2k adds the value of
-// the group member k ranks above it.  All 32 lanes execute every shuffle.
-__device__ __forceinline__ float group_sum(unsigned peers, unsigned rank, unsigned size, float v) {
-    for (unsigned k = 1; k < 32; k <<= 1) {
-        unsigned src_rank = rank + k;
-        bool take = (rank % (2 * k)) == 0 && src_rank < size;
-        int src = take ? (int)__fns(peers, 0, (int)src_rank + 1) : (int)(threadIdx.x & 31);
-        float o = __shfl_sync(0xffffffffu, v, src);
-        if (take) v += o;
+// Sums v[0..5] over the lanes in `peers` (the lanes holding the same key) into
+// the group's lowest lane.  Pointer jumping: every lane adds the partial sum
+// of the next lane of its group and then points past what it has covered, so
+// after k rounds the lane of rank r holds ranks r .. r + 2^k - 1, and the
+// largest group of the warp sets the number of rounds (none in a warp of
+// distinct leaves, five at most).  All 32 lanes execute every shuffle.  The
+// sums are those of a binary tree over the ranks.  Finding each partner with
+// __fns (a software search, five per value) bound the adjoint by instruction
+// issue: 178 us for 3.1 M rays (12 views of 512x512, 256^3), 47 us with this,
+// of which the 0.22 GB it reads would take 32.
+__device__ __forceinline__ void group_sum6(unsigned peers, float (&v)[6]) {
+    const int lane = threadIdx.x & 31;
+    const unsigned above = peers & (0xfffffffeu << lane);
+    int next = above ? __ffs((int)above) - 1 : 32;
+    while (__any_sync(0xffffffffu, next < 32)) {
+        const bool take = next < 32;
+        const int src = take ? next : lane;
+#pragma unroll
+        for (int k = 0; k < 6; ++k) {
+            const float o = __shfl_sync(0xffffffffu, v[k], src);
+            if (take) v[k] += o;
+        }
+        const int nn = __shfl_sync(0xffffffffu, next, src);
+        next = take ? nn : 32;
     }
-    return v;
 }
 
 // Records `leaf` in the touched set the first time any warp adds a gradient
@@ -162,112 +191,141 @@ __device__ __forceinline__ void mark_touched(const DiffArgs &a, uint32_t leaf) {
     if (pos < a.leaf_cap) a.leaf_list[pos] = leaf;
 }
 
-// kRetrace: recompute the hit leaf by traversal instead of reading hit_leaf.
-// kFused: dL/drgb = loss_scale (rgb - target) from the forward pass's rgb
-// instead of a d_rgb array, and the loss summed on the way.
-template <bool kTab, bool kRetrace, bool kFused>
-__global__ void k_diff_backward(DiffArgs a) {
+// Adds a leaf's six gradient values.  Records (kRec) take one 16-byte and one
+// 8-byte vector reduction, each value added on its own as by atomicAdd.
+template <bool kRec>
+__device__ __forceinline__ void add_gradient(const DiffArgs &a, uint32_t leaf, const float (&v)[6]) {
+    float *gr = a.g_rgb + (uint64_t)a.stride * leaf;
+    if constexpr (kRec) {
+        asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(__cvta_generic_to_global(gr)), "f"(v[0]),
+                     "f"(v[1]), "f"(v[2]), "f"(v[3])
+                     : "memory");
+        asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(__cvta_generic_to_global(gr + 4)), "f"(v[4]),
+                     "f"(v[5])
+                     : "memory");
+    } else {
+        float *gn = a.g_n + (uint64_t)a.stride * leaf;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            atomicAdd(gr + k, v[k]);
+            atomicAdd(gn + k, v[3 + k]);
+        }
+    }
+}
+
+// One 8x4 tile of the adjoint.  kRetrace: recompute the hit leaf by traversal
+// instead of reading hit_leaf.  kFused: dL/drgb = loss_scale (rgb - target)
+// from the forward pass's rgb instead of a d_rgb array; returns this lane's
+// squared error.
+template <bool kTab, bool kRetrace, bool kFused, bool kRec>
+__device__ __forceinline__ float adjoint_tile(const DiffArgs &a, uint64_t slot, RayStackFor<kTab> &stk) {
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
-    const unsigned lt = (1u << lane) - 1u;
+    uint32_t idx = 0, view = 0;
+    const bool live = tile_pixel(a, slot, idx, view);
+    uint32_t leaf = 0xFFFFFFFFu;
+    float dx = 0.f, dy = 0.f, dz = 0.f;
+    if (live) {
+        const float2 *r2 = reinterpret_cast<const float2 *>(a.rays) + 3 * (uint64_t)idx;
+        float2 p1 = __ldg(r2 + 1), p2 = __ldg(r2 + 2);
+        dx = p1.y;
+        dy = p2.x;
+        dz = p2.y;
+        if (kRetrace) {
+            float2 p0 = __ldg(r2);
+            RayState st;
+            ray_init_any<kTab>(st, a.oct, a.tab, p0.x, p0.y, p1.x, dx, dy, dz);
+            RayResult res;
+            while (!ray_step_any<kTab, false>(st, stk, a.oct, a.tab, a.n_words, 0.0f, res)) {
+            }
+            if (res.status == kFault) atomicOr(a.status, 1u);
+            if (res.status == kLeafHit) leaf = res.leaf;
+        } else {
+            leaf = a.hit_leaf[idx];
+        }
+    }
+    float sq = 0.f, g0 = 0.f, g1 = 0.f, g2 = 0.f;
+    if (kFused && live) {
+        // every ray adds to the loss; a miss (rgb 0) contributes no gradient
+        const float *c3 = a.rgb + 3 * (uint64_t)idx, *t3 = a.target + 3 * (uint64_t)idx;
+        const float e0 = c3[0] - t3[0], e1 = c3[1] - t3[1], e2 = c3[2] - t3[2];
+        sq = e0 * e0 + e1 * e1 + e2 * e2;
+        g0 = a.loss_scale * e0;
+        g1 = a.loss_scale * e1;
+        g2 = a.loss_scale * e2;
+    }
+    const bool contrib = leaf != 0xFFFFFFFFu;
+    if (!__any_sync(FULL, contrib)) return sq;  // a tile of background
+    float v[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    if (contrib) {
+        float lx = a.lights[3 * view], ly = a.lights[3 * view + 1], lz = a.lights[3 * view + 2];
+        const LeafParams l = load_leaf<kRec>(a, leaf);
+        Shading sh = shade_terms(l, dx, dy, dz, lx, ly, lz);
+        if (!kFused) {
+            g0 = a.d_rgb[3 * (uint64_t)idx];
+            g1 = a.d_rgb[3 * (uint64_t)idx + 1];
+            g2 = a.d_rgb[3 * (uint64_t)idx + 2];
+        }
+        v[0] = g0 * 0.9f * sh.a;
+        v[1] = g1 * 0.9f * sh.a;
+        v[2] = g2 * 0.9f * sh.a;
+        float sgn = sh.ln > 0.0f ? 1.0f : (sh.ln < 0.0f ? -1.0f : 0.0f);
+        float wl = 0.9f * sgn * (g0 * l.c[0] + g1 * l.c[1] + g2 * l.c[2]);
+        float ws = sh.s > 0.0f ? -0.8f * (g0 + g1 + g2) * sh.s : 0.0f;
+        // dL/dn = wl l + ws ((n.d) l + (n.l) d)
+        float gnx = wl * lx + ws * (sh.nd * lx + sh.ln * dx);
+        float gny = wl * ly + ws * (sh.nd * ly + sh.ln * dy);
+        float gnz = wl * lz + ws * (sh.nd * lz + sh.ln * dz);
+        float ndg = sh.nx * gnx + sh.ny * gny + sh.nz * gnz;
+        v[3] = (gnx - sh.nx * ndg) * sh.inv_len;
+        v[4] = (gny - sh.ny * ndg) * sh.inv_len;
+        v[5] = (gnz - sh.nz * ndg) * sh.inv_len;
+    }
+    // warp aggregation by leaf: one set of atomics per distinct leaf.  Lanes
+    // without a leaf are groups of their own (they would only sum zeros).
+    const unsigned lanes = __ballot_sync(FULL, contrib);
+    const unsigned peers = __match_any_sync(FULL, leaf) & (contrib ? lanes : 1u << lane);
+    group_sum6(peers, v);
+    if (contrib && lane == __ffs((int)peers) - 1) {
+        add_gradient<kRec>(a, leaf, v);
+        if (a.touched) mark_touched(a, leaf);
+    }
+    return sq;
+}
+
+// Adds a warp's squared errors to the loss, one atomic per warp.
+__device__ __forceinline__ void add_loss(const DiffArgs &a, double loss) {
+    for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
+    if ((threadIdx.x & 31) == 0) atomicAdd(a.loss_sum, loss);
+}
+
+// The adjoint over recorded hit leaves: short per tile and even, so the tiles
+// are dealt out by a fixed stride over a resident grid.  A lane's squared
+// errors are summed with the running compensation of Kahan ("Further remarks
+// on reducing truncation errors", 1965), so the loss does not depend on how
+// many tiles a lane takes.
+template <bool kFused, bool kRec>
+__global__ void __launch_bounds__(256) k_diff_backward(DiffArgs a) {
+    RayStackFor<false> stk;  // unused: nothing is traced
+    float loss = 0.0f, comp = 0.0f;
+    const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
+    const uint64_t warp0 = (uint64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u);
+    for (uint64_t s0 = warp0; s0 < a.total; s0 += step) {  // uniform per warp
+        const float sq = adjoint_tile<false, false, kFused, kRec>(a, s0 + (threadIdx.x & 31), stk);
+        const float y = sq - comp, t = loss + y;
+        comp = (t - loss) - y;
+        loss = t;
+    }
+    if (kFused && a.loss_sum) add_loss(a, (double)loss - (double)comp);
+}
+
+// The adjoint that traces again: a tile per warp, as the forward pass.
+template <bool kTab, bool kFused, bool kRec>
+__global__ void __launch_bounds__(kTraceThreads) k_diff_retrace(DiffArgs a) {
     RayStackFor<kTab> stk;
-    float loss = 0.0f;  // this lane's share of sum (rgb - target)^2
-    unsigned long long base = 0, end = 0;
-    while (true) {
-        if (base >= end) {
-            if (lane == 0) base = atomicAdd(a.queue, (unsigned long long)kBwdChunk);
-            base = __shfl_sync(FULL, base, 0);
-            if (base >= a.total) break;
-            end = min(base + (unsigned long long)kBwdChunk, (unsigned long long)a.total);
-        }
-        const unsigned long long slot = base + lane;
-        base += 32;
-        uint32_t idx = 0, view = 0;
-        bool live = tile_pixel(a, slot, idx, view);
-        uint32_t leaf = 0xFFFFFFFFu;
-        float dx = 0.f, dy = 0.f, dz = 0.f;
-        if (live) {
-            const float2 *r2 = reinterpret_cast<const float2 *>(a.rays) + 3 * (uint64_t)idx;
-            float2 p1 = __ldg(r2 + 1), p2 = __ldg(r2 + 2);
-            dx = p1.y;
-            dy = p2.x;
-            dz = p2.y;
-            if (kRetrace) {
-                float2 p0 = __ldg(r2);
-                RayState st;
-                ray_init_any<kTab>(st, a.oct, a.tab, p0.x, p0.y, p1.x, dx, dy, dz);
-                RayResult res;
-                while (!ray_step_any<kTab, false>(st, stk, a.oct, a.tab, a.n_words, 0.0f, res)) {
-                }
-                if (res.status == kFault) atomicOr(a.status, 1u);
-                if (res.status == kLeafHit) leaf = res.leaf;
-            } else {
-                leaf = a.hit_leaf[idx];
-            }
-        }
-        float gc0 = 0.f, gc1 = 0.f, gc2 = 0.f, gp0 = 0.f, gp1 = 0.f, gp2 = 0.f;
-        bool contrib = leaf != 0xFFFFFFFFu;
-        float g0 = 0.f, g1 = 0.f, g2 = 0.f;
-        if (kFused && live) {
-            // every ray adds to the loss; a miss (rgb 0) contributes no gradient
-            const float *c3 = a.rgb + 3 * (uint64_t)idx, *t3 = a.target + 3 * (uint64_t)idx;
-            const float e0 = c3[0] - t3[0], e1 = c3[1] - t3[1], e2 = c3[2] - t3[2];
-            loss += e0 * e0 + e1 * e1 + e2 * e2;
-            g0 = a.loss_scale * e0;
-            g1 = a.loss_scale * e1;
-            g2 = a.loss_scale * e2;
-        }
-        if (contrib) {
-            float lx = a.lights[3 * view], ly = a.lights[3 * view + 1], lz = a.lights[3 * view + 2];
-            Shading sh = shade_terms(a.p_n, a.stride, leaf, dx, dy, dz, lx, ly, lz);
-            const float *c = a.p_rgb + (uint64_t)a.stride * leaf;
-            if (!kFused) {
-                g0 = a.d_rgb[3 * (uint64_t)idx];
-                g1 = a.d_rgb[3 * (uint64_t)idx + 1];
-                g2 = a.d_rgb[3 * (uint64_t)idx + 2];
-            }
-            gc0 = g0 * 0.9f * sh.a;
-            gc1 = g1 * 0.9f * sh.a;
-            gc2 = g2 * 0.9f * sh.a;
-            float sgn = sh.ln > 0.0f ? 1.0f : (sh.ln < 0.0f ? -1.0f : 0.0f);
-            float wl = 0.9f * sgn * (g0 * c[0] + g1 * c[1] + g2 * c[2]);
-            float ws = sh.s > 0.0f ? -0.8f * (g0 + g1 + g2) * sh.s : 0.0f;
-            // dL/dn = wl l + ws ((n.d) l + (n.l) d)
-            float gnx = wl * lx + ws * (sh.nd * lx + sh.ln * dx);
-            float gny = wl * ly + ws * (sh.nd * ly + sh.ln * dy);
-            float gnz = wl * lz + ws * (sh.nd * lz + sh.ln * dz);
-            float ndg = sh.nx * gnx + sh.ny * gny + sh.nz * gnz;
-            gp0 = (gnx - sh.nx * ndg) * sh.inv_len;
-            gp1 = (gny - sh.ny * ndg) * sh.inv_len;
-            gp2 = (gnz - sh.nz * ndg) * sh.inv_len;
-        }
-        // warp aggregation by leaf: one set of atomics per distinct leaf
-        unsigned peers = __match_any_sync(FULL, leaf);
-        unsigned rank = __popc(peers & lt), size = __popc(peers);
-        gc0 = group_sum(peers, rank, size, gc0);
-        gc1 = group_sum(peers, rank, size, gc1);
-        gc2 = group_sum(peers, rank, size, gc2);
-        gp0 = group_sum(peers, rank, size, gp0);
-        gp1 = group_sum(peers, rank, size, gp1);
-        gp2 = group_sum(peers, rank, size, gp2);
-        if (contrib && rank == 0) {
-            float *gr = a.g_rgb + (uint64_t)a.stride * leaf;
-            float *gn = a.g_n + (uint64_t)a.stride * leaf;
-            atomicAdd(gr, gc0);
-            atomicAdd(gr + 1, gc1);
-            atomicAdd(gr + 2, gc2);
-            atomicAdd(gn, gp0);
-            atomicAdd(gn + 1, gp1);
-            atomicAdd(gn + 2, gp2);
-            if (a.touched) mark_touched(a, leaf);
-        }
-    }
-    if (kFused && a.loss_sum) {
-        // one atomic per warp, at its end (a per-pass atomic on one address
-        // would serialise the warps)
-        for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(FULL, loss, o);
-        if (lane == 0) atomicAdd(a.loss_sum, (double)loss);
-    }
+    const uint64_t slot = (uint64_t)blockIdx.x * kTraceThreads + threadIdx.x;
+    const float sq = adjoint_tile<kTab, true, kFused, kRec>(a, slot, stk);
+    if (kFused && a.loss_sum) add_loss(a, (double)sq);
 }
 
 int prepare(const svo_octree *oct, const float *rays, uint32_t width, uint32_t height, uint32_t n_views,
@@ -290,21 +348,58 @@ int prepare(const svo_octree *oct, const float *rays, uint32_t width, uint32_t h
     a.p_rgb = p_rgb;
     a.p_n = p_n;
     a.stride = stride;
-    a.queue = oct->d_queue;
     a.status = oct->d_status;
     return SVO_OK;
 }
 
+// Whether the parameters form records that can be read as a float4 and a
+// float2: the normal three floats after the colour, every record on a 16-byte
+// boundary and at least six floats long.
+bool records(const float *rgb, const float *normal, uint32_t stride) {
+    return normal == rgb + 3 && stride >= 6 && stride % 4 == 0 && (reinterpret_cast<uintptr_t>(rgb) & 15) == 0;
+}
+
 template <typename K>
-int launch_persistent(K kern, const DiffArgs &a, cudaStream_t st) {
+int launch_tiles(K kern, const DiffArgs &a, cudaStream_t st) {
+    const uint64_t ctas = (a.total + kTraceThreads - 1) / kTraceThreads;  // at most 2^35 slots (a 1-pixel-wide view pads 8-fold)
+    kern<<<(unsigned)ctas, kTraceThreads, 0, st>>>(a);
+    SVO_CUDA_TRY(cudaGetLastError());
+    return SVO_OK;
+}
+
+template <typename K>
+int launch_resident(K kern, const DiffArgs &a, cudaStream_t st) {
     int dev = 0, sms = 0, resident = 0;
     SVO_CUDA_TRY(cudaGetDevice(&dev));
     SVO_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     SVO_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kern, 256, 0));
-    SVO_CUDA_TRY(cudaMemsetAsync(a.queue, 0, sizeof(unsigned long long), st));
-    kern<<<(unsigned)(sms * (resident > 0 ? resident : 1)), 256, 0, st>>>(a);
+    const uint64_t need = (a.total + 255) / 256, fit = (uint64_t)sms * (resident > 0 ? resident : 1);
+    kern<<<(unsigned)(need < fit ? need : fit), 256, 0, st>>>(a);
     SVO_CUDA_TRY(cudaGetLastError());
     return SVO_OK;
+}
+
+template <bool kFused>
+int launch_backward(const svo_octree *oct, DiffArgs &a, cudaStream_t st) {
+    const bool rec = records(a.p_rgb, a.p_n, a.stride) && records(a.g_rgb, a.g_n, a.stride);
+    if (a.hit_leaf)
+        return rec ? launch_resident(k_diff_backward<kFused, true>, a, st)
+                   : launch_resident(k_diff_backward<kFused, false>, a, st);
+    a.tab = octree_table(oct, st);  // the table only serves the retrace
+    if (a.tab)
+        return rec ? launch_tiles(k_diff_retrace<true, kFused, true>, a, st)
+                   : launch_tiles(k_diff_retrace<true, kFused, false>, a, st);
+    return rec ? launch_tiles(k_diff_retrace<false, kFused, true>, a, st)
+               : launch_tiles(k_diff_retrace<false, kFused, false>, a, st);
+}
+
+template <bool kTab>
+int launch_forward(const DiffArgs &a, cudaStream_t st) {
+    if (records(a.p_rgb, a.p_n, a.stride))
+        return a.hit_leaf ? launch_tiles(k_diff_forward<kTab, true, true>, a, st)
+                          : launch_tiles(k_diff_forward<kTab, false, true>, a, st);
+    return a.hit_leaf ? launch_tiles(k_diff_forward<kTab, true, false>, a, st)
+                      : launch_tiles(k_diff_forward<kTab, false, false>, a, st);
 }
 
 }  // namespace
@@ -325,11 +420,7 @@ int svo_diff_forward_stride(const svo_octree *oct, const float *rays, uint32_t w
     a.rgb = rgb;
     cudaStream_t st = (cudaStream_t)stream;
     a.tab = octree_table(oct, st);
-    if (a.tab)
-        return hit_leaf ? launch_persistent(k_diff_forward<true, true>, a, st)
-                        : launch_persistent(k_diff_forward<true, false>, a, st);
-    return hit_leaf ? launch_persistent(k_diff_forward<false, true>, a, st)
-                    : launch_persistent(k_diff_forward<false, false>, a, st);
+    return a.tab ? launch_forward<true>(a, st) : launch_forward<false>(a, st);
 }
 
 int svo_diff_backward_stride(const svo_octree *oct, const float *rays, uint32_t width, uint32_t height,
@@ -344,11 +435,7 @@ int svo_diff_backward_stride(const svo_octree *oct, const float *rays, uint32_t 
     a.d_rgb = d_rgb;
     a.g_rgb = grad_rgb;
     a.g_n = grad_normal;
-    cudaStream_t st = (cudaStream_t)stream;
-    a.tab = hit_leaf ? nullptr : octree_table(oct, st);  // the table only serves the retrace
-    if (a.tab) return launch_persistent(k_diff_backward<true, true, false>, a, st);
-    return hit_leaf ? launch_persistent(k_diff_backward<false, false, false>, a, st)
-                    : launch_persistent(k_diff_backward<false, true, false>, a, st);
+    return launch_backward<false>(oct, a, (cudaStream_t)stream);
 }
 
 int svo_diff_backward_l2_stride(const svo_octree *oct, const float *rays, uint32_t width, uint32_t height,
@@ -378,11 +465,7 @@ int svo_diff_backward_l2_stride(const svo_octree *oct, const float *rays, uint32
     a.leaf_list = leaf_list;
     a.leaf_count = leaf_count;
     a.leaf_cap = touched ? (uint32_t)oct->n_words : 0u;
-    cudaStream_t st = (cudaStream_t)stream;
-    a.tab = hit_leaf ? nullptr : octree_table(oct, st);
-    if (a.tab) return launch_persistent(k_diff_backward<true, true, true>, a, st);
-    return hit_leaf ? launch_persistent(k_diff_backward<false, false, true>, a, st)
-                    : launch_persistent(k_diff_backward<false, true, true>, a, st);
+    return launch_backward<true>(oct, a, (cudaStream_t)stream);
 }
 
 // The separate-array forms: 3 floats per leaf in each array.

@@ -329,3 +329,74 @@ def test_leaf_records_match_separate_arrays(cuda, svo, problem):
     assert bool((rec[:, 6:] == 7.0).all())
     with pytest.raises(Exception):
         pb["tree"].diff_forward(*geo, p_rgb, p_n, rgb3, param_stride=2)
+
+
+@pytest.mark.parametrize("retrace", [False, True])
+@pytest.mark.parametrize("side,W,H,V,stride,offset", [
+    (8, 64, 40, 1, 8, 0),    # whole tiles on one leaf: lane groups of up to 32, aligned records
+    (32, 37, 5, 3, 8, 0),    # ragged tiles that span views
+    (32, 1, 9, 1, 3, 0),     # a one-pixel-wide image, separate arrays
+    (64, 33, 17, 2, 8, 1),   # records off the 16-byte boundary: the scalar path
+    (64, 33, 17, 2, 12, 0),  # longer records
+    (64, 33, 17, 2, 7, 0),   # a stride no vector load fits
+])
+def test_adjoint_layouts_and_lane_groups(cuda, svo, scenes, side, W, H, V, stride, offset, retrace):
+    """Gradients and the loss over leaf groups from one lane to whole warps
+    and over every layout the vector path accepts or refuses.  Tolerance: a
+    leaf's sum of up to n rays in FP32, in any order, is off by at most about
+    (n + 30) 2^-24 of the sum of its terms' sizes; 1e-5 covers n up to 130,
+    and larger groups are summed pairwise in registers first."""
+    torch = cuda
+    tree = svo.VoxelOctree(svo.VoxelData(scenes.sphere_scene(side, 6, 5)))
+    nw = tree.num_words()
+    cams = scenes.orbit_cameras(V, 4, tree.center(), radius=1.3)
+    rays = np.concatenate([scenes.camera_rays(c, W, H) for c in cams])
+    lights = np.stack([scenes.headlight(c) for c in cams]).astype(np.float32)
+    R = rays.shape[0]
+    rng = np.random.default_rng(side + stride)
+    p = rng.random((nw, 6), dtype=np.float32)
+    target = rng.random((R, 3)).astype(np.float32)
+
+    def layout(values):
+        if stride == 3:
+            a, b = (torch.from_numpy(np.ascontiguousarray(values[:, k:k + 3])).cuda() for k in (0, 3))
+            return a, b, (a, b)
+        flat = torch.full((offset + nw * stride + 8,), 7.0, dtype=torch.float32, device="cuda")
+        rec = flat[offset:offset + nw * stride].view(nw, stride)
+        rec[:, :6] = torch.from_numpy(values).cuda()
+        return rec[:, 0:3], rec[:, 3:6], rec
+
+    d = lambda x: torch.from_numpy(x).cuda()
+    geo = (d(rays), W, H, V, d(lights))
+    c, n, _ = layout(p)
+    gc, gn, g_all = layout(np.zeros((nw, 6), np.float32))
+    rgb = torch.empty((R, 3), dtype=torch.float32, device="cuda")
+    hit = torch.empty(R, dtype=torch.int32, device="cuda")
+    loss = torch.zeros(1, dtype=torch.float64, device="cuda")
+    leaves = svo.LeafSet(nw)
+    scale = 0.25
+    tree.diff_forward(*geo, c, n, rgb, hit_leaf=hit, param_stride=stride)
+    tree.diff_backward_l2(*geo, c, n, rgb, d(target), scale, gc, gn, hit_leaf=None if retrace else hit,
+                          loss_sum=loss, leaves=leaves, param_stride=stride)
+    torch.cuda.synchronize()
+    leaf = hit.cpu().numpy().view(np.uint32)
+    h = leaf != 0xFFFFFFFF
+    li = leaf[h].astype(np.int64)
+    ray_light = np.repeat(lights, W * H, axis=0)
+    shaded = diff_oracle.shade(leaf, rays[:, 3:], ray_light, p[:, :3], p[:, 3:])
+    assert np.max(np.abs(rgb.cpu().numpy() - shaded)) < 2e-6
+    err = rgb.cpu().numpy().astype(np.float64) - target
+    assert abs(loss.item() - (err * err).sum()) <= 1e-6 * (err * err).sum()
+    # one gradient per ray (each ray its own leaf), then summed per leaf
+    m = int(h.sum())
+    per = diff_oracle.gradient(np.arange(m, dtype=np.uint32), rays[h, 3:], ray_light[h], p[li, :3], p[li, 3:],
+                               target[h].astype(np.float64), scale / 2, m)
+    for got, terms in ((gc, per[0]), (gn, per[1])):
+        ref, size = np.zeros((nw, 3)), np.zeros(nw)
+        np.add.at(ref, li, terms)
+        np.add.at(size, li, np.linalg.norm(terms, axis=1))
+        off = np.linalg.norm(got.cpu().numpy() - ref, axis=1)
+        assert np.all(off <= 1e-5 * size)
+    assert leaves.size() == np.unique(li).size
+    if stride > 6:
+        assert bool((g_all[:, 6:] == 7.0).all())
