@@ -316,11 +316,9 @@ int svo_trace_host(svo_octree *oct, const float *rays, uint64_t n, float ray_sca
                    const svo_trace_out *out);
 
 /* svo_trace for rays stored as a row-major width x height image: the same
- * per-ray results, traced by one persistent launch in 8x4-pixel tiles so a
- * warp's rays are neighbours (about 13% faster than svo_trace on camera rays).
- * Outputs are indexed y*width + x.  The launch uses a work counter owned by
- * the handle, so svo_trace_image calls on one handle that could overlap on
- * the GPU (different streams) must be ordered by the caller. */
+ * per-ray results, traced by one launch in 8x4-pixel tiles so a warp's rays
+ * are neighbours (about 13% faster than svo_trace on camera rays).  Outputs
+ * are indexed y*width + x.  Calls on one handle may overlap on the GPU. */
 int svo_trace_image(const svo_octree *oct, const float *rays, uint32_t width, uint32_t height, float ray_scale,
                     const float light[3], const svo_trace_out *out, svo_stream stream);
 

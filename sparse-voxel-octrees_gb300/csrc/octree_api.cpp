@@ -85,22 +85,16 @@ int make_handle(uint32_t *d_words, uint64_t n_words, const float center[3], svo_
     h->n_words = n_words;
     std::memcpy(h->center, center, sizeof(h->center));
     cudaGetDevice(&h->device);
-    // One control block: the work counters, then the error word.
-    const size_t ctrl_bytes = svo_octree::kQueues * sizeof(unsigned long long) + 8;
-    void *ctrl = nullptr;
-    cudaError_t e = cudaMalloc(&ctrl, ctrl_bytes);
+    cudaError_t e = cudaMalloc((void **)&h->d_status, sizeof(uint32_t));
     if (e != cudaSuccess) {
         cudaFree(d_words);
         h->d_words = nullptr;
-        return cuda_fail(e, "cudaMalloc(control block)");
+        return cuda_fail(e, "cudaMalloc(error word)");
     }
-    h->d_queue = static_cast<unsigned long long *>(ctrl);
-    h->d_status = reinterpret_cast<uint32_t *>(static_cast<char *>(ctrl) +
-                                               svo_octree::kQueues * sizeof(unsigned long long));
-    e = cudaMemset(ctrl, 0, ctrl_bytes);
+    e = cudaMemset(h->d_status, 0, sizeof(uint32_t));
     if (e != cudaSuccess) {
         svo_octree_destroy(h.release());
-        return cuda_fail(e, "cudaMemset(control block)");
+        return cuda_fail(e, "cudaMemset(error word)");
     }
     *out = h.release();
     return SVO_OK;
@@ -154,9 +148,9 @@ static std::vector<uint64_t> plan_chunks(uint64_t total, uint64_t target, uint64
 
 // The host-buffer pipeline of svo_trace_host and svo_trace_image_host (and
 // their asynchronous forms).  Chunk k's rays go in on the copy-in stream into
-// staging buffer k % B, are traced on that buffer's trace stream (each with
-// its own work counter, so one chunk's persistent launch fills the tail of the
-// previous one) and come out on the copy-out stream.  A buffer's rays are
+// staging buffer k % B, are traced on that buffer's trace stream (so one
+// chunk's launch fills the tail of the previous one) and come out on the
+// copy-out stream.  A buffer's rays are
 // overwritten only after its previous trace, and its results only after their
 // copy-out.  With two buffers a buffer's whole cycle (copy in, trace, copy
 // out) paced the copy-in stream; with four, the copy-in stream runs back to
@@ -182,7 +176,7 @@ static int host_drain(svo_octree *oct) {
 }
 
 // Enqueues the chunks of `plan` (rays from `rays`, results to `out`, all host
-// memory); launch(d_rays, rays, outputs, stream, buffer) enqueues one chunk's
+// memory); launch(d_rays, rays, outputs, stream) enqueues one chunk's
 // trace.  Called with staging_mtx held.  On an error, everything enqueued so
 // far is drained before returning.
 template <typename Launch>
@@ -245,7 +239,7 @@ static int host_enqueue(svo_octree *oct, const float *rays, const std::vector<ui
             o.word = out.word ? d_word : nullptr;
             o.rgb = out.rgb ? d_rgb : nullptr;
             o.rgba8 = out.rgba8 ? d_rgba8 : nullptr;
-            int rc = launch(d_rays, m, o, sk, h);
+            int rc = launch(d_rays, m, o, sk);
             if (rc) return rc;
             SVO_CUDA_TRY(cudaEventRecord(oct->stage_traced[h], sk));
             SVO_CUDA_TRY(cudaStreamWaitEvent(so, oct->stage_traced[h], 0));
@@ -429,7 +423,7 @@ int svo_octree_destroy(svo_octree *oct) {
     }
     if (oct->d_words) cudaFree(oct->d_words);
     if (oct->d_tab) cudaFree(oct->d_tab);
-    if (oct->d_queue) cudaFree(oct->d_queue);  // the control block (d_status lies inside it)
+    if (oct->d_status) cudaFree(oct->d_status);
     if (oct->stage_dev) cudaFree(oct->stage_dev);
     if (oct->copy_in) cudaStreamDestroy(oct->copy_in);
     if (oct->copy_out) cudaStreamDestroy(oct->copy_out);
@@ -678,7 +672,7 @@ static int trace_host(svo_octree *oct, const float *rays, uint64_t n, float ray_
         const std::vector<uint64_t> plan = plan_chunks(n, kStageRays, 32);
         const float lt[3] = {light ? light[0] : 0.0f, light ? light[1] : 0.0f, light ? light[2] : 0.0f};
         int rc = host_enqueue(oct, rays, plan, *out,
-                              [&](const float *d_rays, uint64_t m, const svo_trace_out &o, cudaStream_t st, int) {
+                              [&](const float *d_rays, uint64_t m, const svo_trace_out &o, cudaStream_t st) {
                                   return launch_trace(oct, d_rays, m, ray_scale, lt, o, st);
                               });
         if (rc) return rc;
@@ -700,10 +694,9 @@ static int trace_image_host(svo_octree *oct, const float *rays, uint32_t width, 
         for (auto &c : plan) c *= width;
         const float lt[3] = {light ? light[0] : 0.0f, light ? light[1] : 0.0f, light ? light[2] : 0.0f};
         int rc = host_enqueue(oct, rays, plan, *out,
-                              [&](const float *d_rays, uint64_t m, const svo_trace_out &o, cudaStream_t st,
-                                  int buffer) {
+                              [&](const float *d_rays, uint64_t m, const svo_trace_out &o, cudaStream_t st) {
                                   return launch_trace_image(oct, d_rays, width, (uint32_t)(m / width), ray_scale,
-                                                            lt, o, st, 1 + buffer);
+                                                            lt, o, st);
                               });
         if (rc) return rc;
     }

@@ -21,10 +21,7 @@ struct svo_octree {
     uint64_t n_words = 0;
     float center[3] = {0.0f, 0.0f, 0.0f};
     int device = 0;
-    // One device control block: kQueues work counters, then d_status.
     uint32_t *d_status = nullptr;  // device error word: bit 0 = a ray ended with kFault
-    unsigned long long *d_queue = nullptr;  // work counters: [0] svo_trace_image and the differentiable
-                                            // launches, [1 + b] svo_trace_image_host's trace stream b
     int index_bits = 32;  // 64: svo_trace uses 64-bit word indices even when n_words fits 32 bits
 
     // Descriptor table of the table traversal (octree_table.cu), built by the
@@ -40,7 +37,6 @@ struct svo_octree {
     // copy-out stream, one trace stream per buffer, and per-buffer events
     // (inputs landed, trace done, outputs copied).
     static constexpr int kStageBuffers = 4;  // stage_used has one flag per buffer
-    static constexpr int kQueues = 1 + kStageBuffers;
     std::mutex staging_mtx;
     void *stage_dev = nullptr;
     size_t stage_dev_bytes = 0;
@@ -106,7 +102,7 @@ int build_voxel_file_streamed(FILE *fp, int w, int h, int d, uint64_t mem, uint6
 int launch_trace(const svo_octree *oct, const float *d_rays, uint64_t n, float ray_scale, const float light[3],
                  const svo_trace_out &out, cudaStream_t st);
 int launch_trace_image(const svo_octree *oct, const float *d_rays, uint32_t width, uint32_t height, float ray_scale,
-                       const float light[3], const svo_trace_out &out, cudaStream_t st, int queue = 0);
+                       const float light[3], const svo_trace_out &out, cudaStream_t st);
 int launch_count_loads(const svo_octree *oct, const float *d_rays, uint64_t n, float ray_scale, uint32_t *loads,
                        cudaStream_t st);
 
