@@ -48,6 +48,7 @@
 #include "sort.cuh"
 #include "svo_device.cuh"
 #include "svo_internal.h"
+#include "tri_box.cuh"
 
 // Device-resident triangle mesh (after PlyLoader's rescale and
 // triangulation).
@@ -66,7 +67,8 @@ namespace {
 // upper (3), padding (3).
 constexpr int kTriFloats = 36;
 constexpr int kTriP = 0, kTriN = 9, kTriC = 18, kTriLo = 27, kTriHi = 30;
-constexpr int kStageFloats = 27;  // p, n, c: what the fold kernel stages
+constexpr int kStageVec = 7;  // float4s of p, n, c that the fold kernel stages
+constexpr int kStageArea = 27;  // its spare 28th float: |(p0 - p1) x (p0 - p2)|
 
 #define SVO_LAUNCH_OK(name)                                                    \
     do {                                                                       \
@@ -103,87 +105,6 @@ struct Dev {
         cudaError_t _e = (buf).alloc((n), st);                                     \
         if (_e != cudaSuccess) return ::svo::cuda_fail(_e, "device allocation in mesh build"); \
     } while (0)
-
-// ---- triangle/box overlap ---------------------------------------------------
-
-// Separating-axis triangle/box test of Akenine-Moller ("Fast 3D
-// triangle-box overlap testing", 2001) in the form third-party/tribox3.c:
-// 132-206 evaluates it: the nine edge-axis tests first (projections of two
-// vertices per axis, with that code's choice of which vertex is tested
-// first for the min), then the box axes, then the triangle's plane.
-__device__ __forceinline__ bool axis_sep(float pa, float pb, bool a_first, float rad) {
-    float mn, mx;
-    if (a_first) {
-        if (pa < pb) { mn = pa; mx = pb; } else { mn = pb; mx = pa; }
-    } else {
-        if (pb < pa) { mn = pb; mx = pa; } else { mn = pa; mx = pb; }
-    }
-    return mn > rad || mx < -rad;
-}
-
-__device__ __forceinline__ bool plane_box(const float n[3], const float v[3], const float h[3]) {
-    float vmin[3], vmax[3];
-#pragma unroll
-    for (int q = 0; q < 3; q++) {
-        if (n[q] > 0.0f) {
-            vmin[q] = -h[q] - v[q];
-            vmax[q] = h[q] - v[q];
-        } else {
-            vmin[q] = h[q] - v[q];
-            vmax[q] = -h[q] - v[q];
-        }
-    }
-    if (n[0] * vmin[0] + n[1] * vmin[1] + n[2] * vmin[2] > 0.0f) return false;
-    if (n[0] * vmax[0] + n[1] * vmax[1] + n[2] * vmax[2] >= 0.0f) return true;
-    return false;
-}
-
-__device__ __forceinline__ bool tri_box(float cx, float cy, float cz, const float h[3], const float *tv) {
-    const float v0[3] = {tv[0] - cx, tv[1] - cy, tv[2] - cz};
-    const float v1[3] = {tv[3] - cx, tv[4] - cy, tv[5] - cz};
-    const float v2[3] = {tv[6] - cx, tv[7] - cy, tv[8] - cz};
-    const float e0[3] = {v1[0] - v0[0], v1[1] - v0[1], v1[2] - v0[2]};
-    const float e1[3] = {v2[0] - v1[0], v2[1] - v1[1], v2[2] - v1[2]};
-    const float e2[3] = {v0[0] - v2[0], v0[1] - v2[1], v0[2] - v2[2]};
-    float fex, fey, fez, a, b;
-
-    fex = fabsf(e0[0]); fey = fabsf(e0[1]); fez = fabsf(e0[2]);
-    a = e0[2]; b = e0[1];
-    if (axis_sep(a * v0[1] - b * v0[2], a * v2[1] - b * v2[2], true, fez * h[1] + fey * h[2])) return false;
-    a = e0[2]; b = e0[0];
-    if (axis_sep(-a * v0[0] + b * v0[2], -a * v2[0] + b * v2[2], true, fez * h[0] + fex * h[2])) return false;
-    a = e0[1]; b = e0[0];
-    if (axis_sep(a * v1[0] - b * v1[1], a * v2[0] - b * v2[1], false, fey * h[0] + fex * h[1])) return false;
-
-    fex = fabsf(e1[0]); fey = fabsf(e1[1]); fez = fabsf(e1[2]);
-    a = e1[2]; b = e1[1];
-    if (axis_sep(a * v0[1] - b * v0[2], a * v2[1] - b * v2[2], true, fez * h[1] + fey * h[2])) return false;
-    a = e1[2]; b = e1[0];
-    if (axis_sep(-a * v0[0] + b * v0[2], -a * v2[0] + b * v2[2], true, fez * h[0] + fex * h[2])) return false;
-    a = e1[1]; b = e1[0];
-    if (axis_sep(a * v0[0] - b * v0[1], a * v1[0] - b * v1[1], true, fey * h[0] + fex * h[1])) return false;
-
-    fex = fabsf(e2[0]); fey = fabsf(e2[1]); fez = fabsf(e2[2]);
-    a = e2[2]; b = e2[1];
-    if (axis_sep(a * v0[1] - b * v0[2], a * v1[1] - b * v1[2], true, fez * h[1] + fey * h[2])) return false;
-    a = e2[2]; b = e2[0];
-    if (axis_sep(-a * v0[0] + b * v0[2], -a * v1[0] + b * v1[2], true, fez * h[0] + fex * h[2])) return false;
-    a = e2[1]; b = e2[0];
-    if (axis_sep(a * v1[0] - b * v1[1], a * v2[0] - b * v2[1], false, fey * h[0] + fex * h[1])) return false;
-
-    const float *vv[3] = {v0, v1, v2};
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        float mn = vv[0][k], mx = vv[0][k];
-        if (vv[1][k] < mn) mn = vv[1][k];
-        if (vv[1][k] > mx) mx = vv[1][k];
-        if (vv[2][k] < mn) mn = vv[2][k];
-        if (vv[2][k] > mx) mx = vv[2][k];
-        if (mn > h[k] || mx < -h[k]) return false;
-    }
-    const float n[3] = {e0[1] * e1[2] - e0[2] * e1[1], e0[2] * e1[0] - e0[0] * e1[2], e0[0] * e1[1] - e0[1] * e1[0]};
-    return plane_box(n, v0, h);
-}
 
 // ---- 1. triangle setup ---------------------------------------------------------
 
@@ -454,22 +375,25 @@ struct FoldArgs {
     int dims[3];
     int log_block;
     uint32_t *slot;
+    int sub_bricks;  // 1: sub-block edges are multiples of the brick edge, so a brick lies in one sub-block
 };
 
-// PlyLoader::writeTriangleCell on a register copy of one buffer cell.
-__device__ __forceinline__ void write_cell(uint32_t &w, uint32_t &cnt, float cx, float cy, float cz, const float *T) {
+// PlyLoader::writeTriangleCell in two halves: what a triangle gives a voxel
+// at (cx, cy, cz), which depends on nothing else, and its running-average
+// write into the cell, which has to follow the list's order.  T also holds
+// the triangle's area term, and ratio[n] is n / (n + 1), both rounded as
+// PlyLoader's own expressions are.
+__device__ __forceinline__ void triangle_sample(float cx, float cy, float cz, const float *T, float &nx, float &ny,
+                                                float &nz, float &shade) {
     const float *p = T + kTriP, *nv = T + kTriN, *cv = T + kTriC;
     // Triangle::barycentric (PlyLoader.cpp:55-64)
     float f1x = p[0] - cx, f1y = p[1] - cy, f1z = p[2] - cz;
     float f2x = p[3] - cx, f2y = p[4] - cy, f2z = p[5] - cz;
     float f3x = p[6] - cx, f3y = p[7] - cy, f3z = p[8] - cz;
-    float ax = p[0] - p[3], ay = p[1] - p[4], az = p[2] - p[5];
-    float bx = p[0] - p[6], by = p[1] - p[7], bz = p[2] - p[8];
-    float qx = ay * bz - az * by, qy = az * bx - ax * bz, qz = ax * by - ay * bx;
-    float area = sqrtf(qx * qx + qy * qy + qz * qz);
-    qx = f2y * f3z - f2z * f3y;
-    qy = f2z * f3x - f2x * f3z;
-    qz = f2x * f3y - f2y * f3x;
+    const float area = T[kStageArea];
+    float qx = f2y * f3z - f2z * f3y;
+    float qy = f2z * f3x - f2x * f3z;
+    float qz = f2x * f3y - f2y * f3x;
     float l1 = sqrtf(qx * qx + qy * qy + qz * qz) / area;
     qx = f3y * f1z - f3z * f1y;
     qy = f3z * f1x - f3x * f1z;
@@ -485,9 +409,9 @@ __device__ __forceinline__ void write_cell(uint32_t &w, uint32_t &cnt, float cx,
         }
     }
     float l3 = 1.0f - l1 - l2;
-    float nx = nv[0] * l1 + nv[3] * l2 + nv[6] * l3;
-    float ny = nv[1] * l1 + nv[4] * l2 + nv[7] * l3;
-    float nz = nv[2] * l1 + nv[5] * l2 + nv[8] * l3;
+    nx = nv[0] * l1 + nv[3] * l2 + nv[6] * l3;
+    ny = nv[1] * l1 + nv[4] * l2 + nv[7] * l3;
+    nz = nv[2] * l1 + nv[5] * l2 + nv[8] * l3;
     float inv = 1.0f / sqrtf(nx * nx + ny * ny + nz * nz);
     nx *= inv;
     ny *= inv;
@@ -495,42 +419,53 @@ __device__ __forceinline__ void write_cell(uint32_t &w, uint32_t &cnt, float cx,
     float r = cv[0] * l1 + cv[3] * l2 + cv[6] * l3;
     float gg = cv[1] * l1 + cv[4] * l2 + cv[7] * l3;
     float b = cv[2] * l1 + cv[5] * l2 + cv[8] * l3;
-    float shade = (r * 0.2126f + gg * 0.7152f + b * 0.0722f) * (1.0f / 256.0f);
+    shade = (r * 0.2126f + gg * 0.7152f + b * 0.0722f) * (1.0f / 256.0f);
+}
+
+__device__ __forceinline__ void blend_cell(uint32_t &w, uint32_t &cnt, float nx, float ny, float nz, float shade,
+                                           const float *ratio) {
     if (w == 0) {
         cnt = 1;
-        w = compress_material(nx, ny, nz, shade);
     } else {
-        float cur = (float)cnt / ((float)cnt + 1.0f);
-        float nr = 1.0f - cur;
+        const float cur = ratio[cnt];
+        const float nr = 1.0f - cur;
         float cnx, cny, cnz, cs;
         decompress_material(w, cnx, cny, cnz, cs);
-        float mx = cnx * cur + nx * nr, my = cny * cur + ny * nr, mz = cnz * cur + nz * nr;
-        float ms = cs * cur + shade * nr;
-        if (mx * mx + my * my + mz * mz < 1e-3f) {
-            mx = cnx;
-            my = cny;
-            mz = cnz;
+        nx = cnx * cur + nx * nr;
+        ny = cny * cur + ny * nr;
+        nz = cnz * cur + nz * nr;
+        shade = cs * cur + shade * nr;
+        if (nx * nx + ny * ny + nz * nz < 1e-3f) {
+            nx = cnx;
+            ny = cny;
+            nz = cnz;
         }
-        w = compress_material(mx, my, mz, ms);
         cnt = cnt + 1 < 255 ? cnt + 1 : 255;
     }
+    w = compress_material(nx, ny, nz, shade);
 }
 
 constexpr int kFoldWarps = 4;   // warps per CTA of the fold kernel
-constexpr int kFoldChunk = 8;   // pairs a warp stages per round (8-bit hit masks)
+constexpr int kFoldChunk = 8;   // pairs a warp stages per round
+constexpr int kFoldCtas = 7;    // per SM: 72 registers a thread (8 CTAs of 64 registers: 596 against 566 us)
+constexpr int kFoldList = 256;  // hits a warp collects before it folds them
 
-struct FoldSmem {
-    float T[kFoldChunk][kStageFloats];  // p, n, c
-    int lo[kFoldChunk][3];              // running-sum start: max(triangle box low, sub-block start)
-    int box[kFoldChunk][6];             // brick-local inclusive range of the clamped box
-    int pre[kFoldChunk + 1];            // prefix of the boxes' voxel counts
-    float C[kFoldChunk][3][8];          // running centres of the brick's E coordinates per axis
-    uint32_t w[512];                    // the brick's buffer words ...
-    uint8_t cnt[512];                   // ... and counts (PlyLoader::_counts)
-    uint32_t mask[128];                 // per voxel, 8 bits: which staged pairs hit it
-    uint16_t list[512];                 // voxels with any hit in this round
-    uint32_t touched[16];
+struct __align__(16) FoldSmem {
+    float T[kFoldChunk][4 * kStageVec];  // p, n, c, area
+    float F[kFoldChunk][kFltFloats];
+    int4 b0[kFoldChunk];                 // brick-local box start x, y, z; first item
+    int4 b1[kFoldChunk];                 // box width in x, y; their 16-bit reciprocals
+    uint32_t w[512];                     // the brick's buffer words, in Morton order ...
+    uint8_t cnt[512];                    // ... and counts (PlyLoader::_counts)
+    float C[kFoldChunk][3][8];           // running centres of the brick's E coordinates per axis
+    int lo[kFoldChunk][3];               // running-sum start: max(triangle box low, sub-block start)
+    uint32_t touched[16];                // the cells folded, a bit each
+    uint16_t list[kFoldList];            // hits: cell x, y, z (3 bits each), staged pair
 };
+
+// ceil(65536 / n): the reciprocals of divmod_small.
+__constant__ int kRcp16[9] = {0, 65536, 32768, 21846, 16384, 13108, 10923, 9363, 8192};
+
 
 // v / n and v % n for v < 1024, n <= 8 by a 16-bit fixed-point reciprocal
 // (exact: the error v / 2^16 stays below 1/n minus the largest fraction).
@@ -539,25 +474,103 @@ __device__ __forceinline__ void divmod_small(int v, int n, int rcp, int &q, int 
     r = v - q * n;
 }
 
+// Brick-local Morton index (edge at most 8) of a cell, and back.
+__device__ __forceinline__ int cell_morton(int x, int y, int z) {
+    auto spread = [](int v) { return (v & 1) | ((v & 2) << 2) | ((v & 4) << 4); };
+    return spread(x) | (spread(y) << 1) | (spread(z) << 2);
+}
+
+__device__ __forceinline__ void brick_cell(int m, int &x, int &y, int &z) {
+    x = (m & 1) | ((m >> 2) & 2) | ((m >> 4) & 4);
+    y = ((m >> 1) & 1) | ((m >> 3) & 2) | ((m >> 5) & 4);
+    z = ((m >> 2) & 1) | ((m >> 4) & 2) | ((m >> 6) & 4);
+}
+
+// Every third bit of a 32-bit Morton code.
+__device__ __forceinline__ uint32_t compact3_32(uint32_t x) {
+    x &= 0x49249249u;
+    x = (x ^ (x >> 2)) & 0xc30c30c3u;
+    x = (x ^ (x >> 4)) & 0x0f00f00fu;
+    x = (x ^ (x >> 8)) & 0xff0000ffu;
+    return (x ^ (x >> 16)) & 0xffffu;
+}
+
+// The exact test of a voxel the filter leaves open: rare, and kept out of the
+// fold's instruction stream.
+__device__ __noinline__ bool tri_box_open(float cx, float cy, float cz, float half, const float *tv) {
+    const float h[3] = {half, half, half};
+    return tri_box(cx, cy, cz, h, tv);
+}
+
+// Folds a warp's collected hits in list order.  Every hit's sample is formed
+// first, a lane per hit; the writes follow, and where lanes of the 32 share a
+// voxel they write one after another in list order.
+__device__ __forceinline__ void fold_hits(FoldSmem &sm, int n, const float *ratio) {
+    const int lane = threadIdx.x & 31;
+    const uint32_t lt = (1u << lane) - 1u;
+    __syncwarp();
+    for (int k0 = 0; k0 < n; k0 += 32) {
+        const bool live = k0 + lane < n;
+        float nx = 0.0f, ny = 0.0f, nz = 0.0f, shade = 0.0f;
+        int m = 512 + lane;  // no cell: a group of its own
+        if (live) {
+            const int e = sm.list[k0 + lane], ix = e & 7, iy = (e >> 3) & 7, iz = (e >> 6) & 7, q = e >> 9;
+            triangle_sample(sm.C[q][0][ix], sm.C[q][1][iy], sm.C[q][2][iz], &sm.T[q][0], nx, ny, nz, shade);
+            m = cell_morton(ix, iy, iz);
+        }
+        const unsigned peers = __match_any_sync(0xffffffffu, m);
+        const unsigned rank = (unsigned)__popc(peers & lt);
+        const unsigned rounds = __reduce_max_sync(0xffffffffu, rank);
+        for (unsigned r = 0; r <= rounds; ++r) {
+            if (live && rank == r) {
+                uint32_t wv = sm.w[m], cv = sm.cnt[m];
+                blend_cell(wv, cv, nx, ny, nz, shade, ratio);
+                sm.w[m] = wv;
+                sm.cnt[m] = (uint8_t)cv;
+                if (r == 0) atomicOr(&sm.touched[m >> 5], 1u << (m & 31));
+            }
+            __syncwarp();
+        }
+    }
+}
+
 // One warp per brick.  The warp loads the brick's buffer cells, then takes
-// the brick's (triangle, sub-block) pairs in list order, 16 per round:
+// the brick's (triangle, sub-block) pairs in list order, kFoldChunk per round:
 //   1. every (pair, voxel of the pair's clamped box inside the brick) item of
 //      the round is spread over the lanes and tested (triangleToVolume's loop
-//      nest, PlyLoader.cpp:338-374), hits recorded as a per-voxel bit mask;
-//   2. the voxels with hits are compacted and each lane folds one voxel's
-//      hits in pair order with writeTriangleCell (PlyLoader.cpp:296-336).
+//      nest, PlyLoader.cpp:338-374): the box axes are tested per coordinate
+//      while the centres are staged and shrink the box, the other ten axes by
+//      the filter, and by tri_box where the filter leaves them open.  Hits
+//      are listed in item order, so a voxel's are in pair order;
+//   2. the listed hits are folded with writeTriangleCell (PlyLoader.cpp:
+//      296-336).
 // A voxel lies in exactly one sub-block, so only pairs of its own cell reach
 // it, in ascending triangle order as that cell's list holds them.
+//
+// Bound by instruction issue.  On a 327,680-triangle mesh at 1024^3 (85,187
+// bricks, 160,202 rounds, 27 M tested voxels, 8.2 M hits) the form before
+// this one ran tri_box on every voxel and one lane per voxel through all its
+// hits: 938 us, 957 M warp instructions, 19 of 32 lanes.  The filter and
+// staging without integer divisions gave 730 us; samples a lane per hit and
+// cells in Morton order 566; tri_box and the fold out of the unrolled code
+// (1.5 of 6.8 stall cycles per instruction were instruction fetches) 509 us,
+// 500 M instructions, 22 lanes, issue 79% active.  Of those instructions the
+// fold takes 46%, the tests 23%, staging 27%.
 template <bool kDirect>
-__global__ void __launch_bounds__(kFoldWarps * 32, 8) k_fold_bricks(FoldArgs a) {
+__global__ void __launch_bounds__(kFoldWarps * 32, kFoldCtas) k_fold_bricks(FoldArgs a) {
     __shared__ FoldSmem smem[kFoldWarps];
+    __shared__ float ratio[256];  // writeTriangleCell's count / (count + 1)
+    const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     FoldSmem &sm = smem[wid];
     const int le = a.log_e, E = 1 << le, E3 = 1 << (3 * le);
-    const float hv[3] = {a.half, a.half, a.half};
     int end0 = a.org[0] + a.buf[0], end1 = a.org[1] + a.buf[1], end2 = a.org[2] + a.buf[2];
     int drop_z = a.drop_z;
     const uint32_t lt = (1u << lane) - 1u;
+    for (int i = threadIdx.x; i < 256; i += kFoldWarps * 32) ratio[i] = (float)i / ((float)i + 1.0f);
+    __syncthreads();
+    // this lane's axis and coordinate when the centres are staged
+    const int cax = lane >> 3, ck = lane & 7;
     // Warps take bricks from a counter: a brick's cost grows with its
     // triangles, and a fixed stride left most warps idle behind the few that
     // drew the heaviest bricks.  Bricks own disjoint buffer cells, so the
@@ -565,11 +578,11 @@ __global__ void __launch_bounds__(kFoldWarps * 32, 8) k_fold_bricks(FoldArgs a) 
     for (;;) {
         uint32_t jt = 0;
         if (lane == 0) jt = atomicAdd(a.next, 1u);
-        const uint32_t j = a.b_first + __shfl_sync(0xffffffffu, jt, 0);
+        const uint32_t j = a.b_first + __shfl_sync(FULL, jt, 0);
         if (j >= a.b_last) break;
         const uint32_t key = a.bkey[j] & a.brick_mask;
-        const int ox = (int)(compact3(key) << le), oy = (int)(compact3((uint64_t)key >> 1) << le),
-                  oz = (int)(compact3((uint64_t)key >> 2) << le);
+        const int ox = (int)(compact3_32(key) << le), oy = (int)(compact3_32(key >> 1) << le),
+                  oz = (int)(compact3_32(key >> 2) << le);
         // a brick the buffer holds only zeros for is not read (the extraction
         // cleared what earlier blocks left, except their dropped slices)
         bool clean = kDirect;
@@ -577,9 +590,7 @@ __global__ void __launch_bounds__(kFoldWarps * 32, 8) k_fold_bricks(FoldArgs a) 
         if (kDirect) {
             // the brick's block: its bounds and dropped slice (VoxelData.cpp:163-170)
             const int lb = a.log_block, B = 1 << lb;
-            const uint64_t blk = (uint64_t)key >> (3 * (lb - le));
-            const int bx = (int)(compact3(blk) << lb), by = (int)(compact3(blk >> 1) << lb),
-                      bz = (int)(compact3(blk >> 2) << lb);
+            const int bx = ox & ~(B - 1), by = oy & ~(B - 1), bz = oz & ~(B - 1);
             end0 = min(bx + B, a.dims[0]);
             end1 = min(by + B, a.dims[1]);
             end2 = min(bz + B, a.dims[2]);
@@ -590,161 +601,242 @@ __global__ void __launch_bounds__(kFoldWarps * 32, 8) k_fold_bricks(FoldArgs a) 
                              (uint32_t)((oz - a.org[2]) >> le));
             if (a.pre_dirty) clean = pm < a.n_pre && a.pre_dirty[pm] == 0;
         }
+        // the sub-block of an aligned brick (the others look theirs up per pair)
+        int st0 = 0, st1 = 0, st2 = 0;
+        if (a.sub_bricks) {
+            st0 = ox / a.sub[0] * a.sub[0];
+            st1 = oy / a.sub[1] * a.sub[1];
+            st2 = oz / a.sub[2] * a.sub[2];
+        }
+        const float h = 2.0f * a.half, mid = 0.5f * (float)(E - 1);
+        const float oc[3] = {((float)ox + mid) * h, ((float)oy + mid) * h, ((float)oz + mid) * h};
         __syncwarp();
-        for (int i = lane; i < E3; i += 32) {
-            int x = ox + (i & (E - 1)), y = oy + ((i >> le) & (E - 1)), z = oz + (i >> (2 * le));
-            uint32_t wv = 0, cv = 0;
-            // a slab's bricks may start below its first slice (z-slabs need not be brick-aligned)
-            if (!clean && x >= a.org[0] && y >= a.org[1] && z >= a.org[2] && x < end0 && y < end1 && z < end2) {
-                uint64_t bi = (uint64_t)(x - a.org[0]) +
-                              (uint64_t)a.buf[0] * ((uint64_t)(y - a.org[1]) + (uint64_t)a.buf[1] * (uint64_t)(z - a.org[2]));
-                wv = a.data[bi];
-                cv = a.counts[bi];
+        if (clean) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) reinterpret_cast<uint4 *>(sm.w)[lane + 32 * i] = make_uint4(0u, 0u, 0u, 0u);
+            reinterpret_cast<uint4 *>(sm.cnt)[lane] = make_uint4(0u, 0u, 0u, 0u);
+        } else {
+            for (int i = lane; i < E3; i += 32) {
+                const int lx = i & (E - 1), ly = (i >> le) & (E - 1), lz = i >> (2 * le);
+                const int x = ox + lx, y = oy + ly, z = oz + lz, m = cell_morton(lx, ly, lz);
+                uint32_t wv = 0, cv = 0;
+                // a slab's bricks may start below its first slice (z-slabs need not be brick-aligned)
+                if (x >= a.org[0] && y >= a.org[1] && z >= a.org[2] && x < end0 && y < end1 && z < end2) {
+                    uint64_t bi = (uint64_t)(x - a.org[0]) +
+                                  (uint64_t)a.buf[0] * ((uint64_t)(y - a.org[1]) + (uint64_t)a.buf[1] * (uint64_t)(z - a.org[2]));
+                    wv = a.data[bi];
+                    cv = a.counts[bi];
+                }
+                sm.w[m] = wv;
+                sm.cnt[m] = (uint8_t)cv;
             }
-            sm.w[i] = wv;
-            sm.cnt[i] = (uint8_t)cv;
         }
         if (lane < 16) sm.touched[lane] = 0;
         const uint32_t s0 = a.bstart[j], s1 = a.bstart[j + 1];
         for (uint32_t c0 = s0; c0 < s1; c0 += kFoldChunk) {
             const int nc = (int)min((uint32_t)kFoldChunk, s1 - c0);
             __syncwarp();
-            for (int i = lane; i < nc * kStageFloats; i += 32) {
-                int q = i / kStageFloats, f = i - q * kStageFloats;
-                sm.T[q][f] = a.tris[(uint64_t)a.pair_tri[c0 + q] * kTriFloats + f];
+            const uint32_t tri = lane < nc ? a.pair_tri[c0 + lane] : 0u;
+            for (int i = lane; i < 2 * 32; i += 32) {
+                const int q = i / kStageVec, f = i - q * kStageVec;
+                const uint32_t t = __shfl_sync(FULL, tri, q & 31);
+                if (q < nc)
+                    reinterpret_cast<float4 *>(sm.T[q])[f] =
+                        __ldg(reinterpret_cast<const float4 *>(a.tris + (uint64_t)t * kTriFloats) + f);
             }
-            for (int i = lane; i < ((E3 + 3) >> 2); i += 32) sm.mask[i] = 0;
-            int items = 0;
+            uint32_t range = 0;  // this lane's pair: brick-local box, 4 bits per bound
             if (lane < nc) {
-                const int32_t *bx = a.box + (uint64_t)a.pair_tri[c0 + lane] * 6;
-                const uint32_t cell = a.pair_cell[c0 + lane];
-                const int g0 = (int)(cell % (uint32_t)a.grid[0]), g12 = (int)(cell / (uint32_t)a.grid[0]);
-                const int g1 = g12 % a.grid[1], g2 = g12 / a.grid[1];
-                const int o[3] = {ox, oy, oz}, st3[3] = {g0 * a.sub[0], g1 * a.sub[1], g2 * a.sub[2]};
+                const int32_t *bx = a.box + (uint64_t)tri * 6;
+                int st3[3] = {st0, st1, st2};
+                if (!a.sub_bricks) {
+                    const uint32_t cell = a.pair_cell[c0 + lane];
+                    const int g0 = (int)(cell % (uint32_t)a.grid[0]), g12 = (int)(cell / (uint32_t)a.grid[0]);
+                    const int g1 = g12 % a.grid[1], g2 = g12 / a.grid[1];
+                    st3[0] = g0 * a.sub[0];
+                    st3[1] = g1 * a.sub[1];
+                    st3[2] = g2 * a.sub[2];
+                }
+                const int o[3] = {ox, oy, oz};
                 const int en[3] = {end0, end1, end2};
-                items = 1;
 #pragma unroll
                 for (int ax = 0; ax < 3; ++ax) {
                     int lo = max(bx[ax], st3[ax]);                                // PlyLoader.cpp:344-346
                     int hi = min(bx[3 + ax], min(st3[ax] + a.sub[ax], en[ax]) - 1);  // :347-349
                     int b0 = max(lo, o[ax]) - o[ax], b1 = min(hi, o[ax] + E - 1) - o[ax];
+                    if (b1 < b0) {
+                        b0 = 8;  // an empty range: no coordinate lies in it
+                        b1 = 0;
+                    }
                     sm.lo[lane][ax] = lo;
-                    sm.box[lane][ax] = b0;
-                    sm.box[lane][3 + ax] = b1;
-                    items *= max(0, b1 - b0 + 1);
+                    range |= (uint32_t)(b0 | (b1 << 4)) << (8 * ax);
                 }
+            }
+            __syncwarp();
+            // running centres, and the box axes' tests per coordinate (the
+            // centres rise with k, so those that pass are consecutive)
+            const float oca = cax == 0 ? oc[0] : (cax == 1 ? oc[1] : oc[2]);
+            const int ov = cax == 0 ? ox : (cax == 1 ? oy : oz);
+            float cdev = 0.0f;
+            unsigned okm = 0;
+            for (int q0 = 0; q0 < nc; q0 += 4) {
+                float c[4];
+                unsigned in = 0;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const int q = q0 + k;
+                    const int b = (int)((__shfl_sync(FULL, range, q) >> (8 * cax)) & 255u);
+                    c[k] = 0.0f;
+                    if (q < nc && lane < 24 && ck >= (b & 15) && ck <= (b >> 4)) {
+                        const int lo = sm.lo[q][cax];
+                        c[k] = __ldg(a.acc + (uint64_t)lo * a.K + (ov + ck - lo));
+                        in |= 1u << k;
+                    }
+                }
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const int q = q0 + k;
+                    bool ok = (in >> k) & 1u;
+                    if (ok) {
+                        sm.C[q][cax][ck] = c[k];
+                        cdev = fmaxf(cdev, fabsf(c[k] - oca));
+                        const float v0 = sm.T[q][kTriP + cax] - c[k], v1 = sm.T[q][kTriP + 3 + cax] - c[k],
+                                    v2 = sm.T[q][kTriP + 6 + cax] - c[k];
+                        float mn = v0, mx = v0;
+                        if (v1 < mn) mn = v1;
+                        if (v1 > mx) mx = v1;
+                        if (v2 < mn) mn = v2;
+                        if (v2 > mx) mx = v2;
+                        ok = !(mn > a.half || mx < -a.half);
+                    }
+                    const unsigned bits = __ballot_sync(FULL, ok);
+                    if (lane == q) okm = bits;
+                }
+            }
+            cdev = __uint_as_float(__reduce_max_sync(FULL, __float_as_uint(cdev)));
+            int items = 0;
+            int b0x = 0, b0y = 0, b0z = 0, nx = 1, ny = 1;
+            if (lane < nc && (okm & 0xFFu) && (okm & 0xFF00u) && (okm & 0xFF0000u)) {
+                const unsigned kx = okm & 0xFFu, ky = (okm >> 8) & 0xFFu, kz = (okm >> 16) & 0xFFu;
+                b0x = __ffs((int)kx) - 1;
+                b0y = __ffs((int)ky) - 1;
+                b0z = __ffs((int)kz) - 1;
+                nx = 32 - __clz((int)kx) - b0x;
+                ny = 32 - __clz((int)ky) - b0y;
+                items = nx * ny * (32 - __clz((int)kz) - b0z);
             }
             // exclusive prefix of the items over the staged pairs
             int incl = items;
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                int n = __shfl_up_sync(0xffffffffu, incl, o);
+            for (int o = 1; o < kFoldChunk; o <<= 1) {
+                int n = __shfl_up_sync(FULL, incl, o);
                 if (lane >= o) incl += n;
             }
-            if (lane < nc) sm.pre[lane] = incl - items;
-            const int total = __shfl_sync(0xffffffffu, incl, 31);
-            __syncwarp();
-            for (int i = lane; i < nc * 3 * E; i += 32) {
-                int q = i / (3 * E), r = i - q * 3 * E, ax = r / E, k = r - ax * E;
-                int ov = ax == 0 ? ox : (ax == 1 ? oy : oz);
-                int lo = sm.lo[q][ax];
-                float c = 0.0f;
-                if (k >= sm.box[q][ax] && k <= sm.box[q][3 + ax]) c = a.acc[(uint64_t)lo * a.K + (ov + k - lo)];
-                sm.C[q][ax][k] = c;
+            if (lane < kFoldChunk) {
+                sm.b0[lane] = make_int4(b0x, b0y, b0z, incl - items);
+                sm.b1[lane] = make_int4(nx, ny, kRcp16[nx], kRcp16[ny]);
+            }
+            const int total = __shfl_sync(FULL, incl, kFoldChunk - 1);
+            // the filter's constants and the blend's area, four lanes a pair
+            if ((lane >> 2) < nc) {
+                float *T = sm.T[lane >> 2];
+                stage_filter(sm.F[lane >> 2], T + kTriP, oc, cdev, a.half, lane & 3);
+                if ((lane & 3) == 3) {
+                    const float *p = T + kTriP;
+                    const float ax = p[0] - p[3], ay = p[1] - p[4], az = p[2] - p[5];
+                    const float bx = p[0] - p[6], by = p[1] - p[7], bz = p[2] - p[8];
+                    const float qx = ay * bz - az * by, qy = az * bx - ax * bz, qz = ax * by - ay * bx;
+                    T[kStageArea] = sqrtf(qx * qx + qy * qy + qz * qz);
+                }
             }
             __syncwarp();
             // 1. tests
-            for (int it = lane; it < total; it += 32) {
-                int q = 0;
-#pragma unroll
-                for (int step = kFoldChunk / 2; step; step >>= 1)
-                    if (q + step < nc && sm.pre[q + step] <= it) q += step;
-                const int v = it - sm.pre[q];
-                const int bx0 = sm.box[q][0], by0 = sm.box[q][1], bz0 = sm.box[q][2];
-                const int nx = sm.box[q][3] - bx0 + 1, ny = sm.box[q][4] - by0 + 1;
-                int r, ix, iy, iz;
-                divmod_small(v, nx, (65536 + nx - 1) / nx, r, ix);
-                divmod_small(r, ny, (65536 + ny - 1) / ny, iz, iy);
-                ix += bx0;
-                iy += by0;
-                iz += bz0;
-                if (tri_box(sm.C[q][0][ix], sm.C[q][1][iy], sm.C[q][2][iz], hv, &sm.T[q][kTriP])) {
-                    const int idx = ix + (iy << le) + (iz << (2 * le));
-                    atomicOr(&sm.mask[idx >> 2], 1u << (q + ((idx & 3) << 3)));
-                }
-            }
-            __syncwarp();
-            // 2. compaction of the voxels with hits, then the ordered fold
             int nhit = 0;
-            for (int b0 = 0; b0 < E3; b0 += 32) {
-                const int idx = b0 + lane;
-                const bool hit = idx < E3 && ((sm.mask[idx >> 2] >> ((idx & 3) << 3)) & 0xFFu) != 0;
-                const uint32_t ball = __ballot_sync(0xffffffffu, hit);
-                if (hit) sm.list[nhit + __popc(ball & lt)] = (uint16_t)idx;
-                nhit += __popc(ball);
-            }
-            __syncwarp();
-            for (int k = lane; k < nhit; k += 32) {
-                const int idx = sm.list[k];
-                uint32_t m = (sm.mask[idx >> 2] >> ((idx & 3) << 3)) & 0xFFu;
-                const int ix = idx & (E - 1), iy = (idx >> le) & (E - 1), iz = idx >> (2 * le);
-                uint32_t wv = sm.w[idx], cv = sm.cnt[idx];
-                while (m) {
-                    const int q = __ffs(m) - 1;
-                    m &= m - 1;
-                    write_cell(wv, cv, sm.C[q][0][ix], sm.C[q][1][iy], sm.C[q][2][iz], &sm.T[q][0]);
+            for (int i0 = 0; i0 < total; i0 += 32) {
+                const int it = i0 + lane;
+                bool hit = false;
+                int entry = 0;
+                if (it < total) {
+                    int q = 0;
+#pragma unroll
+                    for (int step = kFoldChunk / 2; step; step >>= 1)
+                        if (sm.b0[q + step].w <= it) q += step;
+                    const int4 s4 = sm.b0[q], n4 = sm.b1[q];
+                    int r, ix, iy, iz;
+                    divmod_small(it - s4.w, n4.x, n4.z, r, ix);
+                    divmod_small(r, n4.y, n4.w, iz, iy);
+                    ix += s4.x;
+                    iy += s4.y;
+                    iz += s4.z;
+                    const float cx = sm.C[q][0][ix], cy = sm.C[q][1][iy], cz = sm.C[q][2][iz];
+                    float f[kFltFloats];
+#pragma unroll
+                    for (int k = 0; k < kFltFloats / 4; ++k)
+                        reinterpret_cast<float4 *>(f)[k] = reinterpret_cast<const float4 *>(sm.F[q])[k];
+                    const float sep = filter_separation(f, cx - oc[0], cy - oc[1], cz - oc[2]), eps = f[kFltEps];
+                    hit = sep < -eps;
+                    if (!hit && !(sep > eps)) hit = tri_box_open(cx, cy, cz, a.half, &sm.T[q][kTriP]);
+                    entry = ix | (iy << 3) | (iz << 6) | (q << 9);
                 }
-                sm.w[idx] = wv;
-                sm.cnt[idx] = (uint8_t)cv;
-                atomicOr(&sm.touched[idx >> 5], 1u << (idx & 31));
+                const unsigned ball = __ballot_sync(FULL, hit);
+                if (hit) sm.list[nhit + __popc(ball & lt)] = (uint16_t)entry;
+                nhit += __popc(ball);
+                // 2. the ordered fold, after the last test or when the list may not hold another 32
+                if (i0 + 32 >= total || nhit > kFoldList - 32) {
+                    fold_hits(sm, nhit, ratio);
+                    nhit = 0;
+                }
             }
         }
         __syncwarp();
+        // whether every cell of the brick may hold a voxel of the block
+        const bool whole = ox + E <= end0 && oy + E <= end1 && oz + E <= end2 && !(drop_z >= oz && drop_z < oz + E);
         if constexpr (kDirect) {
-            // the brick's voxels outside the dropped slice, in Morton order
-            // (shared memory is x-fastest), compacted into its slot
-            uint32_t n = 0;
+            // the brick's voxels outside the dropped slice, in Morton order,
+            // compacted into its slot: only words with a folded cell are read
+            uint32_t n = 0, mine = 0;
             uint32_t *dst = a.slot + (uint64_t)j * (uint32_t)E3;
-            for (int m0 = 0; m0 < E3; m0 += 32) {
-                const int m = m0 + lane;
-                uint32_t wv = 0;
-                if (m < E3) {
-                    const int lx = (int)compact3((uint64_t)m), ly = (int)compact3((uint64_t)m >> 1),
-                              lz = (int)compact3((uint64_t)m >> 2);
-                    const int x = ox + lx, y = oy + ly, z = oz + lz;
-                    if (x < end0 && y < end1 && z < end2 && z != drop_z) wv = sm.w[lx + (ly << le) + (lz << (2 * le))];
+            const uint32_t folded = lane < 16 ? sm.touched[lane] : 0u;
+            for (unsigned todo = __ballot_sync(FULL, folded != 0); todo; todo &= todo - 1) {
+                const int c = __ffs((int)todo) - 1, m = 32 * c + lane;
+                uint32_t wv = m < E3 ? sm.w[m] : 0u;
+                if (!whole) {
+                    int lx, ly, lz;
+                    brick_cell(m, lx, ly, lz);
+                    if (ox + lx >= end0 || oy + ly >= end1 || oz + lz >= end2 || oz + lz == drop_z) wv = 0;
                 }
-                const uint32_t bits = __ballot_sync(0xffffffffu, wv != 0);
+                const uint32_t bits = __ballot_sync(FULL, wv != 0);
                 if (wv) dst[n + __popc(bits & lt)] = wv;
-                if (lane == 0) a.brick_bits[(uint64_t)j * 16 + (uint64_t)(m0 >> 5)] = bits;
+                if (lane == c) mine = bits;
                 n += (uint32_t)__popc(bits);
             }
+            if (lane < 16) a.brick_bits[(uint64_t)j * 16 + lane] = mine;
             if (lane == 0) a.brick_count[j] = n;
         } else {
             for (int i = lane; i < E3; i += 32) {
-                if (!((sm.touched[i >> 5] >> (i & 31)) & 1u)) continue;
-                int x = ox + (i & (E - 1)), y = oy + ((i >> le) & (E - 1)), z = oz + (i >> (2 * le));
+                const int lx = i & (E - 1), ly = (i >> le) & (E - 1), lz = i >> (2 * le);
+                const int x = ox + lx, y = oy + ly, z = oz + lz, m = cell_morton(lx, ly, lz);
+                if (!((sm.touched[m >> 5] >> (m & 31)) & 1u)) continue;
                 if (x < a.org[0] || y < a.org[1] || z < a.org[2] || x >= end0 || y >= end1 || z >= end2) continue;
                 uint64_t bi = (uint64_t)(x - a.org[0]) +
                               (uint64_t)a.buf[0] * ((uint64_t)(y - a.org[1]) + (uint64_t)a.buf[1] * (uint64_t)(z - a.org[2]));
-                a.data[bi] = sm.w[i];
-                a.counts[bi] = sm.cnt[i];
+                a.data[bi] = sm.w[m];
+                a.counts[bi] = sm.cnt[m];
             }
             if (a.brick_count && pm < a.n_pre) {
                 // the brick's whole buffer state is in shared memory: words read
                 // (or known zero) and folded.  The bits follow the extraction's
-                // order, the brick-local Morton index m (shared memory is x-fastest).
+                // order, the brick-local Morton index m.
                 uint32_t n = 0;
                 for (int m0 = 0; m0 < E3; m0 += 32) {
                     const int m = m0 + lane;
                     bool on = false;
                     if (m < E3) {
-                        const int lx = (int)compact3((uint64_t)m), ly = (int)compact3((uint64_t)m >> 1),
-                                  lz = (int)compact3((uint64_t)m >> 2);
-                        const int x = ox + lx, y = oy + ly, z = oz + lz;
-                        on = x < end0 && y < end1 && z < end2 && z != drop_z && sm.w[lx + (ly << le) + (lz << (2 * le))] != 0;
+                        int lx, ly, lz;
+                        brick_cell(m, lx, ly, lz);
+                        on = (whole || (ox + lx < end0 && oy + ly < end1 && oz + lz < end2 && oz + lz != drop_z)) &&
+                             sm.w[m] != 0;
                     }
-                    const uint32_t bits = __ballot_sync(0xffffffffu, on);
+                    const uint32_t bits = __ballot_sync(FULL, on);
                     if (lane == 0) a.brick_bits[pm * 16 + (uint64_t)(m0 >> 5)] = bits;
                     n += (uint32_t)__popc(bits);
                 }
@@ -1279,7 +1371,7 @@ int build_mesh_device(const svo_mesh *m, int side, int threads, uint64_t mem, cu
     int dev = 0, sms = 0;
     SVO_CUDA_TRY(cudaGetDevice(&dev));
     SVO_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    const unsigned fold_grid = (unsigned)sms * 8, warp_grid = (unsigned)sms * 16;
+    const unsigned fold_grid = (unsigned)(sms * kFoldCtas), warp_grid = (unsigned)sms * 16;
     Dev<uint32_t> fold_next;  // one work counter per fold launch
     const size_t n_next = std::max<size_t>(jobs.size(), 1);
     SVO_ALLOC(fold_next, n_next);
@@ -1306,6 +1398,9 @@ int build_mesh_device(const svo_mesh *m, int side, int threads, uint64_t mem, cu
         fa.half = 0.5f * hx;
         fa.brick_mask = brick_mask;
         fa.drop_z = -1;
+        fa.sub_bricks = 1;
+        for (int k = 0; k < 3; ++k)
+            if (sub[k] % (1 << g.log_e) != 0) fa.sub_bricks = 0;
         return fa;
     };
 
