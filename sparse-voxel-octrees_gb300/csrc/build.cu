@@ -3,7 +3,12 @@
 // Replaces VoxelOctree(VoxelData*) (VoxelOctree.cpp:125-205) with its
 // ChunkedAllocator far-pointer splice (ChunkedAllocator.hpp:76-114).  The
 // reference builds depth first and patches far pointers afterwards; this
-// pipeline computes the same word stream in three data-parallel phases:
+// pipeline computes the same word stream in three data-parallel phases.
+// Voxels that come as bricks (a dense grid's, a mesh fold's) take a shorter
+// way to the same words, over the bricks' occupancy bits and a dense pyramid
+// above them (brick.cuh, build_pyramid); the phases serve streamed files,
+// cache blocks smaller than a brick and, from phase 2 on, the bricks of cubes
+// too large for the pyramid:
 //
 //  1. Extraction.  The grid is read brick by brick (16^3 voxels per CTA,
 //     bricks visited in Morton order) and occupied voxels are emitted as
@@ -33,6 +38,7 @@
 #include <cstdio>
 #include <mutex>
 
+#include "brick.cuh"
 #include "morton.cuh"
 #include "scan.cuh"
 #include "svo_internal.h"
@@ -50,6 +56,12 @@ struct GridGeom {
     int log_block;      // cache-block edge M = 1 << log_block
     uint8_t *topflag;   // per M-block "has any voxel" (Morton-indexed), or null
 };
+
+// Whether the grid's rows start on 16-byte boundaries, so that a uint4 of a
+// 16^3 brick lies wholly inside the grid or outside.
+__device__ __forceinline__ bool grid_vec4(const GridGeom &g) {
+    return (g.w & 3) == 0 && (reinterpret_cast<uintptr_t>(g.grid) & 15) == 0;
+}
 
 // A 16^3 brick wholly inside the grid, whose rows start on 16-byte
 // boundaries, is read as 1024 uint4 (4 per thread of a 256-thread CTA).
@@ -218,6 +230,428 @@ __global__ void __launch_bounds__(kBrickThreads) k_brick_emit(GridGeom g, uint64
     }
 }
 
+// The sum of a tile array before `tile`, by the whole CTA: with up to
+// kSelfScanTiles tiles this replaces a scan launch.
+constexpr uint64_t kSelfScanTiles = 1024;
+
+__device__ __forceinline__ uint32_t tiles_before(const uint32_t *__restrict__ tile_n, uint32_t tile) {
+    uint32_t n = 0;
+    for (uint32_t t = threadIdx.x; t < tile; t += blockDim.x) n += __ldg(tile_n + t);
+    uint32_t total;
+    block_excl_scan<uint32_t>(n, &total);
+    return total;
+}
+
+// ---- bricks of 16^3 cells, straight to the words -------------------------------
+
+// Row-major index, among the 16^3 bricks that cover the grid, of the one at
+// (gx0, gy0, gz0): where its bits are.  (The Morton codes run over the whole
+// cube, which a thin grid fills only in a small part.)
+__device__ __forceinline__ uint64_t brick_linear(const GridGeom &g, int gx0, int gy0, int gz0) {
+    return (uint64_t)(gx0 >> 4) +
+           (uint64_t)((g.w + 15) >> 4) * ((uint64_t)(gy0 >> 4) + (uint64_t)((g.h + 15) >> 4) * (uint64_t)(gz0 >> 4));
+}
+
+// Phase 1 of the brick build: per brick its occupancy bits (128 words by
+// Morton code, written for bricks that hold a voxel), its node's mask and
+// subtree words (0 for an empty brick), and the cache blocks' flags.  A lane's
+// uint4 gives 4 bits of the 32-cell word that its x/4 column shares with 7
+// other lanes, so three shuffles OR the word together and no atomics are
+// needed.  Reads the grid once: bound by HBM, 87 us for the 512^3 cells of a
+// sphere union (0.54 GB at 6.2 TB/s).  6 CTAs of 42 registers per SM: at 8 the
+// word-by-word branch spills.
+// any_of: optionally, whether a brick holds a voxel at all, dropped slice
+// included; list, n_list: optionally, the bricks with surviving voxels, in any
+// order; n_voxels: optionally, those voxels' total.
+__global__ void __launch_bounds__(kBrickThreads, 6) k_brick_bits(GridGeom g, uint64_t n_bricks,
+                                                                 uint32_t *__restrict__ bits,
+                                                                 uint32_t *__restrict__ words_of,
+                                                                 uint8_t *__restrict__ mask_of,
+                                                                 uint8_t *__restrict__ any_of,
+                                                                 uint32_t *__restrict__ list,
+                                                                 uint32_t *__restrict__ n_list,
+                                                                 unsigned long long *__restrict__ n_voxels) {
+    __shared__ __align__(16) uint32_t sbits[2][128];  // alternating: warp 0 may still read the brick before
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    int turn = 0;
+    const int x4 = lane & 3, yl = (lane >> 2) & 3, zl = lane >> 4;
+    const bool vec4 = grid_vec4(g);
+    for (uint64_t b = blockIdx.x; b < n_bricks; b += gridDim.x) {
+        const int gx0 = (int)(compact3(b) << 4), gy0 = (int)(compact3(b >> 1) << 4), gz0 = (int)(compact3(b >> 2) << 4);
+        uint32_t any = 0;
+        uint32_t *const sb = sbits[turn];
+        turn ^= 1;
+        if (gx0 >= g.w || gy0 >= g.h || gz0 >= g.d) {
+            // outside: the cube's padding
+        } else if (vec4) {
+            // warp w takes the columns (y / 4, z / 2) = w, w + 8, w + 16, w + 24
+            uint4 v[4];
+            const int gx = gx0 + 4 * x4, gy = gy0 + 4 * (wid & 3) + yl, gz = gz0 + 2 * (wid >> 2) + zl;
+            const uint32_t *const at = g.grid + (uint64_t)gx + (uint64_t)g.w * ((uint64_t)gy + (uint64_t)g.h * gz);
+            const bool row = gx < g.w && gy < g.h;
+#pragma unroll
+            for (int k = 0; k < 4; ++k)  // wid + 8 k: the same y, z + 4 k
+                v[k] = row && gz + 4 * k < g.d ? __ldg(reinterpret_cast<const uint4 *>(at + (uint64_t)(4 * k) * g.w * g.h))
+                                               : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) any |= v[k].x | v[k].y | v[k].z | v[k].w;
+            any = (uint32_t)__syncthreads_or((int)(any != 0));
+            if (any) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const int c = wid + 8 * k, y4 = c & 3, z2 = c >> 2;
+                    uint32_t w = (uint32_t)(v[k].x != 0u) | ((uint32_t)(v[k].y != 0u) << 1) |
+                                 ((uint32_t)(v[k].z != 0u) << 8) | ((uint32_t)(v[k].w != 0u) << 9);
+                    w <<= ((yl & 1) << 1) | ((yl >> 1) << 4) | (zl << 2);
+                    if (g.drop_last_z && gz0 + 2 * z2 + zl == g.d - 1) w = 0;
+                    w |= __shfl_xor_sync(FULL, w, 4);
+                    w |= __shfl_xor_sync(FULL, w, 8);
+                    w |= __shfl_xor_sync(FULL, w, 16);
+                    if (lane < 4)
+                        sb[(z2 & 1) | ((x4 & 1) << 1) | ((y4 & 1) << 2) | (((z2 >> 1) & 1) << 3) | ((x4 >> 1) << 4) |
+                           ((y4 >> 1) << 5) | ((z2 >> 2) << 6)] = w;
+                }
+            }
+        } else {
+            // a lane per cell of a 32-cell word: the ballot is the word
+            for (int h = 0; h < 16; h += 4) {
+                uint32_t v[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    int x, y, z;
+                    brick_cell((uint32_t)((wid * 16 + h + k) * 32 + lane), x, y, z);
+                    const int gx = gx0 + x, gy = gy0 + y, gz = gz0 + z;
+                    v[k] = gx < g.w && gy < g.h && gz < g.d
+                               ? __ldg(g.grid + (uint64_t)gx + (uint64_t)g.w * ((uint64_t)gy + (uint64_t)g.h * gz))
+                               : 0u;
+                }
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    int x, y, z;
+                    brick_cell((uint32_t)((wid * 16 + h + k) * 32 + lane), x, y, z);
+                    any |= v[k];
+                    const uint32_t w = __ballot_sync(FULL, v[k] != 0u && !(g.drop_last_z && gz0 + z == g.d - 1));
+                    if (lane == 0) sb[wid * 16 + h + k] = w;
+                }
+            }
+            any = (uint32_t)__syncthreads_or((int)(any != 0));
+        }
+        if (!any) {
+            if (threadIdx.x == 0) {
+                words_of[b] = 0;
+                mask_of[b] = 0;
+                if (any_of) any_of[b] = 0;
+            }
+            continue;
+        }
+        __syncthreads();
+        if (wid == 0) {
+            const uint4 w = reinterpret_cast<const uint4 *>(sb)[lane];
+            reinterpret_cast<uint4 *>(bits + brick_linear(g, gx0, gy0, gz0) * 128)[lane] = w;
+            const uint32_t n0 = (uint32_t)(__popc(w.x) + __popc(w.y) + __popc(w.z) + __popc(w.w));
+            const uint32_t n1 = (uint32_t)(__popc(byte_bits(w.x)) + __popc(byte_bits(w.y)) + __popc(byte_bits(w.z)) +
+                                           __popc(byte_bits(w.w)));
+            const uint32_t n2 = (uint32_t)((w.x | w.y) != 0u) + (uint32_t)((w.z | w.w) != 0u);
+            const unsigned full = __ballot_sync(FULL, n2 != 0);
+            uint32_t mask = 0;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) mask |= (uint32_t)(((full >> (4 * i)) & 15u) != 0) << i;
+            const uint32_t total = __reduce_add_sync(FULL, n0 + n1 + n2), cells = __reduce_add_sync(FULL, n0);
+            if (lane == 0) {
+                words_of[b] = total + (uint32_t)__popc(mask);
+                mask_of[b] = (uint8_t)mask;
+                if (any_of) any_of[b] = 1;
+                if (g.topflag) g.topflag[b >> (3 * (g.log_block - 4))] = 1;
+                if (list && cells) list[atomicAdd(n_list, 1u)] = (uint32_t)b;
+                if (n_voxels && cells) atomicAdd(n_voxels, (unsigned long long)cells);
+            }
+        }
+    }
+}
+
+// Where the bricks that hold something are: their keys (the brick's Morton
+// code; key_of[j] where given, else j), masks and subtree words move to
+// consecutive entries, with the brick's own index in src.
+struct BrickNodes {
+    uint64_t n;                   // bricks
+    const uint32_t *key_of;       // or null
+    const uint32_t *words_of;
+    const uint8_t *mask_of;
+    const uint8_t *any_of;        // or null: a brick is kept when it has words
+};
+
+constexpr int kNodeItems = 8, kNodeTile = kBrickThreads * kNodeItems;
+
+__device__ __forceinline__ bool brick_kept(const BrickNodes &b, uint64_t j) {
+    return j < b.n && (b.any_of ? b.any_of[j] != 0 : b.words_of[j] != 0u);
+}
+
+// Thread t of a tile looks at bricks 8t .. 8t + 7.
+__global__ void __launch_bounds__(kBrickThreads) k_brick_keep_count(BrickNodes b, uint32_t *__restrict__ tile_n) {
+    const uint64_t j0 = (uint64_t)blockIdx.x * kNodeTile + (uint64_t)threadIdx.x * kNodeItems;
+    uint32_t n = 0;
+#pragma unroll
+    for (int k = 0; k < kNodeItems; ++k) n += brick_kept(b, j0 + k) ? 1u : 0u;
+    uint32_t total;
+    block_excl_scan<uint32_t>(n, &total);
+    if (threadIdx.x == 0) tile_n[blockIdx.x] = total;
+}
+
+__global__ void __launch_bounds__(kBrickThreads) k_brick_keep(BrickNodes b, const uint32_t *__restrict__ tile_n,
+                                                              const uint32_t *__restrict__ tile_first,
+                                                              uint64_t *__restrict__ key, uint32_t *__restrict__ src,
+                                                              uint8_t *__restrict__ mask, uint8_t *__restrict__ count,
+                                                              uint64_t *__restrict__ S, uint32_t *__restrict__ n_kept) {
+    const uint32_t first = tile_first ? tile_first[blockIdx.x] : tiles_before(tile_n, blockIdx.x);
+    const uint64_t j0 = (uint64_t)blockIdx.x * kNodeTile + (uint64_t)threadIdx.x * kNodeItems;
+    uint32_t n = 0, keep = 0;
+#pragma unroll
+    for (int k = 0; k < kNodeItems; ++k)
+        if (brick_kept(b, j0 + k)) {
+            keep |= 1u << k;
+            ++n;
+        }
+    uint32_t total;
+    uint32_t o = first + block_excl_scan<uint32_t>(n, &total);
+    for (; keep; keep &= keep - 1, ++o) {
+        const uint64_t j = j0 + (uint64_t)(__ffs((int)keep) - 1);
+        key[o] = b.key_of ? (uint64_t)b.key_of[j] : j;
+        src[o] = (uint32_t)j;
+        mask[o] = b.mask_of[j];
+        count[o] = (uint8_t)__popc((uint32_t)b.mask_of[j]);
+        S[o] = b.words_of[j];
+    }
+    if (!tile_first && blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) *n_kept = first + total;
+}
+
+// The bricks to place: n of them, with subtree words and child block position
+// indexed by the brick (dense: words_of, B) or by its entry among the kept
+// nodes (S, B, their keys in key), src holding the bricks (dense) or, for 8^3
+// bricks, the index of their bits and voxels.
+struct BrickPlaces {
+    const uint32_t *n;
+    const uint32_t *src;
+    const uint64_t *key;
+    const uint32_t *words_of;
+    const uint64_t *S, *B;
+};
+
+template <bool kDense>
+__device__ __forceinline__ void brick_place(const BrickPlaces &a, uint64_t p, uint64_t &b, uint64_t &at, uint64_t &size) {
+    if (kDense) {
+        b = a.src[p];
+        at = a.B[b];
+        size = a.words_of[b];
+    } else {
+        b = a.key[p];
+        at = a.B[p];
+        size = a.S[p];
+    }
+}
+
+// The last phase of the brick build: every brick's words, relative to its
+// child block (brick.cuh gives the positions).  The 32 lanes of
+// the first warp scan the level counts, four 32-cell words each; 128 threads
+// write the bottom-level nodes, and the warps copy the voxels, in Morton order
+// with consecutive lanes on consecutive cells.  A range past the word count is
+// reported through *err and not written.
+template <bool kDense>
+__global__ void __launch_bounds__(kBrickThreads) k_place_brick16(GridGeom g, BrickPlaces at_of,
+                                                                 const uint32_t *__restrict__ bits,
+                                                                 uint32_t *__restrict__ words, uint64_t W,
+                                                                 uint32_t *__restrict__ err) {
+    __shared__ __align__(16) uint32_t tile[16 * 16 * 16];  // a whole brick's words by Morton code
+    __shared__ __align__(16) uint32_t sb[128];
+    __shared__ uint16_t cell_at[128];  // per 32-cell word: where its cells go
+    __shared__ uint16_t node_at[128];  // ... and its bottom-level nodes
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const uint32_t lt = (1u << lane) - 1u;
+    const bool vec = grid_vec4(g);
+    const uint32_t n = *at_of.n;
+    for (uint32_t p = blockIdx.x; p < n; p += gridDim.x) {
+        uint64_t b, at, size;
+        brick_place<kDense>(at_of, p, b, at, size);
+        if (size == 0) continue;  // only a dropped slice's voxels: no children
+        if (at + size > W) {
+            if (threadIdx.x == 0) atomicOr(err, 4u);
+            continue;
+        }
+        uint32_t *const out = words + at;
+        const int gx0 = (int)(compact3(b) << 4), gy0 = (int)(compact3(b >> 1) << 4), gz0 = (int)(compact3(b >> 2) << 4);
+        uint4 v[4];
+        if (vec) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const int q = threadIdx.x + k * 256;
+                const int gx = gx0 + ((q & 3) << 2), gy = gy0 + ((q >> 2) & 15), gz = gz0 + (q >> 6);
+                v[k] = gx < g.w && gy < g.h && gz < g.d
+                           ? __ldg(reinterpret_cast<const uint4 *>(
+                                 g.grid + (uint64_t)gx + (uint64_t)g.w * ((uint64_t)gy + (uint64_t)g.h * gz)))
+                           : make_uint4(0u, 0u, 0u, 0u);
+            }
+        }
+        __syncthreads();  // the previous brick's readers are done
+        if (wid == 0) {
+            const uint4 w = __ldg(reinterpret_cast<const uint4 *>(bits + brick_linear(g, gx0, gy0, gz0) * 128) + lane);
+            reinterpret_cast<uint4 *>(sb)[lane] = w;
+            const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
+            uint32_t c0 = 0, c1 = 0;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                c0 += (uint32_t)__popc(ww[k]);
+                c1 += (uint32_t)__popc(byte_bits(ww[k]));
+            }
+            const uint32_t ja = (w.x | w.y) != 0u, jb = (w.z | w.w) != 0u;
+            // cells in bits 0..12, bottom-level nodes in 13..22, level-2 nodes in 23..29
+            const uint32_t own = c0 | (c1 << 13) | ((ja + jb) << 23);
+            const uint32_t incl = warp_incl_scan(own), excl = incl - own;
+            const unsigned full = __ballot_sync(FULL, (ja | jb) != 0u);
+            uint32_t mask = 0;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) mask |= (uint32_t)(((full >> (4 * i)) & 15u) != 0) << i;
+            const uint32_t k3 = (uint32_t)__popc(mask);
+            // the level-3 node of this lane is lanes 4i .. 4i + 3
+            const uint32_t bi = __shfl_sync(FULL, excl, lane & ~3), ti = __shfl_sync(FULL, incl, lane | 3);
+            const uint32_t n2t = ti >> 23;
+            const uint32_t n0 = excl & 0x1FFFu, n1 = (excl >> 13) & 0x3FFu, n2 = excl >> 23;
+            const uint32_t m1[4] = {byte_bits(w.x), byte_bits(w.y), byte_bits(w.z), byte_bits(w.w)};
+            const uint32_t a1 = (uint32_t)__popc(m1[0] | (m1[1] << 4)), p0 = (uint32_t)__popc(w.x);
+            const uint32_t p1 = (uint32_t)__popc(w.y), p2 = (uint32_t)__popc(w.z), a0 = p0 + p1;
+            const uint32_t base = k3 + n2t;
+            cell_at[4 * lane] = (uint16_t)(base + n1 + a1 + n0);
+            cell_at[4 * lane + 1] = (uint16_t)(base + n1 + a1 + n0 + p0);
+            cell_at[4 * lane + 2] = (uint16_t)(base + n1 + c1 + n0 + a0);
+            cell_at[4 * lane + 3] = (uint16_t)(base + n1 + c1 + n0 + a0 + p2);
+            node_at[4 * lane] = (uint16_t)(base + n1 + n0);
+            node_at[4 * lane + 1] = (uint16_t)(base + n1 + (uint32_t)__popc(m1[0]) + n0);
+            node_at[4 * lane + 2] = (uint16_t)(base + n1 + a1 + n0 + a0);
+            node_at[4 * lane + 3] = (uint16_t)(base + n1 + a1 + (uint32_t)__popc(m1[2]) + n0 + a0);
+            // level-2 nodes 2 lane and 2 lane + 1
+            const uint32_t before_i = ((bi >> 13) & 0x3FFu) + (bi & 0x1FFFu);
+            uint32_t pos = k3 + n2 + before_i;
+            if (ja) {
+                const uint32_t m = m1[0] | (m1[1] << 4);
+                out[pos] = (m << 8) | m | ((base + n1 + n0 - pos) << 18);
+                ++pos;
+            }
+            if (jb) {
+                const uint32_t m = m1[2] | (m1[3] << 4);
+                out[pos] = (m << 8) | m | ((base + n1 + a1 + n0 + a0 - pos) << 18);
+            }
+            // level-3 nodes, by the first of their four lanes
+            uint32_t m3 = (ja | (jb << 1)) << (2 * (lane & 3));
+            m3 |= __shfl_xor_sync(FULL, m3, 1);
+            m3 |= __shfl_xor_sync(FULL, m3, 2);
+            if ((lane & 3) == 0 && m3) {
+                const uint32_t r3 = (uint32_t)__popc(mask & ((1u << (lane >> 2)) - 1u));
+                out[r3] = (m3 << 8) | m3 | ((k3 + (bi >> 23) + before_i - r3) << 18);
+            }
+        }
+        if (vec) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const int q = threadIdx.x + k * 256;
+                const uint32_t m = (uint32_t)morton3((uint32_t)((q & 3) << 2), (uint32_t)((q >> 2) & 15), (uint32_t)(q >> 6));
+                tile[m] = v[k].x;
+                tile[m + 1] = v[k].y;
+                tile[m + 8] = v[k].z;
+                tile[m + 9] = v[k].w;
+            }
+        }
+        __syncthreads();
+        if (threadIdx.x < 128) {  // the four bottom-level nodes of a 32-cell word
+            const uint32_t w = sb[threadIdx.x];
+            uint32_t pos = node_at[threadIdx.x], child = cell_at[threadIdx.x];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const uint32_t m = (w >> (8 * k)) & 0xFFu;
+                if (!m) continue;
+                out[pos] = (m << 8) | ((child - pos) << 18);
+                ++pos;
+                child += (uint32_t)__popc(m);
+            }
+        }
+        for (int k = 0; k < 16; ++k) {
+            const int c = wid * 16 + k;
+            const uint32_t w = sb[c];
+            if (!((w >> lane) & 1u)) continue;
+            const uint32_t m = (uint32_t)(c * 32 + lane);
+            uint32_t value;
+            if (vec) {
+                value = tile[m];
+            } else {
+                int x, y, z;
+                brick_cell(m, x, y, z);
+                value = __ldg(g.grid + (uint64_t)(gx0 + x) +
+                              (uint64_t)g.w * ((uint64_t)(gy0 + y) + (uint64_t)g.h * (gz0 + z)));
+            }
+            out[(uint32_t)cell_at[c] + (uint32_t)__popc(w & lt)] = value;
+        }
+    }
+}
+
+// The same for 8^3 bricks whose voxels are already compacted (512 words a
+// brick, Morton order): a warp per brick, a lane per 32-cell word.
+template <bool kDense>
+__global__ void __launch_bounds__(256) k_place_brick8(BrickPlaces at_of, uint64_t n_dense,
+                                                      const uint32_t *__restrict__ bits,
+                                                      const uint32_t *__restrict__ slot, uint32_t *__restrict__ words,
+                                                      uint64_t W, uint32_t *__restrict__ err) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const uint32_t lt = (1u << lane) - 1u;
+    const uint64_t n = kDense ? n_dense : (uint64_t)*at_of.n;
+    const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    for (uint64_t p = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; p < n; p += warps) {
+        uint64_t b, at, size;
+        brick_place<kDense>(at_of, p, b, at, size);
+        const uint64_t j = kDense ? p : (uint64_t)at_of.src[p];
+        if (size == 0) continue;
+        if (at + size > W) {
+            if (lane == 0) atomicOr(err, 4u);
+            continue;
+        }
+        uint32_t *const out = words + at;
+        const uint32_t w = lane < 16 ? __ldg(bits + j * 16 + lane) : 0u;
+        const uint32_t m1 = byte_bits(w), c0 = (uint32_t)__popc(w), c1 = (uint32_t)__popc(m1);
+        const uint32_t own = c0 | (c1 << 16);
+        const uint32_t incl = warp_incl_scan(own), excl = incl - own;
+        const uint32_t other = __shfl_xor_sync(FULL, w, 1), m1o = __shfl_xor_sync(FULL, m1, 1);
+        const bool first = !(lane & 1), has = (w | other) != 0u;
+        const unsigned pairs = __ballot_sync(FULL, first && has);
+        const uint32_t k = (uint32_t)__popc(pairs);
+        // the level-2 node of this lane is its even lane and the next
+        const uint32_t bj = __shfl_sync(FULL, excl, lane & ~1), tj = __shfl_sync(FULL, incl, lane | 1);
+        uint32_t pos = k + (excl >> 16) + (bj & 0xFFFFu);
+        const uint32_t cells = k + (tj >> 16) + (excl & 0xFFFFu);
+        uint32_t child = cells;
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            const uint32_t m = (w >> (8 * t)) & 0xFFu;
+            if (!m) continue;
+            out[pos] = (m << 8) | ((child - pos) << 18);
+            ++pos;
+            child += (uint32_t)__popc(m);
+        }
+        if (first && has) {
+            const uint32_t r = (uint32_t)__popc(pairs & lt), m = m1 | (m1o << 4);
+            out[r] = (m << 8) | m | ((k + (excl >> 16) + (excl & 0xFFFFu) - r) << 18);
+        }
+        const uint32_t *const from = slot + j * 512;
+        for (unsigned todo = __ballot_sync(FULL, w != 0u); todo; todo &= todo - 1) {
+            const int c = __ffs((int)todo) - 1;
+            const uint32_t wc = __shfl_sync(FULL, w, c), cc = __shfl_sync(FULL, cells, c),
+                           fc = __shfl_sync(FULL, excl, c) & 0xFFFFu;
+            if ((wc >> lane) & 1u) {
+                const uint32_t r = (uint32_t)__popc(wc & lt);
+                out[cc + r] = from[fc + r];
+            }
+        }
+    }
+}
+
 // ---- level grouping --------------------------------------------------------
 //
 // Every level kernel takes its element count twice: `n` from the host and
@@ -256,12 +690,29 @@ __global__ void k_child_pidx_from_heads(const uint32_t *__restrict__ head, uint6
     pidx[i] = pidx[i] + head[i] - 1u;
 }
 
+// A node's subtree words and far-pointer decision (VoxelOctree.cpp:172-183)
+// from its k children's subtrees; without them (bottom-level nodes) its k
+// voxels.
+__device__ __forceinline__ void subtree_of(uint32_t k, const uint64_t *__restrict__ childS, uint64_t *S,
+                                           uint8_t *large) {
+    uint64_t run = 0;
+    bool far = false;
+    if (childS) {
+        for (uint32_t i = 0; i < k; ++i) {
+            if ((uint64_t)(k - i) + run > 0x3FFFull) far = true;
+            run += childS[i];
+        }
+    }
+    *S = (uint64_t)k * (far ? 2u : 1u) + run;
+    *large = far ? 1 : 0;
+}
+
 // Fused grouping of one level's children (sorted Morton keys) into parents,
 // in tiles of kLvlTile children.  k_level_count counts each tile's heads
 // (children whose key >> 3 differs from the previous child's); an exclusive
 // scan of those counts gives each tile's first parent; k_level_emit stages
 // the tile's keys in shared memory and writes every parent's key, first
-// child, valid mask and child count.  The keys are read twice and only the
+// child, valid mask, child count, subtree words and far decision.  The keys are read twice and only the
 // parents are written, where head flags, a scan over every child and
 // separate passes for the parents, the children's parent indices and the
 // masks read and wrote about three times as many bytes per child.
@@ -313,9 +764,13 @@ __global__ void __launch_bounds__(kLvlThreads) k_level_count(const uint64_t *__r
 // in the keys that follow the tile, staged in shared memory.
 __global__ void __launch_bounds__(kLvlThreads) k_level_emit(const uint64_t *__restrict__ ckey, uint64_t n,
                                                             const uint32_t *__restrict__ dn,
+                                                            const uint32_t *__restrict__ tile_heads,
                                                             const uint32_t *__restrict__ tile_first,
+                                                            const uint64_t *__restrict__ childS,
                                                             uint64_t *__restrict__ pkey, uint32_t *__restrict__ pstart,
-                                                            uint8_t *__restrict__ pmask, uint8_t *__restrict__ pcount) {
+                                                            uint8_t *__restrict__ pmask, uint8_t *__restrict__ pcount,
+                                                            uint64_t *__restrict__ pS, uint8_t *__restrict__ plarge,
+                                                            uint32_t *__restrict__ n_parents) {
     // sk[0]: the child before the tile; sk[1 + q]: child base + q, for q below
     // kLvlTile + 7
     __shared__ uint64_t sk[kLvlTile + 8];
@@ -365,7 +820,11 @@ __global__ void __launch_bounds__(kLvlThreads) k_level_emit(const uint64_t *__re
         wpre[2 * lane + 1] = ex + a0;
     }
     __syncthreads();
-    const uint32_t first = tile_first[blockIdx.x];
+    // the tile's first parent, from a scan or by summing the earlier tiles'
+    // heads here; then the last tile also leaves the level's total
+    const uint32_t first = tile_first ? tile_first[blockIdx.x] : tiles_before(tile_heads, blockIdx.x);
+    if (!tile_first && blockIdx.x == gridDim.x - 1 && threadIdx.x == 0)
+        *n_parents = first + tile_heads[blockIdx.x];
     const unsigned upto = 0xffffffffu >> (31 - lane);  // lanes 0..lane
     // Pass 2a: each lane's octant bits with its run-mates' after it, and its
     // run's end; each round's leading run (the lanes before its first head,
@@ -425,6 +884,7 @@ __global__ void __launch_bounds__(kLvlThreads) k_level_emit(const uint64_t *__re
         pstart[p] = (uint32_t)i;
         pmask[p] = (uint8_t)mm;
         pcount[p] = (uint8_t)cnt;
+        subtree_of(cnt, childS ? childS + i : nullptr, pS + p, plarge + p);
     }
 }
 
@@ -464,11 +924,17 @@ __global__ void k_child_pidx_from_blocks(const uint64_t *__restrict__ ckey, uint
 
 // The root exists even over an empty grid: a root level with no node gets
 // one, with no children (the device-count form of the host's fix-up).
-__global__ void k_root_node(uint32_t *__restrict__ dn, uint64_t *__restrict__ key, uint32_t *__restrict__ start) {
+__global__ void k_root_node(uint32_t *__restrict__ dn, uint64_t *__restrict__ key, uint32_t *__restrict__ start,
+                            uint8_t *__restrict__ mask, uint8_t *__restrict__ count, uint64_t *__restrict__ S,
+                            uint8_t *__restrict__ large) {
     if (*dn == 0) {
         *dn = 1;
         key[0] = 0;
         start[0] = 0;
+        mask[0] = 0;
+        count[0] = 0;
+        S[0] = 0;
+        large[0] = 0;
     }
 }
 
@@ -520,27 +986,14 @@ __global__ void k_subtree(uint64_t np, const uint32_t *__restrict__ dnp, const u
                           uint64_t *__restrict__ S, uint8_t *__restrict__ large) {
     uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= level_count(np, dnp)) return;
-    uint32_t k = count[p];
-    if (bottom) {
-        S[p] = k;
-        large[p] = 0;
-        return;
-    }
-    uint64_t run = 0;
-    bool far = false;
-    uint32_t s0 = pstart[p];
-    for (uint32_t i = 0; i < k; ++i) {
-        if ((uint64_t)(k - i) + run > 0x3FFFull) far = true;
-        run += childS[s0 + i];
-    }
-    S[p] = (uint64_t)k * (far ? 2u : 1u) + run;
-    large[p] = far ? 1 : 0;
+    subtree_of(count[p], bottom ? nullptr : childS + pstart[p], S + p, large + p);
 }
 
 // ---- placement (top-down) ---------------------------------------------------
 
 __global__ void k_root_word(const uint8_t *__restrict__ mask, const uint8_t *__restrict__ large, int root_is_bottom,
-                            uint32_t *__restrict__ words) {
+                            uint64_t *__restrict__ B, uint32_t *__restrict__ words) {
+    B[0] = 1;
     uint32_t m = mask[0];
     words[0] = (m << 8) | (root_is_bottom ? 0u : m) | (large[0] ? 0x10000u : 0u) | (1u << 18);
 }
@@ -605,8 +1058,9 @@ __global__ void k_place_leaves(uint64_t n, const uint32_t *__restrict__ pidx, ui
     words[dst] = payload[i];
 }
 
-// The same placement with a lane per child: a warp takes 32 consecutive
-// parents, whose children follow one another (at most 256), marks which lane
+// The same placement with a lane per child: a warp takes per_warp consecutive
+// parents (32, or 4 where a level has too few to fill the chip: their
+// children then fit one round of the serial loop below), whose children follow one another (at most 256), marks which lane
 // owns each child in a per-warp table, and places the children 32 at a time.
 // A child's block offset is the sum of the subtree sizes of its earlier
 // siblings: a segmented scan over the round's lanes (runs are at most 8
@@ -619,17 +1073,17 @@ __global__ void __launch_bounds__(256) k_place_warp(uint64_t np, const uint32_t 
                                                     const uint64_t *__restrict__ pB, const uint64_t *__restrict__ cS,
                                                     const uint8_t *__restrict__ cmask,
                                                     const uint8_t *__restrict__ clarge, int child_is_bottom,
-                                                    uint64_t nc, const uint32_t *__restrict__ dnc,
+                                                    uint64_t nc, const uint32_t *__restrict__ dnc, int per_warp,
                                                     uint64_t *__restrict__ cB, uint32_t *__restrict__ words,
                                                     uint64_t W, uint32_t *__restrict__ err) {
     __shared__ uint8_t owner[8][256];  // per warp: the lane whose parent holds child s0 + i
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const unsigned upto = 0xffffffffu >> (31 - lane);
     const uint64_t n = level_count(np, dnp);
-    const uint64_t p0 = ((uint64_t)blockIdx.x * blockDim.x) + (uint64_t)wid * 32;
+    const uint64_t p0 = ((uint64_t)blockIdx.x * 8 + wid) * per_warp;
     if (p0 >= n) return;  // uniform per warp
     const uint64_t p = p0 + lane;
-    const bool live = p < n;
+    const bool live = lane < per_warp && p < n;
     const uint32_t k = live ? count[p] : 0u;
     const uint32_t stride = (live && plarge[p]) ? 2u : 1u;
     const uint64_t s = live ? pstart[p] : 0ull, B = live ? pB[p] : 0ull;
@@ -688,7 +1142,7 @@ __global__ void __launch_bounds__(256) k_place_warp(uint64_t np, const uint32_t 
             cB[c] = blk;
             const uint64_t off = blk - pos;
             const uint32_t m = cmask[c];
-            uint32_t w = (m << 8) | (child_is_bottom ? 0u : m) | (clarge[c] ? 0x10000u : 0u);
+            uint32_t w = (m << 8) | (child_is_bottom ? 0u : m) | (clarge && clarge[c] ? 0x10000u : 0u);
             if (pos + (stl == 2u ? 1u : 0u) >= W) {
                 atomicOr(err, 1u);
             } else {
@@ -761,7 +1215,156 @@ __global__ void __launch_bounds__(256) k_place_leaf_runs(uint64_t np, const uint
     }
 }
 
-__global__ void k_set_u64(uint64_t *p, uint64_t v) { *p = v; }
+// ---- dense pyramid over bricks ------------------------------------------------
+//
+// Above bricks the levels hold few nodes: a 2048^3 cube has 2 M bricks and
+// 300,000 nodes above them.  Up to kPyramidBits bits of brick code, every
+// level is an array over all its cells in Morton order (8 consecutive cells
+// are one parent's children), which needs no keys, no scans and no grouping:
+// one thread per parent going up, one per child coming down.  Levels of at
+// most kTopCells children are handled by one CTA in one launch: with so few
+// nodes a level is its launch and one round of memory latency.
+//
+// A 512^3 sphere union of 37 M voxels (42.6 M words) took 55 launches and 544
+// us of kernels through voxel keys, sorted levels and node arrays, and takes
+// 6 launches and 172 us through bricks: 87 for the bits, 59 to place the
+// bricks, 26 for the five levels above.  Beyond kPyramidBits (a 4096^3 cube or
+// a thin grid in one) the arrays would grow with the cube and not with what it
+// holds, so the bricks are compacted and go through the sorted levels.
+constexpr int kPyramidBits = 21;
+constexpr uint32_t kTopCells = 4096, kTopPlaced = 512;  // going up, coming down
+constexpr int kPyramidMax = kPyramidBits / 3 + 1;  // levels, bricks included
+
+struct Pyramid {
+    int base, top;             // level of the bricks, of the root
+    const uint32_t *words_of;  // bricks: subtree words ...
+    const uint8_t *mask_of;    // ... node mask ...
+    const uint8_t *any_of;     // ... and presence (null: a brick with words)
+    uint64_t *S[kPyramidMax];  // level base + l: subtree words (l >= 1)
+    uint64_t *B[kPyramidMax];  // child block position
+    uint8_t *mask[kPyramidMax], *meta[kPyramidMax];  // valid mask; bit 0 present, bit 1 its children are far
+    const uint8_t *topflag;    // cache blocks that exist at level log_block, or null
+    int log_block;
+};
+
+__device__ __forceinline__ uint32_t pyramid_cells(const Pyramid &p, int level) { return 1u << (3 * (p.top - level)); }
+
+// Node `c` of `level` from its children (VoxelOctree.cpp:139-183).
+__device__ __forceinline__ void pyramid_node(const Pyramid &p, int level, uint32_t c) {
+    const int l = level - p.base;
+    uint32_t mask = 0;
+    uint64_t s[8];
+    if (l == 1) {
+        const uint4 a = reinterpret_cast<const uint4 *>(p.words_of)[2 * c], b = reinterpret_cast<const uint4 *>(p.words_of)[2 * c + 1];
+        const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+        uint2 any = make_uint2(0u, 0u);
+        if (p.any_of) any = reinterpret_cast<const uint2 *>(p.any_of)[c];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            s[i] = w[i];
+            const uint32_t there = p.any_of ? ((i < 4 ? any.x : any.y) >> (8 * (i & 3))) & 255u : w[i];
+            mask |= there ? 1u << i : 0u;
+        }
+    } else {
+        const uint2 m = reinterpret_cast<const uint2 *>(p.meta[l - 1])[c];
+        const ulonglong2 *q = reinterpret_cast<const ulonglong2 *>(p.S[l - 1] + 8ull * c);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const ulonglong2 v = q[i];
+            s[2 * i] = v.x;
+            s[2 * i + 1] = v.y;
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) mask |= (((i < 4 ? m.x : m.y) >> (8 * (i & 3))) & 1u) << i;
+    }
+    const uint32_t k = (uint32_t)__popc(mask);
+    uint64_t run = 0;
+    uint32_t r = 0;
+    bool far = false;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        if (!((mask >> i) & 1u)) continue;
+        if ((uint64_t)(k - r) + run > 0x3FFFull) far = true;
+        run += s[i];
+        ++r;
+    }
+    const bool present = mask != 0 || level == p.top || (p.topflag && level == p.log_block && p.topflag[c] != 0);
+    p.mask[l][c] = (uint8_t)mask;
+    p.meta[l][c] = (uint8_t)((present ? 1u : 0u) | (far ? 2u : 0u));
+    p.S[l][c] = (uint64_t)k * (far ? 2u : 1u) + run;
+}
+
+// Cell `c` of `level` (whole warps call, the 8 lanes of a parent together;
+// cells past the level's do nothing): its position in its parent's child
+// block, its descriptor there and its own child block's position
+// (VoxelOctree.cpp:184-205).
+__device__ __forceinline__ void pyramid_place(const Pyramid &p, int level, uint32_t c, uint32_t *__restrict__ words,
+                                              uint64_t W, uint32_t *__restrict__ err) {
+    const int l = level - p.base;
+    const bool in = c < pyramid_cells(p, level);
+    const uint32_t i = c & 7u, up = in ? c >> 3 : 0u;
+    const uint32_t mask = in ? p.mask[l + 1][up] : 0u, meta = p.meta[l + 1][up];
+    const uint64_t B = p.B[l + 1][up];
+    const bool there = (mask >> i) & 1u;
+    const uint64_t S = !there ? 0ull : (l == 0 ? (uint64_t)p.words_of[c] : p.S[l][c]);
+    uint64_t incl = S;
+#pragma unroll
+    for (int d = 1; d < 8; d <<= 1) {
+        const uint64_t t = __shfl_up_sync(0xffffffffu, incl, d, 8);
+        if (i >= (uint32_t)d) incl += t;
+    }
+    if (!there) return;
+    const uint32_t k = (uint32_t)__popc(mask), r = (uint32_t)__popc(mask & ((1u << i) - 1u)), stride = (meta & 2u) ? 2u : 1u;
+    const uint64_t pos = B + (uint64_t)r * stride, blk = B + (uint64_t)k * stride + (incl - S), off = blk - pos;
+    p.B[l][c] = blk;
+    const uint32_t m = l == 0 ? p.mask_of[c] : p.mask[l][c];
+    uint32_t w = (m << 8) | m | (l > 0 && (p.meta[l][c] & 2u) ? 0x10000u : 0u);
+    if (pos + stride > W) {
+        atomicOr(err, 1u);
+        return;
+    }
+    if (stride == 2u) {
+        w |= 0x20000u | (uint32_t)((off >> 32) << 18);
+        words[pos + 1] = (uint32_t)off;
+    } else {
+        w |= (uint32_t)(off << 18);
+    }
+    words[pos] = w;
+}
+
+__global__ void __launch_bounds__(256) k_pyramid_up(Pyramid p, int level) {
+    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c < pyramid_cells(p, level)) pyramid_node(p, level, c);
+}
+
+__global__ void __launch_bounds__(512) k_pyramid_top_up(Pyramid p, int level) {
+    for (; level <= p.top; ++level) {
+        for (uint32_t c = threadIdx.x; c < pyramid_cells(p, level); c += blockDim.x) pyramid_node(p, level, c);
+        __syncthreads();
+    }
+}
+
+__global__ void __launch_bounds__(256) k_pyramid_down(Pyramid p, int level, uint32_t *__restrict__ words, uint64_t W,
+                                                      uint32_t *__restrict__ err) {
+    pyramid_place(p, level, blockIdx.x * blockDim.x + threadIdx.x, words, W, err);
+}
+
+// The root and every level down to `level`.  Zeroes *err.
+__global__ void __launch_bounds__(kTopPlaced) k_pyramid_top_down(Pyramid p, int level, uint32_t *__restrict__ words,
+                                                           uint64_t W, uint32_t *__restrict__ err) {
+    const int t = p.top - p.base;
+    if (threadIdx.x == 0) {
+        *err = 0;
+        const uint32_t m = t ? p.mask[t][0] : p.mask_of[0];
+        words[0] = (m << 8) | m | (t && (p.meta[t][0] & 2u) ? 0x10000u : 0u) | (1u << 18);
+        p.B[t][0] = 1;
+    }
+    __syncthreads();
+    for (int e = p.top - 1; e >= level; --e) {
+        for (uint32_t c0 = 0; c0 < pyramid_cells(p, e); c0 += blockDim.x) pyramid_place(p, e, c0 + threadIdx.x, words, W, err);
+        __syncthreads();
+    }
+}
 
 inline unsigned blocks_for(uint64_t n, int t = 256) {
     uint64_t b = (n + t - 1) / t;
@@ -844,7 +1447,16 @@ struct LevelArrays {
     DevBuf<uint64_t> key;
     DevBuf<uint32_t> start;
     DevBuf<uint8_t> mask, count, large;
-    DevBuf<uint64_t> S, B;
+    DevBuf<uint64_t> S, B;  // subtree words; child block position (placement)
+    cudaError_t alloc(uint64_t nodes, BuildArena &a) {
+        cudaError_t e = key.alloc(nodes, a);
+        if (e == cudaSuccess) e = start.alloc(nodes, a);
+        if (e == cudaSuccess) e = mask.alloc(nodes, a);
+        if (e == cudaSuccess) e = count.alloc(nodes, a);
+        if (e == cudaSuccess) e = large.alloc(nodes, a);
+        if (e == cudaSuccess) e = S.alloc(nodes, a);
+        return e;
+    }
 };
 
 #define SVO_TRY_ALLOC(expr)                                                   \
@@ -881,33 +1493,41 @@ int scan_on_device(const uint32_t *in, TO *out, uint64_t n, TO *d_total, cudaStr
 // Levels whose children number at most this many are chained on the device.
 constexpr uint64_t kDeviceLevels = 1ull << 20;
 
-}  // namespace
+// Parents per warp of k_place_warp: 4 while that many warps fit the chip at
+// once (152 SMs x 64), else 32.
+int parents_per_warp(uint64_t n) { return n <= 4ull * 152 * 64 ? 4 : 32; }
 
-int build_from_sorted_device(const uint64_t *d_keys, const uint32_t *d_payload, uint64_t N, int log_side,
-                             int log_block, const uint8_t *d_topflag, cudaStream_t st, uint32_t **d_words_out,
-                             uint64_t *n_words_out) {
-    const int D = log_side;
+// Phases 2 and 3 above level `base` (see the top): the levels base + 1 .. D grouped
+// bottom-up with their subtree sizes, then the words allocated, the levels
+// placed top-down, and place_base(words, W, err) writes what lies below the
+// base nodes' descriptors.  Level 0 is the voxels (leaf_keys, n_leaves);
+// above it lv[base] comes with key, mask, count and S (large: none), and its
+// count on the device (dn).  n_voxels: optionally, the voxels' total on the
+// device, refused at 2^32-1 and more.
+template <typename PlaceBase>
+int build_levels(std::vector<LevelArrays> &lv, int base, const uint64_t *leaf_keys, uint64_t n_leaves, int D,
+                 int log_block, const uint8_t *d_topflag, BuildArena &arena, cudaStream_t st,
+                 const unsigned long long *n_voxels, PlaceBase place_base, uint32_t **d_words_out,
+                 uint64_t *n_words_out) {
     const bool multi_block = log_block < D;
     const uint64_t n_blocks = multi_block ? (1ull << (3 * (D - log_block))) : 0;
     if (multi_block && !d_topflag) return set_error(SVO_ERR_INVALID, "build: missing cache-block flags");
-    if (N >= 0xFFFFFFFFull) return set_error(SVO_ERR_LIMIT, "%llu occupied voxels exceed 2^32-1", (unsigned long long)N);
     int rc = SVO_OK;
-    BuildArena arena(st);  // declared first: released after every array below
 
-    // Phase 2: levels e = 1..D (node edge 2^e); level 0 is the leaves.
     // While a level's children number more than kDeviceLevels, the parent
     // count is read back (exact array sizes).  From the first level with
-    // fewer children on, the counts stay on the device (dcount[e]) and the
-    // arrays are sized by upper bounds: no host round trip per level.
-    std::vector<LevelArrays> lv(D + 1);
+    // fewer children on, and everywhere above bricks, the counts stay on the
+    // device (dcount[e]) and the arrays are sized by upper bounds: no host
+    // round trip per level.
     DevBuf<uint32_t> dcount;
     SVO_TRY_ALLOC(dcount.alloc(D + 1, arena));
-    const uint64_t *ckey = d_keys;
-    uint64_t nc = N;              // children: exact count, or an upper bound when cdn != nullptr
-    const uint32_t *cdn = nullptr;  // device count of the children
-    bool on_device = false;
-    for (int e = 1; e <= D; ++e) {
+    const uint64_t *ckey = base ? lv[base].key.p : leaf_keys;
+    uint64_t nc = base ? lv[base].n : n_leaves;  // children: exact count, or an upper bound when cdn != nullptr
+    const uint32_t *cdn = base ? lv[base].dn : nullptr;  // device count of the children
+    bool on_device = cdn != nullptr;
+    for (int e = base + 1; e <= D; ++e) {
         LevelArrays &L = lv[e];
+        const uint64_t *childS = e > 1 ? lv[e - 1].S.p : nullptr;
         if (!on_device && nc <= kDeviceLevels) on_device = true;
         uint32_t *dn = on_device ? dcount.p + e : nullptr;
         // at most one node per cell of edge 2^e, and never more parents than children
@@ -939,10 +1559,7 @@ int build_from_sorted_device(const uint64_t *d_keys, const uint32_t *d_payload, 
             }
             if (rc) return rc;
             if (e == D && L.n == 0) L.n = 1;  // the root (fixed up below)
-            SVO_TRY_ALLOC(L.key.alloc(L.n, arena));
-            SVO_TRY_ALLOC(L.start.alloc(L.n, arena));
-            SVO_TRY_ALLOC(L.mask.alloc(L.n, arena));
-            SVO_TRY_ALLOC(L.count.alloc(L.n, arena));
+            SVO_TRY_ALLOC(L.alloc(L.n, arena));
             // blocks only the top table marks keep mask and count 0
             SVO_CUDA_TRY(cudaMemsetAsync(L.mask.p, 0, L.n, st));
             SVO_CUDA_TRY(cudaMemsetAsync(L.count.p, 0, L.n, st));
@@ -953,21 +1570,25 @@ int build_from_sorted_device(const uint64_t *d_keys, const uint32_t *d_payload, 
                 k_parent_masks_warp<<<blocks_for(nc), 256, 0, st>>>(ckey, nc, cdn, pidx.p, L.mask.p, L.count.p);
                 SVO_LAUNCH_CHECK("k_parent_masks_warp");
             }
+            k_subtree<<<blocks_for(L.n), 256, 0, st>>>(L.n, dn, L.count.p, L.start.p, childS, e == 1, L.S.p, L.large.p);
+            SVO_LAUNCH_CHECK("k_subtree");
         } else {
-            // Fused grouping: tile head counts, their scan, then the parents.
+            // Fused grouping: tile head counts, their scan (a few tiles sum
+            // the earlier ones themselves), then the parents.
             const uint64_t tiles = (nc + kLvlTile - 1) / kLvlTile;
+            const bool self = on_device && tiles <= kSelfScanTiles;
             DevBuf<uint32_t> th, tf;
             SVO_TRY_ALLOC(th.alloc(tiles, arena));
-            SVO_TRY_ALLOC(tf.alloc(tiles, arena));
+            if (!self) SVO_TRY_ALLOC(tf.alloc(tiles, arena));
             if (nc) {
                 k_level_count<<<(unsigned)tiles, kLvlThreads, 0, st>>>(ckey, nc, cdn, th.p);
                 SVO_LAUNCH_CHECK("k_level_count");
             }
             if (on_device) {
-                if (tiles)
-                    rc = scan_on_device<uint32_t>(th.p, tf.p, tiles, dn, st, arena);
-                else
+                if (!tiles)
                     SVO_CUDA_TRY(cudaMemsetAsync(dn, 0, sizeof(uint32_t), st));
+                else if (!self)
+                    rc = scan_on_device<uint32_t>(th.p, tf.p, tiles, dn, st, arena);
                 L.n = std::min(nc, cells);
             } else {
                 uint32_t np = 0;
@@ -976,85 +1597,308 @@ int build_from_sorted_device(const uint64_t *d_keys, const uint32_t *d_payload, 
             }
             if (rc) return rc;
             if (e == D && L.n == 0) L.n = 1;  // the root (fixed up below)
-            SVO_TRY_ALLOC(L.key.alloc(L.n, arena));
-            SVO_TRY_ALLOC(L.start.alloc(L.n, arena));
-            SVO_TRY_ALLOC(L.mask.alloc(L.n, arena));
-            SVO_TRY_ALLOC(L.count.alloc(L.n, arena));
-            if (e == D) {  // a root added over an empty grid has no children
-                SVO_CUDA_TRY(cudaMemsetAsync(L.key.p, 0, sizeof(uint64_t), st));
-                SVO_CUDA_TRY(cudaMemsetAsync(L.start.p, 0, sizeof(uint32_t), st));
-                SVO_CUDA_TRY(cudaMemsetAsync(L.mask.p, 0, 1, st));
-                SVO_CUDA_TRY(cudaMemsetAsync(L.count.p, 0, 1, st));
-            }
+            SVO_TRY_ALLOC(L.alloc(L.n, arena));
             if (nc) {
-                k_level_emit<<<(unsigned)tiles, kLvlThreads, 0, st>>>(ckey, nc, cdn, tf.p, L.key.p, L.start.p,
-                                                                    L.mask.p, L.count.p);
+                k_level_emit<<<(unsigned)tiles, kLvlThreads, 0, st>>>(ckey, nc, cdn, th.p, self ? nullptr : tf.p, childS,
+                                                                    L.key.p, L.start.p, L.mask.p, L.count.p, L.S.p,
+                                                                    L.large.p, dn);
                 SVO_LAUNCH_CHECK("k_level_emit");
             }
-        }
-        // The root always exists, even over an empty grid.
-        if (e == D && on_device) {
-            k_root_node<<<1, 1, 0, st>>>(dn, L.key.p, L.start.p);
-            SVO_LAUNCH_CHECK("k_root_node");
         }
         L.dn = dn;
         ckey = L.key.p;
         nc = L.n;
         cdn = L.dn;
     }
+    // The root always exists, even over an empty grid (its level's count is
+    // on the device: it has at most 8 children).
+    k_root_node<<<1, 1, 0, st>>>(const_cast<uint32_t *>(lv[D].dn), lv[D].key.p, lv[D].start.p, lv[D].mask.p,
+                                 lv[D].count.p, lv[D].S.p, lv[D].large.p);
+    SVO_LAUNCH_CHECK("k_root_node");
 
-    // Subtree sizes, bottom-up.
-    for (int e = 1; e <= D; ++e) {
-        LevelArrays &L = lv[e];
-        SVO_TRY_ALLOC(L.S.alloc(L.n, arena));
-        SVO_TRY_ALLOC(L.large.alloc(L.n, arena));
-        k_subtree<<<blocks_for(L.n), 256, 0, st>>>(L.n, L.dn, L.count.p, L.start.p, e > 1 ? lv[e - 1].S.p : nullptr,
-                                                  e == 1, L.S.p, L.large.p);
-        SVO_LAUNCH_CHECK("k_subtree");
-    }
     uint64_t S_root = 0;
+    unsigned long long voxels = 0;
     SVO_CUDA_TRY(cudaMemcpyAsync(&S_root, lv[D].S.p, sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
+    if (n_voxels) SVO_CUDA_TRY(cudaMemcpyAsync(&voxels, n_voxels, sizeof(voxels), cudaMemcpyDeviceToHost, st));
     SVO_CUDA_TRY(cudaStreamSynchronize(st));
+    if (voxels >= 0xFFFFFFFFull) return set_error(SVO_ERR_LIMIT, "%llu occupied voxels exceed 2^32-1", voxels);
     const uint64_t W = 1 + S_root;
 
     uint32_t *words = nullptr;
     SVO_CUDA_TRY(cudaMallocAsync((void **)&words, (size_t)W * sizeof(uint32_t), st));
-    DevBuf<uint32_t> err;
-    SVO_TRY_ALLOC(err.alloc(1, arena));
-    SVO_CUDA_TRY(cudaMemsetAsync(err.p, 0, sizeof(uint32_t), st));
-
-    // Placement, top-down.
-    SVO_TRY_ALLOC(lv[D].B.alloc(1, arena));
-    k_set_u64<<<1, 1, 0, st>>>(lv[D].B.p, 1);
-    k_root_word<<<1, 1, 0, st>>>(lv[D].mask.p, lv[D].large.p, D == 1, words);
-    for (int e = D; e >= 2; --e) {
-        LevelArrays &P = lv[e];
-        LevelArrays &C = lv[e - 1];
-        SVO_TRY_ALLOC(C.B.alloc(C.n, arena));
-        k_place_warp<<<blocks_for(P.n), 256, 0, st>>>(P.n, P.dn, P.count.p, P.start.p, P.large.p, P.B.p, C.S.p,
-                                                     C.mask.p, C.large.p, e - 1 == 1, C.n, C.dn, C.B.p, words, W,
-                                                     err.p);
-        SVO_LAUNCH_CHECK("k_place_warp");
-    }
-    if (N) {
-        k_place_leaf_runs<<<blocks_for(lv[1].n), 256, 0, st>>>(lv[1].n, lv[1].dn, lv[1].count.p, lv[1].start.p,
-                                                               lv[1].B.p, d_payload, N, words, W, err.p);
-        SVO_LAUNCH_CHECK("k_place_leaf_runs");
-    }
-    uint32_t err_h = 0;
-    cudaError_t e = cudaMemcpyAsync(&err_h, err.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) {
+    auto place = [&]() -> int {
+        DevBuf<uint32_t> err;
+        SVO_TRY_ALLOC(err.alloc(1, arena));
+        SVO_CUDA_TRY(cudaMemsetAsync(err.p, 0, sizeof(uint32_t), st));
+        SVO_TRY_ALLOC(lv[D].B.alloc(1, arena));
+        k_root_word<<<1, 1, 0, st>>>(lv[D].mask.p, lv[D].large.p, D == 1, lv[D].B.p, words);
+        SVO_LAUNCH_CHECK("k_root_word");
+        for (int e = D; e > std::max(base, 1); --e) {
+            LevelArrays &P = lv[e];
+            LevelArrays &C = lv[e - 1];
+            SVO_TRY_ALLOC(C.B.alloc(C.n, arena));
+            const int ppw = parents_per_warp(P.n);
+            k_place_warp<<<blocks_for(P.n, 8 * ppw), 256, 0, st>>>(P.n, P.dn, P.count.p, P.start.p, P.large.p, P.B.p,
+                                                                  C.S.p, C.mask.p, C.large.p, e - 1 == 1, C.n, C.dn,
+                                                                  ppw, C.B.p, words, W, err.p);
+            SVO_LAUNCH_CHECK("k_place_warp");
+        }
+        int r = place_base(words, W, err.p);
+        if (r) return r;
+        uint32_t err_h = 0;
+        SVO_CUDA_TRY(cudaMemcpyAsync(&err_h, err.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+        SVO_CUDA_TRY(cudaStreamSynchronize(st));
+        if (err_h) return set_error(SVO_ERR_DEVICE, "octree build placement check failed (flags %u)", err_h);
+        return SVO_OK;
+    };
+    rc = place();
+    if (rc) {
         cudaFree(words);
-        return cuda_fail(e, "octree build");
-    }
-    if (err_h) {
-        cudaFree(words);
-        return set_error(SVO_ERR_DEVICE, "octree build placement check failed (flags %u)", err_h);
+        return rc;
     }
     *d_words_out = words;
     *n_words_out = W;
     return SVO_OK;
+}
+
+// The kept bricks (at most `most` of them) as nodes of their level, with the
+// count on the device, and their own indices in `src`.
+int keep_bricks(const BrickNodes &b, uint64_t most, LevelArrays &L, DevBuf<uint32_t> &src, DevBuf<uint32_t> &n_kept,
+                BuildArena &arena, cudaStream_t st) {
+    const uint64_t tiles = (b.n + kNodeTile - 1) / kNodeTile;
+    L.n = std::max<uint64_t>(most, 1);
+    SVO_TRY_ALLOC(n_kept.alloc(1, arena));
+    SVO_TRY_ALLOC(src.alloc(L.n, arena));
+    SVO_TRY_ALLOC(L.key.alloc(L.n, arena));
+    SVO_TRY_ALLOC(L.mask.alloc(L.n, arena));
+    SVO_TRY_ALLOC(L.count.alloc(L.n, arena));
+    SVO_TRY_ALLOC(L.S.alloc(L.n, arena));
+    L.dn = n_kept.p;
+    if (tiles == 0) {
+        SVO_CUDA_TRY(cudaMemsetAsync(n_kept.p, 0, sizeof(uint32_t), st));
+        return SVO_OK;
+    }
+    DevBuf<uint32_t> tn, tf;
+    SVO_TRY_ALLOC(tn.alloc(tiles, arena));
+    k_brick_keep_count<<<(unsigned)tiles, kBrickThreads, 0, st>>>(b, tn.p);
+    SVO_LAUNCH_CHECK("k_brick_keep_count");
+    const bool self = tiles <= kSelfScanTiles;
+    if (!self) {
+        SVO_TRY_ALLOC(tf.alloc(tiles, arena));
+        int rc = scan_on_device<uint32_t>(tn.p, tf.p, tiles, n_kept.p, st, arena);
+        if (rc) return rc;
+    }
+    k_brick_keep<<<(unsigned)tiles, kBrickThreads, 0, st>>>(b, tn.p, self ? nullptr : tf.p, L.key.p, src.p, L.mask.p,
+                                                            L.count.p, L.S.p, n_kept.p);
+    SVO_LAUNCH_CHECK("k_brick_keep");
+    return SVO_OK;
+}
+
+}  // namespace
+
+int build_from_sorted_device(const uint64_t *d_keys, const uint32_t *d_payload, uint64_t N, int log_side,
+                             int log_block, const uint8_t *d_topflag, cudaStream_t st, uint32_t **d_words_out,
+                             uint64_t *n_words_out) {
+    const int D = log_side;
+    if (N >= 0xFFFFFFFFull) return set_error(SVO_ERR_LIMIT, "%llu occupied voxels exceed 2^32-1", (unsigned long long)N);
+    BuildArena arena(st);  // declared first: released after every array below
+    std::vector<LevelArrays> lv(D + 1);
+    auto leaves = [&](uint32_t *words, uint64_t W, uint32_t *err) -> int {
+        if (!N) return SVO_OK;
+        k_place_leaf_runs<<<blocks_for(lv[1].n), 256, 0, st>>>(lv[1].n, lv[1].dn, lv[1].count.p, lv[1].start.p,
+                                                               lv[1].B.p, d_payload, N, words, W, err);
+        SVO_LAUNCH_CHECK("k_place_leaf_runs");
+        return SVO_OK;
+    };
+    return build_levels(lv, 0, d_keys, N, D, log_block, d_topflag, arena, st, nullptr, leaves, d_words_out,
+                        n_words_out);
+}
+
+bool bricks_dense(int log_side, int log_brick) { return 3 * (log_side - log_brick) <= kPyramidBits; }
+
+// The build above bricks whose subtree words (and masks, presence) are arrays
+// over all brick codes; place_bricks(places, words, W, err) writes the bricks'
+// own words, places.n, .src and the like left to it.
+template <typename PlaceBricks>
+static int build_pyramid(int base, int D, const uint32_t *words_of, const uint8_t *mask_of, const uint8_t *any_of,
+                         int log_block, const uint8_t *d_topflag, BuildArena &arena, cudaStream_t st,
+                         const unsigned long long *n_voxels, PlaceBricks place_bricks, uint32_t **d_words_out,
+                         uint64_t *n_words_out) {
+    if (log_block < D && !any_of && !d_topflag) return set_error(SVO_ERR_INVALID, "build: missing cache-block flags");
+    Pyramid p{};
+    p.base = base;
+    p.top = D;
+    p.words_of = words_of;
+    p.mask_of = mask_of;
+    p.any_of = any_of;
+    p.topflag = log_block < D ? d_topflag : nullptr;
+    p.log_block = log_block;
+    DevBuf<uint64_t> S[kPyramidMax], B[kPyramidMax];
+    DevBuf<uint8_t> mask[kPyramidMax], meta[kPyramidMax];
+    DevBuf<uint32_t> err;
+    SVO_TRY_ALLOC(err.alloc(1, arena));
+    for (int l = 0; l <= D - base; ++l) {
+        const uint64_t cells = 1ull << (3 * (D - base - l));
+        SVO_TRY_ALLOC(B[l].alloc(cells, arena));
+        p.B[l] = B[l].p;
+        if (!l) continue;
+        SVO_TRY_ALLOC(S[l].alloc(cells, arena));
+        SVO_TRY_ALLOC(mask[l].alloc(cells, arena));
+        SVO_TRY_ALLOC(meta[l].alloc(cells, arena));
+        p.S[l] = S[l].p;
+        p.mask[l] = mask[l].p;
+        p.meta[l] = meta[l].p;
+    }
+    // levels with more than kTopCells children one launch each, the rest in one
+    int e = base + 1;
+    for (; e <= D && (1ull << (3 * (D - e + 1))) > kTopCells; ++e) {
+        const uint64_t cells = 1ull << (3 * (D - e));
+        k_pyramid_up<<<blocks_for(cells), 256, 0, st>>>(p, e);
+        SVO_LAUNCH_CHECK("k_pyramid_up");
+    }
+    if (e <= D) {
+        k_pyramid_top_up<<<1, 512, 0, st>>>(p, e);
+        SVO_LAUNCH_CHECK("k_pyramid_top_up");
+    }
+    uint64_t S_root = 0;
+    unsigned long long voxels = 0;
+    if (D == base) {
+        uint32_t s32 = 0;
+        SVO_CUDA_TRY(cudaMemcpyAsync(&s32, words_of, sizeof(s32), cudaMemcpyDeviceToHost, st));
+        SVO_CUDA_TRY(cudaStreamSynchronize(st));
+        S_root = s32;
+    } else {
+        SVO_CUDA_TRY(cudaMemcpyAsync(&S_root, p.S[D - base], sizeof(S_root), cudaMemcpyDeviceToHost, st));
+        if (n_voxels) SVO_CUDA_TRY(cudaMemcpyAsync(&voxels, n_voxels, sizeof(voxels), cudaMemcpyDeviceToHost, st));
+        SVO_CUDA_TRY(cudaStreamSynchronize(st));
+    }
+    if (voxels >= 0xFFFFFFFFull) return set_error(SVO_ERR_LIMIT, "%llu occupied voxels exceed 2^32-1", voxels);
+    const uint64_t W = 1 + S_root;
+    uint32_t *words = nullptr;
+    SVO_CUDA_TRY(cudaMallocAsync((void **)&words, (size_t)W * sizeof(uint32_t), st));
+    auto place = [&]() -> int {
+        int c = D;
+        while (c > base && (1ull << (3 * (D - c + 1))) <= kTopPlaced) --c;
+        k_pyramid_top_down<<<1, (unsigned)kTopPlaced, 0, st>>>(p, c, words, W, err.p);
+        SVO_LAUNCH_CHECK("k_pyramid_top_down");
+        for (--c; c >= base; --c) {
+            k_pyramid_down<<<blocks_for(1ull << (3 * (D - c))), 256, 0, st>>>(p, c, words, W, err.p);
+            SVO_LAUNCH_CHECK("k_pyramid_down");
+        }
+        BrickPlaces places{};
+        places.words_of = words_of;
+        places.B = p.B[0];
+        int r = place_bricks(places, words, W, err.p);
+        if (r) return r;
+        uint32_t err_h = 0;
+        SVO_CUDA_TRY(cudaMemcpyAsync(&err_h, err.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+        SVO_CUDA_TRY(cudaStreamSynchronize(st));
+        if (err_h) return set_error(SVO_ERR_DEVICE, "octree build placement check failed (flags %u)", err_h);
+        return SVO_OK;
+    };
+    const int rc = place();
+    if (rc) {
+        cudaFree(words);
+        return rc;
+    }
+    *d_words_out = words;
+    *n_words_out = W;
+    return SVO_OK;
+}
+
+int build_from_bricks_device(const MeshBricks &m, int log_side, int log_block, const uint8_t *d_topflag,
+                             cudaStream_t st, uint32_t **d_words_out, uint64_t *n_words_out) {
+    constexpr int kBase = 3;
+    const int D = log_side;
+    BuildArena arena(st);
+    const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((m.n + 7) / 8, 152 * 32));
+    if (bricks_dense(D, kBase)) {
+        auto bricks = [&](BrickPlaces places, uint32_t *words, uint64_t W, uint32_t *err) -> int {
+            places.src = m.key;
+            k_place_brick8<true><<<grid, 256, 0, st>>>(places, m.n, m.bits, m.slot, words, W, err);
+            SVO_LAUNCH_CHECK("k_place_brick8");
+            return SVO_OK;
+        };
+        return build_pyramid(kBase, D, m.words, m.mask, nullptr, log_block, d_topflag, arena, st, m.n_voxels, bricks,
+                             d_words_out, n_words_out);
+    }
+    std::vector<LevelArrays> lv(D + 1);
+    DevBuf<uint32_t> src, n_kept;
+    LevelArrays &L = lv[kBase];
+    const BrickNodes b{m.n, m.key, m.words, m.mask, nullptr};
+    int rc = keep_bricks(b, m.n, L, src, n_kept, arena, st);
+    if (rc) return rc;
+    auto bricks = [&](uint32_t *words, uint64_t W, uint32_t *err) -> int {
+        const BrickPlaces places{n_kept.p, src.p, L.key.p, nullptr, L.S.p, L.B.p};
+        k_place_brick8<false><<<grid, 256, 0, st>>>(places, 0, m.bits, m.slot, words, W, err);
+        SVO_LAUNCH_CHECK("k_place_brick8");
+        return SVO_OK;
+    };
+    return build_levels(lv, kBase, nullptr, 0, D, log_block, d_topflag, arena, st, m.n_voxels, bricks, d_words_out,
+                        n_words_out);
+}
+
+// The dense build through 16^3 bricks: their bits, the levels above them, and
+// every brick's words.  Cache blocks, if several, are at least a brick.
+static int build_dense_bricks(const GridGeom &g, int D, uint64_t n_bricks, cudaStream_t st, uint32_t **d_words_out,
+                              uint64_t *n_words_out) {
+    constexpr int kBase = 4;
+    const bool multi_block = g.log_block < D, dense = bricks_dense(D, kBase);
+    const uint64_t cells = (uint64_t)g.w * (uint64_t)g.h * (uint64_t)g.d;
+    const uint64_t covering = (uint64_t)((g.w + 15) / 16) * (uint64_t)((g.h + 15) / 16) * (uint64_t)((g.d + 15) / 16);
+    BuildArena arena(st);
+    DevBuf<uint32_t> bits, words_of, list, n_list;
+    DevBuf<uint8_t> mask_of, any_of;
+    DevBuf<unsigned long long> n_voxels;
+    SVO_TRY_ALLOC(bits.alloc(covering * 128, st));
+    SVO_TRY_ALLOC(words_of.alloc(n_bricks, arena));
+    SVO_TRY_ALLOC(mask_of.alloc(n_bricks, arena));
+    // where the cache block is a brick, one with only dropped voxels is a
+    // descriptor without children
+    const bool any = multi_block && g.log_block == kBase;
+    if (any) SVO_TRY_ALLOC(any_of.alloc(n_bricks, arena));
+    if (dense) {
+        SVO_TRY_ALLOC(list.alloc(covering, arena));
+        SVO_TRY_ALLOC(n_list.alloc(1, arena));
+        SVO_CUDA_TRY(cudaMemsetAsync(n_list.p, 0, sizeof(uint32_t), st));
+    }
+    if (cells >= 0xFFFFFFFFull) {  // the voxels may exceed the build's limit
+        SVO_TRY_ALLOC(n_voxels.alloc(1, arena));
+        SVO_CUDA_TRY(cudaMemsetAsync(n_voxels.p, 0, sizeof(unsigned long long), st));
+    }
+    const unsigned grid = (unsigned)std::min<uint64_t>(n_bricks, 1ull << 20);
+    k_brick_bits<<<grid, kBrickThreads, 0, st>>>(g, n_bricks, bits.p, words_of.p, mask_of.p, any_of.p, list.p,
+                                                 n_list.p, n_voxels.p);
+    SVO_LAUNCH_CHECK("k_brick_bits");
+    // a cache block that is a brick is a node already
+    const int log_block = any ? D : g.log_block;
+    const uint8_t *const topflag = any ? nullptr : g.topflag;
+    const unsigned pgrid = (unsigned)std::min<uint64_t>(covering, 1ull << 14);
+    if (dense) {
+        auto bricks = [&](BrickPlaces places, uint32_t *words, uint64_t W, uint32_t *err) -> int {
+            places.n = n_list.p;
+            places.src = list.p;
+            k_place_brick16<true><<<pgrid, kBrickThreads, 0, st>>>(g, places, bits.p, words, W, err);
+            SVO_LAUNCH_CHECK("k_place_brick16");
+            return SVO_OK;
+        };
+        return build_pyramid(kBase, D, words_of.p, mask_of.p, any_of.p, log_block, topflag, arena, st, n_voxels.p,
+                             bricks, d_words_out, n_words_out);
+    }
+    std::vector<LevelArrays> lv(D + 1);
+    DevBuf<uint32_t> src, n_kept;
+    LevelArrays &L = lv[kBase];
+    const BrickNodes b{n_bricks, nullptr, words_of.p, mask_of.p, any_of.p};
+    int rc = keep_bricks(b, covering, L, src, n_kept, arena, st);
+    if (rc) return rc;
+    auto bricks = [&](uint32_t *words, uint64_t W, uint32_t *err) -> int {
+        const BrickPlaces places{n_kept.p, nullptr, L.key.p, nullptr, L.S.p, L.B.p};
+        k_place_brick16<false><<<pgrid, kBrickThreads, 0, st>>>(g, places, bits.p, words, W, err);
+        SVO_LAUNCH_CHECK("k_place_brick16");
+        return SVO_OK;
+    };
+    return build_levels(lv, kBase, nullptr, 0, D, log_block, topflag, arena, st, n_voxels.p, bricks, d_words_out,
+                        n_words_out);
 }
 
 int build_dense_device(const uint32_t *d_grid, int w, int h, int d, int log_side, int log_block, cudaStream_t st,
@@ -1084,6 +1928,10 @@ int build_dense_device(const uint32_t *d_grid, int w, int h, int d, int log_side
         SVO_CUDA_TRY(cudaMemsetAsync(topflag.p, 0, n_blocks, st));
         g.topflag = topflag.p;
     }
+    // Brick keys index 32-bit source arrays; smaller cubes and cache blocks
+    // below a brick (budgets of a few KB) take the voxel by voxel form.
+    if (D >= 4 && (!multi_block || log_block >= 4) && n_bricks <= 0xFFFFFFFFull)
+        return build_dense_bricks(g, D, n_bricks, st, d_words_out, n_words_out);
 
     // Phase 1: extraction in Morton order.
     DevBuf<uint32_t> bcount;
@@ -1319,8 +2167,7 @@ int build_dense_noalloc(const uint32_t *d_grid, int w, int h, int d, int log_sid
     SVO_CUDA_TRY(cudaMemsetAsync(err, 0, sizeof(uint32_t), st));
     SVO_ARENA_TAKE(rootB, uint64_t, 1);
     lv[D].B = rootB;
-    k_set_u64<<<1, 1, 0, st>>>(lv[D].B, 1);
-    k_root_word<<<1, 1, 0, st>>>(lv[D].mask, lv[D].large, D == 1, d_words);
+    k_root_word<<<1, 1, 0, st>>>(lv[D].mask, lv[D].large, D == 1, lv[D].B, d_words);
     for (int e = D; e >= 2; --e) {
         ArenaLevel &P = lv[e];
         ArenaLevel &C = lv[e - 1];

@@ -93,6 +93,24 @@ int build_from_sorted_device(const uint64_t *d_keys, const uint32_t *d_payload, 
                              int log_block, const uint8_t *d_topflag, cudaStream_t st, uint32_t **d_words,
                              uint64_t *n_words);
 
+// The same from 8^3 bricks in ascending Morton order (brick.cuh): per brick its
+// key (the Morton code of the brick), 16 words of occupancy bits and 512 words
+// holding its voxels in Morton order; and per brick, or with bricks_dense(
+// log_side, 3) per brick code of the whole cube, the subtree's words (0 where
+// there is no voxel) and the node's mask.  n_voxels: the voxels' total, or
+// null where it is known to be below 2^32-1.  log_block is 4 or more, or
+// log_side.
+struct MeshBricks {
+    uint64_t n;
+    const uint32_t *key, *words;
+    const uint8_t *mask;
+    const uint32_t *bits, *slot;
+    const unsigned long long *n_voxels;
+};
+bool bricks_dense(int log_side, int log_brick);
+int build_from_bricks_device(const MeshBricks &m, int log_side, int log_block, const uint8_t *d_topflag,
+                             cudaStream_t st, uint32_t **d_words, uint64_t *n_words);
+
 // The .voxel build streamed in z slabs of about slab_bytes (voxel_stream.cu);
 // fp is positioned after the 12-byte header.
 int build_voxel_file_streamed(FILE *fp, int w, int h, int d, uint64_t mem, uint64_t slab_bytes, cudaStream_t st,

@@ -42,6 +42,7 @@
 #include <cstring>
 #include <vector>
 
+#include "brick.cuh"
 #include "mesh.h"
 #include "morton.cuh"
 #include "scan.cuh"
@@ -375,6 +376,10 @@ struct FoldArgs {
     int dims[3];
     int log_block;
     uint32_t *slot;
+    uint32_t *node_words;  // or null: per brick (edge 8), its subtree's words and its node's mask (brick.cuh)
+    uint8_t *node_mask;
+    int node_by_key;     // 1: indexed by the brick's key, else by the brick
+    unsigned long long *n_voxels;  // or null: += the bricks' voxels
     int sub_bricks;  // 1: sub-block edges are multiples of the brick edge, so a brick lies in one sub-block
 };
 
@@ -474,16 +479,10 @@ __device__ __forceinline__ void divmod_small(int v, int n, int rcp, int &q, int 
     r = v - q * n;
 }
 
-// Brick-local Morton index (edge at most 8) of a cell, and back.
+// Brick-local Morton index of a cell (edge at most 8).
 __device__ __forceinline__ int cell_morton(int x, int y, int z) {
     auto spread = [](int v) { return (v & 1) | ((v & 2) << 2) | ((v & 4) << 4); };
     return spread(x) | (spread(y) << 1) | (spread(z) << 2);
-}
-
-__device__ __forceinline__ void brick_cell(int m, int &x, int &y, int &z) {
-    x = (m & 1) | ((m >> 2) & 2) | ((m >> 4) & 4);
-    y = ((m >> 1) & 1) | ((m >> 3) & 2) | ((m >> 5) & 4);
-    z = ((m >> 2) & 1) | ((m >> 4) & 2) | ((m >> 6) & 4);
 }
 
 // Every third bit of a 32-bit Morton code.
@@ -801,7 +800,7 @@ __global__ void __launch_bounds__(kFoldWarps * 32, kFoldCtas) k_fold_bricks(Fold
                 uint32_t wv = m < E3 ? sm.w[m] : 0u;
                 if (!whole) {
                     int lx, ly, lz;
-                    brick_cell(m, lx, ly, lz);
+                    brick_cell((uint32_t)m, lx, ly, lz);
                     if (ox + lx >= end0 || oy + ly >= end1 || oz + lz >= end2 || oz + lz == drop_z) wv = 0;
                 }
                 const uint32_t bits = __ballot_sync(FULL, wv != 0);
@@ -810,7 +809,18 @@ __global__ void __launch_bounds__(kFoldWarps * 32, kFoldCtas) k_fold_bricks(Fold
                 n += (uint32_t)__popc(bits);
             }
             if (lane < 16) a.brick_bits[(uint64_t)j * 16 + lane] = mine;
-            if (lane == 0) a.brick_count[j] = n;
+            if (a.node_words) {
+                uint32_t mask, total;
+                brick8_node(lane < 16 ? mine : 0u, mask, total);
+                if (lane == 0) {
+                    const uint32_t at = a.node_by_key ? key : j;
+                    a.node_words[at] = total;
+                    a.node_mask[at] = (uint8_t)mask;
+                    if (a.n_voxels) atomicAdd(a.n_voxels, (unsigned long long)n);
+                }
+            } else if (lane == 0) {
+                a.brick_count[j] = n;
+            }
         } else {
             for (int i = lane; i < E3; i += 32) {
                 const int lx = i & (E - 1), ly = (i >> le) & (E - 1), lz = i >> (2 * le);
@@ -832,7 +842,7 @@ __global__ void __launch_bounds__(kFoldWarps * 32, kFoldCtas) k_fold_bricks(Fold
                     bool on = false;
                     if (m < E3) {
                         int lx, ly, lz;
-                        brick_cell(m, lx, ly, lz);
+                        brick_cell((uint32_t)m, lx, ly, lz);
                         on = (whole || (ox + lx < end0 && oy + ly < end1 && oz + lz < end2 && oz + lz != drop_z)) &&
                              sm.w[m] != 0;
                     }
@@ -1409,16 +1419,18 @@ int build_mesh_device(const svo_mesh *m, int side, int threads, uint64_t mem, cu
         // once, then the walk's voxels (VoxelOctree.cpp:66-103) from the slots
         const uint32_t E3 = 1u << (3 * g.log_e);
         const uint64_t cap = (uint64_t)nb * E3;
+        // 8^3 bricks go to the octree as they are, unless a cache block is no
+        // larger than a brick (budgets of a few KB)
+        const bool as_bricks = g.log_e == 3 && (lb > 3 || lb == D);
         Dev<uint32_t> slot, ccount, cbits, pay;
         Dev<uint64_t> coff, dN, sc64, keys;
+        Dev<uint8_t> nmask;
+        Dev<unsigned long long> n_vox;
+        const bool by_key = as_bricks && bricks_dense(D, 3);
+        const uint64_t nodes = by_key ? 1ull << (3 * (D - 3)) : (uint64_t)nb;
         SVO_ALLOC(slot, cap);
-        SVO_ALLOC(ccount, nb);
+        SVO_ALLOC(ccount, nodes);
         SVO_ALLOC(cbits, (uint64_t)nb * 16);
-        SVO_ALLOC(coff, nb);
-        SVO_ALLOC(dN, 1);
-        SVO_ALLOC(sc64, scan_scratch_elems(nb));
-        SVO_ALLOC(keys, cap);
-        SVO_ALLOC(pay, cap);
         FoldArgs fa = fold_args();
         fa.b_first = 0;
         fa.b_last = nb;
@@ -1426,9 +1438,30 @@ int build_mesh_device(const svo_mesh *m, int side, int threads, uint64_t mem, cu
         fa.slot = slot.p;
         fa.brick_count = ccount.p;
         fa.brick_bits = cbits.p;
+        if (as_bricks) {
+            SVO_ALLOC(nmask, nodes);
+            fa.node_words = ccount.p;
+            fa.node_mask = nmask.p;
+            fa.node_by_key = by_key ? 1 : 0;
+            if (by_key) SVO_CUDA_TRY(cudaMemsetAsync(ccount.p, 0, nodes * sizeof(uint32_t), st));
+            if (cap >= 0xFFFFFFFFull) {  // the voxels may exceed the build's limit
+                SVO_ALLOC(n_vox, 1);
+                SVO_CUDA_TRY(cudaMemsetAsync(n_vox.p, 0, sizeof(unsigned long long), st));
+                fa.n_voxels = n_vox.p;
+            }
+        }
         const unsigned grid = (unsigned)std::min<uint64_t>((nb + kFoldWarps - 1) / kFoldWarps, fold_grid);
         k_fold_bricks<true><<<grid, kFoldWarps * 32, 0, st>>>(fa);
         SVO_LAUNCH_OK("k_fold_bricks<direct>");
+        if (as_bricks) {
+            const MeshBricks mb{nb, bkey.p, ccount.p, nmask.p, cbits.p, slot.p, n_vox.p};
+            return build_from_bricks_device(mb, D, lb, lb < D ? bflag.p : nullptr, st, d_words, n_words);
+        }
+        SVO_ALLOC(coff, nb);
+        SVO_ALLOC(dN, 1);
+        SVO_ALLOC(sc64, scan_scratch_elems(nb));
+        SVO_ALLOC(keys, cap);
+        SVO_ALLOC(pay, cap);
         SVO_CUDA_TRY((exclusive_scan<uint32_t, uint64_t>(ccount.p, coff.p, nb, dN.p, sc64.p, st)));
         k_direct_emit<<<warp_grid, 256, 0, st>>>(nb, g.log_e, bkey.p, cbits.p, slot.p, coff.p, cap, keys.p, pay.p,
                                                 err.p);

@@ -1,0 +1,62 @@
+"""The builds through bricks (16^3 of a dense grid, 8^3 of a mesh fold): one
+brick as the root, ragged and misaligned grids, cache blocks of a brick's size,
+far pointers right above the bricks, and cubes whose brick codes are too many
+for the dense level arrays.  Words bit-exact to the oracle."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def budget(oracle, shape, edge):
+    """A budget whose cache blocks have this edge (None: one block)."""
+    mem = 3000
+    while edge is not None and oracle.cache_block(shape[2], shape[1], shape[0], mem) < edge:
+        mem += mem // 16
+    return 1 << 30 if edge is None else mem
+
+
+@pytest.mark.parametrize("shape,density,edge", [
+    ((16, 16, 16), 1.0, None),      # the brick is the root
+    ((16, 16, 16), 0.01, None),
+    ((15, 13, 16), 0.4, None),      # odd depth: the last slice is dropped
+    ((32, 32, 32), 0.0, None),
+    ((64, 64, 64), 1.0, None),      # every offset above a brick is far
+    ((17, 33, 65), 0.3, None),      # rows off the 16-byte boundary
+    ((50, 47, 100), 0.002, None),   # partial bricks in every direction
+    ((33, 40, 48), 0.1, 16),        # 16^3 cache blocks
+    ((65, 64, 40), 0.05, 32),       # 32^3 cache blocks
+    ((9, 20, 2100), 0.2, None),     # 4096^3 cube: compacted nodes
+    ((35, 36, 2052), 0.1, 64),      # the same with cache blocks
+    ((35, 36, 2052), 0.1, 128),
+])
+def test_dense_builds(svo, oracle, scenes, shape, density, edge):
+    mem = budget(oracle, shape, edge)
+    g = scenes.random_grid(shape, density, sum(shape))
+    if edge is not None:
+        # a cache block whose only voxels lie in the dropped slice
+        assert oracle.cache_block(shape[2], shape[1], shape[0], mem) == edge
+        z = (shape[0] - 1) // edge * edge
+        g[z:, :edge, :edge] = 0
+        g[shape[0] - 1, 3, 5] = 77
+    ow, oc = oracle.build_dense(g, mem)
+    tree = svo.VoxelOctree(svo.VoxelData(g, mem))
+    assert np.array_equal(tree.words(), ow)
+    assert np.array_equal(tree.center(), oc)
+
+
+@pytest.mark.parametrize("side,thin,threads,mem", [
+    (8, 1.0, 2, 1 << 30),         # one 8^3 brick
+    (60, 0.5, 5, 1 << 30),
+    (700, 0.03, 16, 1 << 30),     # 1024^3 cube, a needle
+    (1500, 0.015, 16, 1 << 30),   # 2048^3 cube: compacted nodes
+    (1500, 0.015, 4, 3 << 20),    # the same in small cache blocks
+])
+def test_mesh_builds(svo, oracle, scenes, side, thin, threads, mem):
+    pos, faces, col = scenes.displaced_icosphere(3, side)
+    pos = pos * np.array([1.0, thin, thin], np.float32)
+    col = col.astype(np.float32)
+    tree = svo.VoxelOctree(svo.VoxelData(svo.PlyLoader.from_arrays(pos, faces, colors=col), side, mem, threads))
+    ow, oc = oracle.build_mesh(pos, faces, side, threads, mem, colors=col)
+    assert np.array_equal(tree.words(), ow)
+    assert np.array_equal(tree.center(), oc)
