@@ -12,8 +12,8 @@
 // slowest ray of a fixed 32-ray batch.  Nothing waits on another warp or CTA.
 //
 // Optionally (plain-tile schedule) each warp keeps the first `cache_entries`
-// descriptor-table entries (the top levels: the table is stored breadth
-// first) of one octree in its own slice of shared memory, reloaded when the
+// descriptor-table entries (the top levels: the table starts with them,
+// breadth first) of one octree in its own slice of shared memory, reloaded when the
 // octree of the warp's next 32 slots changes; lanes tracing another octree
 // read the global table.  The cached entries are copies of the global ones,
 // so results do not depend on the cache.  The autotuner picks the depth.

@@ -2,18 +2,41 @@
 // the table traversal (ray_step_tab) walks instead of decoding relative and
 // far offsets with bounds checks at every PUSH.
 //
-// Breadth first from the root, one level at a time:
-//   1. k_table_nodes: per node of the level, table_node's checks
-//      (octree_table.cuh), its entry {descriptor, -, child block, stride} and
-//      its internal-child count;
+// The traversal needs a node's internal children at consecutive entries, in
+// block order, and nothing else of the order.  In the word array they are
+// consecutive descriptors already, so the table holds the top kTopLevels
+// levels breadth first (the batched kernels' shared-memory caches copy the
+// first entries) and every deeper node in word order:
+//   1. k_table_top: the top levels, one CTA;
+//   2. k_table_expand, a launch per level, no host round trip: every node of
+//      the level passes table_node's checks (octree_table.cuh), marks its
+//      internal children in a bitmap over the words and appends them to the
+//      node list, in any order;
+//   3. k_table_tiles, k_table_rank: the bitmap's prefix counts, which are the
+//      entries' positions;
+//   4. k_table_entries: one pass over the words writes every entry.
+// A node reached twice, one between a far block's slots, more nodes than the
+// list holds (a quarter of the words) or more than kWordOrderMost words leave
+// that to the breadth-first form below, which needs a scan and a host round
+// trip per level and keeps shared nodes apart:
+//   1. k_table_nodes: per node of the level, table_node's checks, its entry
+//      {descriptor, -, child block, stride} and its internal-child count;
 //   2. an exclusive scan of the counts gives each node's first child in the
 //      next level;
 //   3. k_table_children: the entry's first-child ordinal, and the next
 //      level's node words (block start + j * stride for its j-th internal
 //      child).
-// A failed check anywhere, a level past 22 or more entries than words (a
-// node reachable twice) leaves the handle without a table.  The table costs
-// 16 bytes per node, about 2 bytes per octree word on the benchmark scenes.
+// A failed check anywhere, a level past 22 or more entries than words leaves
+// the handle without a table.  The table costs 16 bytes per node, about 2
+// bytes per octree word on the benchmark scenes.
+//
+// Measured, first call to ready table, word order against breadth first: 130
+// and 325 us (10,000 words), 235 and 490 (1.8 M), 285 and 570 (14 M), 605 and
+// 815 (63 M), 910 and 980 (113 M), 3,300 and 2,350 (490 M: the list's scattered
+// marks and the pass over all words then cost more than the round trips).
+// Traces run at the same speed over either order (within 0.5% on nine
+// workloads).
+#include <algorithm>
 #include <memory>
 #include <vector>
 
@@ -51,6 +74,175 @@ __global__ void k_table_children(const uint32_t *__restrict__ n_int, const uint3
     entries[i] = e;
 }
 
+// ---- word order --------------------------------------------------------------------
+
+constexpr int kTopLevels = 4;        // breadth first: at most 1 + 8 + 64 + 512 nodes
+constexpr uint64_t kWordOrderMost = 1ull << 27;
+constexpr int kTopNodes = 585;
+constexpr int kTopThreads = 512;
+
+struct WordOrder {
+    const uint32_t *words;
+    uint32_t n_words;
+    uint32_t *list;   // the deeper nodes' words, level by level
+    uint32_t cap;
+    uint32_t *bits;   // one per word: the descriptor of a deeper node
+    uint32_t *rank;   // per 32 words: deeper nodes before them
+    uint32_t *tile;   // per kRankTile words of `bits`: their nodes
+    uint32_t *top;    // top nodes: word, first child's entry (last top level: none yet)
+    uint32_t *ctl;
+};
+// ctl: list entries, error flags, top nodes, top nodes above the last top
+// level, then per level the list's length after it and the CTAs done with it
+constexpr int kCtlTail = 0, kCtlErr = 1, kCtlTop = 2, kCtlInner = 3, kCtlEnd = 4,
+              kCtlDone = kCtlEnd + kTableMaxParentLevel + 4, kCtlWords = kCtlDone + kTableMaxParentLevel + 4;
+constexpr uint32_t kErrBad = 1, kErrFull = 2, kErrOrder = 4;
+constexpr int kRankItems = 8, kRankTile = kScanThreads * kRankItems;
+constexpr uint64_t kRankSelf = 1024;  // tiles up to which each sums those before it itself
+
+// Marks the k internal children of a child block in the bitmap.
+__device__ __forceinline__ void mark_children(const WordOrder &t, uint32_t cb, uint32_t stride, uint32_t k) {
+    const uint64_t m = (stride == 1 ? (1ull << k) - 1 : 0x5555ull & ((1ull << (2 * k)) - 1)) << (cb & 31);
+    atomicOr(t.bits + (cb >> 5), (uint32_t)m);
+    if (m >> 32) atomicOr(t.bits + (cb >> 5) + 1, (uint32_t)(m >> 32));
+}
+
+__device__ __forceinline__ uint32_t rank_of(const WordOrder &t, uint32_t w) {
+    return t.rank[w >> 5] + (uint32_t)__popc(t.bits[w >> 5] & ((1u << (w & 31)) - 1u));
+}
+
+__global__ void __launch_bounds__(kTopThreads) k_table_top(WordOrder t) {
+    __shared__ uint32_t node[kTopNodes], wsum[kTopThreads / 32];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    if (threadIdx.x == 0) node[0] = 0;
+    uint32_t begin = 0, end = 1;
+    for (int L = 0; L < kTopLevels; ++L) {
+        __syncthreads();
+        const bool live = begin + threadIdx.x < end;
+        const uint32_t me = live ? node[begin + threadIdx.x] : 0u;
+        uint32_t cb = 0, stride = 1, k = 0;
+        if (live && !table_node(t.words, t.n_words, me, L, cb, stride, k)) {
+            atomicOr(&t.ctl[kCtlErr], kErrBad);
+            k = 0;
+        }
+        const uint32_t incl = warp_incl_scan(k);
+        if (lane == 31) wsum[wid] = incl;
+        __syncthreads();
+        uint32_t off = incl - k, total = 0;
+        for (int w = 0; w < kTopThreads / 32; ++w) {
+            if (w < wid) off += wsum[w];
+            total += wsum[w];
+        }
+        const bool last = L == kTopLevels - 1;
+        if (live) {
+            t.top[2 * (begin + threadIdx.x)] = me;
+            t.top[2 * (begin + threadIdx.x) + 1] = end + off;
+            if (last && k) mark_children(t, cb, stride, k);
+            for (uint32_t j = 0; j < k; ++j) (last ? t.list : node + end)[off + j] = cb + j * stride;
+        }
+        if (last) {
+            if (threadIdx.x == 0) {
+                t.ctl[kCtlTop] = end;
+                t.ctl[kCtlInner] = begin;
+                t.ctl[kCtlTail] = total;
+                t.ctl[kCtlEnd + kTopLevels] = total;
+            }
+        } else {
+            begin = end;
+            end += total;
+        }
+    }
+}
+
+// Level L's nodes, list[length(L - 1) .. length(L)).  The last CTA to finish
+// notes the list's length for the next level; no CTA waits for another.
+__global__ void __launch_bounds__(256) k_table_expand(WordOrder t, int L) {
+    // after an error the list may hold places that were never written
+    if (t.ctl[kCtlErr]) return;
+    __shared__ uint32_t base;
+    const uint32_t begin = L > kTopLevels ? t.ctl[kCtlEnd + L - 1] : 0u, end = min(t.ctl[kCtlEnd + L], t.cap);
+    for (uint32_t i0 = begin + blockIdx.x * blockDim.x; i0 < end; i0 += gridDim.x * blockDim.x) {
+        const uint32_t i = i0 + threadIdx.x;
+        uint32_t cb = 0, stride = 1, k = 0, total;
+        if (i < end && !table_node(t.words, t.n_words, t.list[i], L, cb, stride, k)) {
+            atomicOr(&t.ctl[kCtlErr], kErrBad);
+            k = 0;
+        }
+        if (!__syncthreads_or((int)k)) continue;
+        const uint32_t off = block_excl_scan<uint32_t>(k, &total);
+        // one reservation per CTA: the list's length is one address
+        if (threadIdx.x == 0) base = atomicAdd(&t.ctl[kCtlTail], total);
+        __syncthreads();
+        const uint32_t at = base + off;
+        if (!k) continue;
+        if (at > t.cap || k > t.cap - at) {
+            atomicOr(&t.ctl[kCtlErr], kErrFull);
+            continue;
+        }
+        mark_children(t, cb, stride, k);
+        for (uint32_t j = 0; j < k; ++j) t.list[at + j] = cb + j * stride;
+    }
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0 && atomicAdd(&t.ctl[kCtlDone + L], 1u) == gridDim.x - 1)
+        t.ctl[kCtlEnd + L + 1] = atomicAdd(&t.ctl[kCtlTail], 0u);
+}
+
+__global__ void __launch_bounds__(kScanThreads) k_table_tiles(WordOrder t, uint64_t n) {
+    const uint64_t i0 = (uint64_t)blockIdx.x * kRankTile + (uint64_t)threadIdx.x * kRankItems;
+    uint32_t c = 0, total;
+    for (int k = 0; k < kRankItems; ++k)
+        if (i0 + k < n) c += (uint32_t)__popc(t.bits[i0 + k]);
+    block_excl_scan<uint32_t>(c, &total);
+    if (threadIdx.x == 0) t.tile[blockIdx.x] = total;
+}
+
+// first: the tiles' scan, or null: this tile adds up those before it, and the
+// last one leaves the total.
+__global__ void __launch_bounds__(kScanThreads) k_table_rank(WordOrder t, uint64_t n, const uint32_t *__restrict__ first,
+                                                             uint32_t *__restrict__ total_out) {
+    uint32_t before = 0, total;
+    if (first) {
+        before = first[blockIdx.x];
+    } else {
+        uint32_t c = 0;
+        for (uint32_t i = threadIdx.x; i < blockIdx.x; i += kScanThreads) c += t.tile[i];
+        block_excl_scan<uint32_t>(c, &before);
+    }
+    const uint64_t i0 = (uint64_t)blockIdx.x * kRankTile + (uint64_t)threadIdx.x * kRankItems;
+    uint32_t c = 0, own[kRankItems];
+    for (int k = 0; k < kRankItems; ++k) {
+        own[k] = i0 + k < n ? (uint32_t)__popc(t.bits[i0 + k]) : 0u;
+        c += own[k];
+    }
+    uint32_t at = before + block_excl_scan<uint32_t>(c, &total);
+    for (int k = 0; k < kRankItems; ++k) {
+        if (i0 + k < n) t.rank[i0 + k] = at;
+        at += own[k];
+    }
+    if (!first && blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) *total_out = before + total;
+}
+
+__global__ void __launch_bounds__(256) k_table_entries(WordOrder t, uint4 *__restrict__ tab) {
+    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t n_top = t.ctl[kCtlTop];
+    if (i < n_top) {  // table_node has passed for every node here
+        uint32_t cb, stride, k, first = t.top[2 * i + 1];
+        table_node(t.words, t.n_words, t.top[2 * i], 0, cb, stride, k);
+        if (i >= t.ctl[kCtlInner]) first = k ? n_top + rank_of(t, cb) : 0u;
+        tab[i] = make_uint4(t.words[t.top[2 * i]], first, cb, 0u);
+    }
+    if (i >= t.n_words || !((t.bits[i >> 5] >> (i & 31)) & 1u)) return;
+    uint32_t cb, stride, k;
+    table_node(t.words, t.n_words, (uint32_t)i, 0, cb, stride, k);
+    // a far block's children are consecutive entries only if the far words
+    // between them are no descriptors
+    if (k && stride == 2)
+        for (uint32_t f = cb + 1; f < cb + 2 * k - 1; f += 2)
+            if ((t.bits[f >> 5] >> (f & 31)) & 1u) atomicOr(&t.ctl[kCtlErr], kErrOrder);
+    tab[n_top + rank_of(t, (uint32_t)i)] = make_uint4(t.words[i], k ? n_top + rank_of(t, cb) : 0u, cb, 0u);
+}
+
 struct Scratch {
     void *p = nullptr;
     cudaStream_t st = nullptr;
@@ -68,6 +260,78 @@ struct Scratch {
 
 inline unsigned grid_for(uint64_t n) { return (unsigned)((n + 255) / 256); }
 
+// The table in word order; *tab stays null when it cannot be had this way.
+int build_word_order(const uint32_t *d_words, uint64_t n_words, cudaStream_t st, uint4 **tab, uint64_t *n_tab) {
+    *tab = nullptr;
+    // a node list as long as the words where that is little memory, else a
+    // quarter of them (about an eighth are nodes on the benchmark scenes)
+    constexpr uint64_t kWholeList = 1ull << 24;
+    const uint64_t nb = (n_words + 31) / 32, tiles = (nb + kRankTile - 1) / kRankTile;
+    const uint64_t cap = std::max<uint64_t>(n_words <= kWholeList ? n_words : n_words / 4, 8 * kTopNodes);
+    const bool self = tiles <= kRankSelf;
+    auto round4 = [](uint64_t n) { return (n + 3) & ~uint64_t(3); };
+    // one block: zeroed ctl and bits (with one more word, for a mark that
+    // reaches past the last), then the rest
+    const uint64_t o_bits = round4(kCtlWords), o_rank = o_bits + round4(nb + 1), o_tile = o_rank + round4(nb),
+                   o_first = o_tile + round4(tiles), o_scan = o_first + (self ? 0 : round4(tiles)),
+                   o_top = o_scan + round4(scan_scratch_elems(tiles)), o_list = o_top + round4(2 * kTopNodes);
+    Scratch mem;
+    SVO_CUDA_TRY(mem.alloc((size_t)(o_list + cap) * sizeof(uint32_t), st));
+    uint32_t *const m = (uint32_t *)mem.p;
+    WordOrder t;
+    t.words = d_words;
+    t.n_words = (uint32_t)n_words;
+    t.ctl = m;
+    t.bits = m + o_bits;
+    t.rank = m + o_rank;
+    t.tile = m + o_tile;
+    t.top = m + o_top;
+    t.list = m + o_list;
+    t.cap = (uint32_t)cap;
+    uint32_t *const first = self ? nullptr : m + o_first;
+    SVO_CUDA_TRY(cudaMemsetAsync(m, 0, (size_t)o_rank * sizeof(uint32_t), st));
+    k_table_top<<<1, kTopThreads, 0, st>>>(t);
+    SVO_CUDA_TRY(cudaGetLastError());
+    // twelve levels (a 4096^3 cube's) before the host looks, and if they end
+    // there the ranks are there too
+    uint32_t h[kCtlWords];
+    uint32_t n = 0;
+    for (int L = kTopLevels;;) {
+        const int to = std::min(L == kTopLevels ? 12 : L + 6, kTableMaxParentLevel + 2);
+        for (; L < to; ++L) {
+            const uint64_t most = L < 8 ? std::min<uint64_t>(cap, 1ull << (3 * L)) : cap;
+            k_table_expand<<<(unsigned)std::min<uint64_t>((most + 255) / 256, 152 * 8), 256, 0, st>>>(t, L);
+            SVO_CUDA_TRY(cudaGetLastError());
+        }
+        k_table_tiles<<<(unsigned)tiles, kScanThreads, 0, st>>>(t, nb);
+        SVO_CUDA_TRY(cudaGetLastError());
+        if (!self)
+            SVO_CUDA_TRY((exclusive_scan<uint32_t, uint32_t>(t.tile, first, tiles, t.ctl + kCtlWords - 1, m + o_scan, st)));
+        k_table_rank<<<(unsigned)tiles, kScanThreads, 0, st>>>(t, nb, first, t.ctl + kCtlWords - 1);
+        SVO_CUDA_TRY(cudaGetLastError());
+        SVO_CUDA_TRY(cudaMemcpyAsync(h, t.ctl, sizeof(h), cudaMemcpyDeviceToHost, st));
+        SVO_CUDA_TRY(cudaStreamSynchronize(st));
+        if (h[kCtlErr]) return SVO_OK;
+        if (h[kCtlEnd + L] == h[kCtlEnd + L - 1]) break;  // the last level expanded added nothing
+        if (L >= kTableMaxParentLevel + 2) return SVO_OK;
+    }
+    if (h[kCtlWords - 1] != h[kCtlTail]) return SVO_OK;  // a node reached twice
+    n = h[kCtlTop] + h[kCtlTail];
+    uint4 *e = nullptr;
+    SVO_CUDA_TRY(cudaMalloc((void **)&e, (size_t)n * sizeof(uint4)));
+    k_table_entries<<<grid_for(std::max<uint64_t>(n_words, kTopNodes)), 256, 0, st>>>(t, e);
+    cudaError_t er = cudaGetLastError();
+    if (er == cudaSuccess) er = cudaMemcpyAsync(h, t.ctl, sizeof(h), cudaMemcpyDeviceToHost, st);
+    if (er == cudaSuccess) er = cudaStreamSynchronize(st);
+    if (er != cudaSuccess || h[kCtlErr]) {
+        cudaFree(e);
+        return er != cudaSuccess ? cuda_fail(er, "descriptor table") : SVO_OK;
+    }
+    *tab = e;
+    *n_tab = n;
+    return SVO_OK;
+}
+
 // Builds the table on `st` and waits for it.  Returns SVO_OK with *tab set
 // (cudaMalloc'd, n_tab entries) or with *tab = nullptr when the octree does
 // not qualify; an error code only for CUDA failures.
@@ -76,6 +340,10 @@ int build_table(const uint32_t *d_words, uint64_t n_words, cudaStream_t st, uint
     *n_tab = 0;
     if (n_words == 0 || n_words > kMaxNarrowWords) return SVO_OK;
     const uint32_t W = (uint32_t)n_words;
+    if (n_words <= kWordOrderMost) {
+        const int rc = build_word_order(d_words, n_words, st, tab, n_tab);
+        if (rc != SVO_OK || *tab) return rc;
+    }
     std::unique_ptr<Scratch[]> lv_entries(new Scratch[kTableMaxParentLevel + 2]);
     std::vector<uint32_t> lv_n;
     Scratch err, cur, total;

@@ -1,11 +1,11 @@
 // octree_table.cuh — the per-node check behind the descriptor table that the
 // table traversal (ray_step_tab in svo_device.cuh) walks.
 //
-// The table is built breadth first from the root (octree_table.cu): level 0
-// is the root, the internal children of the level-L nodes, in node order and
-// within a node in block order, are level L+1, and entry k holds
+// Entry 0 is the root, the internal children of a node have consecutive
+// entries in block order, and entry k holds
 //   {descriptor word, ordinal of its first internal child, word index of its
 //    child block, 0}.
+// The top levels come first, breadth first; octree_table.cu says what follows.
 // A table is built only when every node reachable from the root passes
 // table_node; otherwise the octree keeps the checked traversal, which ends a
 // ray at the first out-of-range index with kFault exactly where it did.

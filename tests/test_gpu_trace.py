@@ -366,3 +366,49 @@ def test_table_refused_for_corrupt_trees(cuda, svo):
         tree = svo.VoxelOctree.from_words(np.array(words, np.uint32), (0.5, 0.5, 0.5))
         assert tree.table_size() == 0
         tree.close()
+
+
+def _chain(depth):
+    """One child per level, always octant 0: `depth` internal nodes, a
+    bottom node and its voxel."""
+    w = [(1 << 18) | (0x80 << 8) | 0x80] * depth + [(1 << 18) | (0x80 << 8), 12345]
+    return np.array(w, np.uint32)
+
+
+def _shared_subtree(words):
+    """A root whose octants 0 and 1 are the same subtree: two internal
+    children need two slots, so a second-level node per octant points to one
+    child block."""
+    n = words.size
+    root = (1 << 18) | (0xC0 << 8) | 0xC0  # slots: octant 1, octant 0
+    a = (2 << 18) | (0x80 << 8) | 0x80
+    b = (1 << 18) | (0x80 << 8) | 0x80
+    return np.concatenate([np.array([root, a, b], np.uint32), words]), n
+
+
+@pytest.mark.parametrize("kind", ["chain_6", "chain_13", "chain_21", "shared", "far"])
+def test_table_orders(cuda, svo, oracle, scenes, kind):
+    """Trees the table build treats differently: deeper than the levels it
+    expands before the host looks, a subtree reached twice (breadth-first form,
+    both occurrences kept) and children with far words between them."""
+    center = np.full(3, 0.5, np.float32)
+    rays = scenes.random_rays(20_000, 23)
+    if kind.startswith("chain"):
+        words = _chain(int(kind[6:]))
+        nodes = words.size - 1
+        # towards the corner that octant 0 nests into
+        rays = np.concatenate([rays, rays])
+        rays[20_000:, 3:] = np.float32(1.0) - rays[20_000:, :3] + np.float32(1e-7)
+        rays[20_000:, 3:] /= np.linalg.norm(rays[20_000:, 3:], axis=1, keepdims=True)
+    elif kind == "shared":
+        sub, _ = oracle.build_dense(scenes.random_grid((16, 16, 16), 0.3, 5))
+        words, _ = _shared_subtree(sub)
+        t = svo.VoxelOctree.from_words(sub, center)
+        nodes = 3 + 2 * t.table_size()
+    else:
+        words, center = oracle.build_dense(scenes.random_grid((64, 64, 64), 0.9, 9))
+        nodes = None
+    tree = svo.VoxelOctree.from_words(words, center)
+    assert tree.table_size() == (nodes if nodes is not None else tree.validate()[0])
+    ref = oracle.raymarch(words, rays, threads=4)
+    _assert_same(_device_trace(cuda, svo, tree, rays), ref)
