@@ -80,8 +80,9 @@ void svo_free(void *p);
 int svo_octree_from_words(const uint32_t *words, uint64_t n_words, const float center[3], svo_octree **out);
 
 /* The builds keep their freed scratch memory in a per-device pool of the
- * library for the next build; this returns that memory to the driver (after
- * a device synchronisation). */
+ * library for the next build, and destroyed octrees up to 1 GiB of theirs in
+ * another; this returns that memory to the driver (after a device
+ * synchronisation). */
 int svo_trim_memory(void);
 
 /* Frees the handle and its device memory. */

@@ -1625,7 +1625,7 @@ int build_levels(std::vector<LevelArrays> &lv, int base, const uint64_t *leaf_ke
     const uint64_t W = 1 + S_root;
 
     uint32_t *words = nullptr;
-    SVO_CUDA_TRY(cudaMallocAsync((void **)&words, (size_t)W * sizeof(uint32_t), st));
+    SVO_CUDA_TRY(alloc_words(&words, W, st));
     auto place = [&]() -> int {
         DevBuf<uint32_t> err;
         SVO_TRY_ALLOC(err.alloc(1, arena));
@@ -1653,7 +1653,7 @@ int build_levels(std::vector<LevelArrays> &lv, int base, const uint64_t *leaf_ke
     };
     rc = place();
     if (rc) {
-        cudaFree(words);
+        cudaFreeAsync(words, st);
         return rc;
     }
     *d_words_out = words;
@@ -1775,7 +1775,7 @@ static int build_pyramid(int base, int D, const uint32_t *words_of, const uint8_
     if (voxels >= 0xFFFFFFFFull) return set_error(SVO_ERR_LIMIT, "%llu occupied voxels exceed 2^32-1", voxels);
     const uint64_t W = 1 + S_root;
     uint32_t *words = nullptr;
-    SVO_CUDA_TRY(cudaMallocAsync((void **)&words, (size_t)W * sizeof(uint32_t), st));
+    SVO_CUDA_TRY(alloc_words(&words, W, st));
     auto place = [&]() -> int {
         int c = D;
         while (c > base && (1ull << (3 * (D - c + 1))) <= kTopPlaced) --c;
@@ -1798,7 +1798,7 @@ static int build_pyramid(int base, int D, const uint32_t *words_of, const uint8_
     };
     const int rc = place();
     if (rc) {
-        cudaFree(words);
+        cudaFreeAsync(words, st);
         return rc;
     }
     *d_words_out = words;

@@ -1,4 +1,4 @@
-// mem_pool.cpp — the library's stream-ordered scratch pool.
+// mem_pool.cpp — the library's stream-ordered memory pools.
 //
 // Builds allocate and free their working arrays on the build's stream.  The
 // device's default pool hands freed memory back to the driver at every
@@ -6,6 +6,13 @@
 // MB for a 1024^3 mesh build).  The library therefore keeps one pool per
 // device whose release threshold is unbounded: freed scratch stays mapped
 // for the next build until svo_trim_memory() returns it.
+//
+// Octrees themselves (words and descriptor tables) live in a second pool that
+// keeps at most kHandleKeep of freed memory mapped, so that a program that
+// replaces an octree every frame does not map and unmap it each time: a
+// rebuilt 200x131x177 volume spent 130 us freeing the octree before it and 100
+// allocating its own, of 385.  A pool holding more than that in live octrees
+// returns whatever is freed at the next synchronisation, as before.
 #include <mutex>
 
 #include "svo_internal.h"
@@ -14,17 +21,20 @@ namespace svo {
 
 namespace {
 constexpr int kMaxDevices = 64;
+constexpr uint64_t kHandleKeep = 1ull << 30;
+enum Pool { kScratch, kHandles, kPools };
 std::mutex g_pool_mtx;
-cudaMemPool_t g_pools[kMaxDevices] = {};
-}  // namespace
+cudaMemPool_t g_pools[kMaxDevices][kPools] = {};
+cudaStream_t g_streams[kMaxDevices] = {};
 
-cudaError_t pool_for_current_device(cudaMemPool_t *out) {
+cudaError_t pool_for_current_device(Pool which, cudaMemPool_t *out) {
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     if (dev < 0 || dev >= kMaxDevices) return cudaErrorInvalidDevice;
     std::lock_guard<std::mutex> lk(g_pool_mtx);
-    if (!g_pools[dev]) {
+    cudaMemPool_t &slot = g_pools[dev][which];
+    if (!slot) {
         cudaMemPoolProps props = {};
         props.allocType = cudaMemAllocationTypePinned;
         props.location.type = cudaMemLocationTypeDevice;
@@ -32,23 +42,59 @@ cudaError_t pool_for_current_device(cudaMemPool_t *out) {
         cudaMemPool_t pool;
         e = cudaMemPoolCreate(&pool, &props);
         if (e != cudaSuccess) return e;
-        uint64_t keep = ~0ull;
+        uint64_t keep = which == kScratch ? ~0ull : kHandleKeep;
         e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
         if (e != cudaSuccess) {
             cudaMemPoolDestroy(pool);
             return e;
         }
-        g_pools[dev] = pool;
+        slot = pool;
     }
-    *out = g_pools[dev];
+    *out = slot;
     return cudaSuccess;
 }
 
-cudaError_t scratch_alloc(void **p, size_t bytes, cudaStream_t st) {
+cudaError_t pool_alloc(Pool which, void **p, size_t bytes, cudaStream_t st) {
     cudaMemPool_t pool;
-    cudaError_t e = pool_for_current_device(&pool);
+    cudaError_t e = pool_for_current_device(which, &pool);
     if (e != cudaSuccess) return e;
     return cudaMallocFromPoolAsync(p, bytes, pool, st);
+}
+}  // namespace
+
+cudaError_t scratch_alloc(void **p, size_t bytes, cudaStream_t st) { return pool_alloc(kScratch, p, bytes, st); }
+
+cudaError_t handle_alloc(void **p, size_t bytes, cudaStream_t st) { return pool_alloc(kHandles, p, bytes, st); }
+
+cudaError_t alloc_words(uint32_t **words, uint64_t n, cudaStream_t st) {
+    void *p = nullptr;
+    const uint64_t at = status_offset(n);
+    cudaError_t e = handle_alloc(&p, (size_t)(at + kStatusWords) * sizeof(uint32_t), st);
+    if (e != cudaSuccess) return e;
+    e = cudaMemsetAsync((uint32_t *)p + at, 0, kStatusWords * sizeof(uint32_t), st);
+    if (e != cudaSuccess) {
+        cudaFreeAsync(p, st);
+        return e;
+    }
+    *words = (uint32_t *)p;
+    return cudaSuccess;
+}
+
+cudaError_t library_stream(cudaStream_t *out) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev < 0 || dev >= kMaxDevices) return cudaErrorInvalidDevice;
+    std::lock_guard<std::mutex> lk(g_pool_mtx);
+    if (!g_streams[dev]) {
+        e = cudaStreamCreateWithFlags(&g_streams[dev], cudaStreamNonBlocking);
+        if (e != cudaSuccess) {
+            g_streams[dev] = nullptr;
+            return e;
+        }
+    }
+    *out = g_streams[dev];
+    return cudaSuccess;
 }
 
 }  // namespace svo
@@ -58,14 +104,18 @@ extern "C" int svo_trim_memory(void) {
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return svo::cuda_fail(e, "cudaGetDevice");
-    cudaMemPool_t pool = nullptr;
+    cudaMemPool_t pools[svo::kPools] = {};
     {
         std::lock_guard<std::mutex> lk(svo::g_pool_mtx);
-        if (dev >= 0 && dev < svo::kMaxDevices) pool = svo::g_pools[dev];
+        for (int k = 0; k < svo::kPools; ++k)
+            if (dev >= 0 && dev < svo::kMaxDevices) pools[k] = svo::g_pools[dev][k];
     }
-    if (!pool) return SVO_OK;
+    bool any = false;
+    for (cudaMemPool_t p : pools) any = any || p;
+    if (!any) return SVO_OK;
     e = cudaDeviceSynchronize();
-    if (e == cudaSuccess) e = cudaMemPoolTrimTo(pool, 0);
-    if (e != cudaSuccess) return svo::cuda_fail(e, "trimming the scratch pool");
+    for (cudaMemPool_t p : pools)
+        if (p && e == cudaSuccess) e = cudaMemPoolTrimTo(p, 0);
+    if (e != cudaSuccess) return svo::cuda_fail(e, "trimming the memory pools");
     return SVO_OK;
 }

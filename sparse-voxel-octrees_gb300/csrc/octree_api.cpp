@@ -76,7 +76,6 @@ int cache_block_log2(int w, int h, int d, uint64_t mem, uint64_t cell_cost) {
 }
 
 }  // namespace svo
-extern "C" int svo_octree_destroy(svo_octree *oct);
 namespace svo {
 
 int make_handle(uint32_t *d_words, uint64_t n_words, const float center[3], svo_octree **out) {
@@ -85,17 +84,7 @@ int make_handle(uint32_t *d_words, uint64_t n_words, const float center[3], svo_
     h->n_words = n_words;
     std::memcpy(h->center, center, sizeof(h->center));
     cudaGetDevice(&h->device);
-    cudaError_t e = cudaMalloc((void **)&h->d_status, sizeof(uint32_t));
-    if (e != cudaSuccess) {
-        cudaFree(d_words);
-        h->d_words = nullptr;
-        return cuda_fail(e, "cudaMalloc(error word)");
-    }
-    e = cudaMemset(h->d_status, 0, sizeof(uint32_t));
-    if (e != cudaSuccess) {
-        svo_octree_destroy(h.release());
-        return cuda_fail(e, "cudaMemset(error word)");
-    }
+    h->d_status = d_words + status_offset(n_words);
     *out = h.release();
     return SVO_OK;
 }
@@ -103,10 +92,13 @@ int make_handle(uint32_t *d_words, uint64_t n_words, const float center[3], svo_
 static int upload_words(const uint32_t *words, uint64_t n, const float center[3], svo_octree **out) {
     if (n == 0) return set_error(SVO_ERR_FORMAT, "octree has no words");
     uint32_t *d = nullptr;
-    SVO_CUDA_TRY(cudaMalloc((void **)&d, n * sizeof(uint32_t)));
-    cudaError_t e = cudaMemcpy(d, words, n * sizeof(uint32_t), cudaMemcpyHostToDevice);
+    cudaStream_t st = nullptr;
+    SVO_CUDA_TRY(library_stream(&st));
+    SVO_CUDA_TRY(alloc_words(&d, n, st));
+    cudaError_t e = cudaMemcpyAsync(d, words, n * sizeof(uint32_t), cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) {
-        cudaFree(d);
+        cudaFreeAsync(d, st);
         return cuda_fail(e, "upload octree words");
     }
     return make_handle(d, n, center, out);
@@ -421,9 +413,17 @@ int svo_octree_destroy(svo_octree *oct) {
         std::lock_guard<std::mutex> lock(oct->staging_mtx);
         host_drain(oct);
     }
-    if (oct->d_words) cudaFree(oct->d_words);
-    if (oct->d_tab) cudaFree(oct->d_tab);
-    if (oct->d_status) cudaFree(oct->d_status);
+    // what the octree's own device still runs may use its memory: wait for
+    // it, after which the pool may hand the memory out again
+    int dev = oct->device;
+    cudaGetDevice(&dev);
+    if (dev != oct->device) cudaSetDevice(oct->device);
+    cudaStream_t st = nullptr;
+    cudaDeviceSynchronize();
+    library_stream(&st);
+    if (oct->d_words) cudaFreeAsync(oct->d_words, st);
+    if (oct->d_tab) cudaFreeAsync(oct->d_tab, st);
+    if (dev != oct->device) cudaSetDevice(dev);
     if (oct->stage_dev) cudaFree(oct->stage_dev);
     if (oct->copy_in) cudaStreamDestroy(oct->copy_in);
     if (oct->copy_out) cudaStreamDestroy(oct->copy_out);

@@ -318,13 +318,13 @@ int build_word_order(const uint32_t *d_words, uint64_t n_words, cudaStream_t st,
     if (h[kCtlWords - 1] != h[kCtlTail]) return SVO_OK;  // a node reached twice
     n = h[kCtlTop] + h[kCtlTail];
     uint4 *e = nullptr;
-    SVO_CUDA_TRY(cudaMalloc((void **)&e, (size_t)n * sizeof(uint4)));
+    SVO_CUDA_TRY(handle_alloc((void **)&e, (size_t)n * sizeof(uint4), st));
     k_table_entries<<<grid_for(std::max<uint64_t>(n_words, kTopNodes)), 256, 0, st>>>(t, e);
     cudaError_t er = cudaGetLastError();
     if (er == cudaSuccess) er = cudaMemcpyAsync(h, t.ctl, sizeof(h), cudaMemcpyDeviceToHost, st);
     if (er == cudaSuccess) er = cudaStreamSynchronize(st);
     if (er != cudaSuccess || h[kCtlErr]) {
-        cudaFree(e);
+        cudaFreeAsync(e, st);
         return er != cudaSuccess ? cuda_fail(er, "descriptor table") : SVO_OK;
     }
     *tab = e;
@@ -333,7 +333,7 @@ int build_word_order(const uint32_t *d_words, uint64_t n_words, cudaStream_t st,
 }
 
 // Builds the table on `st` and waits for it.  Returns SVO_OK with *tab set
-// (cudaMalloc'd, n_tab entries) or with *tab = nullptr when the octree does
+// (handle_alloc'd, n_tab entries) or with *tab = nullptr when the octree does
 // not qualify; an error code only for CUDA failures.
 int build_table(const uint32_t *d_words, uint64_t n_words, cudaStream_t st, uint4 **tab, uint64_t *n_tab) {
     *tab = nullptr;
@@ -395,20 +395,20 @@ int build_table(const uint32_t *d_words, uint64_t n_words, cudaStream_t st, uint
     SVO_CUDA_TRY(cudaStreamSynchronize(st));
     if (!ok || err_h) return SVO_OK;
     uint4 *t = nullptr;
-    SVO_CUDA_TRY(cudaMalloc((void **)&t, (size_t)base * sizeof(uint4)));
+    SVO_CUDA_TRY(handle_alloc((void **)&t, (size_t)base * sizeof(uint4), st));
     uint64_t at = 0;
     for (size_t L = 0; L < lv_n.size(); ++L) {
         cudaError_t e = cudaMemcpyAsync(t + at, lv_entries[L].p, (size_t)lv_n[L] * sizeof(uint4),
                                         cudaMemcpyDeviceToDevice, st);
         if (e != cudaSuccess) {
-            cudaFree(t);
+            cudaFreeAsync(t, st);
             return cuda_fail(e, "descriptor table copy");
         }
         at += lv_n[L];
     }
     cudaError_t e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) {
-        cudaFree(t);
+        cudaFreeAsync(t, st);
         return cuda_fail(e, "descriptor table");
     }
     *tab = t;
@@ -429,11 +429,10 @@ const uint4 *octree_table(const svo_octree *oct, cudaStream_t caller) {
     std::lock_guard<std::mutex> lock(oct->tab_mtx);
     if (oct->tab_state == 0) {
         cudaStream_t st = nullptr;
-        if (cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess) return nullptr;
+        if (library_stream(&st) != cudaSuccess) return nullptr;
         uint4 *t = nullptr;
         uint64_t nt = 0;
         int rc = build_table(oct->d_words, oct->n_words, st, &t, &nt);
-        cudaStreamDestroy(st);
         if (rc != SVO_OK) {
             // A CUDA failure (device memory, most likely): keep the word
             // traversal for this handle rather than retry on every call.

@@ -21,7 +21,7 @@ struct svo_octree {
     uint64_t n_words = 0;
     float center[3] = {0.0f, 0.0f, 0.0f};
     int device = 0;
-    uint32_t *d_status = nullptr;  // device error word: bit 0 = a ray ended with kFault
+    uint32_t *d_status = nullptr;  // device error word, behind the words: bit 0 = a ray ended with kFault
     int index_bits = 32;  // 64: svo_trace uses 64-bit word indices even when n_words fits 32 bits
 
     // Descriptor table of the table traversal (octree_table.cu), built by the
@@ -76,6 +76,19 @@ int lz4_decompress_block(const uint8_t *src, size_t src_len, uint8_t *out, size_
 // release with cudaFreeAsync.
 cudaError_t scratch_alloc(void **p, size_t bytes, cudaStream_t st);
 
+// Memory that a handle keeps, from a pool of its own; release with
+// cudaFreeAsync once nothing on the device uses it any more.
+cudaError_t handle_alloc(void **p, size_t bytes, cudaStream_t st);
+
+// An octree's words from that pool, with the handle's zeroed error word behind
+// them, at status_offset(n) words.
+constexpr uint64_t kStatusWords = 32;
+inline uint64_t status_offset(uint64_t n_words) { return (n_words + 31) / 32 * 32; }
+cudaError_t alloc_words(uint32_t **words, uint64_t n, cudaStream_t st);
+
+// A non-blocking stream per device, shared by the library's own work.
+cudaError_t library_stream(cudaStream_t *out);
+
 // VoxelData::init cache-block search (VoxelData.cpp:211-244): log2 of the
 // cache-block edge, or -1 when no partition fits `mem`.
 int cache_block_log2(int w, int h, int d, uint64_t mem, uint64_t cell_cost);
@@ -124,7 +137,8 @@ int launch_trace_image(const svo_octree *oct, const float *d_rays, uint32_t widt
 int launch_count_loads(const svo_octree *oct, const float *d_rays, uint64_t n, float ray_scale, uint32_t *loads,
                        cudaStream_t st);
 
-// Creates a handle around device words (takes ownership).
+// Creates a handle around device words from alloc_words, complete on the
+// device (takes ownership).
 int make_handle(uint32_t *d_words, uint64_t n_words, const float center[3], svo_octree **out);
 
 // The handle's descriptor table (octree_table.cu), built on first use; null
