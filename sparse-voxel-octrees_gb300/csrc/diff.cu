@@ -293,39 +293,56 @@ __device__ __forceinline__ float adjoint_tile(const DiffArgs &a, uint64_t slot, 
     return sq;
 }
 
-// Adds a warp's squared errors to the loss, one atomic per warp.
-__device__ __forceinline__ void add_loss(const DiffArgs &a, double loss) {
-    for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
-    if ((threadIdx.x & 31) == 0) atomicAdd(a.loss_sum, loss);
+// The loss is summed in groups of four tiles: a lane adds its four squared
+// errors and the lanes are added by halves, in float, and the groups' sums are
+// added in double.  Both adjoint kernels group alike.
+constexpr int kLossTiles = 4;
+
+__device__ __forceinline__ float lanes_sum(float v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
 }
 
-// The adjoint over recorded hit leaves: short per tile and even, so the tiles
-// are dealt out by a fixed stride over a resident grid.  A lane's squared
-// errors are summed with the running compensation of Kahan ("Further remarks
-// on reducing truncation errors", 1965), so the loss does not depend on how
-// many tiles a lane takes.
+// The adjoint over recorded hit leaves: short per tile and even, so the groups
+// of tiles are dealt out by a fixed stride over a resident grid, with one
+// atomic on the loss per warp.
 template <bool kFused, bool kRec>
 __global__ void __launch_bounds__(256) k_diff_backward(DiffArgs a) {
     RayStackFor<false> stk;  // unused: nothing is traced
-    float loss = 0.0f, comp = 0.0f;
-    const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
-    const uint64_t warp0 = (uint64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u);
-    for (uint64_t s0 = warp0; s0 < a.total; s0 += step) {  // uniform per warp
-        const float sq = adjoint_tile<false, false, kFused, kRec>(a, s0 + (threadIdx.x & 31), stk);
-        const float y = sq - comp, t = loss + y;
-        comp = (t - loss) - y;
-        loss = t;
+    double loss = 0.0;
+    const uint64_t step = (uint64_t)gridDim.x * blockDim.x * kLossTiles;
+    const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    for (uint64_t s0 = warp * (32 * kLossTiles); s0 < a.total; s0 += step) {  // uniform per warp
+        float group = 0.0f;
+#pragma unroll 1
+        for (int t = 0; t < kLossTiles; ++t)
+            group += adjoint_tile<false, false, kFused, kRec>(a, s0 + (uint64_t)(32 * t) + (threadIdx.x & 31), stk);
+        if (kFused && a.loss_sum) loss += (double)lanes_sum(group);
     }
-    if (kFused && a.loss_sum) add_loss(a, (double)loss - (double)comp);
+    if (kFused && a.loss_sum && (threadIdx.x & 31) == 0 && loss != 0.0) atomicAdd(a.loss_sum, loss);
 }
 
-// The adjoint that traces again: a tile per warp, as the forward pass.
+// The adjoint that traces again: a tile per warp, as the forward pass, and a
+// group of tiles per CTA.
 template <bool kTab, bool kFused, bool kRec>
 __global__ void __launch_bounds__(kTraceThreads) k_diff_retrace(DiffArgs a) {
+    static_assert(kTraceThreads == 32 * kLossTiles, "a CTA's tiles are a group");
     RayStackFor<kTab> stk;
     const uint64_t slot = (uint64_t)blockIdx.x * kTraceThreads + threadIdx.x;
     const float sq = adjoint_tile<kTab, true, kFused, kRec>(a, slot, stk);
-    if (kFused && a.loss_sum) add_loss(a, (double)sq);
+    if (kFused && a.loss_sum) {
+        __shared__ float tile_sq[kTraceThreads];
+        tile_sq[threadIdx.x] = sq;
+        __syncthreads();
+        if (threadIdx.x < 32) {
+            float group = 0.0f;
+#pragma unroll
+            for (int t = 0; t < kLossTiles; ++t) group += tile_sq[32 * t + threadIdx.x];
+            group = lanes_sum(group);
+            if (threadIdx.x == 0) atomicAdd(a.loss_sum, (double)group);
+        }
+    }
 }
 
 int prepare(const svo_octree *oct, const float *rays, uint32_t width, uint32_t height, uint32_t n_views,
