@@ -336,8 +336,9 @@ constexpr int kImageThreads = 128;
 constexpr int kImageTileW = 8, kImageTileH = 4;
 
 template <bool kTab, bool kLod>
-__global__ void __launch_bounds__(kImageThreads) k_trace_single(JobDev J, uint32_t *status) {
+__global__ void __launch_bounds__(kImageThreads) k_trace_single(JobDev J, uint32_t *status, uint32_t *carry) {
     const uint64_t slot = (uint64_t)blockIdx.x * kImageThreads + threadIdx.x;
+    if (slot == 0) carry_status(carry, status);
     const uint32_t tile = (uint32_t)(slot >> 5), r = (uint32_t)(slot & 31);  // tile < 2^30
     const uint32_t ty = tile / J.tiles_x, tx = tile - ty * J.tiles_x;
     const uint32_t px = tx * kImageTileW + (r & 7u), py = ty * kImageTileH + (r >> 3);
@@ -378,7 +379,7 @@ bool config_ok(const svo_trace_config &c) {
 // svo_trace_image: rays in row-major image order, traced in 8x4-pixel tiles
 // by one launch.
 int launch_trace_image(const svo_octree *oct, const float *d_rays, uint32_t width, uint32_t height, float ray_scale,
-                       const float light[3], const svo_trace_out &out, cudaStream_t st) {
+                       const float light[3], const svo_trace_out &out, cudaStream_t st, uint32_t *status) {
     if (width == 0 || height == 0) return SVO_OK;
     if (wide_octree(oct)) return set_error(SVO_ERR_LIMIT, "image tracing takes octrees of up to 2^32-1 words");
     JobDev J;
@@ -401,10 +402,11 @@ int launch_trace_image(const svo_octree *oct, const float *d_rays, uint32_t widt
     J.rgba8 = out.rgba8;
     J.tab = octree_table(oct, st);
     const uint64_t slots = (uint64_t)J.tiles_x * ((height + kImageTileH - 1) / kImageTileH) * 32;  // at most 2^35
-    void (*kern)(JobDev, uint32_t *) =
+    void (*kern)(JobDev, uint32_t *, uint32_t *) =
         J.tab ? (ray_scale != 0.0f ? k_trace_single<true, true> : k_trace_single<true, false>)
               : (ray_scale != 0.0f ? k_trace_single<false, true> : k_trace_single<false, false>);
-    kern<<<(unsigned)((slots + kImageThreads - 1) / kImageThreads), kImageThreads, 0, st>>>(J, oct->d_status);
+    kern<<<(unsigned)((slots + kImageThreads - 1) / kImageThreads), kImageThreads, 0, st>>>(
+        J, status ? status : oct->d_status, status ? oct->d_status : nullptr);
     SVO_CUDA_TRY(cudaGetLastError());
     return SVO_OK;
 }

@@ -14,6 +14,7 @@
 // allocating its own, of 385.  A pool holding more than that in live octrees
 // returns whatever is freed at the next synchronisation, as before.
 #include <mutex>
+#include <vector>
 
 #include "svo_internal.h"
 
@@ -26,6 +27,11 @@ enum Pool { kScratch, kHandles, kPools };
 std::mutex g_pool_mtx;
 cudaMemPool_t g_pools[kMaxDevices][kPools] = {};
 cudaStream_t g_streams[kMaxDevices] = {};
+// host slots: a call takes one for its duration, so the calls of up to
+// kMaxSlots threads run side by side
+constexpr int kMaxSlots = 16;
+std::vector<HostSlot *> g_free_slots[kMaxDevices];
+int g_slots[kMaxDevices] = {};
 
 cudaError_t pool_for_current_device(Pool which, cudaMemPool_t *out) {
     int dev = 0;
@@ -97,6 +103,56 @@ cudaError_t library_stream(cudaStream_t *out) {
     return cudaSuccess;
 }
 
+static void host_slot_free(HostSlot *s) {
+    if (s->st) cudaStreamDestroy(s->st);
+    if (s->host) cudaFreeHost(s->host);
+    delete s;
+}
+
+HostSlot *host_slot_take() {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return nullptr;
+    {
+        std::lock_guard<std::mutex> lk(g_pool_mtx);
+        if (!g_free_slots[dev].empty()) {
+            HostSlot *s = g_free_slots[dev].back();
+            g_free_slots[dev].pop_back();
+            return s;
+        }
+        if (g_slots[dev] >= kMaxSlots) return nullptr;
+        ++g_slots[dev];
+    }
+    HostSlot *s = new HostSlot{dev, nullptr, nullptr, nullptr};
+    void *h = nullptr, *d = nullptr;
+    cudaError_t e = cudaHostAlloc(&h, kHostSlotBytes, cudaHostAllocMapped);
+    s->host = (char *)h;
+    if (e == cudaSuccess) e = cudaHostGetDevicePointer(&d, h, 0);
+    s->dev = (char *)d;
+    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&s->st, cudaStreamNonBlocking);
+    if (e == cudaSuccess) return s;
+    cudaGetLastError();  // the call takes the staged path instead
+    host_slot_free(s);
+    std::lock_guard<std::mutex> lk(g_pool_mtx);
+    --g_slots[dev];
+    return nullptr;
+}
+
+void host_slot_give(HostSlot *s) {
+    std::lock_guard<std::mutex> lk(g_pool_mtx);
+    g_free_slots[s->device].push_back(s);
+}
+
+// Frees the idle slots of a device.
+static void host_slots_trim(int dev) {
+    std::vector<HostSlot *> idle;
+    {
+        std::lock_guard<std::mutex> lk(g_pool_mtx);
+        idle.swap(g_free_slots[dev]);
+        g_slots[dev] -= (int)idle.size();
+    }
+    for (HostSlot *s : idle) host_slot_free(s);
+}
+
 }  // namespace svo
 
 extern "C" int svo_trim_memory(void) {
@@ -104,6 +160,7 @@ extern "C" int svo_trim_memory(void) {
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return svo::cuda_fail(e, "cudaGetDevice");
+    if (dev >= 0 && dev < svo::kMaxDevices) svo::host_slots_trim(dev);
     cudaMemPool_t pools[svo::kPools] = {};
     {
         std::lock_guard<std::mutex> lk(svo::g_pool_mtx);

@@ -114,13 +114,17 @@ static int ensure_staging(svo_octree *oct, size_t dev_bytes) {
     return SVO_OK;
 }
 
+static int traversal_fault() {
+    return set_error(SVO_ERR_DEVICE, "a ray hit the traversal step cap or an out-of-range word index "
+                                     "(corrupt octree?)");
+}
+
 static int check_device_status(const svo_octree *oct) {
     uint32_t flags = 0;
     SVO_CUDA_TRY(cudaMemcpy(&flags, oct->d_status, sizeof(flags), cudaMemcpyDeviceToHost));
     if (flags) {
         cudaMemset(oct->d_status, 0, sizeof(uint32_t));
-        return set_error(SVO_ERR_DEVICE, "a ray hit the traversal step cap or an out-of-range word index "
-                                         "(corrupt octree?)");
+        return traversal_fault();
     }
     return SVO_OK;
 }
@@ -257,6 +261,54 @@ static int host_enqueue(svo_octree *oct, const float *rays, const std::vector<ui
         oct->stage_pending = false;
     }
     return rc;
+}
+
+// Up to this many rays a host call is bound by its copies', events' and waits'
+// latency: through the staged pipeline one ray takes 77 us, 1,000 rays 107 and
+// 16,000 rays 131 (1024^3 terrain); in place 28, 62 and 98.  At 60,000 rays
+// the two are equal (152 us): there the host's own copies count.
+constexpr uint64_t kSmallRays = 16384;
+static_assert(kSmallRays * 53 + 8 * 256 <= kHostSlotBytes, "a slot holds the rays and every output");
+
+// A waiting host call of at most kSmallRays rays: the rays go through a slot
+// of page-locked memory that the kernel reads and writes in place, one launch
+// and one wait, no copies on the device.  Sets `done` unless no slot can be
+// had.  launch(d_rays, outputs, stream, status) enqueues the trace.  Called
+// without staging_mtx, with nothing pending on the handle.
+template <typename Launch>
+static int trace_small(const float *rays, uint64_t n, const svo_trace_out &out, Launch launch, bool &done) {
+    done = false;
+    HostSlot *s = host_slot_take();
+    if (!s) return SVO_OK;
+    std::unique_ptr<HostSlot, void (*)(HostSlot *)> guard(s, host_slot_give);
+    size_t used = 0;
+    auto take = [&](size_t bytes) {
+        const size_t at = used;
+        used += (bytes + 255) & ~size_t(255);
+        return at;
+    };
+    const size_t o_status = take(4), o_rays = take(n * 24);
+    struct Part {
+        void *user;
+        size_t bytes, at;
+    } parts[6] = {{out.hit, n, 0},     {out.t, n * 4, 0},    {out.leaf, n * 4, 0},
+                  {out.word, n * 4, 0}, {out.rgb, n * 12, 0}, {out.rgba8, n * 4, 0}};
+    for (Part &p : parts)
+        if (p.user) p.at = take(p.bytes);
+    auto dev = [&](int k) -> void * { return parts[k].user ? s->dev + parts[k].at : nullptr; };
+    const svo_trace_out o = {(uint8_t *)dev(0), (float *)dev(1), (uint32_t *)dev(2),
+                             (uint32_t *)dev(3), (float *)dev(4), (uint32_t *)dev(5)};
+    uint32_t &status = *(uint32_t *)(s->host + o_status);
+    status = 0;
+    std::memcpy(s->host + o_rays, rays, n * 24);
+    const int rc = launch((const float *)(s->dev + o_rays), o, s->st, (uint32_t *)(s->dev + o_status));
+    const cudaError_t e = cudaStreamSynchronize(s->st);  // also after a failure: the slot goes back idle
+    if (rc) return rc;
+    if (e != cudaSuccess) return cuda_fail(e, "host trace");
+    done = true;
+    for (const Part &p : parts)
+        if (p.user) std::memcpy(p.user, s->host + p.at, p.bytes);
+    return status ? traversal_fault() : SVO_OK;
 }
 
 }  // namespace svo
@@ -666,7 +718,19 @@ static int trace_host(svo_octree *oct, const float *rays, uint64_t n, float ray_
                       const svo_trace_out *out, bool wait) {
     if (!oct || (!rays && n) || !out) return set_error(SVO_ERR_INVALID, "null argument");
     if (n > 0xFFFFFFFFull) return set_error(SVO_ERR_LIMIT, "more than 2^32-1 rays");
-    std::lock_guard<std::mutex> lock(oct->staging_mtx);
+    std::unique_lock<std::mutex> lock(oct->staging_mtx);
+    if (wait && n && n <= kSmallRays && !oct->stage_pending) {
+        lock.unlock();
+        bool done = false;
+        const float lt[3] = {light ? light[0] : 0.0f, light ? light[1] : 0.0f, light ? light[2] : 0.0f};
+        const int rc = trace_small(rays, n, *out,
+                                   [&](const float *d_rays, const svo_trace_out &o, cudaStream_t st, uint32_t *status) {
+                                       return launch_trace(oct, d_rays, n, ray_scale, lt, o, st, status);
+                                   },
+                                   done);
+        if (rc || done) return rc;
+        lock.lock();
+    }
     if (n) {
         // warp-aligned chunks
         const std::vector<uint64_t> plan = plan_chunks(n, kStageRays, 32);
@@ -684,7 +748,20 @@ static int trace_image_host(svo_octree *oct, const float *rays, uint32_t width, 
                             const float light[3], const svo_trace_out *out, bool wait) {
     if (!oct || (!rays && width && height) || !out) return set_error(SVO_ERR_INVALID, "null argument");
     if ((uint64_t)width * height > 0xFFFFFFFFull) return set_error(SVO_ERR_LIMIT, "more than 2^32-1 pixels");
-    std::lock_guard<std::mutex> lock(oct->staging_mtx);
+    std::unique_lock<std::mutex> lock(oct->staging_mtx);
+    const uint64_t n = (uint64_t)width * height;
+    if (wait && n && n <= kSmallRays && !oct->stage_pending) {
+        lock.unlock();
+        bool done = false;
+        const float lt[3] = {light ? light[0] : 0.0f, light ? light[1] : 0.0f, light ? light[2] : 0.0f};
+        const int rc = trace_small(rays, n, *out,
+                                   [&](const float *d_rays, const svo_trace_out &o, cudaStream_t st, uint32_t *status) {
+                                       return launch_trace_image(oct, d_rays, width, height, ray_scale, lt, o, st, status);
+                                   },
+                                   done);
+        if (rc || done) return rc;
+        lock.lock();
+    }
     if (width && height) {
         // Chunks of whole rows, a multiple of the 4-row tile height (all but
         // the last), about kStageRays rays at full size; each chunk is traced

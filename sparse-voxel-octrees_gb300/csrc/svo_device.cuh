@@ -100,6 +100,17 @@ __device__ __forceinline__ uint32_t pack_rgba8(float grey) {
 
 enum : int { kMiss = 0, kLeafHit = 1, kLodHit = 2, kFault = 3 };
 
+#ifdef __CUDACC__
+// Moves the flags that earlier calls left in the error word `carry` (null:
+// none) to *status.
+__device__ __forceinline__ void carry_status(uint32_t *carry, uint32_t *status) {
+    if (carry && *carry) {
+        const uint32_t f = atomicExch(carry, 0u);
+        if (f) atomicOr(status, f);
+    }
+}
+#endif
+
 // Per-ray traversal state of VoxelOctree::raymarch (VoxelOctree.cpp:207-346),
 // split into ray_init (setup, :213-250) and ray_step (one pass of the loop
 // body, :252-339) so a persistent kernel can suspend a ray between steps and

@@ -89,6 +89,19 @@ cudaError_t alloc_words(uint32_t **words, uint64_t n, cudaStream_t st);
 // A non-blocking stream per device, shared by the library's own work.
 cudaError_t library_stream(cudaStream_t *out);
 
+// Page-locked memory that the device reads and writes in place, with a stream,
+// for host calls too small for copies to pay (mem_pool.cpp).  host_slot_take
+// returns null when none can be had; a slot is idle on the device when it is
+// given back.
+constexpr size_t kHostSlotBytes = 1u << 20;
+struct HostSlot {
+    int device;
+    char *host, *dev;  // the same memory
+    cudaStream_t st;
+};
+HostSlot *host_slot_take();
+void host_slot_give(HostSlot *slot);
+
 // VoxelData::init cache-block search (VoxelData.cpp:211-244): log2 of the
 // cache-block edge, or -1 when no partition fits `mem`.
 int cache_block_log2(int w, int h, int d, uint64_t mem, uint64_t cell_cost);
@@ -129,11 +142,13 @@ int build_from_bricks_device(const MeshBricks &m, int log_side, int log_block, c
 int build_voxel_file_streamed(FILE *fp, int w, int h, int d, uint64_t mem, uint64_t slab_bytes, cudaStream_t st,
                               uint32_t **d_words, uint64_t *n_words, float center[3]);
 
-// Trace launchers (trace.cu).
+// Trace launchers (trace.cu).  status: null for the handle's error word, else
+// the word that gets this call's flags and those the handle's word holds.
 int launch_trace(const svo_octree *oct, const float *d_rays, uint64_t n, float ray_scale, const float light[3],
-                 const svo_trace_out &out, cudaStream_t st);
+                 const svo_trace_out &out, cudaStream_t st, uint32_t *status = nullptr);
 int launch_trace_image(const svo_octree *oct, const float *d_rays, uint32_t width, uint32_t height, float ray_scale,
-                       const float light[3], const svo_trace_out &out, cudaStream_t st);
+                       const float light[3], const svo_trace_out &out, cudaStream_t st,
+                       uint32_t *status = nullptr);
 int launch_count_loads(const svo_octree *oct, const float *d_rays, uint64_t n, float ray_scale, uint32_t *loads,
                        cudaStream_t st);
 

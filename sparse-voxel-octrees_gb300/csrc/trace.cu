@@ -29,6 +29,7 @@ struct TraceArgs {
     float *rgb;
     uint32_t *rgba8;
     uint32_t *status;
+    uint32_t *carry;  // or null: an error word whose flags move to *status
 };
 
 __device__ __forceinline__ void load_ray(const float *rays, uint64_t i, float &ox, float &oy, float &oz, float &dx,
@@ -63,6 +64,7 @@ __device__ __forceinline__ void store_result(const TraceArgs &a, uint64_t i, con
 template <typename Idx>
 __global__ void __launch_bounds__(256) k_trace_plain(TraceArgs a) {
     uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i == 0) carry_status(a.carry, a.status);
     if (i >= a.n) return;
     float ox, oy, oz, dx, dy, dz;
     load_ray(a.rays, i, ox, oy, oz, dx, dy, dz);
@@ -80,6 +82,7 @@ constexpr int kTabThreads = 128;
 
 __global__ void __launch_bounds__(kTabThreads) k_trace_plain_tab(TraceArgs a) {
     const uint64_t i = (uint64_t)blockIdx.x * kTabThreads + threadIdx.x;
+    if (i == 0) carry_status(a.carry, a.status);
     if (i >= a.n) return;
     float ox, oy, oz, dx, dy, dz;
     load_ray(a.rays, i, ox, oy, oz, dx, dy, dz);
@@ -103,7 +106,7 @@ __global__ void __launch_bounds__(256) k_count_loads(const uint32_t *oct, uint32
 }  // namespace
 
 int launch_trace(const svo_octree *oct, const float *d_rays, uint64_t n, float ray_scale, const float light[3],
-                 const svo_trace_out &out, cudaStream_t st) {
+                 const svo_trace_out &out, cudaStream_t st, uint32_t *status) {
     if (n == 0) return SVO_OK;
     if (out.leaf && wide_octree(oct))
         return set_error(SVO_ERR_LIMIT, "leaf indices of an octree of %llu words do not fit the 32-bit leaf output",
@@ -123,7 +126,8 @@ int launch_trace(const svo_octree *oct, const float *d_rays, uint64_t n, float r
     a.word = out.word;
     a.rgb = out.rgb;
     a.rgba8 = out.rgba8;
-    a.status = oct->d_status;
+    a.status = status ? status : oct->d_status;
+    a.carry = status ? oct->d_status : nullptr;
     a.tab = nullptr;
     const unsigned grid = (unsigned)((n + 255) / 256);
     if (wide_octree(oct) || oct->index_bits == 64)

@@ -412,3 +412,39 @@ def test_table_orders(cuda, svo, oracle, scenes, kind):
     assert tree.table_size() == (nodes if nodes is not None else tree.validate()[0])
     ref = oracle.raymarch(words, rays, threads=4)
     _assert_same(_device_trace(cuda, svo, tree, rays), ref)
+
+
+@pytest.mark.parametrize("n", [1, 33, 16384, 16385])
+def test_host_calls_around_the_in_place_limit(cuda, svo, oracle, scenes, n):
+    """Waiting host calls of up to 16,384 rays are traced in page-locked memory
+    in place, larger ones through the staged pipeline, and so is any call with
+    an asynchronous one queued before it: the same results and error reports."""
+    torch = cuda
+    grid = scenes.sphere_scene(64, 12, 0)
+    words, center = oracle.build_dense(grid)
+    tree = svo.VoxelOctree.from_words(words, center)
+    rays = scenes.random_rays(n, 3)
+    light = np.array([0.6, 0.0, 0.8], np.float32)
+    ref = oracle.raymarch(words, rays, light=light)
+    names = ("hit", "t", "leaf", "word", "rgb")
+    _assert_same(tree.trace_host(rays, light=light, outputs=names), ref)
+    pending = tree.trace_host(rays, light=light, outputs=names, wait=False)
+    _assert_same(tree.trace_host(rays, light=light, outputs=names), ref)
+    tree.synchronize()
+    _assert_same(pending, ref)
+    w = 128 if n >= 16384 else n
+    h = n // w
+    _assert_same(tree.trace_image_host(rays[:w * h], w, h, light=light, outputs=names),
+                 oracle.raymarch(words, rays[:w * h], light=light))
+    one = tree.trace_host(rays, outputs=("t",))
+    assert list(one) == ["t"] and np.array_equal(one["t"].view(np.uint32), ref["t"].view(np.uint32))
+    # a device trace that met a bounds check is reported by the next host call, once
+    bad = svo.VoxelOctree.from_words(np.array([(0x3FFF << 18) | 0xFFFF], np.uint32), (0.5, 0.5, 0.5))
+    down = np.array([[1.5, 1.5, -1.0, 0.0, 0.0, 1.0]], np.float32)
+    away = np.tile(np.array([[5.0, 5.0, 5.0, 0.6, 0.0, 0.8]], np.float32), (n, 1))
+    bad.trace(torch.from_numpy(down).cuda(), out={"hit": torch.empty(1, dtype=torch.uint8, device="cuda")})
+    torch.cuda.synchronize()
+    with pytest.raises(svo.SvoError) as e:
+        bad.trace_host(away)
+    assert e.value.code == svo.SVO_ERR_DEVICE
+    assert not bad.trace_host(away)["hit"].any()
