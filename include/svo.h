@@ -309,7 +309,7 @@ int svo_trace(const svo_octree *oct, const float *rays, uint64_t n, float ray_sc
               const svo_trace_out *out, svo_stream stream);
 
 /* Same as svo_trace with host arrays: rays are copied in and results out
- * through the handle's four staging buffers in chunks of about 4 M rays, on
+ * through the handle's four staging buffers in chunks of at most 4 M rays, on
  * internal copy-in, copy-out and per-buffer trace streams, so copies overlap
  * tracing.  Returns when results are on the host (after any work queued
  * earlier by the asynchronous forms below). */

@@ -21,7 +21,7 @@ namespace svo {
 namespace {
 thread_local std::string g_last_error;
 constexpr uint64_t kOctBlock = 64ull * 1024 * 1024;  // VoxelOctree.cpp:55
-constexpr uint64_t kStageRays = 1ull << 22;          // rays per staging chunk
+constexpr uint64_t kStageRays = 1ull << 22;          // rays per staging chunk, at most
 }  // namespace
 
 int set_error(int code, const char *fmt, ...) {
@@ -140,6 +140,36 @@ static std::vector<uint64_t> plan_chunks(uint64_t total, uint64_t target, uint64
     std::vector<uint64_t> plan;
     for (uint64_t s = 0; s < total; s += t) plan.push_back(std::min(t, total - s));
     return plan;
+}
+
+// Whether every array of a host call is page-locked, so that its copies run
+// beside its traces.
+static bool page_locked(const float *rays, const svo_trace_out &out) {
+    const void *const p[7] = {rays, out.hit, out.t, out.leaf, out.word, out.rgb, out.rgba8};
+    for (const void *q : p) {
+        if (!q) continue;
+        cudaPointerAttributes a;
+        if (cudaPointerGetAttributes(&a, q) != cudaSuccess) {
+            cudaGetLastError();  // not CUDA's: pageable
+            return false;
+        }
+        if (a.type != cudaMemoryTypeHost) return false;
+    }
+    return true;
+}
+
+// Rays per chunk of a host call of n rays.  In one chunk a call's copy in, its
+// trace and its copies out follow one another; in four they overlap, as long
+// as a chunk's copy is longer than the 20 us its calls take on the host.
+// 1024x768 pinned rays (256^3): 242 us in one chunk, 200 in 2, 193 in 3, 195 in
+// 4, 200 in 6, 206 in 8; 640x480: 137, 120, 126, 130, 135, 135; 1920x1080: 515,
+// 419, 392, 384, 379, 381; 3840x2160: 1,445 in two, 1,270 in four.  A pageable
+// copy is staged by the driver, waits for it and costs about 60 us each, so
+// those calls keep whole chunks (1024x768: 256 us in one, 455 in four).
+static uint64_t chunk_rays(const float *rays, uint64_t n, const svo_trace_out &out) {
+    constexpr uint64_t kParts = 4, kLeast = 160 * 1024;
+    if (n <= kLeast || !page_locked(rays, out)) return kStageRays;
+    return std::min(kStageRays, std::max((n + kParts - 1) / kParts, kLeast));
 }
 
 // The host-buffer pipeline of svo_trace_host and svo_trace_image_host (and
@@ -733,7 +763,7 @@ static int trace_host(svo_octree *oct, const float *rays, uint64_t n, float ray_
     }
     if (n) {
         // warp-aligned chunks
-        const std::vector<uint64_t> plan = plan_chunks(n, kStageRays, 32);
+        const std::vector<uint64_t> plan = plan_chunks(n, chunk_rays(rays, n, *out), 32);
         const float lt[3] = {light ? light[0] : 0.0f, light ? light[1] : 0.0f, light ? light[2] : 0.0f};
         int rc = host_enqueue(oct, rays, plan, *out,
                               [&](const float *d_rays, uint64_t m, const svo_trace_out &o, cudaStream_t st) {
@@ -764,9 +794,8 @@ static int trace_image_host(svo_octree *oct, const float *rays, uint32_t width, 
     }
     if (width && height) {
         // Chunks of whole rows, a multiple of the 4-row tile height (all but
-        // the last), about kStageRays rays at full size; each chunk is traced
-        // as an image of its own.
-        const uint64_t rows = std::max<uint64_t>(4, (kStageRays / width) & ~uint64_t(3));
+        // the last); each chunk is traced as an image of its own.
+        const uint64_t rows = std::max<uint64_t>(4, (chunk_rays(rays, n, *out) / width) & ~uint64_t(3));
         std::vector<uint64_t> plan = plan_chunks(height, rows, 4);
         for (auto &c : plan) c *= width;
         const float lt[3] = {light ? light[0] : 0.0f, light ? light[1] : 0.0f, light ? light[2] : 0.0f};

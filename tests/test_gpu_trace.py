@@ -448,3 +448,30 @@ def test_host_calls_around_the_in_place_limit(cuda, svo, oracle, scenes, n):
         bad.trace_host(away)
     assert e.value.code == svo.SVO_ERR_DEVICE
     assert not bad.trace_host(away)["hit"].any()
+
+
+@pytest.mark.parametrize("W,H", [(640, 256), (641, 257), (1024, 643)])
+def test_page_locked_host_calls_in_chunks(cuda, svo, oracle, scenes, W, H):
+    """Page-locked arrays go through the host pipeline in chunks (from 163,841
+    rays on), pageable ones whole: the same results, chunk edges included."""
+    torch = cuda
+    words, center = oracle.build_dense(scenes.sphere_scene(64, 12, 0))
+    tree = svo.VoxelOctree.from_words(words, center)
+    rays = scenes.camera_rays(scenes.orbit_cameras(1, 3, center, radius=1.6)[0], W, H)
+    R = W * H
+    ref = oracle.raymarch(words, rays, light=(0.0, 0.0, 1.0))
+    keep = [torch.from_numpy(rays).pin_memory()]
+    kinds = {"hit": torch.uint8, "t": torch.float32, "leaf": torch.int32, "word": torch.int32}
+    for call in (tree.trace_host, lambda r, **kw: tree.trace_image_host(r, W, H, **kw)):
+        for wait in (True, False):
+            out = {}
+            for k, d in kinds.items():
+                keep.append(torch.zeros(R, dtype=d).pin_memory())
+                out[k] = keep[-1].numpy()
+            keep.append(torch.zeros((R, 3)).pin_memory())
+            out["rgb"] = keep[-1].numpy()
+            call(keep[0].numpy(), out=out, wait=wait)
+            tree.synchronize()
+            out["leaf"], out["word"] = out["leaf"].view(np.uint32), out["word"].view(np.uint32)
+            _assert_same(out, ref)
+    _assert_same(tree.trace_image_host(rays, W, H, outputs=("hit", "t", "leaf", "word", "rgb")), ref)
