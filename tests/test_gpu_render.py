@@ -56,3 +56,15 @@ def test_frames_match_reference_renderer(cuda, svo, golden):
         img = tree.render_frame(rot, pos, 1280, 720, 16, 3 if half else 1).cpu().numpy().view(np.uint32)
         assert np.array_equal(img, ref)
     assert tree.device_status() == 0
+
+
+@pytest.mark.parametrize("W,H,strips", [(320, 200, 4), (61, 45, 3), (9, 7, 2)])
+@pytest.mark.parametrize("stride", [2, 4, 5, 7, 8])
+def test_strided_frames_match_oracle(cuda, svo, golden, oracle, scenes, W, H, strips, stride):
+    """Every pixel stride: from 16 colours a tile down to one, tiles that share
+    a warp across strip and frame edges."""
+    g = golden["dragon"]
+    tree = svo.VoxelOctree.from_words(g["words"], g["center"])
+    cam = scenes.orbit_cameras(1, W + stride, g["center"], radius=1.2)[0]
+    img = _frame(cuda, tree, cam, width=W, height=H, n_strips=strips, pixel_stride=stride)
+    assert np.array_equal(img, oracle.render_frame(g["words"], cam[:9], cam[9:12], W, H, strips, stride))
