@@ -3,8 +3,9 @@
 //
 // Work is a global space of ray slots: each view contributes either one slot
 // per ray (linear views) or 32 slots per tile_w x tile_h pixel tile (image
-// views, so a warp's lanes start on neighbouring pixels).  A persistent grid
-// of SMs x blocks_per_sm CTAs drains the space: each warp takes `chunk`
+// views, so a warp's lanes start on neighbouring pixels).  Without lane refill
+// or table cache a launch has a thread per slot (k_trace_slots).  Otherwise a
+// persistent grid of SMs x blocks_per_sm CTAs drains the space: each warp takes `chunk`
 // consecutive slots from one device counter with a single atomicAdd and hands
 // them to its idle lanes in ballot-rank order.  Lanes whose ray finishes go
 // idle; once at least `refill_idle` lanes of a warp are idle the warp refills
@@ -323,6 +324,33 @@ __global__ void __maxnreg__(48) k_trace_persistent_r48(BatchArgs a) {
     trace_refill<kTab, kLod>(a, s_dyn);
 }
 
+// A ray slot per thread, in small CTAs that the hardware starts one after
+// another: what whole-warp schedules (refill_idle 0 or 32) come to where the
+// launch shape does not hold the grid below what fits.  The persistent form
+// pays for the queue, for its longest warps at the end of each CTA's share and
+// for registers (48 to 64 against 40): 12 octrees of depth 7 to 10 took 444 us
+// with its 48-register build and take 393, 3 small ones 128 and 100, 48 ones
+// 1,589 and 1,574.
+constexpr int kSlotThreads = 128;
+
+template <bool kTab, bool kLod>
+__global__ void __launch_bounds__(kSlotThreads) k_trace_slots(BatchArgs a) {
+    const uint64_t slot = (uint64_t)blockIdx.x * kSlotThreads + threadIdx.x;
+    if (slot >= a.total) return;
+    RayStackFor<kTab> stk;
+    RayState st;
+    int job;
+    uint32_t out_idx, nw;
+    const uint32_t *oct;
+    const uint4 *tab;
+    float rs, rdx, rdy, rdz;
+    if (!setup_slot<kTab>(a, a.begin, slot, st, job, out_idx, oct, tab, nw, rs, rdx, rdy, rdz)) return;
+    RayResult res;
+    while (!ray_step_any<kTab, kLod>(st, stk, oct, tab, nw, rs, res)) {
+    }
+    write_result(a, job, out_idx, res, rdx, rdy, rdz);
+}
+
 // One image view, passed by value (svo_trace_image): an 8x4-pixel tile per
 // warp, in small CTAs that the hardware starts one after another.  A large
 // image is bound by instruction issue and gains nothing over a persistent
@@ -533,6 +561,14 @@ int enqueue_trace(svo_batch *b, const svo_trace_config &c, cudaStream_t st) {
     int resident = 0;
     SVO_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kern, c.block_threads, smem));
     int per_sm = std::max(1, std::min(c.blocks_per_sm, resident));
+    const uint64_t ctas = std::max<uint64_t>(1, (b->total + kSlotThreads - 1) / kSlotThreads);
+    if (!cache && (c.refill_idle == 0 || c.refill_idle == 32) && c.blocks_per_sm >= resident && ctas <= 0x7FFFFFFFull) {
+        BatchKernel slots = b->all_tab ? (b->any_lod ? k_trace_slots<true, true> : k_trace_slots<true, false>)
+                                       : (b->any_lod ? k_trace_slots<false, true> : k_trace_slots<false, false>);
+        slots<<<(unsigned)ctas, kSlotThreads, 0, st>>>(a);
+        SVO_CUDA_TRY(cudaGetLastError());
+        return SVO_OK;
+    }
     SVO_CUDA_TRY(cudaMemsetAsync(b->queue_d, 0, sizeof(unsigned long long), st));
     dim3 grid((unsigned)(b->num_sms * per_sm));
     kern<<<grid, c.block_threads, smem, st>>>(a);
@@ -762,10 +798,12 @@ int svo_batch_autotune(svo_batch *b, svo_trace_config *best, float *best_ms, svo
     };
     // table cache depths: none; 64 entries (levels 0-1 hold at most 9 nodes,
     // level 2 at most 64 more); 256 entries (levels 0-2 hold at most 73)
+    // (without a cache the launch does not depend on the CTA and chunk sizes)
     for (int cache : {0, 64, 256})
         for (int bt : {128, 256, 512})
             for (int tw : {4, 8, 16})
-                for (int chunk : {32, 128}) add(bt, 0, 1, tw, chunk, cache);  // whole-warp tiles, no refill
+                for (int chunk : {32, 128})
+                    if (cache || (bt == 256 && chunk == 32)) add(bt, 0, 1, tw, chunk, cache);  // whole-warp tiles, no refill
     // lane refill, default build (64 registers) or 48-register build
     for (int cap : {0, 48})
         for (int bt : {128, 256})

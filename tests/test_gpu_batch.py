@@ -186,3 +186,19 @@ def test_batch_matches_plain_kernel(cuda, svo, oracle, scenes, golden):
     p, q = _host(plain), _host(batched)
     for k in p:
         assert np.array_equal(p[k], q[k]), k
+
+
+@pytest.mark.parametrize("cfg", [dict(refill_idle=32), dict(refill_idle=0, tile_w=32), dict(refill_idle=32, tile_w=4),
+                                 # a grid held below what fits stays persistent
+                                 dict(refill_idle=0, blocks_per_sm=1), dict(refill_idle=32, blocks_per_sm=1),
+                                 dict(refill_idle=32, blocks_per_sm=1, reg_cap=48, chunk=32)])
+def test_batch_whole_warp_schedules(cuda, svo, scene, cfg):
+    torch = cuda
+    views, refs = scene
+    b = svo.Batch(views)
+    b.capture_graph(svo.default_config(**cfg))
+    for _ in range(2):
+        _clear(torch, views)
+        b.launch_graph()
+        _check(torch, views, refs)
+    assert b.status() == 0
