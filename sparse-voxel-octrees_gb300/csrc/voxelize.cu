@@ -14,32 +14,36 @@
 //  1. Triangle setup (one thread per triangle): rescale to the unit cube,
 //     gather the fan triangle's vertices, flat normal when the file has none,
 //     bounds (PlyLoader.cpp:40-53, 167-224).
-//  2. Sub-block lists (one thread per triangle): the cells of
+//  2. Sub-block lists (a thread, or for large ones a warp, per triangle): the cells of
 //     iterateOverlappingBlocks (PlyLoader.cpp:233-270), culled by the same
 //     triangle/box test with the same incrementally accumulated centres; each
 //     member cell marks its cache block non-empty (isBlockEmpty) and emits
 //     one (brick, triangle) pair per 8^3 brick (smaller when sub-blocks are)
 //     of the cell that the triangle's clamped voxel box touches.
-//  3. A stable radix sort of the pairs by brick (sort.cuh): each brick's
-//     triangles in ascending index, the order a sub-block list holds them.
-//  4. Cache blocks in the reference's visiting order (ascending Morton code
-//     of the blocks the lists mark), each against the one persistent
-//     buffer: one warp per brick folds the brick's triangles in order with
-//     writeTriangleCell's blend (PlyLoader.cpp:296-336), its lanes covering
-//     each triangle's clamped box inside the brick; voxel-box centres are
-//     the reference's running sums (lo - 0.5) * h + h + ... + h, read from a
-//     table of those sums.  Then the block's nonzero words are extracted in
-//     Morton order and cleared, except a dropped odd last slice, from the
-//     bricks that can hold any: the folded ones and those under earlier
-//     blocks' dropped slices.
-//  5. The octree from the Morton-ordered voxels and the block flags
-//     (build_from_sorted_device).
+//  3. The pairs by brick, each brick's triangles in ascending index, the order
+//     a sub-block list holds them: through a table of counts per brick where
+//     the cube's brick codes fit one, else a stable radix sort (sort.cuh).
+//  4. The fold: one warp per brick blends the brick's triangles in order with
+//     writeTriangleCell's formula (PlyLoader.cpp:296-336), its lanes covering
+//     each triangle's clamped box inside the brick; voxel-box centres are the
+//     reference's running sums (lo - 0.5) * h + h + ... + h, read from a table
+//     of those sums.  Where no dropped slice reaches a later block, all bricks
+//     are folded at once (the direct fold).  Else cache blocks follow one
+//     another in the reference's visiting order (ascending Morton code of the
+//     blocks the lists mark) against the one persistent buffer, and each
+//     block's nonzero words are extracted in Morton order and cleared, except
+//     a dropped odd last slice, from the bricks that can hold any: the folded
+//     ones and those under earlier blocks' dropped slices.
+//  5. The octree: from the folded 8^3 bricks (build_from_bricks_device), or
+//     from the Morton-ordered voxels (build_from_sorted_device), and the block
+//     flags.
 #include <algorithm>
 #include <memory>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "brick.cuh"
@@ -175,91 +179,323 @@ struct ListGeom {
 
 __device__ __forceinline__ int point_to_grid(float p, float s) { return (int)(p * s + 1.0f); }
 
-// mode 0: count pairs per triangle (and store the triangle's voxel box,
-// mark blocks); mode 1: emit pairs at out_off[t].
-template <int kMode>
-__global__ void k_tri_pairs(uint64_t n_tris, const float *__restrict__ tris, ListGeom g, int32_t *__restrict__ box,
-                            uint8_t *__restrict__ block_flag, uint32_t *__restrict__ count,
-                            const uint64_t *__restrict__ out_off, uint32_t *__restrict__ pair_key,
-                            uint32_t *__restrict__ pair_tri, uint32_t *__restrict__ pair_cell,
-                            uint32_t *__restrict__ err) {
-    uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n_tris) return;
-    const float *T = tris + t * kTriFloats;
-    int lo[3], hi[3];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        lo[k] = point_to_grid(T[kTriLo + k], g.grid_scale);
-        hi[k] = point_to_grid(T[kTriHi + k], g.grid_scale);
-    }
-    if (kMode == 0) {
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            box[6 * t + k] = lo[k];
-            box[6 * t + 3 + k] = hi[k];
-        }
-    }
-    float tv[9];
-#pragma unroll
-    for (int k = 0; k < 9; ++k) tv[k] = T[kTriP + k];
-    int lg[3], ug[3];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        lg[k] = lo[k] / g.sub[k];
-        ug[k] = (hi[k] + 1) / g.sub[k];
-    }
-    const int max_side = max(ug[0] - lg[0], max(ug[1] - lg[1], ug[2] - lg[2]));
-    uint32_t n = 0;
-    uint64_t o = kMode == 1 ? out_off[t] : 0;
+// mode 0: count pairs per triangle and, with brick_n, per brick (and store the
+// triangle's voxel box, mark blocks); mode 1: emit pairs at out_off[t]; mode 2:
+// emit each pair's triangle and cell at the next place of its brick
+// (brick_n[key], moved on).
+//
+// A thread per triangle, per_warp of them in a warp; the triangles whose box
+// meets more than kWarpTriangle bricks are left to the whole warp, one after
+// another.  A thread's loop is a chain (in mode 2 of atomics that return): the
+// build of 1,280 triangles of hundreds of bricks each at 1024^3 takes 3.5 ms
+// with it, 1.6 ms so.  Of 327,680 small triangles a pass takes 32 us, bound by
+// the scattered atomics (one per brick and warp by match_any: 36 us).
+constexpr int kWarpTriangle = 32;
 
-    auto member = [&](int gx, int gy, int gz) {
-        if (gx < 0 || gy < 0 || gz < 0 || gx >= g.grid[0] || gy >= g.grid[1] || gz >= g.grid[2]) {
-            atomicOr(err, 1u);  // the reference would index past its block offsets
-            return;
-        }
-        const uint32_t slab = g.slab_mode ? (uint32_t)(gz / g.part[2]) : 0u;
-        if (kMode == 0) {
-            uint64_t blk = g.slab_mode ? (uint64_t)slab
-                                       : morton3((uint32_t)(gx / g.part[0]), (uint32_t)(gy / g.part[1]),
-                                                 (uint32_t)(gz / g.part[2]));
-            if (blk < g.n_blocks) block_flag[blk] = 1;
-            else atomicOr(err, 2u);
-        }
-        const int c0[3] = {gx * g.sub[0], gy * g.sub[1], gz * g.sub[2]};
-        int a[3], b[3];
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            a[k] = max(lo[k], c0[k]);
-            b[k] = min(hi[k], min(c0[k] + g.sub[k] - 1, g.dims[k] - 1));
-        }
-        if (a[0] > b[0] || a[1] > b[1] || a[2] > b[2]) return;
-        for (int bz = a[2] >> g.log_e; bz <= (b[2] >> g.log_e); ++bz)
-            for (int by = a[1] >> g.log_e; by <= (b[1] >> g.log_e); ++by)
-                for (int bx = a[0] >> g.log_e; bx <= (b[0] >> g.log_e); ++bx) {
-                    if (kMode == 1) {
-                        pair_key[o + n] = (slab << g.brick_bits) | (uint32_t)morton3((uint32_t)bx, (uint32_t)by, (uint32_t)bz);
-                        pair_tri[o + n] = (uint32_t)t;
-                        pair_cell[o + n] = (uint32_t)gx + (uint32_t)g.grid[0] * ((uint32_t)gy + (uint32_t)g.grid[1] * (uint32_t)gz);
-                    }
-                    ++n;
-                }
+// Morton code of three 10-bit coordinates (brick codes have at most 30 bits).
+__device__ __forceinline__ uint32_t morton3_32(uint32_t x, uint32_t y, uint32_t z) {
+    auto spread = [](uint32_t v) {
+        v = (v | (v << 16)) & 0x030000FFu;
+        v = (v | (v << 8)) & 0x0300F00Fu;
+        v = (v | (v << 4)) & 0x030C30C3u;
+        return (v | (v << 2)) & 0x09249249u;
     };
+    return spread(x) | (spread(y) << 1) | (spread(z) << 2);
+}
 
-    if (max_side > 0) {
-        const float half[3] = {0.5f * g.cell_h[0], 0.5f * g.cell_h[1], 0.5f * g.cell_h[2]};
-        float cz = ((float)lg[2] + 0.5f) * g.cell_h[2];
-        for (int z = lg[2]; z <= ug[2]; ++z, cz += g.cell_h[2]) {
-            float cy = ((float)lg[1] + 0.5f) * g.cell_h[1];
-            for (int y = lg[1]; y <= ug[1]; ++y, cy += g.cell_h[1]) {
-                float cx = ((float)lg[0] + 0.5f) * g.cell_h[0];
-                for (int x = lg[0]; x <= ug[0]; ++x, cx += g.cell_h[0])
-                    if (tri_box(cx, cy, cz, half, tv)) member(x, y, z);
+template <int kMode>
+__global__ void __launch_bounds__(128, 8) k_tri_pairs(uint64_t n_tris, int per_warp, const float *__restrict__ tris, ListGeom g,
+                                                   int32_t *__restrict__ box, uint8_t *__restrict__ block_flag,
+                                                   uint32_t *__restrict__ count, const uint64_t *__restrict__ out_off,
+                                                   uint32_t *__restrict__ pair_key, uint32_t *__restrict__ pair_tri,
+                                                   uint32_t *__restrict__ pair_cell, uint32_t *__restrict__ brick_n,
+                                                   uint32_t *__restrict__ err) {
+    const int lane = threadIdx.x & 31;
+    const uint64_t t0 = ((uint64_t)blockIdx.x * 4 + (threadIdx.x >> 5)) * (uint64_t)per_warp;
+    uint32_t left = 0;  // the warp's large triangles
+    for (bool own = true;; own = false) {
+        uint64_t t = lane < per_warp ? t0 + lane : n_tris;
+        uint32_t first = 0, step = 1;  // this thread's share of the triangle's pairs
+        if (!own) {
+            if (!left) break;
+            t = t0 + (__ffs(left) - 1);
+            left &= left - 1;
+            first = lane;
+            step = 32;
+        }
+        const float *T = tris + t * kTriFloats;
+        int lo[3] = {0, 0, 0}, hi[3] = {-1, -1, -1};
+        if (t < n_tris) {
+            if (kMode == 0) {
+                static_assert(kTriLo == 27 && kTriHi == 30 && kTriFloats % 4 == 0, "bounds at floats 27..32");
+                const float4 m = *reinterpret_cast<const float4 *>(T + 28);
+                const float bound[6] = {T[27], m.x, m.y, m.z, m.w, T[32]};
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    lo[k] = point_to_grid(bound[k], g.grid_scale);
+                    hi[k] = point_to_grid(bound[3 + k], g.grid_scale);
+                }
+            } else {
+                const int2 *v = reinterpret_cast<const int2 *>(box) + 3 * t;
+                const int2 u0 = v[0], u1 = v[1], u2 = v[2];
+                lo[0] = u0.x, lo[1] = u0.y, lo[2] = u1.x;
+                hi[0] = u1.y, hi[1] = u2.x, hi[2] = u2.y;
             }
         }
-    } else {
-        member(lg[0], lg[1], lg[2]);
+        if (own) {
+            float bricks = 1.0f;
+#pragma unroll
+            for (int k = 0; k < 3; ++k) bricks *= (float)((hi[k] >> g.log_e) - (lo[k] >> g.log_e) + 1);
+            const bool large = t < n_tris && bricks > (float)kWarpTriangle;
+            left = __ballot_sync(0xffffffffu, large);
+            if (large || t >= n_tris) continue;
+        }
+        if (kMode == 0 && first == 0) {
+            int2 *v = reinterpret_cast<int2 *>(box) + 3 * t;
+            v[0] = make_int2(lo[0], lo[1]);
+            v[1] = make_int2(lo[2], hi[0]);
+            v[2] = make_int2(hi[1], hi[2]);
+        }
+        int lg[3], ug[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            lg[k] = lo[k] / g.sub[k];
+            ug[k] = (hi[k] + 1) / g.sub[k];
+        }
+        const int max_side = max(ug[0] - lg[0], max(ug[1] - lg[1], ug[2] - lg[2]));
+        uint32_t n = 0;
+        const uint64_t o = kMode == 1 ? out_off[t] : 0;
+
+        auto member = [&](int gx, int gy, int gz) {
+            if (gx < 0 || gy < 0 || gz < 0 || gx >= g.grid[0] || gy >= g.grid[1] || gz >= g.grid[2]) {
+                atomicOr(err, 1u);  // the reference would index past its block offsets
+                return;
+            }
+            const uint32_t slab = g.slab_mode ? (uint32_t)(gz / g.part[2]) : 0u;
+            if (kMode == 0 && first == 0) {
+                uint64_t blk = g.slab_mode ? (uint64_t)slab
+                                           : morton3((uint32_t)(gx / g.part[0]), (uint32_t)(gy / g.part[1]),
+                                                     (uint32_t)(gz / g.part[2]));
+                if (blk >= g.n_blocks) atomicOr(err, 2u);
+                else if (!block_flag[blk]) block_flag[blk] = 1;  // most triangles find it marked
+            }
+            const int c0[3] = {gx * g.sub[0], gy * g.sub[1], gz * g.sub[2]};
+            int a[3], b[3];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                a[k] = max(lo[k], c0[k]);
+                b[k] = min(hi[k], min(c0[k] + g.sub[k] - 1, g.dims[k] - 1));
+            }
+            if (a[0] > b[0] || a[1] > b[1] || a[2] > b[2]) return;
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                a[k] >>= g.log_e;
+                b[k] = (b[k] >> g.log_e) - a[k] + 1;
+            }
+            const uint32_t pairs = (uint32_t)b[0] * (uint32_t)b[1] * (uint32_t)b[2];
+            const uint32_t cell = (uint32_t)gx + (uint32_t)g.grid[0] * ((uint32_t)gy + (uint32_t)g.grid[1] * (uint32_t)gz);
+            int x = 0, y = 0, z = 0;
+            for (uint32_t f = first; f < pairs; f += step) {
+                if (kMode == 0 && !brick_n) break;
+                if (step != 1) {
+                    const uint32_t yz = f / (uint32_t)b[0];
+                    x = (int)(f - yz * (uint32_t)b[0]);
+                    z = (int)(yz / (uint32_t)b[1]);
+                    y = (int)yz - z * b[1];
+                } else if (f && ++x == b[0]) {
+                    x = 0;
+                    if (++y == b[1]) {
+                        y = 0;
+                        ++z;
+                    }
+                }
+                const uint32_t key = morton3_32((uint32_t)(a[0] + x), (uint32_t)(a[1] + y), (uint32_t)(a[2] + z));
+                if (kMode == 0) atomicAdd(brick_n + key, 1u);
+                if (kMode == 1) {
+                    pair_key[o + n + f] = (slab << g.brick_bits) | key;
+                    pair_tri[o + n + f] = (uint32_t)t;
+                    pair_cell[o + n + f] = cell;
+                }
+                if (kMode == 2) {
+                    const uint32_t at = atomicAdd(brick_n + key, 1u);
+                    pair_tri[at] = (uint32_t)t;
+                    if (pair_cell) pair_cell[at] = cell;
+                }
+            }
+            n += pairs;
+        };
+
+        if (max_side > 0) {
+            const float4 p0 = reinterpret_cast<const float4 *>(T + kTriP)[0], p1 = reinterpret_cast<const float4 *>(T + kTriP)[1];
+            const float tv[9] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w, T[kTriP + 8]};
+            const float half[3] = {0.5f * g.cell_h[0], 0.5f * g.cell_h[1], 0.5f * g.cell_h[2]};
+            float cz = ((float)lg[2] + 0.5f) * g.cell_h[2];
+            for (int z = lg[2]; z <= ug[2]; ++z, cz += g.cell_h[2]) {
+                float cy = ((float)lg[1] + 0.5f) * g.cell_h[1];
+                for (int y = lg[1]; y <= ug[1]; ++y, cy += g.cell_h[1]) {
+                    float cx = ((float)lg[0] + 0.5f) * g.cell_h[0];
+                    for (int x = lg[0]; x <= ug[0]; ++x, cx += g.cell_h[0])
+                        if (tri_box(cx, cy, cz, half, tv)) member(x, y, z);
+                }
+            }
+        } else {
+            member(lg[0], lg[1], lg[2]);
+        }
+        if (kMode == 0 && first == 0) count[t] = n;
     }
-    if (kMode == 0) count[t] = n;
+}
+
+// ---- 3. pairs by brick -----------------------------------------------------------
+//
+// Where the brick codes of the whole cube fit a table, the pairs are counted
+// per brick, the counts scanned, and every pair dropped into its brick's range
+// in any order; each brick's few triangles are then sorted by a warp, or, in
+// the bricks that hold more than kWarpSort, by a CTA.  A radix sort of the
+// pairs moves all of them once per key digit and needs head flags, scans and
+// gathers of its own.  Whole builds, radix sort / table (us): 1,280 triangles
+// at 64^3 400 / 230, 20,480 at 256^3 470 / 270, 327,680 at 128^3 890 / 700 and
+// at 1024^3 1130 / 850.  The radix sort stays for larger cubes, z-slabs, the
+// block buffer, and meshes with more than kSortedInBrick pairs in one brick.
+constexpr int kWarpSort = 128, kSortedInBrick = 4096;
+constexpr int kBrickTile = 2048;  // 256 threads x 8
+
+// Bricks and pairs of a tile: bricks above bit 40, pairs below.
+__device__ __forceinline__ uint64_t tile_sum(const uint32_t *n, uint64_t i0, uint64_t cells, uint32_t (&c)[8]) {
+    uint64_t s = 0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        c[k] = i0 + k < cells ? n[i0 + k] : 0u;
+        s += (uint64_t)c[k] + (c[k] ? 1ull << 40 : 0ull);
+    }
+    return s;
+}
+
+__global__ void __launch_bounds__(256) k_brick_tiles(const uint32_t *__restrict__ n, uint64_t cells,
+                                                     uint64_t *__restrict__ tiles, uint32_t *__restrict__ largest) {
+    uint32_t c[8], most = 0;
+    const uint64_t s = tile_sum(n, (uint64_t)blockIdx.x * kBrickTile + (uint64_t)threadIdx.x * 8, cells, c);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) most = max(most, c[k]);
+    most = __reduce_max_sync(0xffffffffu, most);
+    if ((threadIdx.x & 31) == 0 && most) atomicMax(largest, most);
+    uint64_t total;
+    block_excl_scan<uint64_t>(s, &total);
+    if (threadIdx.x == 0) tiles[blockIdx.x] = total;
+}
+
+// The non-empty bricks' keys and first pairs, in key order, and in n each
+// brick's first pair in place of its count.
+__global__ void __launch_bounds__(256) k_brick_layout(uint32_t *__restrict__ n, uint64_t cells,
+                                                      const uint64_t *__restrict__ tiles, uint32_t *__restrict__ bkey,
+                                                      uint32_t *__restrict__ bstart, uint64_t *__restrict__ totals) {
+    uint64_t before = 0, total;
+    for (uint32_t t = threadIdx.x; t < blockIdx.x; t += 256) before += tiles[t];
+    block_excl_scan<uint64_t>(before, &total);
+    before = total;
+    const uint64_t i0 = (uint64_t)blockIdx.x * kBrickTile + (uint64_t)threadIdx.x * 8;
+    uint32_t c[8];
+    const uint64_t s = tile_sum(n, i0, cells, c);
+    uint64_t at = before + block_excl_scan<uint64_t>(s, &total);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        if (!c[k]) continue;
+        n[i0 + k] = (uint32_t)at;
+        bkey[at >> 40] = (uint32_t)(i0 + k);
+        bstart[at >> 40] = (uint32_t)at;
+        at += (uint64_t)c[k] + (1ull << 40);
+    }
+    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {
+        bstart[(before + total) >> 40] = (uint32_t)(before + total);
+        *totals = before + total;
+    }
+}
+
+// A brick's pairs into the order of the sub-block lists: ascending triangles,
+// and a triangle's cells ascending (where a brick lies in one sub-block each
+// triangle is there once, and cell is null).
+template <bool kCells>
+using PairKey = std::conditional_t<kCells, uint64_t, uint32_t>;
+
+template <bool kCells>
+__device__ __forceinline__ PairKey<kCells> pair_at(const uint32_t *tri, const uint32_t *cell, uint32_t i) {
+    if constexpr (kCells) return ((uint64_t)tri[i] << 32) | cell[i];
+    else return tri[i];
+}
+
+template <bool kCells>
+__device__ __forceinline__ void put_pair(uint32_t *tri, uint32_t *cell, uint32_t i, PairKey<kCells> v) {
+    if constexpr (kCells) {
+        tri[i] = (uint32_t)(v >> 32);
+        cell[i] = (uint32_t)v;
+    } else {
+        tri[i] = v;
+    }
+}
+
+// A warp per brick of at most kWarpSort pairs: each pair's place is the count
+// of those before it (no two are equal).
+constexpr int kBrickSortWarps = 4;
+
+template <bool kCells>
+__global__ void __launch_bounds__(kBrickSortWarps * 32) k_sort_bricks(uint32_t nb, const uint32_t *__restrict__ bstart,
+                                                                      uint32_t *tri, uint32_t *cell) {
+    using Key = PairKey<kCells>;
+    __shared__ alignas(16) Key buf[kBrickSortWarps][kWarpSort];
+    const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const uint32_t j = blockIdx.x * kBrickSortWarps + wid;
+    if (j >= nb) return;
+    const uint32_t s0 = bstart[j], n = bstart[j + 1] - s0;
+    if (n <= 1 || n > (uint32_t)kWarpSort) return;
+    Key *const key = buf[wid], v[kWarpSort / 32];
+#pragma unroll
+    for (int q = 0; q < kWarpSort / 32; ++q) {
+        const uint32_t i = lane + 32 * q;
+        v[q] = i < n ? pair_at<kCells>(tri, cell, s0 + i) : ~Key(0);
+        key[i] = v[q];
+    }
+    __syncwarp();
+#pragma unroll
+    for (int q = 0; q < kWarpSort / 32; ++q) {
+        if (32u * q >= n) break;
+        uint32_t r = 0;
+        for (uint32_t k = 0; k < n; k += 4) {
+#pragma unroll
+            for (int m = 0; m < 4; ++m) r += key[k + m] < v[q] ? 1u : 0u;
+        }
+        if (lane + 32 * q < n) put_pair<kCells>(tri, cell, s0 + r, v[q]);
+    }
+}
+
+// A CTA per brick of more: a bitonic sort in shared memory.
+template <bool kCells>
+__global__ void __launch_bounds__(256) k_sort_large(uint32_t nb, const uint32_t *__restrict__ bstart, uint32_t *tri,
+                                                    uint32_t *cell) {
+    using Key = PairKey<kCells>;
+    __shared__ Key key[kSortedInBrick];
+    for (uint32_t j = blockIdx.x; j < nb; j += gridDim.x) {
+        const uint32_t s0 = bstart[j], n = bstart[j + 1] - s0;
+        if (n <= (uint32_t)kWarpSort || n > (uint32_t)kSortedInBrick) continue;  // the host has checked the largest
+        uint32_t size = kWarpSort;
+        while (size < n) size *= 2;
+        for (uint32_t i = threadIdx.x; i < size; i += 256)
+            key[i] = i < n ? pair_at<kCells>(tri, cell, s0 + i) : ~Key(0);
+        for (uint32_t k = 2; k <= size; k *= 2) {
+            for (uint32_t d = k / 2; d > 0; d /= 2) {
+                __syncthreads();
+                for (uint32_t p = threadIdx.x; p < size / 2; p += 256) {
+                    const uint32_t i = 2 * p - (p & (d - 1)), l = i + d;
+                    const Key a = key[i], b = key[l];
+                    if ((a > b) == ((i & k) == 0)) {
+                        key[i] = b;
+                        key[l] = a;
+                    }
+                }
+            }
+        }
+        __syncthreads();
+        for (uint32_t i = threadIdx.x; i < n; i += 256) put_pair<kCells>(tri, cell, s0 + i, key[i]);
+        __syncthreads();
+    }
 }
 
 __global__ void k_iota(uint32_t *__restrict__ v, uint64_t n) {
@@ -324,14 +560,25 @@ __global__ void k_gather_blocks(const uint8_t *__restrict__ flag, uint64_t n, co
 
 // Running centres: acc[l * K + k] = ((l - 0.5) * h) + h + ... (k additions),
 // the value the reference's loop holds at voxel l + k (PlyLoader.cpp:363-368).
-__global__ void k_center_table(int n_l, int K, float h, float *__restrict__ acc) {
-    int l = blockIdx.x * blockDim.x + threadIdx.x;
-    if (l >= n_l) return;
-    float c = ((float)l - 0.5f) * h;
-    float *row = acc + (uint64_t)l * K;
-    for (int k = 0; k < K; ++k) {
-        row[k] = c;
-        c += h;
+// A thread per row and kCenterRows rows a CTA, staged so that the rows go out
+// in whole segments: 1025 rows of 512 additions take 9 us, 36 us with a CTA per
+// 256 rows and each thread storing along its own row.
+constexpr int kCenterRows = 32, kCenterSpan = 32;
+
+__global__ void __launch_bounds__(kCenterRows) k_center_table(int n_l, int K, float h, float *__restrict__ acc) {
+    __shared__ float buf[kCenterRows][kCenterSpan + 1];
+    const int l0 = blockIdx.x * kCenterRows, lane = threadIdx.x;
+    float c = ((float)(l0 + lane) - 0.5f) * h;
+    for (int k0 = 0; k0 < K; k0 += kCenterSpan) {
+#pragma unroll
+        for (int k = 0; k < kCenterSpan; ++k) {
+            buf[lane][k] = c;
+            c += h;
+        }
+        __syncwarp();
+        for (int r = 0; r < kCenterRows && l0 + r < n_l; ++r)
+            if (k0 + lane < K) acc[(uint64_t)(l0 + r) * K + k0 + lane] = buf[r][lane];
+        __syncwarp();
     }
 }
 
@@ -1052,6 +1299,74 @@ struct BlockJob {
     uint32_t morton, first, last;
 };
 
+// SVO_MESH_BLOCK_BUFFER=1 keeps the per-block buffer path (same words)
+bool block_buffer_asked() {
+    const char *env = std::getenv("SVO_MESH_BLOCK_BUFFER");
+    return env && *env && *env != '0';
+}
+
+// PlyLoader::processBlock (PlyLoader.cpp:439-458) of every block at once, then
+// the walk's voxels (VoxelOctree.cpp:66-103) from the slots, and the octree of
+// them.  fa: what every fold launch shares.
+int fold_direct(FoldArgs fa, uint32_t *next, uint32_t nb, const uint8_t *bflag, uint32_t *err, int D, int lb,
+                unsigned fold_grid, unsigned warp_grid, cudaStream_t st, uint32_t **d_words, uint64_t *n_words) {
+    const uint64_t cap = (uint64_t)nb << (3 * fa.log_e);
+    // 8^3 bricks go to the octree as they are, unless a cache block is no
+    // larger than a brick (budgets of a few KB)
+    const bool as_bricks = fa.log_e == 3 && (lb > 3 || lb == D);
+    Dev<uint32_t> slot, ccount, cbits, pay;
+    Dev<uint64_t> coff, dN, sc64, keys;
+    Dev<uint8_t> nmask;
+    Dev<unsigned long long> n_vox;
+    const bool by_key = as_bricks && bricks_dense(D, 3);
+    const uint64_t nodes = by_key ? 1ull << (3 * (D - 3)) : (uint64_t)nb;
+    SVO_ALLOC(slot, cap);
+    SVO_ALLOC(ccount, nodes);
+    SVO_ALLOC(cbits, (uint64_t)nb * 16);
+    fa.b_first = 0;
+    fa.b_last = nb;
+    fa.next = next;
+    fa.slot = slot.p;
+    fa.brick_count = ccount.p;
+    fa.brick_bits = cbits.p;
+    if (as_bricks) {
+        SVO_ALLOC(nmask, nodes);
+        fa.node_words = ccount.p;
+        fa.node_mask = nmask.p;
+        fa.node_by_key = by_key ? 1 : 0;
+        if (by_key) SVO_CUDA_TRY(cudaMemsetAsync(ccount.p, 0, nodes * sizeof(uint32_t), st));
+        if (cap >= 0xFFFFFFFFull) {  // the voxels may exceed the build's limit
+            SVO_ALLOC(n_vox, 1);
+            SVO_CUDA_TRY(cudaMemsetAsync(n_vox.p, 0, sizeof(unsigned long long), st));
+            fa.n_voxels = n_vox.p;
+        }
+    }
+    const unsigned grid = (unsigned)std::min<uint64_t>((nb + kFoldWarps - 1) / kFoldWarps, fold_grid);
+    k_fold_bricks<true><<<grid, kFoldWarps * 32, 0, st>>>(fa);
+    SVO_LAUNCH_OK("k_fold_bricks<direct>");
+    if (as_bricks) {
+        const MeshBricks mb{nb, fa.bkey, ccount.p, nmask.p, cbits.p, slot.p, n_vox.p};
+        return build_from_bricks_device(mb, D, lb, lb < D ? bflag : nullptr, st, d_words, n_words);
+    }
+    SVO_ALLOC(coff, nb);
+    SVO_ALLOC(dN, 1);
+    SVO_ALLOC(sc64, scan_scratch_elems(nb));
+    SVO_ALLOC(keys, cap);
+    SVO_ALLOC(pay, cap);
+    SVO_CUDA_TRY((exclusive_scan<uint32_t, uint64_t>(ccount.p, coff.p, nb, dN.p, sc64.p, st)));
+    k_direct_emit<<<warp_grid, 256, 0, st>>>(nb, fa.log_e, fa.bkey, cbits.p, slot.p, coff.p, cap, keys.p, pay.p, err);
+    SVO_LAUNCH_OK("k_direct_emit");
+    uint64_t N = 0;
+    uint32_t e_h = 0;
+    SVO_CUDA_TRY(cudaMemcpyAsync(&N, dN.p, sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
+    SVO_CUDA_TRY(cudaMemcpyAsync(&e_h, err, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+    SVO_CUDA_TRY(cudaStreamSynchronize(st));
+    if (e_h) return set_error(SVO_ERR_DEVICE, "mesh build: voxel extraction check failed (flags %u)", e_h);
+    slot.release();
+    if (N >= 0xFFFFFFFFull) return set_error(SVO_ERR_LIMIT, "%llu voxels exceed 2^32-1", (unsigned long long)N);
+    return build_from_sorted_device(keys.p, pay.p, N, D, lb, lb < D ? bflag : nullptr, st, d_words, n_words);
+}
+
 }  // namespace
 
 // Mesh dimensions for a side length: PlyLoader::suggestedDimensions
@@ -1188,25 +1503,161 @@ int build_mesh_device(const svo_mesh *m, int side, int threads, uint64_t mem, cu
         return set_error(SVO_ERR_LIMIT, "voxel-centre table of %d x %d entries is too large", n_l, K);
 
     const uint64_t nt = m->n_tris;
-    Dev<uint32_t> err;
-    SVO_ALLOC(err, 1);
-    SVO_CUDA_TRY(cudaMemsetAsync(err.p, 0, sizeof(uint32_t), st));
-    Dev<uint8_t> bflag;
-    SVO_ALLOC(bflag, g.n_blocks);
-    SVO_CUDA_TRY(cudaMemsetAsync(bflag.p, 0, g.n_blocks, st));
+    // what the host reads after the count (totals of the table of bricks, the
+    // largest, the error word), then the block flags
+    Dev<uint64_t> info;
+    SVO_ALLOC(info, 2 + (g.n_blocks + 7) / 8);
+    SVO_CUDA_TRY(cudaMemsetAsync(info.p, 0, 16 + g.n_blocks, st));
+    uint32_t *const largest = (uint32_t *)info.p + 2, *const err = (uint32_t *)info.p + 3;
+    uint8_t *const bflag = (uint8_t *)(info.p + 2);
 
-    // 2. pairs: count, offsets, emit (triangle-major order)
+    // the running centres, first: they depend on the size alone
+    Dev<float> acc;
+    SVO_ALLOC(acc, (uint64_t)n_l * K);
+    const float hx = 1.0f / (float)(side - 4);
+    k_center_table<<<(unsigned)((n_l + kCenterRows - 1) / kCenterRows), kCenterRows, 0, st>>>(n_l, K, hx, acc.p);
+    SVO_LAUNCH_OK("k_center_table");
+
+    // sub-block edges are multiples of the brick edge: a brick lies in one sub-block
+    bool sub_bricks = true;
+    for (int k = 0; k < 3; ++k)
+        if (sub[k] % (1 << g.log_e) != 0) sub_bricks = false;
+
+    // whether the bricks of these blocks, in this order, can all be folded at
+    // once, without the buffer: the direct fold, below
+    auto direct_blocks = [&](const std::vector<BlockJob> &blocks) {
+        std::vector<std::pair<uint64_t, uint64_t>> gs;  // flat ranges of the dropped slices so far
+        for (const BlockJob &j : blocks) {
+            int o[3] = {(int)(compact3(j.morton) << lb), (int)(compact3((uint64_t)j.morton >> 1) << lb),
+                        (int)(compact3((uint64_t)j.morton >> 2) << lb)};
+            int bb[3];
+            bool inside = true;
+            for (int k = 0; k < 3; ++k) {
+                bb[k] = std::min(B, dims[k] - o[k]);
+                if (bb[k] <= 0) inside = false;
+            }
+            if (!inside) continue;
+            const uint64_t vol = (uint64_t)bb[0] * bb[1] * bb[2];
+            for (const auto &r : gs)
+                if (std::min(r.second, vol) > r.first) return false;
+            if ((bb[2] & 1) && lb >= 2) {
+                const uint64_t plane = (uint64_t)bb[0] * bb[1];
+                gs.emplace_back(plane * (uint64_t)(bb[2] - 1), plane * (uint64_t)bb[2]);
+            }
+        }
+        return true;
+    };
+    // 2. pairs: count per triangle, and per brick where all brick codes fit a
+    // table.  That path wants 8^3 bricks (sub-blocks are halved cache blocks,
+    // so a brick's block is one that its pairs mark), the direct fold whichever
+    // blocks are marked, and no brick count that could wrap (a triangle meets
+    // a brick in at most 8^3 sub-blocks).
+    bool table = !volume && nt > 0 && g.log_e == 3 && (lb > 3 || lb == D) && bricks_dense(D, 3) &&
+                 nt < (sub_bricks ? 1ull << 32 : 1ull << 23) && g.n_blocks <= 4096 && !block_buffer_asked();
+    if (table) {
+        std::vector<BlockJob> all((size_t)g.n_blocks);
+        for (size_t k = 0; k < all.size(); ++k) all[k] = {(uint32_t)k, 0, 0};
+        table = direct_blocks(all);
+    }
+    const uint64_t brick_cells = table ? 1ull << (3 * (D - 3)) : 0, brick_tiles = (brick_cells + kBrickTile - 1) / kBrickTile;
     Dev<int32_t> box;
-    Dev<uint32_t> pcount;
-    Dev<uint64_t> poff;
+    Dev<uint32_t> pcount, brick_n, bkey, bstart;
+    Dev<uint64_t> poff, tiles;
     SVO_ALLOC(box, nt * 6);
     SVO_ALLOC(pcount, nt);
-    SVO_ALLOC(poff, nt);
+    if (table) {
+        SVO_ALLOC(brick_n, brick_cells);
+        SVO_ALLOC(tiles, brick_tiles);
+        SVO_ALLOC(bkey, brick_cells);
+        SVO_ALLOC(bstart, brick_cells + 1);
+        SVO_CUDA_TRY(cudaMemsetAsync(brick_n.p, 0, brick_cells * sizeof(uint32_t), st));
+    }
+    int dev = 0, sms = 0;
+    SVO_CUDA_TRY(cudaGetDevice(&dev));
+    SVO_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    // triangles a warp of k_tri_pairs takes: fewer where 32 would leave SMs
+    // idle (1,280 large triangles at 1024^3: 1.6 ms, 2.0 ms with 32 a warp)
+    int per_warp = 32;
+    while (per_warp > 1 && nt / (uint64_t)per_warp < (uint64_t)sms * 16) per_warp /= 2;
+    const unsigned pair_grid = (unsigned)((nt + 4 * per_warp - 1) / (4 * per_warp));
+    if (nt) {
+        k_tri_pairs<0><<<pair_grid, 128, 0, st>>>(nt, per_warp, m->d_tris, g, box.p, bflag, pcount.p, nullptr, nullptr,
+                                                          nullptr, nullptr, brick_n.p, err);
+        SVO_LAUNCH_OK("k_tri_pairs<count>");
+    }
+    const unsigned fold_grid = (unsigned)(sms * kFoldCtas), warp_grid = (unsigned)sms * 16;
+    const uint32_t brick_mask = g.slab_mode ? (uint32_t)((1ull << g.brick_bits) - 1) : 0xFFFFFFFFu;
+    // what every fold launch shares
+    auto fold_args = [&](const uint32_t *pair_tri, const uint32_t *pair_cell) -> FoldArgs {
+        FoldArgs fa{};
+        for (int k = 0; k < 3; ++k) {
+            fa.sub[k] = sub[k];
+            fa.grid[k] = g.grid[k];
+            fa.dims[k] = dims[k];
+        }
+        fa.tris = m->d_tris;
+        fa.box = box.p;
+        fa.pair_tri = pair_tri;
+        fa.pair_cell = pair_cell;
+        fa.bkey = bkey.p;
+        fa.bstart = bstart.p;
+        fa.log_e = g.log_e;
+        fa.log_block = lb;
+        fa.acc = acc.p;
+        fa.K = K;
+        fa.half = 0.5f * hx;
+        fa.brick_mask = brick_mask;
+        fa.drop_z = -1;
+        fa.sub_bricks = sub_bricks ? 1 : 0;
+        return fa;
+    };
+    // the direct fold's scratch (a slot of E^3 words per brick, besides the keys and words
+    // both paths hold) must fit comfortably
+    auto direct_fits = [&](uint64_t bricks) {
+        size_t free_b = 0, total_b = 0;
+        return cudaMemGetInfo(&free_b, &total_b) != cudaSuccess ||
+               bricks * (1ull << (3 * g.log_e)) * 16ull <= (uint64_t)free_b / 2;
+    };
+    Dev<uint32_t> fold_next;  // one work counter per fold launch
+
+    if (table) {
+        k_brick_tiles<<<(unsigned)brick_tiles, 256, 0, st>>>(brick_n.p, brick_cells, tiles.p, largest);
+        k_brick_layout<<<(unsigned)brick_tiles, 256, 0, st>>>(brick_n.p, brick_cells, tiles.p, bkey.p, bstart.p, info.p);
+        SVO_LAUNCH_OK("k_brick_layout");
+        uint64_t h[2];
+        SVO_CUDA_TRY(cudaMemcpyAsync(h, info.p, sizeof h, cudaMemcpyDeviceToHost, st));
+        SVO_CUDA_TRY(cudaStreamSynchronize(st));
+        const uint32_t nb = (uint32_t)(h[0] >> 40), h_largest = (uint32_t)h[1], h_err = (uint32_t)(h[1] >> 32);
+        const uint64_t pairs = h[0] & ((1ull << 40) - 1);
+        if (h_err) return set_error(SVO_ERR_DEVICE, "mesh build: sub-block lists out of range (flags %u)", h_err);
+        if (nb > 0 && h_largest <= (uint32_t)kSortedInBrick && pairs < 0xFFFFFFFFull && direct_fits(nb)) {
+            Dev<uint32_t> ptri, pcell;
+            SVO_ALLOC(ptri, pairs);
+            if (!sub_bricks) SVO_ALLOC(pcell, pairs);
+            k_tri_pairs<2><<<pair_grid, 128, 0, st>>>(nt, per_warp, m->d_tris, g, box.p, bflag, nullptr, nullptr, nullptr,
+                                                              ptri.p, pcell.p, brick_n.p, err);
+            SVO_LAUNCH_OK("k_tri_pairs<emit>");
+            auto sort_bricks = [&](auto cells) {
+                constexpr bool kCells = decltype(cells)::value;
+                k_sort_bricks<kCells><<<(nb + kBrickSortWarps - 1) / kBrickSortWarps, kBrickSortWarps * 32, 0, st>>>(
+                    nb, bstart.p, ptri.p, pcell.p);
+                if (h_largest > (uint32_t)kWarpSort)
+                    k_sort_large<kCells><<<std::min<uint32_t>(nb, (uint32_t)sms * 4), 256, 0, st>>>(nb, bstart.p, ptri.p,
+                                                                                                  pcell.p);
+            };
+            if (sub_bricks) sort_bricks(std::false_type());
+            else sort_bricks(std::true_type());
+            SVO_LAUNCH_OK("k_sort_bricks");
+            SVO_ALLOC(fold_next, 1);
+            SVO_CUDA_TRY(cudaMemsetAsync(fold_next.p, 0, sizeof(uint32_t), st));
+            return fold_direct(fold_args(ptri.p, pcell.p), fold_next.p, nb, bflag, err, D, lb, fold_grid, warp_grid, st,
+                               d_words, n_words);
+        }
+    }
+
     uint64_t n_pairs = 0;
     if (nt) {
-        k_tri_pairs<0><<<grid_for(nt, 128), 128, 0, st>>>(nt, m->d_tris, g, box.p, bflag.p, pcount.p, nullptr,
-                                                          nullptr, nullptr, nullptr, err.p);
-        SVO_LAUNCH_OK("k_tri_pairs<count>");
+        SVO_ALLOC(poff, nt);
         int rc = scan_total<uint32_t, uint64_t>(pcount.p, poff.p, nt, &n_pairs, st);
         if (rc) return rc;
     }
@@ -1220,8 +1671,8 @@ int build_mesh_device(const svo_mesh *m, int side, int threads, uint64_t mem, cu
     SVO_ALLOC(pk2, n_pairs);
     SVO_ALLOC(pi2, n_pairs);
     if (n_pairs) {
-        k_tri_pairs<1><<<grid_for(nt, 128), 128, 0, st>>>(nt, m->d_tris, g, box.p, bflag.p, pcount.p, poff.p, pk.p,
-                                                          pt.p, pc.p, err.p);
+        k_tri_pairs<1><<<pair_grid, 128, 0, st>>>(nt, per_warp, m->d_tris, g, box.p, bflag, pcount.p, poff.p, pk.p,
+                                                          pt.p, pc.p, nullptr, err);
         SVO_LAUNCH_OK("k_tri_pairs<emit>");
         k_iota<<<grid_for(n_pairs), 256, 0, st>>>(pi.p, n_pairs);
         SVO_LAUNCH_OK("k_iota");
@@ -1246,7 +1697,7 @@ int build_mesh_device(const svo_mesh *m, int side, int threads, uint64_t mem, cu
     const uint32_t *scell = scell_buf.p;
 
     // unique bricks and per-block brick ranges
-    Dev<uint32_t> head, hidx, bkey, bstart, rfirst, rlast;
+    Dev<uint32_t> head, hidx, rfirst, rlast;
     SVO_ALLOC(head, n_pairs);
     SVO_ALLOC(hidx, n_pairs);
     uint32_t nb = 0;
@@ -1256,6 +1707,9 @@ int build_mesh_device(const svo_mesh *m, int side, int threads, uint64_t mem, cu
         int rc = scan_total<uint32_t, uint32_t>(head.p, hidx.p, n_pairs, &nb, st);
         if (rc) return rc;
     }
+    bkey.release();
+    bstart.release();
+    brick_n.release();
     SVO_ALLOC(bkey, nb);
     SVO_ALLOC(bstart, (uint64_t)nb + 1);
     SVO_ALLOC(rfirst, g.n_blocks);
@@ -1269,7 +1723,7 @@ int build_mesh_device(const svo_mesh *m, int side, int threads, uint64_t mem, cu
     if (nb) {
         k_brick_table<<<grid_for(n_pairs), 256, 0, st>>>(skey, n_pairs, head.p, hidx.p, bkey.p, bstart.p);
         k_block_ranges<<<grid_for(nb), 256, 0, st>>>(bkey.p, nb, 3 * (lb - g.log_e), g.n_blocks, rfirst.p, rlast.p,
-                                                    err.p);
+                                                    err);
         SVO_LAUNCH_OK("k_block_ranges");
     }
     head.release();
@@ -1281,14 +1735,14 @@ int build_mesh_device(const svo_mesh *m, int side, int threads, uint64_t mem, cu
         Dev<uint32_t> f32, fidx, packed;
         SVO_ALLOC(f32, g.n_blocks);
         SVO_ALLOC(fidx, g.n_blocks);
-        k_flag_to_u32<<<grid_for(g.n_blocks), 256, 0, st>>>(bflag.p, g.n_blocks, f32.p);
+        k_flag_to_u32<<<grid_for(g.n_blocks), 256, 0, st>>>(bflag, g.n_blocks, f32.p);
         SVO_LAUNCH_OK("k_flag_to_u32");
         uint32_t n_jobs = 0;
         int rc = scan_total<uint32_t, uint32_t>(f32.p, fidx.p, g.n_blocks, &n_jobs, st);
         if (rc) return rc;
         SVO_ALLOC(packed, (uint64_t)n_jobs * 3);
         if (n_jobs) {
-            k_gather_blocks<<<grid_for(g.n_blocks), 256, 0, st>>>(bflag.p, g.n_blocks, fidx.p, rfirst.p, rlast.p,
+            k_gather_blocks<<<grid_for(g.n_blocks), 256, 0, st>>>(bflag, g.n_blocks, fidx.p, rfirst.p, rlast.p,
                                                                  packed.p);
             SVO_LAUNCH_OK("k_gather_blocks");
         }
@@ -1297,7 +1751,7 @@ int build_mesh_device(const svo_mesh *m, int side, int threads, uint64_t mem, cu
             SVO_CUDA_TRY(cudaMemcpyAsync(jobs.data(), packed.p, (size_t)n_jobs * 3 * sizeof(uint32_t),
                                          cudaMemcpyDeviceToHost, st));
         uint32_t e_h = 0;
-        SVO_CUDA_TRY(cudaMemcpyAsync(&e_h, err.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+        SVO_CUDA_TRY(cudaMemcpyAsync(&e_h, err, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
         SVO_CUDA_TRY(cudaStreamSynchronize(st));
         if (e_h) return set_error(SVO_ERR_DEVICE, "mesh build: sub-block lists out of range (flags %u)", e_h);
     }
@@ -1312,42 +1766,16 @@ int build_mesh_device(const svo_mesh *m, int side, int threads, uint64_t mem, cu
     // and one scan places them.  Bricks are sorted by key and blocks are
     // visited in Morton order, so the bricks of consecutive blocks follow
     // one another and the result is in Morton order.
-    bool direct = !volume && nb > 0;
-    if (direct) {
+    bool direct = !volume && nb > 0 && !block_buffer_asked() && direct_blocks(jobs) && direct_fits(nb);
+    {
         uint32_t next = 0;
-        std::vector<std::pair<uint64_t, uint64_t>> gs;  // flat ranges of the dropped slices so far
         for (const BlockJob &j : jobs) {
             if (j.last > j.first) {
                 if (j.first != next) direct = false;
                 next = j.last;
             }
-            int o[3] = {(int)(compact3(j.morton) << lb), (int)(compact3((uint64_t)j.morton >> 1) << lb),
-                        (int)(compact3((uint64_t)j.morton >> 2) << lb)};
-            int bb[3];
-            bool inside = true;
-            for (int k = 0; k < 3; ++k) {
-                bb[k] = std::min(B, dims[k] - o[k]);
-                if (bb[k] <= 0) inside = false;
-            }
-            if (!inside) continue;
-            const uint64_t vol = (uint64_t)bb[0] * bb[1] * bb[2];
-            for (const auto &r : gs)
-                if (std::min(r.second, vol) > r.first) direct = false;
-            if ((bb[2] & 1) && lb >= 2) {
-                const uint64_t plane = (uint64_t)bb[0] * bb[1];
-                gs.emplace_back(plane * (uint64_t)(bb[2] - 1), plane * (uint64_t)bb[2]);
-            }
         }
         if (next != nb) direct = false;
-        // the direct fold's scratch (a slot of E^3 words per brick, besides
-        // the keys and words both paths hold) must fit comfortably
-        size_t free_b = 0, total_b = 0;
-        if (direct && cudaMemGetInfo(&free_b, &total_b) == cudaSuccess &&
-            (uint64_t)nb * (1ull << (3 * g.log_e)) * 16ull > (uint64_t)free_b / 2)
-            direct = false;
-        // SVO_MESH_BLOCK_BUFFER=1 keeps the per-block buffer path (same words)
-        const char *env = std::getenv("SVO_MESH_BLOCK_BUFFER");
-        if (env && *env && *env != '0') direct = false;
     }
 
     // the persistent block buffer (VoxelData::_bufferedData, zeroed) and the
@@ -1364,7 +1792,6 @@ int build_mesh_device(const svo_mesh *m, int side, int threads, uint64_t mem, cu
     }
     Dev<uint32_t> data;
     Dev<uint8_t> counts;
-    Dev<float> acc;
     // the conversion folds every slab in place in its output (region 0 zeroed here)
     if (!volume && !direct) SVO_ALLOC(data, buf_cells);
     uint32_t *const data_p = volume ? d_volume : data.p;
@@ -1373,110 +1800,14 @@ int build_mesh_device(const svo_mesh *m, int side, int threads, uint64_t mem, cu
         SVO_CUDA_TRY(cudaMemsetAsync(data_p, 0, buf_cells * sizeof(uint32_t), st));
         SVO_CUDA_TRY(cudaMemsetAsync(counts.p, 0, buf_cells, st));
     }
-    SVO_ALLOC(acc, (uint64_t)n_l * K);
-    const float hx = 1.0f / (float)(side - 4);
-    k_center_table<<<grid_for(n_l), 256, 0, st>>>(n_l, K, hx, acc.p);
-    SVO_LAUNCH_OK("k_center_table");
 
-    int dev = 0, sms = 0;
-    SVO_CUDA_TRY(cudaGetDevice(&dev));
-    SVO_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    const unsigned fold_grid = (unsigned)(sms * kFoldCtas), warp_grid = (unsigned)sms * 16;
-    Dev<uint32_t> fold_next;  // one work counter per fold launch
     const size_t n_next = std::max<size_t>(jobs.size(), 1);
     SVO_ALLOC(fold_next, n_next);
     SVO_CUDA_TRY(cudaMemsetAsync(fold_next.p, 0, n_next * sizeof(uint32_t), st));
-    const uint32_t brick_mask = g.slab_mode ? (uint32_t)((1ull << g.brick_bits) - 1) : 0xFFFFFFFFu;
-    // what every fold launch shares
-    auto fold_args = [&]() -> FoldArgs {
-        FoldArgs fa{};
-        for (int k = 0; k < 3; ++k) {
-            fa.sub[k] = sub[k];
-            fa.grid[k] = g.grid[k];
-            fa.dims[k] = dims[k];
-        }
-        fa.tris = m->d_tris;
-        fa.box = box.p;
-        fa.pair_tri = stri;
-        fa.pair_cell = scell;
-        fa.bkey = bkey.p;
-        fa.bstart = bstart.p;
-        fa.log_e = g.log_e;
-        fa.log_block = lb;
-        fa.acc = acc.p;
-        fa.K = K;
-        fa.half = 0.5f * hx;
-        fa.brick_mask = brick_mask;
-        fa.drop_z = -1;
-        fa.sub_bricks = 1;
-        for (int k = 0; k < 3; ++k)
-            if (sub[k] % (1 << g.log_e) != 0) fa.sub_bricks = 0;
-        return fa;
-    };
 
-    if (direct) {
-        // PlyLoader::processBlock (PlyLoader.cpp:439-458) of every block at
-        // once, then the walk's voxels (VoxelOctree.cpp:66-103) from the slots
-        const uint32_t E3 = 1u << (3 * g.log_e);
-        const uint64_t cap = (uint64_t)nb * E3;
-        // 8^3 bricks go to the octree as they are, unless a cache block is no
-        // larger than a brick (budgets of a few KB)
-        const bool as_bricks = g.log_e == 3 && (lb > 3 || lb == D);
-        Dev<uint32_t> slot, ccount, cbits, pay;
-        Dev<uint64_t> coff, dN, sc64, keys;
-        Dev<uint8_t> nmask;
-        Dev<unsigned long long> n_vox;
-        const bool by_key = as_bricks && bricks_dense(D, 3);
-        const uint64_t nodes = by_key ? 1ull << (3 * (D - 3)) : (uint64_t)nb;
-        SVO_ALLOC(slot, cap);
-        SVO_ALLOC(ccount, nodes);
-        SVO_ALLOC(cbits, (uint64_t)nb * 16);
-        FoldArgs fa = fold_args();
-        fa.b_first = 0;
-        fa.b_last = nb;
-        fa.next = fold_next.p;
-        fa.slot = slot.p;
-        fa.brick_count = ccount.p;
-        fa.brick_bits = cbits.p;
-        if (as_bricks) {
-            SVO_ALLOC(nmask, nodes);
-            fa.node_words = ccount.p;
-            fa.node_mask = nmask.p;
-            fa.node_by_key = by_key ? 1 : 0;
-            if (by_key) SVO_CUDA_TRY(cudaMemsetAsync(ccount.p, 0, nodes * sizeof(uint32_t), st));
-            if (cap >= 0xFFFFFFFFull) {  // the voxels may exceed the build's limit
-                SVO_ALLOC(n_vox, 1);
-                SVO_CUDA_TRY(cudaMemsetAsync(n_vox.p, 0, sizeof(unsigned long long), st));
-                fa.n_voxels = n_vox.p;
-            }
-        }
-        const unsigned grid = (unsigned)std::min<uint64_t>((nb + kFoldWarps - 1) / kFoldWarps, fold_grid);
-        k_fold_bricks<true><<<grid, kFoldWarps * 32, 0, st>>>(fa);
-        SVO_LAUNCH_OK("k_fold_bricks<direct>");
-        if (as_bricks) {
-            const MeshBricks mb{nb, bkey.p, ccount.p, nmask.p, cbits.p, slot.p, n_vox.p};
-            return build_from_bricks_device(mb, D, lb, lb < D ? bflag.p : nullptr, st, d_words, n_words);
-        }
-        SVO_ALLOC(coff, nb);
-        SVO_ALLOC(dN, 1);
-        SVO_ALLOC(sc64, scan_scratch_elems(nb));
-        SVO_ALLOC(keys, cap);
-        SVO_ALLOC(pay, cap);
-        SVO_CUDA_TRY((exclusive_scan<uint32_t, uint64_t>(ccount.p, coff.p, nb, dN.p, sc64.p, st)));
-        k_direct_emit<<<warp_grid, 256, 0, st>>>(nb, g.log_e, bkey.p, cbits.p, slot.p, coff.p, cap, keys.p, pay.p,
-                                                err.p);
-        SVO_LAUNCH_OK("k_direct_emit");
-        uint64_t N = 0;
-        uint32_t e_h = 0;
-        SVO_CUDA_TRY(cudaMemcpyAsync(&N, dN.p, sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
-        SVO_CUDA_TRY(cudaMemcpyAsync(&e_h, err.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-        SVO_CUDA_TRY(cudaStreamSynchronize(st));
-        if (e_h) return set_error(SVO_ERR_DEVICE, "mesh build: voxel extraction check failed (flags %u)", e_h);
-        slot.release();
-        acc.release();
-        if (N >= 0xFFFFFFFFull) return set_error(SVO_ERR_LIMIT, "%llu voxels exceed 2^32-1", (unsigned long long)N);
-        return build_from_sorted_device(keys.p, pay.p, N, D, lb, lb < D ? bflag.p : nullptr, st, d_words, n_words);
-    }
+    if (direct)
+        return fold_direct(fold_args(stri, scell), fold_next.p, nb, bflag, err, D, lb, fold_grid, warp_grid, st, d_words,
+                           n_words);
 
     // PlyLoader::processBlock (PlyLoader.cpp:439-458) of job ji, whose buffer
     // `data` starts at org with edges buf: its bricks' pairs folded into it
@@ -1485,7 +1816,7 @@ int build_mesh_device(const svo_mesh *m, int side, int threads, uint64_t mem, cu
                           int drop_z) -> int {
         const BlockJob &j = jobs[ji];
         if (j.last <= j.first) return SVO_OK;
-        FoldArgs fa = fold_args();
+        FoldArgs fa = fold_args(stri, scell);
         for (int k = 0; k < 3; ++k) {
             fa.org[k] = org[k];
             fa.buf[k] = buf[k];
@@ -1532,7 +1863,7 @@ int build_mesh_device(const svo_mesh *m, int side, int threads, uint64_t mem, cu
             }
         }
         uint32_t e_v = 0;
-        SVO_CUDA_TRY(cudaMemcpyAsync(&e_v, err.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+        SVO_CUDA_TRY(cudaMemcpyAsync(&e_v, err, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
         SVO_CUDA_TRY(cudaStreamSynchronize(st));
         if (e_v) return set_error(SVO_ERR_DEVICE, "mesh conversion check failed (flags %u)", e_v);
         if (ji != jobs.size()) return set_error(SVO_ERR_DEVICE, "mesh conversion: slab jobs out of order");
@@ -1617,7 +1948,7 @@ int build_mesh_device(const svo_mesh *m, int side, int threads, uint64_t mem, cu
             SVO_LAUNCH_OK("k_ghost_count");
         }
         SVO_CUDA_TRY((exclusive_scan<uint32_t, uint64_t>(ccount.p, coff.p, n_e, bn.p, sc64.p, st)));
-        k_cand_emit<<<warp_grid, 256, 0, st>>>(ea, cbits.p, ccount.p, coff.p, dN.p, cap, keys.p, pay.p, err.p);
+        k_cand_emit<<<warp_grid, 256, 0, st>>>(ea, cbits.p, ccount.p, coff.p, dN.p, cap, keys.p, pay.p, err);
         SVO_LAUNCH_OK("k_cand_emit");
         k_add_u64<<<1, 1, 0, st>>>(dN.p, bn.p);
         if (drop) {  // the walk never reads this slice; it stays in the buffer
@@ -1629,7 +1960,7 @@ int build_mesh_device(const svo_mesh *m, int side, int threads, uint64_t mem, cu
     uint64_t N = 0;
     uint32_t e_h = 0;
     SVO_CUDA_TRY(cudaMemcpyAsync(&N, dN.p, sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
-    SVO_CUDA_TRY(cudaMemcpyAsync(&e_h, err.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+    SVO_CUDA_TRY(cudaMemcpyAsync(&e_h, err, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     SVO_CUDA_TRY(cudaStreamSynchronize(st));
     if (e_h) return set_error(SVO_ERR_DEVICE, "mesh build: voxel extraction check failed (flags %u)", e_h);
     data.release();
@@ -1638,7 +1969,7 @@ int build_mesh_device(const svo_mesh *m, int side, int threads, uint64_t mem, cu
     if (N >= 0xFFFFFFFFull) return set_error(SVO_ERR_LIMIT, "%llu voxels exceed 2^32-1", (unsigned long long)N);
 
     // 5. octree from the (already Morton-ordered) voxels
-    return build_from_sorted_device(keys.p, pay.p, N, D, lb, lb < D ? bflag.p : nullptr, st, d_words, n_words);
+    return build_from_sorted_device(keys.p, pay.p, N, D, lb, lb < D ? bflag : nullptr, st, d_words, n_words);
 }
 
 }  // namespace svo

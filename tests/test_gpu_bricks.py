@@ -60,3 +60,34 @@ def test_mesh_builds(svo, oracle, scenes, side, thin, threads, mem):
     ow, oc = oracle.build_mesh(pos, faces, side, threads, mem, colors=col)
     assert np.array_equal(tree.words(), ow)
     assert np.array_equal(tree.center(), oc)
+
+
+def _fan(n, rng):
+    """n small triangles in one corner of the unit cube, and one across it."""
+    at = rng.uniform(0.1, 0.104, (n, 1, 3))
+    pos = np.concatenate([(at + rng.uniform(-0.004, 0.004, (n, 3, 3))).reshape(-1, 3),
+                          [[0.0, 0.0, 0.0], [1.0, 0.2, 0.9], [0.9, 1.0, 0.1]]]).astype(np.float32)
+    return pos, np.arange(3 * (n + 1), dtype=np.int32).reshape(-1, 3)
+
+
+@pytest.mark.parametrize("side,n,threads,mem", [
+    (64, 40, 4, 1 << 30), (64, 480, 4, 1 << 30),    # one brick holds tens, hundreds of triangles
+    (64, 900, 4, 1 << 30), (64, 4000, 4, 1 << 30),  # thousands, a CTA's sort
+    (64, 4600, 4, 1 << 30),                         # and more than that sorts
+    (16, 30, 512, 1 << 30), (40, 60, 4096, 1 << 30),  # sub-blocks inside a brick: several pairs of one triangle
+    (40, 60, 512, 5 * 16 ** 3 + 3000),              # and several cache blocks
+    (1027, 50, 8, 1 << 30),                         # beyond the table of brick codes
+])
+def test_mesh_pairs_by_brick(svo, oracle, monkeypatch, side, n, threads, mem):
+    """Pairs laid out through the table of brick codes, and sorted: the words
+    of the block-after-block fold, and of the oracle."""
+    rng = np.random.default_rng(side + n)
+    pos, faces = _fan(n, rng)
+    col = rng.uniform(0, 1, pos.shape).astype(np.float32)
+    got = svo.VoxelOctree(svo.VoxelData(svo.PlyLoader.from_arrays(pos, faces, colors=col), side, mem, threads)).words()
+    monkeypatch.setenv("SVO_MESH_BLOCK_BUFFER", "1")
+    want = svo.VoxelOctree(svo.VoxelData(svo.PlyLoader.from_arrays(pos, faces, colors=col), side, mem, threads)).words()
+    assert np.array_equal(got, want)
+    if side <= 64:
+        ow, _ = oracle.build_mesh(pos, faces, side, threads, mem, colors=col)
+        assert np.array_equal(got, ow)
