@@ -39,6 +39,7 @@
 #include <mutex>
 
 #include "brick.cuh"
+#include "chain.cuh"
 #include "morton.cuh"
 #include "scan.cuh"
 #include "svo_internal.h"
@@ -271,6 +272,7 @@ __global__ void __launch_bounds__(kBrickThreads, 6) k_brick_bits(GridGeom g, uin
                                                                  uint32_t *__restrict__ list,
                                                                  uint32_t *__restrict__ n_list,
                                                                  unsigned long long *__restrict__ n_voxels) {
+    chain_begin();
     __shared__ __align__(16) uint32_t sbits[2][128];  // alternating: warp 0 may still read the brick before
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -461,6 +463,7 @@ __global__ void __launch_bounds__(kBrickThreads) k_place_brick16(GridGeom g, Bri
                                                                  const uint32_t *__restrict__ bits,
                                                                  uint32_t *__restrict__ words, uint64_t W,
                                                                  uint32_t *__restrict__ err) {
+    chain_begin();
     __shared__ __align__(16) uint32_t tile[16 * 16 * 16];  // a whole brick's words by Morton code
     __shared__ __align__(16) uint32_t sb[128];
     __shared__ uint16_t cell_at[128];  // per 32-cell word: where its cells go
@@ -599,6 +602,7 @@ __global__ void __launch_bounds__(256) k_place_brick8(BrickPlaces at_of, uint64_
                                                       const uint32_t *__restrict__ bits,
                                                       const uint32_t *__restrict__ slot, uint32_t *__restrict__ words,
                                                       uint64_t W, uint32_t *__restrict__ err) {
+    chain_begin();
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const uint32_t lt = (1u << lane) - 1u;
@@ -1333,11 +1337,13 @@ __device__ __forceinline__ void pyramid_place(const Pyramid &p, int level, uint3
 }
 
 __global__ void __launch_bounds__(256) k_pyramid_up(Pyramid p, int level) {
+    chain_begin();
     const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c < pyramid_cells(p, level)) pyramid_node(p, level, c);
 }
 
 __global__ void __launch_bounds__(512) k_pyramid_top_up(Pyramid p, int level) {
+    chain_begin();
     for (; level <= p.top; ++level) {
         for (uint32_t c = threadIdx.x; c < pyramid_cells(p, level); c += blockDim.x) pyramid_node(p, level, c);
         __syncthreads();
@@ -1346,12 +1352,14 @@ __global__ void __launch_bounds__(512) k_pyramid_top_up(Pyramid p, int level) {
 
 __global__ void __launch_bounds__(256) k_pyramid_down(Pyramid p, int level, uint32_t *__restrict__ words, uint64_t W,
                                                       uint32_t *__restrict__ err) {
+    chain_begin();
     pyramid_place(p, level, blockIdx.x * blockDim.x + threadIdx.x, words, W, err);
 }
 
 // The root and every level down to `level`.  Zeroes *err.
 __global__ void __launch_bounds__(kTopPlaced) k_pyramid_top_down(Pyramid p, int level, uint32_t *__restrict__ words,
                                                            uint64_t W, uint32_t *__restrict__ err) {
+    chain_begin();
     const int t = p.top - p.base;
     if (threadIdx.x == 0) {
         *err = 0;
@@ -1753,12 +1761,10 @@ static int build_pyramid(int base, int D, const uint32_t *words_of, const uint8_
     int e = base + 1;
     for (; e <= D && (1ull << (3 * (D - e + 1))) > kTopCells; ++e) {
         const uint64_t cells = 1ull << (3 * (D - e));
-        k_pyramid_up<<<blocks_for(cells), 256, 0, st>>>(p, e);
-        SVO_LAUNCH_CHECK("k_pyramid_up");
+        SVO_CUDA_TRY(launch_chained(k_pyramid_up, blocks_for(cells), 256, st, p, e));
     }
     if (e <= D) {
-        k_pyramid_top_up<<<1, 512, 0, st>>>(p, e);
-        SVO_LAUNCH_CHECK("k_pyramid_top_up");
+        SVO_CUDA_TRY(launch_chained(k_pyramid_top_up, 1, 512, st, p, e));
     }
     uint64_t S_root = 0;
     unsigned long long voxels = 0;
@@ -1782,8 +1788,7 @@ static int build_pyramid(int base, int D, const uint32_t *words_of, const uint8_
         k_pyramid_top_down<<<1, (unsigned)kTopPlaced, 0, st>>>(p, c, words, W, err.p);
         SVO_LAUNCH_CHECK("k_pyramid_top_down");
         for (--c; c >= base; --c) {
-            k_pyramid_down<<<blocks_for(1ull << (3 * (D - c))), 256, 0, st>>>(p, c, words, W, err.p);
-            SVO_LAUNCH_CHECK("k_pyramid_down");
+            SVO_CUDA_TRY(launch_chained(k_pyramid_down, blocks_for(1ull << (3 * (D - c))), 256, st, p, c, words, W, err.p));
         }
         BrickPlaces places{};
         places.words_of = words_of;
@@ -1815,8 +1820,7 @@ int build_from_bricks_device(const MeshBricks &m, int log_side, int log_block, c
     if (bricks_dense(D, kBase)) {
         auto bricks = [&](BrickPlaces places, uint32_t *words, uint64_t W, uint32_t *err) -> int {
             places.src = m.key;
-            k_place_brick8<true><<<grid, 256, 0, st>>>(places, m.n, m.bits, m.slot, words, W, err);
-            SVO_LAUNCH_CHECK("k_place_brick8");
+            SVO_CUDA_TRY(launch_chained(k_place_brick8<true>, grid, 256, st, places, m.n, m.bits, m.slot, words, W, err));
             return SVO_OK;
         };
         return build_pyramid(kBase, D, m.words, m.mask, nullptr, log_block, d_topflag, arena, st, m.n_voxels, bricks,
@@ -1878,8 +1882,7 @@ static int build_dense_bricks(const GridGeom &g, int D, uint64_t n_bricks, cudaS
         auto bricks = [&](BrickPlaces places, uint32_t *words, uint64_t W, uint32_t *err) -> int {
             places.n = n_list.p;
             places.src = list.p;
-            k_place_brick16<true><<<pgrid, kBrickThreads, 0, st>>>(g, places, bits.p, words, W, err);
-            SVO_LAUNCH_CHECK("k_place_brick16");
+            SVO_CUDA_TRY(launch_chained(k_place_brick16<true>, pgrid, kBrickThreads, st, g, places, bits.p, words, W, err));
             return SVO_OK;
         };
         return build_pyramid(kBase, D, words_of.p, mask_of.p, any_of.p, log_block, topflag, arena, st, n_voxels.p,

@@ -78,10 +78,11 @@ int cache_block_log2(int w, int h, int d, uint64_t mem, uint64_t cell_cost) {
 }  // namespace svo
 namespace svo {
 
-int make_handle(uint32_t *d_words, uint64_t n_words, const float center[3], svo_octree **out) {
+int make_handle(uint32_t *d_words, uint64_t n_words, const float center[3], svo_octree **out, int levels) {
     std::unique_ptr<svo_octree> h(new svo_octree());
     h->d_words = d_words;
     h->n_words = n_words;
+    h->levels = levels;
     std::memcpy(h->center, center, sizeof(h->center));
     cudaGetDevice(&h->device);
     h->d_status = d_words + status_offset(n_words);
@@ -656,7 +657,7 @@ int svo_octree_build_dense(const uint32_t *grid, int w, int h, int d, uint64_t m
     if (owned) cudaFree(owned);
     if (rc) return rc;
     float center[3] = {(float)w * 0.5f / (float)side, (float)h * 0.5f / (float)side, (float)d * 0.5f / (float)side};
-    return make_handle(dw, nw, center, out);
+    return make_handle(dw, nw, center, out, log2_exact((uint64_t)side));
 }
 
 // The .voxel build: the whole grid on the device when it fits in half the
@@ -692,7 +693,7 @@ static int build_voxel_file_impl(const char *path, uint64_t mem, uint64_t slab_b
         float center[3];
         int rc = build_voxel_file_streamed(fp, w, h, d, mem, slab_bytes, (cudaStream_t)stream, &dw, &nw, center);
         if (rc) return rc;
-        return make_handle(dw, nw, center, out);
+        return make_handle(dw, nw, center, out, log2_exact((uint64_t)side));
     }
     uint32_t *dg = nullptr;
     SVO_CUDA_TRY(cudaMalloc((void **)&dg, slab * d * 4));

@@ -30,16 +30,19 @@
 // the handle without a table.  The table costs 16 bytes per node, about 2
 // bytes per octree word on the benchmark scenes.
 //
-// Measured, first call to ready table, word order against breadth first: 130
-// and 325 us (10,000 words), 235 and 490 (1.8 M), 285 and 570 (14 M), 605 and
-// 815 (63 M), 910 and 980 (113 M), 3,300 and 2,350 (490 M: the list's scattered
-// marks and the pass over all words then cost more than the round trips).
+// Measured, first call to ready table (us), word order against breadth first:
+// 63 and 320 (10,000 words), 89 and 428 (1.8 M), 156 and 498 (14 M), 471 and 727
+// (63 M), 776 and 836 (113 M), 3,240 and 2,290 (490 M: the list's scattered marks
+// and the pass over all words then cost more than the round trips).  The
+// table of a 200x131x177 volume takes 118 without chained launches (chain.cuh),
+// 92 with them, 83 when the levels are known.
 // Traces run at the same speed over either order (within 0.5% on nine
 // workloads).
 #include <algorithm>
 #include <memory>
 #include <vector>
 
+#include "chain.cuh"
 #include "octree_table.cuh"
 #include "scan.cuh"
 #include "svo_internal.h"
@@ -112,6 +115,7 @@ __device__ __forceinline__ uint32_t rank_of(const WordOrder &t, uint32_t w) {
 }
 
 __global__ void __launch_bounds__(kTopThreads) k_table_top(WordOrder t) {
+    chain_begin();
     __shared__ uint32_t node[kTopNodes], wsum[kTopThreads / 32];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     if (threadIdx.x == 0) node[0] = 0;
@@ -157,6 +161,7 @@ __global__ void __launch_bounds__(kTopThreads) k_table_top(WordOrder t) {
 // Level L's nodes, list[length(L - 1) .. length(L)).  The last CTA to finish
 // notes the list's length for the next level; no CTA waits for another.
 __global__ void __launch_bounds__(256) k_table_expand(WordOrder t, int L) {
+    chain_begin();
     // after an error the list may hold places that were never written
     if (t.ctl[kCtlErr]) return;
     __shared__ uint32_t base;
@@ -189,6 +194,7 @@ __global__ void __launch_bounds__(256) k_table_expand(WordOrder t, int L) {
 }
 
 __global__ void __launch_bounds__(kScanThreads) k_table_tiles(WordOrder t, uint64_t n) {
+    chain_begin();
     const uint64_t i0 = (uint64_t)blockIdx.x * kRankTile + (uint64_t)threadIdx.x * kRankItems;
     uint32_t c = 0, total;
     for (int k = 0; k < kRankItems; ++k)
@@ -201,6 +207,7 @@ __global__ void __launch_bounds__(kScanThreads) k_table_tiles(WordOrder t, uint6
 // last one leaves the total.
 __global__ void __launch_bounds__(kScanThreads) k_table_rank(WordOrder t, uint64_t n, const uint32_t *__restrict__ first,
                                                              uint32_t *__restrict__ total_out) {
+    chain_begin();
     uint32_t before = 0, total;
     if (first) {
         before = first[blockIdx.x];
@@ -261,7 +268,8 @@ struct Scratch {
 inline unsigned grid_for(uint64_t n) { return (unsigned)((n + 255) / 256); }
 
 // The table in word order; *tab stays null when it cannot be had this way.
-int build_word_order(const uint32_t *d_words, uint64_t n_words, cudaStream_t st, uint4 **tab, uint64_t *n_tab) {
+int build_word_order(const uint32_t *d_words, uint64_t n_words, int levels, cudaStream_t st, uint4 **tab,
+                     uint64_t *n_tab) {
     *tab = nullptr;
     // a node list as long as the words where that is little memory, else a
     // quarter of them (about an eighth are nodes on the benchmark scenes)
@@ -292,23 +300,23 @@ int build_word_order(const uint32_t *d_words, uint64_t n_words, cudaStream_t st,
     SVO_CUDA_TRY(cudaMemsetAsync(m, 0, (size_t)o_rank * sizeof(uint32_t), st));
     k_table_top<<<1, kTopThreads, 0, st>>>(t);
     SVO_CUDA_TRY(cudaGetLastError());
-    // twelve levels (a 4096^3 cube's) before the host looks, and if they end
-    // there the ranks are there too
+    // a built cube's levels, or twelve (a 4096^3 cube's), before the host looks,
+    // and if they end there the ranks are there too; an empty level costs 3 us
+    const int expect = levels > kTopLevels ? levels : levels ? kTopLevels + 1 : 12;
     uint32_t h[kCtlWords];
     uint32_t n = 0;
     for (int L = kTopLevels;;) {
-        const int to = std::min(L == kTopLevels ? 12 : L + 6, kTableMaxParentLevel + 2);
+        const int to = std::min(L == kTopLevels ? expect : L + 6, kTableMaxParentLevel + 2);
         for (; L < to; ++L) {
             const uint64_t most = L < 8 ? std::min<uint64_t>(cap, 1ull << (3 * L)) : cap;
-            k_table_expand<<<(unsigned)std::min<uint64_t>((most + 255) / 256, 152 * 8), 256, 0, st>>>(t, L);
-            SVO_CUDA_TRY(cudaGetLastError());
+            SVO_CUDA_TRY(launch_chained(k_table_expand, (unsigned)std::min<uint64_t>((most + 255) / 256, 152 * 8), 256, st,
+                                        t, L));
         }
-        k_table_tiles<<<(unsigned)tiles, kScanThreads, 0, st>>>(t, nb);
-        SVO_CUDA_TRY(cudaGetLastError());
+        SVO_CUDA_TRY(launch_chained(k_table_tiles, (unsigned)tiles, kScanThreads, st, t, nb));
         if (!self)
             SVO_CUDA_TRY((exclusive_scan<uint32_t, uint32_t>(t.tile, first, tiles, t.ctl + kCtlWords - 1, m + o_scan, st)));
-        k_table_rank<<<(unsigned)tiles, kScanThreads, 0, st>>>(t, nb, first, t.ctl + kCtlWords - 1);
-        SVO_CUDA_TRY(cudaGetLastError());
+        SVO_CUDA_TRY(launch_chained(k_table_rank, (unsigned)tiles, kScanThreads, st, t, nb, first,
+                                    t.ctl + kCtlWords - 1));
         SVO_CUDA_TRY(cudaMemcpyAsync(h, t.ctl, sizeof(h), cudaMemcpyDeviceToHost, st));
         SVO_CUDA_TRY(cudaStreamSynchronize(st));
         if (h[kCtlErr]) return SVO_OK;
@@ -335,13 +343,13 @@ int build_word_order(const uint32_t *d_words, uint64_t n_words, cudaStream_t st,
 // Builds the table on `st` and waits for it.  Returns SVO_OK with *tab set
 // (handle_alloc'd, n_tab entries) or with *tab = nullptr when the octree does
 // not qualify; an error code only for CUDA failures.
-int build_table(const uint32_t *d_words, uint64_t n_words, cudaStream_t st, uint4 **tab, uint64_t *n_tab) {
+int build_table(const uint32_t *d_words, uint64_t n_words, int levels, cudaStream_t st, uint4 **tab, uint64_t *n_tab) {
     *tab = nullptr;
     *n_tab = 0;
     if (n_words == 0 || n_words > kMaxNarrowWords) return SVO_OK;
     const uint32_t W = (uint32_t)n_words;
     if (n_words <= kWordOrderMost) {
-        const int rc = build_word_order(d_words, n_words, st, tab, n_tab);
+        const int rc = build_word_order(d_words, n_words, levels, st, tab, n_tab);
         if (rc != SVO_OK || *tab) return rc;
     }
     std::unique_ptr<Scratch[]> lv_entries(new Scratch[kTableMaxParentLevel + 2]);
@@ -432,7 +440,7 @@ const uint4 *octree_table(const svo_octree *oct, cudaStream_t caller) {
         if (library_stream(&st) != cudaSuccess) return nullptr;
         uint4 *t = nullptr;
         uint64_t nt = 0;
-        int rc = build_table(oct->d_words, oct->n_words, st, &t, &nt);
+        int rc = build_table(oct->d_words, oct->n_words, oct->levels, st, &t, &nt);
         if (rc != SVO_OK) {
             // A CUDA failure (device memory, most likely): keep the word
             // traversal for this handle rather than retry on every call.

@@ -20,6 +20,7 @@
 #include <algorithm>
 #include <cmath>
 
+#include "chain.cuh"
 #include "svo_device.cuh"
 #include "svo_internal.h"
 
@@ -70,6 +71,7 @@ __device__ __forceinline__ int strip_rows_of(const FrameArgs &f, int s, int &y0)
 // additions for 1280 pixels).
 template <bool kTab>
 __global__ void __launch_bounds__(kFrameThreads) k_corners(FrameArgs f, int warps_x) {
+    chain_begin();
     const int lane = threadIdx.x & 31, w = (blockIdx.x * kFrameThreads + threadIdx.x) >> 5, s = blockIdx.y;
     const int tx = (w % warps_x) * 8 + (lane & 7), ty = (w / warps_x) * 4 + (lane >> 3);
     if (tx >= f.tiles_x) return;
@@ -135,6 +137,7 @@ __device__ __forceinline__ uint32_t pixel_color(const FrameArgs &f, const TilePl
 // A warp per 8x4 half tile.
 template <bool kTab>
 __global__ void __launch_bounds__(kFrameThreads) k_tiles(FrameArgs f, int total_tiles) {
+    chain_begin();
     const int lane = threadIdx.x & 31;
     const int w = (int)(((uint64_t)blockIdx.x * kFrameThreads + threadIdx.x) >> 5);
     if ((w >> 1) >= total_tiles) return;
@@ -151,6 +154,7 @@ __global__ void __launch_bounds__(kFrameThreads) k_tiles(FrameArgs f, int total_
 // traced, 90 with this.
 template <bool kTab>
 __global__ void __launch_bounds__(kFrameThreads) k_tiles_coarse(FrameArgs f, int total_tiles, int edge, int per_warp) {
+    chain_begin();
     const int lane = threadIdx.x & 31;
     const int w = (int)(((uint64_t)blockIdx.x * kFrameThreads + threadIdx.x) >> 5);
     const int first = w * per_warp, n = min(per_warp, total_tiles - first);
@@ -241,17 +245,11 @@ extern "C" int svo_render_frame(const svo_octree *oct, const float rot[9], const
         const int edge = (kTile + f.pixel_stride - 1) / f.pixel_stride, per_warp = 32 / std::min(32, edge * edge);
         const uint64_t warps2 = f.pixel_stride == 1 ? 2ull * total_tiles : ((uint64_t)total_tiles + per_warp - 1) / per_warp;
         const unsigned g2 = (unsigned)((warps2 * 32 + kFrameThreads - 1) / kFrameThreads);
-        if (f.pixel_stride > 1) {
-            if (f.tab)
-                k_tiles_coarse<true><<<g2, kFrameThreads, 0, st>>>(f, total_tiles, edge, per_warp);
-            else
-                k_tiles_coarse<false><<<g2, kFrameThreads, 0, st>>>(f, total_tiles, edge, per_warp);
-        } else if (f.tab) {
-            k_tiles<true><<<g2, kFrameThreads, 0, st>>>(f, total_tiles);
-        } else {
-            k_tiles<false><<<g2, kFrameThreads, 0, st>>>(f, total_tiles);
-        }
-        e = cudaGetLastError();
+        if (f.pixel_stride > 1)
+            e = launch_chained(f.tab ? k_tiles_coarse<true> : k_tiles_coarse<false>, g2, kFrameThreads, st, f, total_tiles,
+                               edge, per_warp);
+        else
+            e = launch_chained(f.tab ? k_tiles<true> : k_tiles<false>, g2, kFrameThreads, st, f, total_tiles);
     }
     cudaFreeAsync(scratch, st);
     if (e != cudaSuccess) return cuda_fail(e, "svo_render_frame");

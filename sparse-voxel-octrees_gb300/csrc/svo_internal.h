@@ -21,6 +21,7 @@ struct svo_octree {
     uint64_t n_words = 0;
     float center[3] = {0.0f, 0.0f, 0.0f};
     int device = 0;
+    int levels = 0;  // descriptor levels, 0: not known
     uint32_t *d_status = nullptr;  // device error word, behind the words: bit 0 = a ray ended with kFault
     int index_bits = 32;  // 64: svo_trace uses 64-bit word indices even when n_words fits 32 bits
 
@@ -154,7 +155,8 @@ int launch_count_loads(const svo_octree *oct, const float *d_rays, uint64_t n, f
 
 // Creates a handle around device words from alloc_words, complete on the
 // device (takes ownership).
-int make_handle(uint32_t *d_words, uint64_t n_words, const float center[3], svo_octree **out);
+// levels: the built cube's descriptor levels, or 0 where they are not known
+int make_handle(uint32_t *d_words, uint64_t n_words, const float center[3], svo_octree **out, int levels = 0);
 
 // The handle's descriptor table (octree_table.cu), built on first use; null
 // when the octree does not qualify (over 2^32-1 words, or a reachable node

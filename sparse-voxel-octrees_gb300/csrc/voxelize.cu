@@ -47,6 +47,7 @@
 #include <vector>
 
 #include "brick.cuh"
+#include "chain.cuh"
 #include "mesh.h"
 #include "morton.cuh"
 #include "scan.cuh"
@@ -210,6 +211,7 @@ __global__ void __launch_bounds__(128, 8) k_tri_pairs(uint64_t n_tris, int per_w
                                                    uint32_t *__restrict__ pair_key, uint32_t *__restrict__ pair_tri,
                                                    uint32_t *__restrict__ pair_cell, uint32_t *__restrict__ brick_n,
                                                    uint32_t *__restrict__ err) {
+    chain_begin();
     const int lane = threadIdx.x & 31;
     const uint64_t t0 = ((uint64_t)blockIdx.x * 4 + (threadIdx.x >> 5)) * (uint64_t)per_warp;
     uint32_t left = 0;  // the warp's large triangles
@@ -372,6 +374,7 @@ __device__ __forceinline__ uint64_t tile_sum(const uint32_t *n, uint64_t i0, uin
 
 __global__ void __launch_bounds__(256) k_brick_tiles(const uint32_t *__restrict__ n, uint64_t cells,
                                                      uint64_t *__restrict__ tiles, uint32_t *__restrict__ largest) {
+    chain_begin();
     uint32_t c[8], most = 0;
     const uint64_t s = tile_sum(n, (uint64_t)blockIdx.x * kBrickTile + (uint64_t)threadIdx.x * 8, cells, c);
 #pragma unroll
@@ -388,6 +391,7 @@ __global__ void __launch_bounds__(256) k_brick_tiles(const uint32_t *__restrict_
 __global__ void __launch_bounds__(256) k_brick_layout(uint32_t *__restrict__ n, uint64_t cells,
                                                       const uint64_t *__restrict__ tiles, uint32_t *__restrict__ bkey,
                                                       uint32_t *__restrict__ bstart, uint64_t *__restrict__ totals) {
+    chain_begin();
     uint64_t before = 0, total;
     for (uint32_t t = threadIdx.x; t < blockIdx.x; t += 256) before += tiles[t];
     block_excl_scan<uint64_t>(before, &total);
@@ -439,6 +443,7 @@ constexpr int kBrickSortWarps = 4;
 template <bool kCells>
 __global__ void __launch_bounds__(kBrickSortWarps * 32) k_sort_bricks(uint32_t nb, const uint32_t *__restrict__ bstart,
                                                                       uint32_t *tri, uint32_t *cell) {
+    chain_begin();
     using Key = PairKey<kCells>;
     __shared__ alignas(16) Key buf[kBrickSortWarps][kWarpSort];
     const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -470,6 +475,7 @@ __global__ void __launch_bounds__(kBrickSortWarps * 32) k_sort_bricks(uint32_t n
 template <bool kCells>
 __global__ void __launch_bounds__(256) k_sort_large(uint32_t nb, const uint32_t *__restrict__ bstart, uint32_t *tri,
                                                     uint32_t *cell) {
+    chain_begin();
     using Key = PairKey<kCells>;
     __shared__ Key key[kSortedInBrick];
     for (uint32_t j = blockIdx.x; j < nb; j += gridDim.x) {
@@ -566,6 +572,7 @@ __global__ void k_gather_blocks(const uint8_t *__restrict__ flag, uint64_t n, co
 constexpr int kCenterRows = 32, kCenterSpan = 32;
 
 __global__ void __launch_bounds__(kCenterRows) k_center_table(int n_l, int K, float h, float *__restrict__ acc) {
+    chain_begin();
     __shared__ float buf[kCenterRows][kCenterSpan + 1];
     const int l0 = blockIdx.x * kCenterRows, lane = threadIdx.x;
     float c = ((float)(l0 + lane) - 0.5f) * h;
@@ -804,6 +811,7 @@ __device__ __forceinline__ void fold_hits(FoldSmem &sm, int n, const float *rati
 // fold takes 46%, the tests 23%, staging 27%.
 template <bool kDirect>
 __global__ void __launch_bounds__(kFoldWarps * 32, kFoldCtas) k_fold_bricks(FoldArgs a) {
+    chain_begin();
     __shared__ FoldSmem smem[kFoldWarps];
     __shared__ float ratio[256];  // writeTriangleCell's count / (count + 1)
     const unsigned FULL = 0xffffffffu;
@@ -1342,8 +1350,7 @@ int fold_direct(FoldArgs fa, uint32_t *next, uint32_t nb, const uint8_t *bflag, 
         }
     }
     const unsigned grid = (unsigned)std::min<uint64_t>((nb + kFoldWarps - 1) / kFoldWarps, fold_grid);
-    k_fold_bricks<true><<<grid, kFoldWarps * 32, 0, st>>>(fa);
-    SVO_LAUNCH_OK("k_fold_bricks<direct>");
+    SVO_CUDA_TRY(launch_chained(k_fold_bricks<true>, grid, kFoldWarps * 32, st, fa));
     if (as_bricks) {
         const MeshBricks mb{nb, fa.bkey, ccount.p, nmask.p, cbits.p, slot.p, n_vox.p};
         return build_from_bricks_device(mb, D, lb, lb < D ? bflag : nullptr, st, d_words, n_words);
@@ -1582,7 +1589,7 @@ int build_mesh_device(const svo_mesh *m, int side, int threads, uint64_t mem, cu
     const unsigned pair_grid = (unsigned)((nt + 4 * per_warp - 1) / (4 * per_warp));
     if (nt) {
         k_tri_pairs<0><<<pair_grid, 128, 0, st>>>(nt, per_warp, m->d_tris, g, box.p, bflag, pcount.p, nullptr, nullptr,
-                                                          nullptr, nullptr, brick_n.p, err);
+                                                  nullptr, nullptr, brick_n.p, err);
         SVO_LAUNCH_OK("k_tri_pairs<count>");
     }
     const unsigned fold_grid = (unsigned)(sms * kFoldCtas), warp_grid = (unsigned)sms * 16;
@@ -1621,9 +1628,9 @@ int build_mesh_device(const svo_mesh *m, int side, int threads, uint64_t mem, cu
     Dev<uint32_t> fold_next;  // one work counter per fold launch
 
     if (table) {
-        k_brick_tiles<<<(unsigned)brick_tiles, 256, 0, st>>>(brick_n.p, brick_cells, tiles.p, largest);
-        k_brick_layout<<<(unsigned)brick_tiles, 256, 0, st>>>(brick_n.p, brick_cells, tiles.p, bkey.p, bstart.p, info.p);
-        SVO_LAUNCH_OK("k_brick_layout");
+        SVO_CUDA_TRY(launch_chained(k_brick_tiles, (unsigned)brick_tiles, 256, st, brick_n.p, brick_cells, tiles.p, largest));
+        SVO_CUDA_TRY(launch_chained(k_brick_layout, (unsigned)brick_tiles, 256, st, brick_n.p, brick_cells, tiles.p, bkey.p,
+                                    bstart.p, info.p));
         uint64_t h[2];
         SVO_CUDA_TRY(cudaMemcpyAsync(h, info.p, sizeof h, cudaMemcpyDeviceToHost, st));
         SVO_CUDA_TRY(cudaStreamSynchronize(st));
@@ -1634,22 +1641,21 @@ int build_mesh_device(const svo_mesh *m, int side, int threads, uint64_t mem, cu
             Dev<uint32_t> ptri, pcell;
             SVO_ALLOC(ptri, pairs);
             if (!sub_bricks) SVO_ALLOC(pcell, pairs);
+            SVO_ALLOC(fold_next, 1);
+            SVO_CUDA_TRY(cudaMemsetAsync(fold_next.p, 0, sizeof(uint32_t), st));
             k_tri_pairs<2><<<pair_grid, 128, 0, st>>>(nt, per_warp, m->d_tris, g, box.p, bflag, nullptr, nullptr, nullptr,
                                                               ptri.p, pcell.p, brick_n.p, err);
             SVO_LAUNCH_OK("k_tri_pairs<emit>");
-            auto sort_bricks = [&](auto cells) {
+            auto sort_bricks = [&](auto cells) -> cudaError_t {
                 constexpr bool kCells = decltype(cells)::value;
-                k_sort_bricks<kCells><<<(nb + kBrickSortWarps - 1) / kBrickSortWarps, kBrickSortWarps * 32, 0, st>>>(
-                    nb, bstart.p, ptri.p, pcell.p);
-                if (h_largest > (uint32_t)kWarpSort)
-                    k_sort_large<kCells><<<std::min<uint32_t>(nb, (uint32_t)sms * 4), 256, 0, st>>>(nb, bstart.p, ptri.p,
-                                                                                                  pcell.p);
+                cudaError_t e = launch_chained(k_sort_bricks<kCells>, (nb + kBrickSortWarps - 1) / kBrickSortWarps,
+                                               kBrickSortWarps * 32, st, nb, bstart.p, ptri.p, pcell.p);
+                if (e == cudaSuccess && h_largest > (uint32_t)kWarpSort)
+                    e = launch_chained(k_sort_large<kCells>, std::min<uint32_t>(nb, (uint32_t)sms * 4), 256, st, nb,
+                                       bstart.p, ptri.p, pcell.p);
+                return e;
             };
-            if (sub_bricks) sort_bricks(std::false_type());
-            else sort_bricks(std::true_type());
-            SVO_LAUNCH_OK("k_sort_bricks");
-            SVO_ALLOC(fold_next, 1);
-            SVO_CUDA_TRY(cudaMemsetAsync(fold_next.p, 0, sizeof(uint32_t), st));
+            SVO_CUDA_TRY(sub_bricks ? sort_bricks(std::false_type()) : sort_bricks(std::true_type()));
             return fold_direct(fold_args(ptri.p, pcell.p), fold_next.p, nb, bflag, err, D, lb, fold_grid, warp_grid, st,
                                d_words, n_words);
         }
@@ -2079,7 +2085,10 @@ extern "C" int svo_octree_build_mesh(const svo_mesh *m, int side, int threads, u
     float center[3];
     int rc = build_mesh_device(m, side, threads, mem, (cudaStream_t)stream, &dw, &nw, center, nullptr);
     if (rc) return rc;
-    return make_handle(dw, nw, center, out);
+    int dims[3];
+    mesh_dims(m, side, dims);
+    const uint64_t cube = round_pow2((uint64_t)std::max(dims[0], std::max(dims[1], dims[2])));
+    return make_handle(dw, nw, center, out, log2_floor(cube));
 }
 
 extern "C" int svo_mesh_to_volume(const svo_mesh *m, int side, int threads, uint64_t mem, uint32_t *d_volume,

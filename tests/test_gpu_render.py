@@ -68,3 +68,38 @@ def test_strided_frames_match_oracle(cuda, svo, golden, oracle, scenes, W, H, st
     cam = scenes.orbit_cameras(1, W + stride, g["center"], radius=1.2)[0]
     img = _frame(cuda, tree, cam, width=W, height=H, n_strips=strips, pixel_stride=stride)
     assert np.array_equal(img, oracle.render_frame(g["words"], cam[:9], cam[9:12], W, H, strips, stride))
+
+
+@pytest.mark.parametrize("stride", [1, 3])
+def test_frames_in_a_row_and_captured(cuda, svo, golden, scenes, stride):
+    """Frames queued without a wait between them, the corner pass of each
+    behind the tiles of the last, and the same from a captured graph."""
+    torch = cuda
+    g = golden["dragon"]
+    tree = svo.VoxelOctree.from_words(g["words"], g["center"])
+    cams = scenes.orbit_cameras(6, 11, g["center"], radius=1.2)
+    want = []
+    for c in cams:
+        want.append(tree.render_frame(c[:9], c[9:12], 320, 200, 4, stride).clone())
+        torch.cuda.synchronize()
+    st = torch.cuda.Stream()
+    out = [torch.zeros_like(want[0]) for _ in cams]
+    torch.cuda.synchronize()
+
+    def frames():
+        for c, o in zip(cams, out):
+            tree.render_frame(c[:9], c[9:12], 320, 200, 4, stride, out=o, stream=st)
+
+    frames()
+    st.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(want, out))
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=st):
+        frames()
+    for o in out:
+        o.zero_()
+    torch.cuda.synchronize()
+    for _ in range(3):
+        graph.replay()
+    torch.cuda.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(want, out))
