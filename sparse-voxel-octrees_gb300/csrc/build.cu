@@ -1661,7 +1661,7 @@ int build_levels(std::vector<LevelArrays> &lv, int base, const uint64_t *leaf_ke
     };
     rc = place();
     if (rc) {
-        cudaFreeAsync(words, st);
+        free_words(words, W, st);
         return rc;
     }
     *d_words_out = words;
@@ -1803,7 +1803,7 @@ static int build_pyramid(int base, int D, const uint32_t *words_of, const uint8_
     };
     const int rc = place();
     if (rc) {
-        cudaFreeAsync(words, st);
+        free_words(words, W, st);
         return rc;
     }
     *d_words_out = words;

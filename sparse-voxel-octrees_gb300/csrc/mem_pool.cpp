@@ -12,7 +12,10 @@
 // replaces an octree every frame does not map and unmap it each time: a
 // rebuilt 200x131x177 volume spent 130 us freeing the octree before it and 100
 // allocating its own, of 385.  A pool holding more than that in live octrees
-// returns whatever is freed at the next synchronisation, as before.
+// returns whatever is freed at the next synchronisation, as before.  Arrays of
+// kHandleDirect bytes or more, which it would not keep for long, are the
+// driver's, for the pool maps memory more slowly: with a 1 GB table the first
+// trace of a 2048^3 terrain waited 3.2 ms for it, 2.3 ms with the driver's.
 #include <mutex>
 #include <vector>
 
@@ -23,6 +26,7 @@ namespace svo {
 namespace {
 constexpr int kMaxDevices = 64;
 constexpr uint64_t kHandleKeep = 1ull << 30;
+constexpr size_t kHandleDirect = 512ull << 20;
 enum Pool { kScratch, kHandles, kPools };
 std::mutex g_pool_mtx;
 cudaMemPool_t g_pools[kMaxDevices][kPools] = {};
@@ -70,20 +74,32 @@ cudaError_t pool_alloc(Pool which, void **p, size_t bytes, cudaStream_t st) {
 
 cudaError_t scratch_alloc(void **p, size_t bytes, cudaStream_t st) { return pool_alloc(kScratch, p, bytes, st); }
 
-cudaError_t handle_alloc(void **p, size_t bytes, cudaStream_t st) { return pool_alloc(kHandles, p, bytes, st); }
+cudaError_t handle_alloc(void **p, size_t bytes, cudaStream_t st) {
+    return bytes < kHandleDirect ? pool_alloc(kHandles, p, bytes, st) : cudaMalloc(p, bytes);
+}
+
+cudaError_t handle_free(void *p, size_t bytes, cudaStream_t st) {
+    return bytes < kHandleDirect ? cudaFreeAsync(p, st) : cudaFree(p);
+}
+
+size_t words_bytes(uint64_t n) { return (size_t)(status_offset(n) + kStatusWords) * sizeof(uint32_t); }
 
 cudaError_t alloc_words(uint32_t **words, uint64_t n, cudaStream_t st) {
     void *p = nullptr;
     const uint64_t at = status_offset(n);
-    cudaError_t e = handle_alloc(&p, (size_t)(at + kStatusWords) * sizeof(uint32_t), st);
+    cudaError_t e = handle_alloc(&p, words_bytes(n), st);
     if (e != cudaSuccess) return e;
     e = cudaMemsetAsync((uint32_t *)p + at, 0, kStatusWords * sizeof(uint32_t), st);
     if (e != cudaSuccess) {
-        cudaFreeAsync(p, st);
+        handle_free(p, words_bytes(n), st);
         return e;
     }
     *words = (uint32_t *)p;
     return cudaSuccess;
+}
+
+void free_words(uint32_t *words, uint64_t n, cudaStream_t st) {
+    if (words) handle_free(words, words_bytes(n), st);
 }
 
 cudaError_t library_stream(cudaStream_t *out) {

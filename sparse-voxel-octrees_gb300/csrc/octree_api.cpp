@@ -99,7 +99,7 @@ static int upload_words(const uint32_t *words, uint64_t n, const float center[3]
     cudaError_t e = cudaMemcpyAsync(d, words, n * sizeof(uint32_t), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) {
-        cudaFreeAsync(d, st);
+        free_words(d, n, st);
         return cuda_fail(e, "upload octree words");
     }
     return make_handle(d, n, center, out);
@@ -504,8 +504,8 @@ int svo_octree_destroy(svo_octree *oct) {
     cudaStream_t st = nullptr;
     cudaDeviceSynchronize();
     library_stream(&st);
-    if (oct->d_words) cudaFreeAsync(oct->d_words, st);
-    if (oct->d_tab) cudaFreeAsync(oct->d_tab, st);
+    free_words(oct->d_words, oct->n_words, st);
+    if (oct->d_tab) handle_free(oct->d_tab, (size_t)oct->n_tab * sizeof(uint4), st);
     if (dev != oct->device) cudaSetDevice(dev);
     if (oct->stage_dev) cudaFree(oct->stage_dev);
     if (oct->copy_in) cudaStreamDestroy(oct->copy_in);

@@ -19,20 +19,20 @@
 // list holds (a quarter of the words) or more than kWordOrderMost words leave
 // that to the breadth-first form below, which needs a scan and a host round
 // trip per level and keeps shared nodes apart:
-//   1. k_table_nodes: per node of the level, table_node's checks, its entry
-//      {descriptor, -, child block, stride} and its internal-child count;
+//   1. k_table_count: per node of the level, table_node's checks and its
+//      internal-child count;
 //   2. an exclusive scan of the counts gives each node's first child in the
 //      next level;
-//   3. k_table_children: the entry's first-child ordinal, and the next
-//      level's node words (block start + j * stride for its j-th internal
-//      child).
+//   3. k_table_children: the next level's node words (block start + j * stride
+//      for a node's j-th internal child);
+//   4. k_table_write, once all levels are known: the entries.
 // A failed check anywhere, a level past 22 or more entries than words leaves
 // the handle without a table.  The table costs 16 bytes per node, about 2
 // bytes per octree word on the benchmark scenes.
 //
 // Measured, first call to ready table (us), word order against breadth first:
 // 63 and 320 (10,000 words), 89 and 428 (1.8 M), 156 and 498 (14 M), 471 and 727
-// (63 M), 776 and 836 (113 M), 3,240 and 2,290 (490 M: the list's scattered marks
+// (63 M), 776 and 836 (113 M), 3,240 and 2,100 (490 M: the list's scattered marks
 // and the pass over all words then cost more than the round trips).  The
 // table of a 200x131x177 volume takes 118 without chained launches (chain.cuh),
 // 92 with them, 83 when the levels are known.
@@ -50,31 +50,42 @@
 namespace svo {
 namespace {
 
-__global__ void k_table_nodes(const uint32_t *__restrict__ words, uint32_t n_words, const uint32_t *__restrict__ level,
-                              uint32_t n, int L, uint4 *__restrict__ entries, uint32_t *__restrict__ n_int,
-                              uint32_t *__restrict__ err) {
+// ---- breadth first -----------------------------------------------------------------
+
+__global__ void __launch_bounds__(256) k_table_count(const uint32_t *__restrict__ words, uint32_t n_words,
+                                                     const uint32_t *__restrict__ level, uint32_t n, int L,
+                                                     uint32_t *__restrict__ n_int, uint32_t *__restrict__ err) {
+    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    uint32_t cb, stride, k;
+    if (!table_node(words, n_words, level[i], L, cb, stride, k)) {
+        atomicOr(err, 1u);
+        k = 0;
+    }
+    n_int[i] = k;
+}
+
+__global__ void __launch_bounds__(256) k_table_children(const uint32_t *__restrict__ words, uint32_t n_words,
+                                                        const uint32_t *__restrict__ level, uint32_t n, int L,
+                                                        const uint32_t *__restrict__ first, uint32_t *__restrict__ next) {
+    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    uint32_t cb, stride, k;
+    if (!table_node(words, n_words, level[i], L, cb, stride, k)) return;
+    const uint32_t o = first[i];
+    for (uint32_t j = 0; j < k; ++j) next[o + j] = cb + j * stride;
+}
+
+__global__ void __launch_bounds__(256) k_table_write(const uint32_t *__restrict__ words, uint32_t n_words,
+                                                     const uint32_t *__restrict__ level, uint32_t n, int L,
+                                                     const uint32_t *__restrict__ first, uint32_t next_base,
+                                                     uint4 *__restrict__ entries) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const uint32_t d = level[i];
     uint32_t cb, stride, k;
-    if (!table_node(words, n_words, d, L, cb, stride, k)) {
-        atomicOr(err, 1u);
-        k = 0;
-    }
-    entries[i] = make_uint4(words[d], 0u, cb, stride);
-    n_int[i] = k;
-}
-
-__global__ void k_table_children(const uint32_t *__restrict__ n_int, const uint32_t *__restrict__ first, uint32_t n,
-                                 uint32_t next_base, uint4 *__restrict__ entries, uint32_t *__restrict__ next) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    uint4 e = entries[i];
-    const uint32_t k = n_int[i], o = first[i], stride = e.w;
-    for (uint32_t j = 0; j < k; ++j) next[o + j] = e.z + j * stride;
-    e.y = next_base + o;
-    e.w = 0;
-    entries[i] = e;
+    table_node(words, n_words, d, L, cb, stride, k);
+    entries[i] = make_uint4(words[d], next_base + first[i], cb, 0u);
 }
 
 // ---- word order --------------------------------------------------------------------
@@ -332,7 +343,7 @@ int build_word_order(const uint32_t *d_words, uint64_t n_words, int levels, cuda
     if (er == cudaSuccess) er = cudaMemcpyAsync(h, t.ctl, sizeof(h), cudaMemcpyDeviceToHost, st);
     if (er == cudaSuccess) er = cudaStreamSynchronize(st);
     if (er != cudaSuccess || h[kCtlErr]) {
-        cudaFreeAsync(e, st);
+        handle_free(e, (size_t)n * sizeof(uint4), st);
         return er != cudaSuccess ? cuda_fail(er, "descriptor table") : SVO_OK;
     }
     *tab = e;
@@ -352,51 +363,50 @@ int build_table(const uint32_t *d_words, uint64_t n_words, int levels, cudaStrea
         const int rc = build_word_order(d_words, n_words, levels, st, tab, n_tab);
         if (rc != SVO_OK || *tab) return rc;
     }
-    std::unique_ptr<Scratch[]> lv_entries(new Scratch[kTableMaxParentLevel + 2]);
+    // per level, the nodes' words and their first children within the next:
+    // 8 bytes a node until the table itself can be had
+    constexpr int kMost = kTableMaxParentLevel + 2;
+    std::unique_ptr<Scratch[]> nodes(new Scratch[kMost + 1]), first(new Scratch[kMost + 1]);
     std::vector<uint32_t> lv_n;
-    Scratch err, cur, total;
+    Scratch err, total;
     SVO_CUDA_TRY(err.alloc(sizeof(uint32_t), st));
     SVO_CUDA_TRY(total.alloc(sizeof(uint32_t), st));
     SVO_CUDA_TRY(cudaMemsetAsync(err.p, 0, sizeof(uint32_t), st));
-    SVO_CUDA_TRY(cur.alloc(sizeof(uint32_t), st));
-    SVO_CUDA_TRY(cudaMemsetAsync(cur.p, 0, sizeof(uint32_t), st));  // level 0: the root at word 0
+    SVO_CUDA_TRY(nodes[0].alloc(sizeof(uint32_t), st));
+    SVO_CUDA_TRY(cudaMemsetAsync(nodes[0].p, 0, sizeof(uint32_t), st));  // level 0: the root at word 0
     uint32_t n = 1;
     uint64_t base = 0;
     bool ok = true;
     for (int L = 0; n > 0; ++L) {
-        if (L > kTableMaxParentLevel + 1 || base + n > n_words) {
+        if (L >= kMost || base + n > n_words) {
             ok = false;
             break;
         }
-        Scratch &ent = lv_entries[L];
-        SVO_CUDA_TRY(ent.alloc((size_t)n * sizeof(uint4), st));
-        Scratch c, f, sc;
+        const uint32_t *const at = (const uint32_t *)nodes[L].p;
+        Scratch c, sc;
         SVO_CUDA_TRY(c.alloc((size_t)n * sizeof(uint32_t), st));
-        SVO_CUDA_TRY(f.alloc((size_t)n * sizeof(uint32_t), st));
+        SVO_CUDA_TRY(first[L].alloc((size_t)n * sizeof(uint32_t), st));
         SVO_CUDA_TRY(sc.alloc(scan_scratch_elems(n) * sizeof(uint32_t), st));
-        k_table_nodes<<<grid_for(n), 256, 0, st>>>(d_words, W, (const uint32_t *)cur.p, n, L, (uint4 *)ent.p,
-                                                   (uint32_t *)c.p, (uint32_t *)err.p);
+        uint32_t *const f = (uint32_t *)first[L].p;
+        k_table_count<<<grid_for(n), 256, 0, st>>>(d_words, W, at, n, L, (uint32_t *)c.p, (uint32_t *)err.p);
         SVO_CUDA_TRY(cudaGetLastError());
-        SVO_CUDA_TRY((exclusive_scan<uint32_t, uint32_t>((const uint32_t *)c.p, (uint32_t *)f.p, n,
-                                                         (uint32_t *)total.p, (uint32_t *)sc.p, st)));
+        SVO_CUDA_TRY((exclusive_scan<uint32_t, uint32_t>((const uint32_t *)c.p, f, n, (uint32_t *)total.p,
+                                                         (uint32_t *)sc.p, st)));
         uint32_t next_n = 0;
         SVO_CUDA_TRY(cudaMemcpyAsync(&next_n, total.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
         SVO_CUDA_TRY(cudaStreamSynchronize(st));
-        Scratch nxt;
-        SVO_CUDA_TRY(nxt.alloc((size_t)next_n * sizeof(uint32_t), st));
-        const uint64_t next_base = base + n;
-        if (next_base + next_n > n_words) {
-            lv_n.push_back(n);
+        lv_n.push_back(n);
+        base += n;
+        if (base + next_n > n_words) {
             ok = false;
             break;
         }
-        k_table_children<<<grid_for(n), 256, 0, st>>>((const uint32_t *)c.p, (const uint32_t *)f.p, n,
-                                                      (uint32_t)next_base, (uint4 *)ent.p, (uint32_t *)nxt.p);
-        SVO_CUDA_TRY(cudaGetLastError());
-        lv_n.push_back(n);
-        base = next_base;
+        if (next_n) {
+            SVO_CUDA_TRY(nodes[L + 1].alloc((size_t)next_n * sizeof(uint32_t), st));
+            k_table_children<<<grid_for(n), 256, 0, st>>>(d_words, W, at, n, L, f, (uint32_t *)nodes[L + 1].p);
+            SVO_CUDA_TRY(cudaGetLastError());
+        }
         n = next_n;
-        std::swap(cur.p, nxt.p);  // nxt now owns the finished level's node list
     }
     uint32_t err_h = 0;
     SVO_CUDA_TRY(cudaMemcpyAsync(&err_h, err.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
@@ -406,17 +416,18 @@ int build_table(const uint32_t *d_words, uint64_t n_words, int levels, cudaStrea
     SVO_CUDA_TRY(handle_alloc((void **)&t, (size_t)base * sizeof(uint4), st));
     uint64_t at = 0;
     for (size_t L = 0; L < lv_n.size(); ++L) {
-        cudaError_t e = cudaMemcpyAsync(t + at, lv_entries[L].p, (size_t)lv_n[L] * sizeof(uint4),
-                                        cudaMemcpyDeviceToDevice, st);
+        k_table_write<<<grid_for(lv_n[L]), 256, 0, st>>>(d_words, W, (const uint32_t *)nodes[L].p, lv_n[L], (int)L,
+                                                         (const uint32_t *)first[L].p, (uint32_t)(at + lv_n[L]), t + at);
+        cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) {
-            cudaFreeAsync(t, st);
-            return cuda_fail(e, "descriptor table copy");
+            handle_free(t, (size_t)base * sizeof(uint4), st);
+            return cuda_fail(e, "descriptor table");
         }
         at += lv_n[L];
     }
     cudaError_t e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) {
-        cudaFreeAsync(t, st);
+        handle_free(t, (size_t)base * sizeof(uint4), st);
         return cuda_fail(e, "descriptor table");
     }
     *tab = t;

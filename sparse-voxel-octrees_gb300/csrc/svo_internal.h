@@ -77,15 +77,18 @@ int lz4_decompress_block(const uint8_t *src, size_t src_len, uint8_t *out, size_
 // release with cudaFreeAsync.
 cudaError_t scratch_alloc(void **p, size_t bytes, cudaStream_t st);
 
-// Memory that a handle keeps, from a pool of its own; release with
-// cudaFreeAsync once nothing on the device uses it any more.
+// Memory that a handle keeps, from a pool of its own or, when large, the
+// driver's; release with handle_free (and the same size) once nothing on the
+// device uses it any more.
 cudaError_t handle_alloc(void **p, size_t bytes, cudaStream_t st);
+cudaError_t handle_free(void *p, size_t bytes, cudaStream_t st);
 
 // An octree's words from that pool, with the handle's zeroed error word behind
 // them, at status_offset(n) words.
 constexpr uint64_t kStatusWords = 32;
 inline uint64_t status_offset(uint64_t n_words) { return (n_words + 31) / 32 * 32; }
 cudaError_t alloc_words(uint32_t **words, uint64_t n, cudaStream_t st);
+void free_words(uint32_t *words, uint64_t n, cudaStream_t st);  // of alloc_words, or null
 
 // A non-blocking stream per device, shared by the library's own work.
 cudaError_t library_stream(cudaStream_t *out);
