@@ -1342,11 +1342,18 @@ __global__ void __launch_bounds__(256) k_pyramid_up(Pyramid p, int level) {
     if (c < pyramid_cells(p, level)) pyramid_node(p, level, c);
 }
 
-__global__ void __launch_bounds__(512) k_pyramid_top_up(Pyramid p, int level) {
+// The levels from `level` up to the root.  Reports the root's subtree words
+// and, where counted, the voxels.
+__global__ void __launch_bounds__(512) k_pyramid_top_up(Pyramid p, int level, const unsigned long long *n_voxels,
+                                                        uint64_t *report) {
     chain_begin();
     for (; level <= p.top; ++level) {
         for (uint32_t c = threadIdx.x; c < pyramid_cells(p, level); c += blockDim.x) pyramid_node(p, level, c);
         __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        report[0] = p.S[p.top - p.base][0];
+        report[1] = n_voxels ? *n_voxels : 0;
     }
 }
 
@@ -1356,13 +1363,12 @@ __global__ void __launch_bounds__(256) k_pyramid_down(Pyramid p, int level, uint
     pyramid_place(p, level, blockIdx.x * blockDim.x + threadIdx.x, words, W, err);
 }
 
-// The root and every level down to `level`.  Zeroes *err.
+// The root and every level down to `level`.
 __global__ void __launch_bounds__(kTopPlaced) k_pyramid_top_down(Pyramid p, int level, uint32_t *__restrict__ words,
                                                            uint64_t W, uint32_t *__restrict__ err) {
     chain_begin();
     const int t = p.top - p.base;
     if (threadIdx.x == 0) {
-        *err = 0;
         const uint32_t m = t ? p.mask[t][0] : p.mask_of[0];
         words[0] = (m << 8) | m | (t && (p.meta[t][0] & 2u) ? 0x10000u : 0u) | (1u << 18);
         p.B[t][0] = 1;
@@ -1743,8 +1749,8 @@ static int build_pyramid(int base, int D, const uint32_t *words_of, const uint8_
     p.log_block = log_block;
     DevBuf<uint64_t> S[kPyramidMax], B[kPyramidMax];
     DevBuf<uint8_t> mask[kPyramidMax], meta[kPyramidMax];
-    DevBuf<uint32_t> err;
-    SVO_TRY_ALLOC(err.alloc(1, arena));
+    Report report;  // root's words, voxels (64 bits each), errors
+    SVO_CUDA_TRY(report.open(st));
     for (int l = 0; l <= D - base; ++l) {
         const uint64_t cells = 1ull << (3 * (D - base - l));
         SVO_TRY_ALLOC(B[l].alloc(cells, arena));
@@ -1764,7 +1770,7 @@ static int build_pyramid(int base, int D, const uint32_t *words_of, const uint8_
         SVO_CUDA_TRY(launch_chained(k_pyramid_up, blocks_for(cells), 256, st, p, e));
     }
     if (e <= D) {
-        SVO_CUDA_TRY(launch_chained(k_pyramid_top_up, 1, 512, st, p, e));
+        SVO_CUDA_TRY(launch_chained(k_pyramid_top_up, 1, 512, st, p, e, n_voxels, (uint64_t *)report.device()));
     }
     uint64_t S_root = 0;
     unsigned long long voxels = 0;
@@ -1774,31 +1780,30 @@ static int build_pyramid(int base, int D, const uint32_t *words_of, const uint8_
         SVO_CUDA_TRY(cudaStreamSynchronize(st));
         S_root = s32;
     } else {
-        SVO_CUDA_TRY(cudaMemcpyAsync(&S_root, p.S[D - base], sizeof(S_root), cudaMemcpyDeviceToHost, st));
-        if (n_voxels) SVO_CUDA_TRY(cudaMemcpyAsync(&voxels, n_voxels, sizeof(voxels), cudaMemcpyDeviceToHost, st));
-        SVO_CUDA_TRY(cudaStreamSynchronize(st));
+        SVO_CUDA_TRY(report.wait());
+        S_root = ((const uint64_t *)report.words())[0];
+        voxels = ((const uint64_t *)report.words())[1];
     }
     if (voxels >= 0xFFFFFFFFull) return set_error(SVO_ERR_LIMIT, "%llu occupied voxels exceed 2^32-1", voxels);
     const uint64_t W = 1 + S_root;
     uint32_t *words = nullptr;
     SVO_CUDA_TRY(alloc_words(&words, W, st));
     auto place = [&]() -> int {
+        uint32_t *const err = report.device() + 4;
         int c = D;
         while (c > base && (1ull << (3 * (D - c + 1))) <= kTopPlaced) --c;
-        k_pyramid_top_down<<<1, (unsigned)kTopPlaced, 0, st>>>(p, c, words, W, err.p);
+        k_pyramid_top_down<<<1, (unsigned)kTopPlaced, 0, st>>>(p, c, words, W, err);
         SVO_LAUNCH_CHECK("k_pyramid_top_down");
         for (--c; c >= base; --c) {
-            SVO_CUDA_TRY(launch_chained(k_pyramid_down, blocks_for(1ull << (3 * (D - c))), 256, st, p, c, words, W, err.p));
+            SVO_CUDA_TRY(launch_chained(k_pyramid_down, blocks_for(1ull << (3 * (D - c))), 256, st, p, c, words, W, err));
         }
         BrickPlaces places{};
         places.words_of = words_of;
         places.B = p.B[0];
-        int r = place_bricks(places, words, W, err.p);
+        int r = place_bricks(places, words, W, err);
         if (r) return r;
-        uint32_t err_h = 0;
-        SVO_CUDA_TRY(cudaMemcpyAsync(&err_h, err.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-        SVO_CUDA_TRY(cudaStreamSynchronize(st));
-        if (err_h) return set_error(SVO_ERR_DEVICE, "octree build placement check failed (flags %u)", err_h);
+        SVO_CUDA_TRY(report.wait());
+        if (const uint32_t err_h = report.words()[4]) return set_error(SVO_ERR_DEVICE, "octree build placement check failed (flags %u)", err_h);
         return SVO_OK;
     };
     const int rc = place();

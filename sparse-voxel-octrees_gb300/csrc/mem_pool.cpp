@@ -16,6 +16,7 @@
 // kHandleDirect bytes or more, which it would not keep for long, are the
 // driver's, for the pool maps memory more slowly: with a 1 GB table the first
 // trace of a 2048^3 terrain waited 3.2 ms for it, 2.3 ms with the driver's.
+#include <cstring>
 #include <mutex>
 #include <vector>
 
@@ -156,6 +157,38 @@ HostSlot *host_slot_take() {
 void host_slot_give(HostSlot *s) {
     std::lock_guard<std::mutex> lk(g_pool_mtx);
     g_free_slots[s->device].push_back(s);
+}
+
+cudaError_t Report::open(cudaStream_t st) {
+    st_ = st;
+    slot_ = host_slot_take();
+    if (slot_) {
+        std::memset(slot_->host, 0, kWords * sizeof(uint32_t));
+        dev_ = (uint32_t *)slot_->dev;
+        return cudaSuccess;
+    }
+    void *p = nullptr;
+    cudaError_t e = scratch_alloc(&p, kWords * sizeof(uint32_t), st);
+    if (e != cudaSuccess) return e;
+    dev_ = (uint32_t *)p;
+    return cudaMemsetAsync(dev_, 0, kWords * sizeof(uint32_t), st);
+}
+
+cudaError_t Report::wait() {
+    cudaError_t e = cudaSuccess;
+    if (!slot_) e = cudaMemcpyAsync(copy_, dev_, sizeof copy_, cudaMemcpyDeviceToHost, st_);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st_);
+    busy_ = e != cudaSuccess;
+    return e;
+}
+
+Report::~Report() {
+    if (slot_) {
+        if (busy_) cudaStreamSynchronize(st_);  // a call that ended early: its kernels may still write
+        host_slot_give(slot_);
+    } else if (dev_) {
+        cudaFreeAsync(dev_, st_);
+    }
 }
 
 // Frees the idle slots of a device.

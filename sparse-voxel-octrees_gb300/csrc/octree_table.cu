@@ -31,14 +31,16 @@
 // bytes per octree word on the benchmark scenes.
 //
 // Measured, first call to ready table (us), word order against breadth first:
-// 63 and 320 (10,000 words), 89 and 428 (1.8 M), 156 and 498 (14 M), 471 and 727
-// (63 M), 776 and 836 (113 M), 3,240 and 2,100 (490 M: the list's scattered marks
+// 49 and 309 (10,000 words), 70 and 413 (1.8 M), 140 and 492 (14 M), 458 and 706
+// (63 M), 759 and 833 (113 M), 3,240 and 2,100 (490 M: the list's scattered marks
 // and the pass over all words then cost more than the round trips).  The
-// table of a 200x131x177 volume takes 118 without chained launches (chain.cuh),
-// 92 with them, 83 when the levels are known.
+// table of a 200x131x177 volume took 118 without chained launches (chain.cuh),
+// 92 with them, 83 with the levels known, and 65 since the kernels write what
+// the host waits for into its own memory.
 // Traces run at the same speed over either order (within 0.5% on nine
 // workloads).
 #include <algorithm>
+#include <cstring>
 #include <memory>
 #include <vector>
 
@@ -214,10 +216,10 @@ __global__ void __launch_bounds__(kScanThreads) k_table_tiles(WordOrder t, uint6
     if (threadIdx.x == 0) t.tile[blockIdx.x] = total;
 }
 
-// first: the tiles' scan, or null: this tile adds up those before it, and the
-// last one leaves the total.
+// first: the tiles' scan, or null: this tile adds up those before it.  Reports
+// ctl to the host, and as its last word the bitmap's total.
 __global__ void __launch_bounds__(kScanThreads) k_table_rank(WordOrder t, uint64_t n, const uint32_t *__restrict__ first,
-                                                             uint32_t *__restrict__ total_out) {
+                                                             uint32_t *__restrict__ report) {
     chain_begin();
     uint32_t before = 0, total;
     if (first) {
@@ -238,10 +240,11 @@ __global__ void __launch_bounds__(kScanThreads) k_table_rank(WordOrder t, uint64
         if (i0 + k < n) t.rank[i0 + k] = at;
         at += own[k];
     }
-    if (!first && blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) *total_out = before + total;
+    if (blockIdx.x == 0 && threadIdx.x < kCtlWords - (first ? 0 : 1)) report[threadIdx.x] = t.ctl[threadIdx.x];
+    if (!first && blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) report[kCtlWords - 1] = before + total;
 }
 
-__global__ void __launch_bounds__(256) k_table_entries(WordOrder t, uint4 *__restrict__ tab) {
+__global__ void __launch_bounds__(256) k_table_entries(WordOrder t, uint4 *__restrict__ tab, uint32_t *__restrict__ err) {
     const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t n_top = t.ctl[kCtlTop];
     if (i < n_top) {  // table_node has passed for every node here
@@ -257,7 +260,7 @@ __global__ void __launch_bounds__(256) k_table_entries(WordOrder t, uint4 *__res
     // between them are no descriptors
     if (k && stride == 2)
         for (uint32_t f = cb + 1; f < cb + 2 * k - 1; f += 2)
-            if ((t.bits[f >> 5] >> (f & 31)) & 1u) atomicOr(&t.ctl[kCtlErr], kErrOrder);
+            if ((t.bits[f >> 5] >> (f & 31)) & 1u) atomicOr(err, kErrOrder);
     tab[n_top + rank_of(t, (uint32_t)i)] = make_uint4(t.words[i], k ? n_top + rank_of(t, cb) : 0u, cb, 0u);
 }
 
@@ -314,6 +317,9 @@ int build_word_order(const uint32_t *d_words, uint64_t n_words, int levels, cuda
     // a built cube's levels, or twelve (a 4096^3 cube's), before the host looks,
     // and if they end there the ranks are there too; an empty level costs 3 us
     const int expect = levels > kTopLevels ? levels : levels ? kTopLevels + 1 : 12;
+    static_assert(kCtlWords <= Report::kWords && kCtlWords <= kScanThreads, "one report");
+    Report report;
+    SVO_CUDA_TRY(report.open(st));
     uint32_t h[kCtlWords];
     uint32_t n = 0;
     for (int L = kTopLevels;;) {
@@ -327,9 +333,9 @@ int build_word_order(const uint32_t *d_words, uint64_t n_words, int levels, cuda
         if (!self)
             SVO_CUDA_TRY((exclusive_scan<uint32_t, uint32_t>(t.tile, first, tiles, t.ctl + kCtlWords - 1, m + o_scan, st)));
         SVO_CUDA_TRY(launch_chained(k_table_rank, (unsigned)tiles, kScanThreads, st, t, nb, first,
-                                    t.ctl + kCtlWords - 1));
-        SVO_CUDA_TRY(cudaMemcpyAsync(h, t.ctl, sizeof(h), cudaMemcpyDeviceToHost, st));
-        SVO_CUDA_TRY(cudaStreamSynchronize(st));
+                                    report.device()));
+        SVO_CUDA_TRY(report.wait());
+        std::memcpy(h, report.words(), sizeof(h));
         if (h[kCtlErr]) return SVO_OK;
         if (h[kCtlEnd + L] == h[kCtlEnd + L - 1]) break;  // the last level expanded added nothing
         if (L >= kTableMaxParentLevel + 2) return SVO_OK;
@@ -338,11 +344,10 @@ int build_word_order(const uint32_t *d_words, uint64_t n_words, int levels, cuda
     n = h[kCtlTop] + h[kCtlTail];
     uint4 *e = nullptr;
     SVO_CUDA_TRY(handle_alloc((void **)&e, (size_t)n * sizeof(uint4), st));
-    k_table_entries<<<grid_for(std::max<uint64_t>(n_words, kTopNodes)), 256, 0, st>>>(t, e);
+    k_table_entries<<<grid_for(std::max<uint64_t>(n_words, kTopNodes)), 256, 0, st>>>(t, e, report.device() + kCtlErr);
     cudaError_t er = cudaGetLastError();
-    if (er == cudaSuccess) er = cudaMemcpyAsync(h, t.ctl, sizeof(h), cudaMemcpyDeviceToHost, st);
-    if (er == cudaSuccess) er = cudaStreamSynchronize(st);
-    if (er != cudaSuccess || h[kCtlErr]) {
+    if (er == cudaSuccess) er = report.wait();
+    if (er != cudaSuccess || report.words()[kCtlErr]) {
         handle_free(e, (size_t)n * sizeof(uint4), st);
         return er != cudaSuccess ? cuda_fail(er, "descriptor table") : SVO_OK;
     }

@@ -387,10 +387,12 @@ __global__ void __launch_bounds__(256) k_brick_tiles(const uint32_t *__restrict_
 }
 
 // The non-empty bricks' keys and first pairs, in key order, and in n each
-// brick's first pair in place of its count.
+// brick's first pair in place of its count.  Reports the bricks and pairs
+// (packed as above), the largest brick and the error word.
 __global__ void __launch_bounds__(256) k_brick_layout(uint32_t *__restrict__ n, uint64_t cells,
                                                       const uint64_t *__restrict__ tiles, uint32_t *__restrict__ bkey,
-                                                      uint32_t *__restrict__ bstart, uint64_t *__restrict__ totals) {
+                                                      uint32_t *__restrict__ bstart, const uint32_t *largest,
+                                                      const uint32_t *err, uint64_t *__restrict__ report) {
     chain_begin();
     uint64_t before = 0, total;
     for (uint32_t t = threadIdx.x; t < blockIdx.x; t += 256) before += tiles[t];
@@ -410,7 +412,8 @@ __global__ void __launch_bounds__(256) k_brick_layout(uint32_t *__restrict__ n, 
     }
     if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {
         bstart[(before + total) >> 40] = (uint32_t)(before + total);
-        *totals = before + total;
+        report[0] = before + total;
+        report[1] = *largest | ((uint64_t)*err << 32);
     }
 }
 
@@ -1510,12 +1513,11 @@ int build_mesh_device(const svo_mesh *m, int side, int threads, uint64_t mem, cu
         return set_error(SVO_ERR_LIMIT, "voxel-centre table of %d x %d entries is too large", n_l, K);
 
     const uint64_t nt = m->n_tris;
-    // what the host reads after the count (totals of the table of bricks, the
-    // largest, the error word), then the block flags
-    Dev<uint64_t> info;
-    SVO_ALLOC(info, 2 + (g.n_blocks + 7) / 8);
-    SVO_CUDA_TRY(cudaMemsetAsync(info.p, 0, 16 + g.n_blocks, st));
-    uint32_t *const largest = (uint32_t *)info.p + 2, *const err = (uint32_t *)info.p + 3;
+    // the largest brick's pairs, the error word and the block flags
+    Dev<uint32_t> info;
+    SVO_ALLOC(info, 2 + (g.n_blocks + 3) / 4);
+    SVO_CUDA_TRY(cudaMemsetAsync(info.p, 0, 8 + g.n_blocks, st));
+    uint32_t *const largest = info.p, *const err = info.p + 1;
     uint8_t *const bflag = (uint8_t *)(info.p + 2);
 
     // the running centres, first: they depend on the size alone
@@ -1628,12 +1630,17 @@ int build_mesh_device(const svo_mesh *m, int side, int threads, uint64_t mem, cu
     Dev<uint32_t> fold_next;  // one work counter per fold launch
 
     if (table) {
-        SVO_CUDA_TRY(launch_chained(k_brick_tiles, (unsigned)brick_tiles, 256, st, brick_n.p, brick_cells, tiles.p, largest));
-        SVO_CUDA_TRY(launch_chained(k_brick_layout, (unsigned)brick_tiles, 256, st, brick_n.p, brick_cells, tiles.p, bkey.p,
-                                    bstart.p, info.p));
         uint64_t h[2];
-        SVO_CUDA_TRY(cudaMemcpyAsync(h, info.p, sizeof h, cudaMemcpyDeviceToHost, st));
-        SVO_CUDA_TRY(cudaStreamSynchronize(st));
+        {
+            Report report;
+            SVO_CUDA_TRY(report.open(st));
+            SVO_CUDA_TRY(launch_chained(k_brick_tiles, (unsigned)brick_tiles, 256, st, brick_n.p, brick_cells, tiles.p,
+                                        largest));
+            SVO_CUDA_TRY(launch_chained(k_brick_layout, (unsigned)brick_tiles, 256, st, brick_n.p, brick_cells, tiles.p,
+                                        bkey.p, bstart.p, largest, err, (uint64_t *)report.device()));
+            SVO_CUDA_TRY(report.wait());
+            std::memcpy(h, report.words(), sizeof(h));
+        }
         const uint32_t nb = (uint32_t)(h[0] >> 40), h_largest = (uint32_t)h[1], h_err = (uint32_t)(h[1] >> 32);
         const uint64_t pairs = h[0] & ((1ull << 40) - 1);
         if (h_err) return set_error(SVO_ERR_DEVICE, "mesh build: sub-block lists out of range (flags %u)", h_err);

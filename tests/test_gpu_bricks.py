@@ -91,3 +91,34 @@ def test_mesh_pairs_by_brick(svo, oracle, monkeypatch, side, n, threads, mem):
     if side <= 64:
         ow, _ = oracle.build_mesh(pos, faces, side, threads, mem, colors=col)
         assert np.array_equal(got, ow)
+
+
+@pytest.mark.parametrize("n_threads", [1, 24])
+def test_builds_side_by_side(svo, oracle, scenes, n_threads):
+    """More builds, tables and mesh builds at a time than there are page-locked
+    report slots: the rest report through copies."""
+    import threading
+    grid = scenes.sphere_scene(64, 9, 3)
+    want, _ = oracle.build_dense(grid)
+    pos, faces, col = scenes.displaced_icosphere(2, 5)
+    mw, _ = oracle.build_mesh(pos, faces, 40, 4, 1 << 30, colors=col.astype(np.float32))
+    entries = svo.VoxelOctree.from_words(want, np.full(3, 0.5, np.float32)).table_size()
+    go, bad = threading.Barrier(n_threads), []
+
+    def work():
+        go.wait()
+        for _ in range(6):
+            t = svo.VoxelOctree(svo.VoxelData(grid, 1 << 30))
+            if not (np.array_equal(t.words(), want) and t.table_size() == entries):
+                bad.append("dense")
+            m = svo.VoxelOctree(svo.VoxelData(svo.PlyLoader.from_arrays(pos, faces, colors=col.astype(np.float32)), 40,
+                                              1 << 30, 4))
+            if not np.array_equal(m.words(), mw):
+                bad.append("mesh")
+
+    ts = [threading.Thread(target=work) for _ in range(n_threads)]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert not bad
