@@ -272,7 +272,6 @@ __global__ void __launch_bounds__(kBrickThreads, 6) k_brick_bits(GridGeom g, uin
                                                                  uint32_t *__restrict__ list,
                                                                  uint32_t *__restrict__ n_list,
                                                                  unsigned long long *__restrict__ n_voxels) {
-    chain_begin();
     __shared__ __align__(16) uint32_t sbits[2][128];  // alternating: warp 0 may still read the brick before
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -1366,7 +1365,6 @@ __global__ void __launch_bounds__(256) k_pyramid_down(Pyramid p, int level, uint
 // The root and every level down to `level`.
 __global__ void __launch_bounds__(kTopPlaced) k_pyramid_top_down(Pyramid p, int level, uint32_t *__restrict__ words,
                                                            uint64_t W, uint32_t *__restrict__ err) {
-    chain_begin();
     const int t = p.top - p.base;
     if (threadIdx.x == 0) {
         const uint32_t m = t ? p.mask[t][0] : p.mask_of[0];

@@ -128,7 +128,6 @@ __device__ __forceinline__ uint32_t rank_of(const WordOrder &t, uint32_t w) {
 }
 
 __global__ void __launch_bounds__(kTopThreads) k_table_top(WordOrder t) {
-    chain_begin();
     __shared__ uint32_t node[kTopNodes], wsum[kTopThreads / 32];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     if (threadIdx.x == 0) node[0] = 0;

@@ -71,7 +71,7 @@ __device__ __forceinline__ int strip_rows_of(const FrameArgs &f, int s, int &y0)
 // additions for 1280 pixels).
 template <bool kTab>
 __global__ void __launch_bounds__(kFrameThreads) k_corners(FrameArgs f, int warps_x) {
-    chain_begin();
+    chain_next();
     const int lane = threadIdx.x & 31, w = (blockIdx.x * kFrameThreads + threadIdx.x) >> 5, s = blockIdx.y;
     const int tx = (w % warps_x) * 8 + (lane & 7), ty = (w / warps_x) * 4 + (lane >> 3);
     if (tx >= f.tiles_x) return;

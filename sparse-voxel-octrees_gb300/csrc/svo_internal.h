@@ -108,10 +108,10 @@ void host_slot_give(HostSlot *slot);
 
 // A few words that kernels of a call report to the host.  They lie in a host
 // slot's page-locked memory, which the kernels write themselves, so that the
-// host only waits for the stream.  A copy of a few bytes to pageable memory costs
-// 10 us more: the octree, table and first view of a 200x131x177 volume, four
-// such waits, took 207 us with copies and 170 without.  Where no slot can be had they lie on the device and
-// wait() copies them.
+// host only waits for the stream.  A copy of a few bytes to pageable memory
+// costs 10 us more: the octree, table and first view of a 200x131x177 volume,
+// four such waits, took 207 us with copies and 170 without.  Where no slot can
+// be had they lie on the device and wait() copies them.
 class Report {
   public:
     static constexpr uint32_t kWords = 64;

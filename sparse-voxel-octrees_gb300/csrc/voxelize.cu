@@ -211,7 +211,6 @@ __global__ void __launch_bounds__(128, 8) k_tri_pairs(uint64_t n_tris, int per_w
                                                    uint32_t *__restrict__ pair_key, uint32_t *__restrict__ pair_tri,
                                                    uint32_t *__restrict__ pair_cell, uint32_t *__restrict__ brick_n,
                                                    uint32_t *__restrict__ err) {
-    chain_begin();
     const int lane = threadIdx.x & 31;
     const uint64_t t0 = ((uint64_t)blockIdx.x * 4 + (threadIdx.x >> 5)) * (uint64_t)per_warp;
     uint32_t left = 0;  // the warp's large triangles
@@ -575,7 +574,6 @@ __global__ void k_gather_blocks(const uint8_t *__restrict__ flag, uint64_t n, co
 constexpr int kCenterRows = 32, kCenterSpan = 32;
 
 __global__ void __launch_bounds__(kCenterRows) k_center_table(int n_l, int K, float h, float *__restrict__ acc) {
-    chain_begin();
     __shared__ float buf[kCenterRows][kCenterSpan + 1];
     const int l0 = blockIdx.x * kCenterRows, lane = threadIdx.x;
     float c = ((float)(l0 + lane) - 0.5f) * h;
