@@ -595,7 +595,13 @@ __global__ void __launch_bounds__(kBrickThreads) k_place_brick16(GridGeom g, Bri
 }
 
 // The same for 8^3 bricks whose voxels are already compacted (512 words a
-// brick, Morton order): a warp per brick, a lane per 32-cell word.
+// brick, Morton order): a warp per brick, a lane per 32-cell word of its bits.
+// A brick is two waits long: its bits and its place are read together, then
+// the first 128 voxels while the nodes are written.  Compacted voxel i of the
+// level-2 node j goes to k + n_1(through j) + i, so the copy reads whole
+// segments and needs the bounds of eight nodes only.  The 85,187 bricks of a
+// mesh at 1024^3: 33 us; 47 with a read and a write of 32 cells at a time and
+// the place, the bits and the voxels read one after another.
 template <bool kDense>
 __global__ void __launch_bounds__(256) k_place_brick8(BrickPlaces at_of, uint64_t n_dense,
                                                       const uint32_t *__restrict__ bits,
@@ -608,19 +614,24 @@ __global__ void __launch_bounds__(256) k_place_brick8(BrickPlaces at_of, uint64_
     const uint64_t n = kDense ? n_dense : (uint64_t)*at_of.n;
     const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
     for (uint64_t p = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; p < n; p += warps) {
+        const uint64_t j = kDense ? p : (uint64_t)at_of.src[p];
+        const uint32_t w = lane < 16 ? __ldg(bits + j * 16 + lane) : 0u;
         uint64_t b, at, size;
         brick_place<kDense>(at_of, p, b, at, size);
-        const uint64_t j = kDense ? p : (uint64_t)at_of.src[p];
+        const uint32_t m1 = byte_bits(w);
+        const uint32_t own = (uint32_t)__popc(w) | ((uint32_t)__popc(m1) << 16);
+        const uint32_t incl = warp_incl_scan(own), excl = incl - own;  // cells below, level-1 nodes above
+        const uint32_t cells = __shfl_sync(FULL, incl, 31) & 0xFFFFu;
+        const uint32_t *const from = slot + j * 512;
+        uint32_t v[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) v[q] = lane + 32u * q < cells ? __ldg(from + lane + 32 * q) : 0u;
         if (size == 0) continue;
         if (at + size > W) {
             if (lane == 0) atomicOr(err, 4u);
             continue;
         }
         uint32_t *const out = words + at;
-        const uint32_t w = lane < 16 ? __ldg(bits + j * 16 + lane) : 0u;
-        const uint32_t m1 = byte_bits(w), c0 = (uint32_t)__popc(w), c1 = (uint32_t)__popc(m1);
-        const uint32_t own = c0 | (c1 << 16);
-        const uint32_t incl = warp_incl_scan(own), excl = incl - own;
         const uint32_t other = __shfl_xor_sync(FULL, w, 1), m1o = __shfl_xor_sync(FULL, m1, 1);
         const bool first = !(lane & 1), has = (w | other) != 0u;
         const unsigned pairs = __ballot_sync(FULL, first && has);
@@ -628,8 +639,7 @@ __global__ void __launch_bounds__(256) k_place_brick8(BrickPlaces at_of, uint64_
         // the level-2 node of this lane is its even lane and the next
         const uint32_t bj = __shfl_sync(FULL, excl, lane & ~1), tj = __shfl_sync(FULL, incl, lane | 1);
         uint32_t pos = k + (excl >> 16) + (bj & 0xFFFFu);
-        const uint32_t cells = k + (tj >> 16) + (excl & 0xFFFFu);
-        uint32_t child = cells;
+        uint32_t child = k + (tj >> 16) + (excl & 0xFFFFu);
 #pragma unroll
         for (int t = 0; t < 4; ++t) {
             const uint32_t m = (w >> (8 * t)) & 0xFFu;
@@ -642,15 +652,23 @@ __global__ void __launch_bounds__(256) k_place_brick8(BrickPlaces at_of, uint64_
             const uint32_t r = (uint32_t)__popc(pairs & lt), m = m1 | (m1o << 4);
             out[r] = (m << 8) | m | ((k + (excl >> 16) + (excl & 0xFFFFu) - r) << 18);
         }
-        const uint32_t *const from = slot + j * 512;
-        for (unsigned todo = __ballot_sync(FULL, w != 0u); todo; todo &= todo - 1) {
-            const int c = __ffs((int)todo) - 1;
-            const uint32_t wc = __shfl_sync(FULL, w, c), cc = __shfl_sync(FULL, cells, c),
-                           fc = __shfl_sync(FULL, excl, c) & 0xFFFFu;
-            if ((wc >> lane) & 1u) {
-                const uint32_t r = (uint32_t)__popc(wc & lt);
-                out[cc + r] = from[fc + r];
+        uint32_t through[8];  // per level-2 node: cells and level-1 nodes up to its end
+#pragma unroll
+        for (int q = 0; q < 8; ++q) through[q] = __shfl_sync(FULL, incl, 2 * q + 1);
+        for (uint32_t i0 = 0;;) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const uint32_t i = i0 + lane + 32u * q;
+                uint32_t n1 = through[7] >> 16;
+#pragma unroll
+                for (int t = 6; t >= 0; --t)
+                    if (i < (through[t] & 0xFFFFu)) n1 = through[t] >> 16;
+                if (i < cells) out[k + n1 + i] = v[q];
             }
+            i0 += 128;
+            if (i0 >= cells) break;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) v[q] = i0 + lane + 32u * q < cells ? __ldg(from + i0 + lane + 32 * q) : 0u;
         }
     }
 }
@@ -1819,7 +1837,7 @@ int build_from_bricks_device(const MeshBricks &m, int log_side, int log_block, c
     constexpr int kBase = 3;
     const int D = log_side;
     BuildArena arena(st);
-    const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((m.n + 7) / 8, 152 * 32));
+    const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((m.n + 7) / 8, 1ull << 20));
     if (bricks_dense(D, kBase)) {
         auto bricks = [&](BrickPlaces places, uint32_t *words, uint64_t W, uint32_t *err) -> int {
             places.src = m.key;
