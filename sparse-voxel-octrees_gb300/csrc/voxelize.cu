@@ -706,21 +706,24 @@ __device__ __forceinline__ void blend_cell(uint32_t &w, uint32_t &cnt, float nx,
 }
 
 constexpr int kFoldWarps = 4;   // warps per CTA of the fold kernel
-constexpr int kFoldChunk = 8;   // pairs a warp stages per round
+constexpr int kFoldChunk = 8;   // pairs a warp stages per round ...
+constexpr int kDenseChunk = 16; // ... in the direct fold of bricks with many pairs
 constexpr int kFoldCtas = 7;    // per SM: 72 registers a thread (8 CTAs of 64 registers: 596 against 566 us)
+constexpr int kDenseCtas = 5;   // by shared memory
 constexpr int kFoldList = 256;  // hits a warp collects before it folds them
 
+template <int kChunk>
 struct __align__(16) FoldSmem {
-    float T[kFoldChunk][4 * kStageVec];  // p, n, c, area
-    float F[kFoldChunk][kFltFloats];
-    int4 b0[kFoldChunk];                 // brick-local box start x, y, z; first item
-    int4 b1[kFoldChunk];                 // box width in x, y; their 16-bit reciprocals
-    uint32_t w[512];                     // the brick's buffer words, in Morton order ...
-    uint8_t cnt[512];                    // ... and counts (PlyLoader::_counts)
-    float C[kFoldChunk][3][8];           // running centres of the brick's E coordinates per axis
-    int lo[kFoldChunk][3];               // running-sum start: max(triangle box low, sub-block start)
-    uint32_t touched[16];                // the cells folded, a bit each
-    uint16_t list[kFoldList];            // hits: cell x, y, z (3 bits each), staged pair
+    float T[kChunk][4 * kStageVec];  // p, n, c, area
+    float F[kChunk][kFltFloats];
+    int4 b0[kChunk];                 // brick-local box start x, y, z; first item
+    int4 b1[kChunk];                 // box width in x, y; their 16-bit reciprocals
+    uint32_t w[512];                 // the brick's buffer words, in Morton order ...
+    uint8_t cnt[512];                // ... and counts (PlyLoader::_counts)
+    float C[kChunk][3][8];           // running centres of the brick's E coordinates per axis
+    int lo[kChunk][3];               // running-sum start: max(triangle box low, sub-block start)
+    uint32_t touched[16];            // the cells folded, a bit each
+    uint16_t list[kFoldList];        // hits: cell x, y, z (3 bits each), staged pair
 };
 
 // ceil(65536 / n): the reciprocals of divmod_small.
@@ -759,7 +762,8 @@ __device__ __noinline__ bool tri_box_open(float cx, float cy, float cz, float ha
 // Folds a warp's collected hits in list order.  Every hit's sample is formed
 // first, a lane per hit; the writes follow, and where lanes of the 32 share a
 // voxel they write one after another in list order.
-__device__ __forceinline__ void fold_hits(FoldSmem &sm, int n, const float *ratio) {
+template <int kChunk>
+__device__ __forceinline__ void fold_hits(FoldSmem<kChunk> &sm, int n, const float *ratio) {
     const int lane = threadIdx.x & 31;
     const uint32_t lt = (1u << lane) - 1u;
     __syncwarp();
@@ -789,7 +793,7 @@ __device__ __forceinline__ void fold_hits(FoldSmem &sm, int n, const float *rati
 }
 
 // One warp per brick.  The warp loads the brick's buffer cells, then takes
-// the brick's (triangle, sub-block) pairs in list order, kFoldChunk per round:
+// the brick's (triangle, sub-block) pairs in list order, kChunk per round:
 //   1. every (pair, voxel of the pair's clamped box inside the brick) item of
 //      the round is spread over the lanes and tested (triangleToVolume's loop
 //      nest, PlyLoader.cpp:338-374): the box axes are tested per coordinate
@@ -810,14 +814,15 @@ __device__ __forceinline__ void fold_hits(FoldSmem &sm, int n, const float *rati
 // (1.5 of 6.8 stall cycles per instruction were instruction fetches) 509 us,
 // 500 M instructions, 22 lanes, issue 79% active.  Of those instructions the
 // fold takes 46%, the tests 23%, staging 27%.
-template <bool kDirect>
-__global__ void __launch_bounds__(kFoldWarps * 32, kFoldCtas) k_fold_bricks(FoldArgs a) {
+template <bool kDirect, int kChunk = kFoldChunk>
+__global__ void __launch_bounds__(kFoldWarps * 32, kChunk == kDenseChunk ? kDenseCtas : kFoldCtas) k_fold_bricks(FoldArgs a) {
+    static_assert((kChunk & (kChunk - 1)) == 0 && kChunk <= 32, "the search for an item's pair halves kChunk");
     chain_begin();
-    __shared__ FoldSmem smem[kFoldWarps];
+    __shared__ FoldSmem<kChunk> smem[kFoldWarps];
     __shared__ float ratio[256];  // writeTriangleCell's count / (count + 1)
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    FoldSmem &sm = smem[wid];
+    FoldSmem<kChunk> &sm = smem[wid];
     const int le = a.log_e, E = 1 << le, E3 = 1 << (3 * le);
     int end0 = a.org[0] + a.buf[0], end1 = a.org[1] + a.buf[1], end2 = a.org[2] + a.buf[2];
     int drop_z = a.drop_z;
@@ -888,11 +893,12 @@ __global__ void __launch_bounds__(kFoldWarps * 32, kFoldCtas) k_fold_bricks(Fold
         }
         if (lane < 16) sm.touched[lane] = 0;
         const uint32_t s0 = a.bstart[j], s1 = a.bstart[j + 1];
-        for (uint32_t c0 = s0; c0 < s1; c0 += kFoldChunk) {
-            const int nc = (int)min((uint32_t)kFoldChunk, s1 - c0);
+        for (uint32_t c0 = s0; c0 < s1; c0 += kChunk) {
+            const int nc = (int)min((uint32_t)kChunk, s1 - c0);
             __syncwarp();
             const uint32_t tri = lane < nc ? a.pair_tri[c0 + lane] : 0u;
-            for (int i = lane; i < 2 * 32; i += 32) {
+#pragma unroll
+            for (int i = lane; i < (kChunk * kStageVec + 31) / 32 * 32; i += 32) {
                 const int q = i / kStageVec, f = i - q * kStageVec;
                 const uint32_t t = __shfl_sync(FULL, tri, q & 31);
                 if (q < nc)
@@ -982,19 +988,19 @@ __global__ void __launch_bounds__(kFoldWarps * 32, kFoldCtas) k_fold_bricks(Fold
             // exclusive prefix of the items over the staged pairs
             int incl = items;
 #pragma unroll
-            for (int o = 1; o < kFoldChunk; o <<= 1) {
+            for (int o = 1; o < kChunk; o <<= 1) {
                 int n = __shfl_up_sync(FULL, incl, o);
                 if (lane >= o) incl += n;
             }
-            if (lane < kFoldChunk) {
+            if (lane < kChunk) {
                 sm.b0[lane] = make_int4(b0x, b0y, b0z, incl - items);
                 sm.b1[lane] = make_int4(nx, ny, kRcp16[nx], kRcp16[ny]);
             }
-            const int total = __shfl_sync(FULL, incl, kFoldChunk - 1);
+            const int total = __shfl_sync(FULL, incl, kChunk - 1);
             // the filter's constants and the blend's area, four lanes a pair
-            if ((lane >> 2) < nc) {
-                float *T = sm.T[lane >> 2];
-                stage_filter(sm.F[lane >> 2], T + kTriP, oc, cdev, a.half, lane & 3);
+            for (int q = lane >> 2; q < nc; q += 8) {
+                float *T = sm.T[q];
+                stage_filter(sm.F[q], T + kTriP, oc, cdev, a.half, lane & 3);
                 if ((lane & 3) == 3) {
                     const float *p = T + kTriP;
                     const float ax = p[0] - p[3], ay = p[1] - p[4], az = p[2] - p[5];
@@ -1013,7 +1019,7 @@ __global__ void __launch_bounds__(kFoldWarps * 32, kFoldCtas) k_fold_bricks(Fold
                 if (it < total) {
                     int q = 0;
 #pragma unroll
-                    for (int step = kFoldChunk / 2; step; step >>= 1)
+                    for (int step = kChunk / 2; step; step >>= 1)
                         if (sm.b0[q + step].w <= it) q += step;
                     const int4 s4 = sm.b0[q], n4 = sm.b1[q];
                     int r, ix, iy, iz;
@@ -1317,8 +1323,8 @@ bool block_buffer_asked() {
 // PlyLoader::processBlock (PlyLoader.cpp:439-458) of every block at once, then
 // the walk's voxels (VoxelOctree.cpp:66-103) from the slots, and the octree of
 // them.  fa: what every fold launch shares.
-int fold_direct(FoldArgs fa, uint32_t *next, uint32_t nb, const uint8_t *bflag, uint32_t *err, int D, int lb,
-                unsigned fold_grid, unsigned warp_grid, cudaStream_t st, uint32_t **d_words, uint64_t *n_words) {
+int fold_direct(FoldArgs fa, uint32_t *next, uint32_t nb, uint64_t pairs, const uint8_t *bflag, uint32_t *err, int D,
+                int lb, int sms, unsigned warp_grid, cudaStream_t st, uint32_t **d_words, uint64_t *n_words) {
     const uint64_t cap = (uint64_t)nb << (3 * fa.log_e);
     // 8^3 bricks go to the octree as they are, unless a cache block is no
     // larger than a brick (budgets of a few KB)
@@ -1350,8 +1356,15 @@ int fold_direct(FoldArgs fa, uint32_t *next, uint32_t nb, const uint8_t *bflag, 
             fa.n_voxels = n_vox.p;
         }
     }
-    const unsigned grid = (unsigned)std::min<uint64_t>((nb + kFoldWarps - 1) / kFoldWarps, fold_grid);
-    SVO_CUDA_TRY(launch_chained(k_fold_bricks<true>, grid, kFoldWarps * 32, st, fa));
+    // Bricks of many pairs in rounds of 16: fewer half-filled folds, for 20 warps
+    // an SM instead of 28.  Whole builds, rounds of 8 / 16 (us): 327,680
+    // triangles at 128^3 (280 pairs a brick) 645 / 558, 200^3 430 / 407, 256^3
+    // 403 / 382, 400^3 402 / 395, 512^3 433 / 437, 1024^3 (11 a brick) 775 / 822.
+    const bool dense = pairs >= 64ull * nb;
+    const unsigned grid = (unsigned)std::min<uint64_t>((nb + kFoldWarps - 1) / kFoldWarps,
+                                                       (uint64_t)sms * (dense ? kDenseCtas : kFoldCtas));
+    SVO_CUDA_TRY(launch_chained(dense ? k_fold_bricks<true, kDenseChunk> : k_fold_bricks<true>, grid, kFoldWarps * 32, st,
+                                fa));
     if (as_bricks) {
         const MeshBricks mb{nb, fa.bkey, ccount.p, nmask.p, cbits.p, slot.p, n_vox.p};
         return build_from_bricks_device(mb, D, lb, lb < D ? bflag : nullptr, st, d_words, n_words);
@@ -1661,7 +1674,7 @@ int build_mesh_device(const svo_mesh *m, int side, int threads, uint64_t mem, cu
                 return e;
             };
             SVO_CUDA_TRY(sub_bricks ? sort_bricks(std::false_type()) : sort_bricks(std::true_type()));
-            return fold_direct(fold_args(ptri.p, pcell.p), fold_next.p, nb, bflag, err, D, lb, fold_grid, warp_grid, st,
+            return fold_direct(fold_args(ptri.p, pcell.p), fold_next.p, nb, pairs, bflag, err, D, lb, sms, warp_grid, st,
                                d_words, n_words);
         }
     }
@@ -1817,8 +1830,8 @@ int build_mesh_device(const svo_mesh *m, int side, int threads, uint64_t mem, cu
     SVO_CUDA_TRY(cudaMemsetAsync(fold_next.p, 0, n_next * sizeof(uint32_t), st));
 
     if (direct)
-        return fold_direct(fold_args(stri, scell), fold_next.p, nb, bflag, err, D, lb, fold_grid, warp_grid, st, d_words,
-                           n_words);
+        return fold_direct(fold_args(stri, scell), fold_next.p, nb, n_pairs, bflag, err, D, lb, sms, warp_grid, st,
+                           d_words, n_words);
 
     // PlyLoader::processBlock (PlyLoader.cpp:439-458) of job ji, whose buffer
     // `data` starts at org with edges buf: its bricks' pairs folded into it

@@ -76,6 +76,7 @@ def _fan(n, rng):
     (64, 4600, 4, 1 << 30),                         # and more than that sorts
     (16, 30, 512, 1 << 30), (40, 60, 4096, 1 << 30),  # sub-blocks inside a brick: several pairs of one triangle
     (40, 60, 512, 5 * 16 ** 3 + 3000),              # and several cache blocks
+    (16, 600, 4, 1 << 30), (16, 3001, 512, 1 << 30),  # hundreds of pairs in every brick: rounds of 16
     (1027, 50, 8, 1 << 30),                         # beyond the table of brick codes
 ])
 def test_mesh_pairs_by_brick(svo, oracle, monkeypatch, side, n, threads, mem):
