@@ -812,8 +812,9 @@ __device__ __forceinline__ void fold_hits(FoldSmem<kChunk> &sm, int n, const flo
 // staging without integer divisions gave 730 us; samples a lane per hit and
 // cells in Morton order 566; tri_box and the fold out of the unrolled code
 // (1.5 of 6.8 stall cycles per instruction were instruction fetches) 509 us,
-// 500 M instructions, 22 lanes, issue 79% active.  Of those instructions the
-// fold takes 46%, the tests 23%, staging 27%.
+// 500 M instructions, 22 lanes, issue 79% active, of those instructions the
+// fold 46%, the tests 23%, staging 27%; staging unrolled 493 us.  Samples held
+// over to the next round, so that every fold has 32, cost 515 us.
 template <bool kDirect, int kChunk = kFoldChunk>
 __global__ void __launch_bounds__(kFoldWarps * 32, kChunk == kDenseChunk ? kDenseCtas : kFoldCtas) k_fold_bricks(FoldArgs a) {
     static_assert((kChunk & (kChunk - 1)) == 0 && kChunk <= 32, "the search for an item's pair halves kChunk");
