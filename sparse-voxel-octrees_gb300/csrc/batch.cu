@@ -4,11 +4,12 @@
 // Work is a global space of ray slots: each view contributes either one slot
 // per ray (linear views) or 32 slots per tile_w x tile_h pixel tile (image
 // views, so a warp's lanes start on neighbouring pixels).  Without lane refill
-// or table cache a launch has a thread per slot (k_trace_slots).  Otherwise a
-// persistent grid of SMs x blocks_per_sm CTAs drains the space: each warp takes `chunk`
-// consecutive slots from one device counter with a single atomicAdd and hands
-// them to its idle lanes in ballot-rank order.  Lanes whose ray finishes go
-// idle; once at least `refill_idle` lanes of a warp are idle the warp refills
+// or table cache a launch of up to kSlotsMost slots has a thread per slot
+// (k_trace_slots).  Otherwise a persistent grid of SMs x blocks_per_sm CTAs
+// drains the space: each warp takes `chunk` consecutive slots from one device
+// counter with a single atomicAdd and hands them to its idle lanes in
+// ballot-rank order.  Lanes whose ray finishes go idle; once at least
+// `refill_idle` lanes of a warp are idle the warp refills
 // them, so lanes keep doing traversal steps instead of waiting for the
 // slowest ray of a fixed 32-ray batch.  Nothing waits on another warp or CTA.
 //
@@ -330,8 +331,11 @@ __global__ void __maxnreg__(48) k_trace_persistent_r48(BatchArgs a) {
 // pays for the queue, for its longest warps at the end of each CTA's share and
 // for registers (48 to 64 against 40): 12 octrees of depth 7 to 10 took 444 us
 // with its 48-register build and take 393, 3 small ones 128 and 100, 48 ones
-// 1,589 and 1,574.
+// 1,589 and 1,574.  More than kSlotsMost slots keep the persistent form: 96
+// octrees (47 M rays) take 3,118 us with it and 3,139 without, 32 1080p images
+// and their shadow rays (93 M) 11.1 and 11.5 ms.
 constexpr int kSlotThreads = 128;
+constexpr uint64_t kSlotsMost = 1ull << 25;
 
 template <bool kTab, bool kLod>
 __global__ void __launch_bounds__(kSlotThreads) k_trace_slots(BatchArgs a) {
@@ -352,16 +356,21 @@ __global__ void __launch_bounds__(kSlotThreads) k_trace_slots(BatchArgs a) {
 }
 
 // One image view, passed by value (svo_trace_image): an 8x4-pixel tile per
-// warp, in small CTAs that the hardware starts one after another.  A large
-// image is bound by instruction issue and gains nothing over a persistent
-// grid fed from a counter (1080p over a 2048^3 terrain: 291 us either way);
-// a small one, bound by its longest ray's chain of steps, saves the counter's
-// reset and reads (256x256 over 128^3: 27.7 to 25.3 us a call).  32, 64, 128
-// and 256 threads: 25.6, 25.4, 25.3, 25.3 us and 313, 292, 291, 293 us.
-// Fewer rays per warp (16, 8 or 4, for shorter divergent chains) gave at most
-// 10% on images below 4,096 pixels and cost more above.
-constexpr int kImageThreads = 128;
+// warp, in small CTAs that the hardware starts one after another, or (kQueue,
+// images of more than kImageQueue tile slots) a persistent grid whose warps
+// take the next tile from a counter.  An image is bound by instruction issue,
+// a small one by its longest ray's chain of steps.  The small CTAs save the
+// counter's reset and reads, but a CTA's slots wait for its slowest warp.
+// Counter / small CTAs (us): 256x256 over 128^3 27.7 / 25.3; 1080p images of a
+// 2048^3 terrain 275 / 256, two stacked 501 / 486, four 960 / 972, eight 1,690 /
+// 1,745, 32 6,752 / 7,032.  32, 64, 128 and 256 threads without the counter:
+// 25.6, 25.4, 25.3, 25.3 us and 313, 292, 291, 293 us.  Several tiles a warp one
+// after another instead of the counter: 32 images 7,450 to 7,800 us.  Fewer
+// rays per warp (16, 8 or 4, for shorter divergent chains) gave at most 10% on
+// images below 4,096 pixels and cost more above.
+constexpr int kImageThreads = 128, kImageQueueThreads = 256;
 constexpr int kImageTileW = 8, kImageTileH = 4;
+constexpr uint64_t kImageQueue = 1ull << 22;
 
 template <bool kTab, bool kLod>
 __global__ void __launch_bounds__(kImageThreads) k_trace_single(JobDev J, uint32_t *status, uint32_t *carry) {
@@ -384,6 +393,43 @@ __global__ void __launch_bounds__(kImageThreads) k_trace_single(JobDev J, uint32
     a.jobs = &J;
     a.status = status;
     write_result(a, 0, out_idx, res, p1.y, p2.x, p2.y);
+}
+
+// The loop over [base, end) runs once; the code compiled for this form is 2%
+// faster than for the tile's body alone (32 1080p images 6,762 and 6,902 us).
+template <bool kTab, bool kLod>
+__global__ void k_trace_image_queue(JobDev J, uint64_t slots, unsigned long long *queue, uint32_t *status,
+                                    uint32_t *carry) {
+    const int lane = threadIdx.x & 31;
+    if (blockIdx.x == 0 && threadIdx.x == 0) carry_status(carry, status);
+    RayStackFor<kTab> stk;
+    BatchArgs a;  // only the fields write_result reads
+    a.jobs = &J;
+    a.status = status;
+    while (true) {
+        unsigned long long base = 0;
+        if (lane == 0) base = atomicAdd(queue, 32ull);
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (base >= slots) break;
+        const unsigned long long end = min(base + 32ull, (unsigned long long)slots);
+        for (unsigned long long s0 = base; s0 < end; s0 += 32) {
+            const uint64_t slot = s0 + lane;
+            if (slot >= end) continue;
+            const uint32_t tile = (uint32_t)(slot >> 5), r = (uint32_t)(slot & 31);
+            const uint32_t ty = tile / J.tiles_x, tx = tile - ty * J.tiles_x;
+            const uint32_t px = tx * kImageTileW + (r & 7u), py = ty * kImageTileH + (r >> 3);
+            if (px >= J.width || py >= J.height) continue;
+            const uint32_t out_idx = py * J.width + px;
+            const float2 *r2 = reinterpret_cast<const float2 *>(J.rays) + 3 * (uint64_t)out_idx;
+            float2 p0 = __ldg(r2), p1 = __ldg(r2 + 1), p2 = __ldg(r2 + 2);
+            RayState st;
+            ray_init_any<kTab>(st, J.oct, J.tab, p0.x, p0.y, p1.x, p1.y, p2.x, p2.y);
+            RayResult res;
+            while (!ray_step_any<kTab, kLod>(st, stk, J.oct, J.tab, J.n_words, J.ray_scale, res)) {
+            }
+            write_result(a, 0, out_idx, res, p1.y, p2.x, p2.y);
+        }
+    }
 }
 
 int log2_of(int v) {
@@ -430,11 +476,31 @@ int launch_trace_image(const svo_octree *oct, const float *d_rays, uint32_t widt
     J.rgba8 = out.rgba8;
     J.tab = octree_table(oct, st);
     const uint64_t slots = (uint64_t)J.tiles_x * ((height + kImageTileH - 1) / kImageTileH) * 32;  // at most 2^35
+    uint32_t *const to = status ? status : oct->d_status, *const carry = status ? oct->d_status : nullptr;
+    if (slots > kImageQueue) {
+        void (*kern)(JobDev, uint64_t, unsigned long long *, uint32_t *, uint32_t *) =
+            J.tab ? (ray_scale != 0.0f ? k_trace_image_queue<true, true> : k_trace_image_queue<true, false>)
+                  : (ray_scale != 0.0f ? k_trace_image_queue<false, true> : k_trace_image_queue<false, false>);
+        int dev = 0, sms = 0, resident = 0;
+        SVO_CUDA_TRY(cudaGetDevice(&dev));
+        SVO_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        SVO_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kern, kImageQueueThreads, 0));
+        void *q = nullptr;
+        SVO_CUDA_TRY(scratch_alloc(&q, sizeof(unsigned long long), st));
+        cudaError_t e = cudaMemsetAsync(q, 0, sizeof(unsigned long long), st);
+        if (e == cudaSuccess) {
+            kern<<<(unsigned)(sms * std::max(1, resident)), kImageQueueThreads, 0, st>>>(J, slots,
+                                                                                        (unsigned long long *)q, to, carry);
+            e = cudaGetLastError();
+        }
+        cudaFreeAsync(q, st);
+        if (e != cudaSuccess) return cuda_fail(e, "svo_trace_image");
+        return SVO_OK;
+    }
     void (*kern)(JobDev, uint32_t *, uint32_t *) =
         J.tab ? (ray_scale != 0.0f ? k_trace_single<true, true> : k_trace_single<true, false>)
               : (ray_scale != 0.0f ? k_trace_single<false, true> : k_trace_single<false, false>);
-    kern<<<(unsigned)((slots + kImageThreads - 1) / kImageThreads), kImageThreads, 0, st>>>(
-        J, status ? status : oct->d_status, status ? oct->d_status : nullptr);
+    kern<<<(unsigned)((slots + kImageThreads - 1) / kImageThreads), kImageThreads, 0, st>>>(J, to, carry);
     SVO_CUDA_TRY(cudaGetLastError());
     return SVO_OK;
 }
@@ -562,7 +628,7 @@ int enqueue_trace(svo_batch *b, const svo_trace_config &c, cudaStream_t st) {
     SVO_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kern, c.block_threads, smem));
     int per_sm = std::max(1, std::min(c.blocks_per_sm, resident));
     const uint64_t ctas = std::max<uint64_t>(1, (b->total + kSlotThreads - 1) / kSlotThreads);
-    if (!cache && (c.refill_idle == 0 || c.refill_idle == 32) && c.blocks_per_sm >= resident && ctas <= 0x7FFFFFFFull) {
+    if (!cache && (c.refill_idle == 0 || c.refill_idle == 32) && c.blocks_per_sm >= resident && b->total <= kSlotsMost) {
         BatchKernel slots = b->all_tab ? (b->any_lod ? k_trace_slots<true, true> : k_trace_slots<true, false>)
                                        : (b->any_lod ? k_trace_slots<false, true> : k_trace_slots<false, false>);
         slots<<<(unsigned)ctas, kSlotThreads, 0, st>>>(a);
@@ -798,12 +864,14 @@ int svo_batch_autotune(svo_batch *b, svo_trace_config *best, float *best_ms, svo
     };
     // table cache depths: none; 64 entries (levels 0-1 hold at most 9 nodes,
     // level 2 at most 64 more); 256 entries (levels 0-2 hold at most 73)
-    // (without a cache the launch does not depend on the CTA and chunk sizes)
+    // (without a cache, launches of a thread per slot do not depend on the CTA
+    // and chunk sizes)
     for (int cache : {0, 64, 256})
         for (int bt : {128, 256, 512})
             for (int tw : {4, 8, 16})
                 for (int chunk : {32, 128})
-                    if (cache || (bt == 256 && chunk == 32)) add(bt, 0, 1, tw, chunk, cache);  // whole-warp tiles, no refill
+                    if (cache || b->total > kSlotsMost || (bt == 256 && chunk == 32))
+                        add(bt, 0, 1, tw, chunk, cache);  // whole-warp tiles, no refill
     // lane refill, default build (64 registers) or 48-register build
     for (int cap : {0, 48})
         for (int bt : {128, 256})

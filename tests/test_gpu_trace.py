@@ -475,3 +475,50 @@ def test_page_locked_host_calls_in_chunks(cuda, svo, oracle, scenes, W, H):
             out["leaf"], out["word"] = out["leaf"].view(np.uint32), out["word"].view(np.uint32)
             _assert_same(out, ref)
     _assert_same(tree.trace_image_host(rays, W, H, outputs=("hit", "t", "leaf", "word", "rgb")), ref)
+
+
+def test_large_sets_of_rays(cuda, svo, scenes):
+    """Images and ray lists on both sides of the sizes from which their warps
+    take work from a counter, and a batch above its own: the rays traced in
+    parts."""
+    torch = cuda
+    grid = scenes.sphere_scene(64, 9, 3)
+    tree = svo.VoxelOctree(svo.VoxelData(grid, 1 << 30))
+    light = np.float32([0.3, -0.5, 0.8])
+
+    def outputs(n):
+        return {"hit": torch.zeros(n, dtype=torch.uint8, device="cuda"), "t": torch.zeros(n, device="cuda"),
+                "leaf": torch.zeros(n, dtype=torch.int32, device="cuda"),
+                "rgba8": torch.zeros(n, dtype=torch.int32, device="cuda")}
+
+    def equal(a, b):
+        return all(torch.equal(a[k].view(torch.int8), b[k].view(torch.int8)) for k in a)
+
+    cam = scenes.orbit_cameras(1, 5, tree.center())[0]
+    for W, H in ((2051, 2045), (2049, 2053), (4001, 1061)):  # about 2^22 slots, ragged tiles
+        rays = scenes.gpu_camera_rays(cam, W, H)
+        n = W * H
+        want, image, linear = outputs(n), outputs(n), outputs(n)
+        for i in range(0, n, 1 << 20):
+            m = min(1 << 20, n - i)
+            tree.trace(rays[i:i + m], light=light, out={k: v[i:i + m] for k, v in want.items()})
+        tree.trace_image(rays, W, H, light=light, out=image)
+        tree.trace(rays, light=light, out=linear)
+        torch.cuda.synchronize()
+        assert 0 < int(want["hit"].sum()) < n
+        assert equal(image, want) and equal(linear, want)
+        # the counter is each call's own, also from a captured graph
+        st = torch.cuda.Stream()
+        st.wait_stream(torch.cuda.current_stream())
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=st):
+            tree.trace_image(rays, W, H, light=light, out=image, stream=st)
+            tree.trace(rays, light=light, out=linear, stream=st)
+        for _ in range(2):
+            for o in (image, linear):
+                for v in o.values():
+                    v.zero_()
+            graph.replay()
+            torch.cuda.synchronize()
+            assert equal(image, want) and equal(linear, want)
+    assert tree.device_status() == 0
