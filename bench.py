@@ -566,7 +566,7 @@ def run_ours(args):
     traffic, traffic_source = profiled_traffic(Rp)
     roofline = {"bound": "hbm", "achieved": round(achieved, 1), "peak": peaks["hbm_gbs"], "unit": "GB/s",
                 "frac": round(achieved / peaks["hbm_gbs"], 4), "traffic": traffic, "traffic_source": traffic_source,
-                "kernel": "k_trace_single (svo_trace_image, primary rays)", "peak_kind": peak_kind,
+                "kernel": "k_trace_image_queue (svo_trace_image, primary rays)", "peak_kind": peak_kind,
                 "algorithmic_bytes_per_launch": bytes_prim, "bytes_per_ray": round(bytes_prim / Rp, 2),
                 "launch_ms": round(t_prim_avg, 3), "issue_bound": profiled_issue()}
 
@@ -874,8 +874,8 @@ def run_batched(args, torch, svo, scenes, tune_cache=None):
            "speedup_vs_best_plain": round(ms_best_plain / ms_batched, 3),
            "best_plain": "svo_trace_image" if ms_image <= ms_plain else "svo_trace",
            "exact_hit_parity": bool(exact and exact_image),
-           "plain_apis": {"plain": "96 svo_trace launches (persistent, 32 rays per queue access, row order)",
-                          "plain_image": "96 svo_trace_image launches (persistent, 8x4-pixel tiles)"},
+           "plain_apis": {"plain": "96 svo_trace launches (row order)",
+                          "plain_image": "96 svo_trace_image launches (8x4-pixel tiles)"},
            "config": cfg.as_dict(), "autotune_s": round(tune_s, 1), "setup_s": round(setup_s, 1),
            "launches": {"plain": len(views), "plain_image": len(views), "batched": 1}}
     depth_hi = min(11, args.max_side.bit_length() - 1) if args.max_side else 11

@@ -190,7 +190,8 @@ __device__ __forceinline__ int point_to_grid(float p, float s) { return (int)(p 
 // another.  A thread's loop is a chain (in mode 2 of atomics that return): the
 // build of 1,280 triangles of hundreds of bricks each at 1024^3 takes 3.5 ms
 // with it, 1.6 ms so.  Of 327,680 small triangles a pass takes 32 us, bound by
-// the scattered atomics (one per brick and warp by match_any: 36 us).
+// instruction issue at 11 of 32 lanes (issue 68% active, DRAM 19%; with one
+// atomic per brick and warp by match_any 36 us).
 constexpr int kWarpTriangle = 32;
 
 // Morton code of three 10-bit coordinates (brick codes have at most 30 bits).
@@ -813,7 +814,7 @@ __device__ __forceinline__ void fold_hits(FoldSmem<kChunk> &sm, int n, const flo
 // cells in Morton order 566; tri_box and the fold out of the unrolled code
 // (1.5 of 6.8 stall cycles per instruction were instruction fetches) 509 us,
 // 500 M instructions, 22 lanes, issue 79% active, of those instructions the
-// fold 46%, the tests 23%, staging 27%; staging unrolled 493 us.  Samples held
+// fold 46%, the tests 23%, staging 27%; staging unrolled 493 us, 480 M.  Samples held
 // over to the next round, so that every fold has 32, cost 515 us.
 template <bool kDirect, int kChunk = kFoldChunk>
 __global__ void __launch_bounds__(kFoldWarps * 32, kChunk == kDenseChunk ? kDenseCtas : kFoldCtas) k_fold_bricks(FoldArgs a) {
