@@ -166,10 +166,13 @@ static bool page_locked(const float *rays, const svo_trace_out &out) {
 // 4, 200 in 6, 206 in 8; 640x480: 137, 120, 126, 130, 135, 135; 1920x1080: 515,
 // 419, 392, 384, 379, 381; 3840x2160: 1,445 in two, 1,270 in four.  A pageable
 // copy is staged by the driver, waits for it and costs about 60 us each, so
-// those calls keep whole chunks (1024x768: 256 us in one, 455 in four).
-static uint64_t chunk_rays(const float *rays, uint64_t n, const svo_trace_out &out) {
+// those calls keep whole chunks (1024x768: 256 us in one, 455 in four).  So do
+// calls that do not wait: the next call's copies overlap their traces, and
+// smaller chunks only add to the queue (twelve 1024x768 views and one
+// synchronize: 1,405 us whole, 1,541 in quarters).
+static uint64_t chunk_rays(const float *rays, uint64_t n, const svo_trace_out &out, bool wait) {
     constexpr uint64_t kParts = 4, kLeast = 160 * 1024;
-    if (n <= kLeast || !page_locked(rays, out)) return kStageRays;
+    if (!wait || n <= kLeast || !page_locked(rays, out)) return kStageRays;
     return std::min(kStageRays, std::max((n + kParts - 1) / kParts, kLeast));
 }
 
@@ -764,7 +767,7 @@ static int trace_host(svo_octree *oct, const float *rays, uint64_t n, float ray_
     }
     if (n) {
         // warp-aligned chunks
-        const std::vector<uint64_t> plan = plan_chunks(n, chunk_rays(rays, n, *out), 32);
+        const std::vector<uint64_t> plan = plan_chunks(n, chunk_rays(rays, n, *out, wait), 32);
         const float lt[3] = {light ? light[0] : 0.0f, light ? light[1] : 0.0f, light ? light[2] : 0.0f};
         int rc = host_enqueue(oct, rays, plan, *out,
                               [&](const float *d_rays, uint64_t m, const svo_trace_out &o, cudaStream_t st) {
@@ -796,7 +799,7 @@ static int trace_image_host(svo_octree *oct, const float *rays, uint32_t width, 
     if (width && height) {
         // Chunks of whole rows, a multiple of the 4-row tile height (all but
         // the last); each chunk is traced as an image of its own.
-        const uint64_t rows = std::max<uint64_t>(4, (chunk_rays(rays, n, *out) / width) & ~uint64_t(3));
+        const uint64_t rows = std::max<uint64_t>(4, (chunk_rays(rays, n, *out, wait) / width) & ~uint64_t(3));
         std::vector<uint64_t> plan = plan_chunks(height, rows, 4);
         for (auto &c : plan) c *= width;
         const float lt[3] = {light ? light[0] : 0.0f, light ? light[1] : 0.0f, light ? light[2] : 0.0f};
