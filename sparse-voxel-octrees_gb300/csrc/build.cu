@@ -272,7 +272,11 @@ __global__ void __launch_bounds__(kBrickThreads, 6) k_brick_bits(GridGeom g, uin
                                                                  uint32_t *__restrict__ list,
                                                                  uint32_t *__restrict__ n_list,
                                                                  unsigned long long *__restrict__ n_voxels) {
-    __shared__ __align__(16) uint32_t sbits[2][128];  // alternating: warp 0 may still read the brick before
+    // Alternating: warp 0 may still read the brick before.  Every brick that
+    // takes a buffer passes a barrier after writing it, so the bits written to
+    // a buffer follow, by the barrier of the brick between, the reads of its
+    // last use.
+    __shared__ __align__(16) uint32_t sbits[2][128];
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     int turn = 0;
@@ -281,10 +285,11 @@ __global__ void __launch_bounds__(kBrickThreads, 6) k_brick_bits(GridGeom g, uin
     for (uint64_t b = blockIdx.x; b < n_bricks; b += gridDim.x) {
         const int gx0 = (int)(compact3(b) << 4), gy0 = (int)(compact3(b >> 1) << 4), gz0 = (int)(compact3(b >> 2) << 4);
         uint32_t any = 0;
+        const bool inside = gx0 < g.w && gy0 < g.h && gz0 < g.d;  // else the cube's padding
         uint32_t *const sb = sbits[turn];
-        turn ^= 1;
-        if (gx0 >= g.w || gy0 >= g.h || gz0 >= g.d) {
-            // outside: the cube's padding
+        if (inside) turn ^= 1;
+        if (!inside) {
+            // no barrier is passed here, so the buffer stays for the next brick
         } else if (vec4) {
             // warp w takes the columns (y / 4, z / 2) = w, w + 8, w + 16, w + 24
             uint4 v[4];

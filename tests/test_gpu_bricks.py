@@ -45,6 +45,28 @@ def test_dense_builds(svo, oracle, scenes, shape, density, edge):
     assert np.array_equal(tree.center(), oc)
 
 
+@pytest.mark.parametrize("shape,offset", [
+    ((9, 20, 2101), 0),    # rows off the 16-byte boundary
+    ((70, 20, 2050), 0),
+    ((20, 2101, 40), 1),   # whole rows, the first off it
+    ((2101, 36, 17), 3),
+])
+def test_unaligned_rows_in_large_cubes(cuda, svo, oracle, scenes, shape, offset):
+    """4096^3 cubes, in which a CTA visits sixteen bricks and those inside the
+    grid have padding between them, read a word at a time: the bits of one
+    brick while the next one's are formed."""
+    torch = cuda
+    g = scenes.random_grid(shape, 0.3, sum(shape))
+    flat = torch.zeros(g.size + offset, dtype=torch.int32, device="cuda")
+    dev = flat[offset:].view(shape)
+    dev.copy_(torch.from_numpy(g.view(np.int32)))
+    ow, oc = oracle.build_dense(g)
+    for _ in range(3):
+        tree = svo.VoxelOctree(svo.VoxelData(dev, 1 << 30))
+        assert np.array_equal(tree.words(), ow)
+        assert np.array_equal(tree.center(), oc)
+
+
 @pytest.mark.parametrize("side,thin,threads,mem", [
     (8, 1.0, 2, 1 << 30),         # one 8^3 brick
     (60, 0.5, 5, 1 << 30),
