@@ -192,7 +192,16 @@ __device__ __forceinline__ int point_to_grid(float p, float s) { return (int)(p 
 // with it, 1.6 ms so.  Of 327,680 small triangles a pass takes 32 us, bound by
 // instruction issue at 11 of 32 lanes (issue 68% active, DRAM 19%; with one
 // atomic per brick and warp by match_any 36 us).
+//
+// brick_n is counted only while the pairs can still be laid out: *wide_pairs
+// sums those of the large triangles before they are counted, and from
+// kPairLimit on, where the build refuses, they are left out of brick_n (not of
+// count).  So brick_n sums to less than 2^38: 2^37 pairs of small triangles
+// (32 bricks each, of fewer than 2^32 triangles, or fewer than 2^23 where a
+// brick lies in up to 512 sub-blocks), kPairLimit, and one member of at most
+// 2^21 bricks for each of the fewer than 2^14 warps on the chip.
 constexpr int kWarpTriangle = 32;
+constexpr uint64_t kPairLimit = 0xFFFFFFFFull;
 
 // Morton code of three 10-bit coordinates (brick codes have at most 30 bits).
 __device__ __forceinline__ uint32_t morton3_32(uint32_t x, uint32_t y, uint32_t z) {
@@ -211,7 +220,7 @@ __global__ void __launch_bounds__(128, 8) k_tri_pairs(uint64_t n_tris, int per_w
                                                    uint32_t *__restrict__ count, const uint64_t *__restrict__ out_off,
                                                    uint32_t *__restrict__ pair_key, uint32_t *__restrict__ pair_tri,
                                                    uint32_t *__restrict__ pair_cell, uint32_t *__restrict__ brick_n,
-                                                   uint32_t *__restrict__ err) {
+                                                   unsigned long long *wide_pairs, uint32_t *__restrict__ err) {
     const int lane = threadIdx.x & 31;
     const uint64_t t0 = ((uint64_t)blockIdx.x * 4 + (threadIdx.x >> 5)) * (uint64_t)per_warp;
     uint32_t left = 0;  // the warp's large triangles
@@ -296,9 +305,15 @@ __global__ void __launch_bounds__(128, 8) k_tri_pairs(uint64_t n_tris, int per_w
             }
             const uint32_t pairs = (uint32_t)b[0] * (uint32_t)b[1] * (uint32_t)b[2];
             const uint32_t cell = (uint32_t)gx + (uint32_t)g.grid[0] * ((uint32_t)gy + (uint32_t)g.grid[1] * (uint32_t)gz);
+            bool each = kMode != 0 || brick_n != nullptr;
+            if (kMode == 0 && each && step != 1) {  // the whole warp, on one triangle and cell
+                volatile unsigned long long *const sum = wide_pairs;
+                if (first == 0 && *sum < kPairLimit) atomicAdd(wide_pairs, (unsigned long long)pairs);
+                __syncwarp();
+                each = *sum < kPairLimit;
+            }
             int x = 0, y = 0, z = 0;
-            for (uint32_t f = first; f < pairs; f += step) {
-                if (kMode == 0 && !brick_n) break;
+            for (uint32_t f = first; each && f < pairs; f += step) {
                 if (step != 1) {
                     const uint32_t yz = f / (uint32_t)b[0];
                     x = (int)(f - yz * (uint32_t)b[0]);
@@ -361,7 +376,8 @@ __global__ void __launch_bounds__(128, 8) k_tri_pairs(uint64_t n_tris, int per_w
 constexpr int kWarpSort = 128, kSortedInBrick = 4096;
 constexpr int kBrickTile = 2048;  // 256 threads x 8
 
-// Bricks and pairs of a tile: bricks above bit 40, pairs below.
+// Bricks and pairs of a tile: bricks above bit 40, pairs below (k_tri_pairs
+// keeps them under 2^38).
 __device__ __forceinline__ uint64_t tile_sum(const uint32_t *n, uint64_t i0, uint64_t cells, uint32_t (&c)[8]) {
     uint64_t s = 0;
 #pragma unroll
@@ -388,11 +404,13 @@ __global__ void __launch_bounds__(256) k_brick_tiles(const uint32_t *__restrict_
 
 // The non-empty bricks' keys and first pairs, in key order, and in n each
 // brick's first pair in place of its count.  Reports the bricks and pairs
-// (packed as above), the largest brick and the error word.
+// (packed as above), the largest brick and the error word, and the large
+// triangles' pairs.
 __global__ void __launch_bounds__(256) k_brick_layout(uint32_t *__restrict__ n, uint64_t cells,
                                                       const uint64_t *__restrict__ tiles, uint32_t *__restrict__ bkey,
                                                       uint32_t *__restrict__ bstart, const uint32_t *largest,
-                                                      const uint32_t *err, uint64_t *__restrict__ report) {
+                                                      const uint32_t *err, const unsigned long long *wide_pairs,
+                                                      uint64_t *__restrict__ report) {
     chain_begin();
     uint64_t before = 0, total;
     for (uint32_t t = threadIdx.x; t < blockIdx.x; t += 256) before += tiles[t];
@@ -414,6 +432,7 @@ __global__ void __launch_bounds__(256) k_brick_layout(uint32_t *__restrict__ n, 
         bstart[(before + total) >> 40] = (uint32_t)(before + total);
         report[0] = before + total;
         report[1] = *largest | ((uint64_t)*err << 32);
+        report[2] = *wide_pairs;
     }
 }
 
@@ -1526,12 +1545,13 @@ int build_mesh_device(const svo_mesh *m, int side, int threads, uint64_t mem, cu
         return set_error(SVO_ERR_LIMIT, "voxel-centre table of %d x %d entries is too large", n_l, K);
 
     const uint64_t nt = m->n_tris;
-    // the largest brick's pairs, the error word and the block flags
+    // the largest brick's pairs, the error word, the large triangles' pairs and the block flags
     Dev<uint32_t> info;
-    SVO_ALLOC(info, 2 + (g.n_blocks + 3) / 4);
-    SVO_CUDA_TRY(cudaMemsetAsync(info.p, 0, 8 + g.n_blocks, st));
+    SVO_ALLOC(info, 4 + (g.n_blocks + 3) / 4);
+    SVO_CUDA_TRY(cudaMemsetAsync(info.p, 0, 16 + g.n_blocks, st));
     uint32_t *const largest = info.p, *const err = info.p + 1;
-    uint8_t *const bflag = (uint8_t *)(info.p + 2);
+    unsigned long long *const wide_pairs = (unsigned long long *)(info.p + 2);
+    uint8_t *const bflag = (uint8_t *)(info.p + 4);
 
     // the running centres, first: they depend on the size alone
     Dev<float> acc;
@@ -1604,7 +1624,7 @@ int build_mesh_device(const svo_mesh *m, int side, int threads, uint64_t mem, cu
     const unsigned pair_grid = (unsigned)((nt + 4 * per_warp - 1) / (4 * per_warp));
     if (nt) {
         k_tri_pairs<0><<<pair_grid, 128, 0, st>>>(nt, per_warp, m->d_tris, g, box.p, bflag, pcount.p, nullptr, nullptr,
-                                                  nullptr, nullptr, brick_n.p, err);
+                                                  nullptr, nullptr, brick_n.p, wide_pairs, err);
         SVO_LAUNCH_OK("k_tri_pairs<count>");
     }
     const unsigned fold_grid = (unsigned)(sms * kFoldCtas), warp_grid = (unsigned)sms * 16;
@@ -1643,28 +1663,29 @@ int build_mesh_device(const svo_mesh *m, int side, int threads, uint64_t mem, cu
     Dev<uint32_t> fold_next;  // one work counter per fold launch
 
     if (table) {
-        uint64_t h[2];
+        uint64_t h[3];
         {
             Report report;
             SVO_CUDA_TRY(report.open(st));
             SVO_CUDA_TRY(launch_chained(k_brick_tiles, (unsigned)brick_tiles, 256, st, brick_n.p, brick_cells, tiles.p,
                                         largest));
             SVO_CUDA_TRY(launch_chained(k_brick_layout, (unsigned)brick_tiles, 256, st, brick_n.p, brick_cells, tiles.p,
-                                        bkey.p, bstart.p, largest, err, (uint64_t *)report.device()));
+                                        bkey.p, bstart.p, largest, err, wide_pairs, (uint64_t *)report.device()));
             SVO_CUDA_TRY(report.wait());
             std::memcpy(h, report.words(), sizeof(h));
         }
         const uint32_t nb = (uint32_t)(h[0] >> 40), h_largest = (uint32_t)h[1], h_err = (uint32_t)(h[1] >> 32);
         const uint64_t pairs = h[0] & ((1ull << 40) - 1);
         if (h_err) return set_error(SVO_ERR_DEVICE, "mesh build: sub-block lists out of range (flags %u)", h_err);
-        if (nb > 0 && h_largest <= (uint32_t)kSortedInBrick && pairs < 0xFFFFFFFFull && direct_fits(nb)) {
+        if (nb > 0 && h_largest <= (uint32_t)kSortedInBrick && h[2] < kPairLimit && pairs < kPairLimit &&
+            direct_fits(nb)) {
             Dev<uint32_t> ptri, pcell;
             SVO_ALLOC(ptri, pairs);
             if (!sub_bricks) SVO_ALLOC(pcell, pairs);
             SVO_ALLOC(fold_next, 1);
             SVO_CUDA_TRY(cudaMemsetAsync(fold_next.p, 0, sizeof(uint32_t), st));
             k_tri_pairs<2><<<pair_grid, 128, 0, st>>>(nt, per_warp, m->d_tris, g, box.p, bflag, nullptr, nullptr, nullptr,
-                                                              ptri.p, pcell.p, brick_n.p, err);
+                                                              ptri.p, pcell.p, brick_n.p, nullptr, err);
             SVO_LAUNCH_OK("k_tri_pairs<emit>");
             auto sort_bricks = [&](auto cells) -> cudaError_t {
                 constexpr bool kCells = decltype(cells)::value;
@@ -1687,7 +1708,7 @@ int build_mesh_device(const svo_mesh *m, int side, int threads, uint64_t mem, cu
         int rc = scan_total<uint32_t, uint64_t>(pcount.p, poff.p, nt, &n_pairs, st);
         if (rc) return rc;
     }
-    if (n_pairs >= 0xFFFFFFFFull)
+    if (n_pairs >= kPairLimit)
         return set_error(SVO_ERR_LIMIT, "%llu brick/triangle pairs exceed 2^32-1", (unsigned long long)n_pairs);
     Dev<uint32_t> pk, pt, pc, pi, pk2, pi2, stri_buf, scell_buf, sort_scratch;
     SVO_ALLOC(pk, n_pairs);
@@ -1698,7 +1719,7 @@ int build_mesh_device(const svo_mesh *m, int side, int threads, uint64_t mem, cu
     SVO_ALLOC(pi2, n_pairs);
     if (n_pairs) {
         k_tri_pairs<1><<<pair_grid, 128, 0, st>>>(nt, per_warp, m->d_tris, g, box.p, bflag, pcount.p, poff.p, pk.p,
-                                                          pt.p, pc.p, nullptr, err);
+                                                          pt.p, pc.p, nullptr, nullptr, err);
         SVO_LAUNCH_OK("k_tri_pairs<emit>");
         k_iota<<<grid_for(n_pairs), 256, 0, st>>>(pi.p, n_pairs);
         SVO_LAUNCH_OK("k_iota");

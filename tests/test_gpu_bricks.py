@@ -116,6 +116,25 @@ def test_mesh_pairs_by_brick(svo, oracle, monkeypatch, side, n, threads, mem):
         assert np.array_equal(got, ow)
 
 
+@pytest.mark.parametrize("n", [4096, 1 << 19])
+@pytest.mark.parametrize("threads", [1, 16])
+def test_more_pairs_than_can_be_laid_out(svo, n, threads):
+    """Triangles across a 1024^3 cube in sub-blocks of all or a sixteenth of
+    it, 2^31 to 2^40 (brick, triangle) pairs: refused, after a count that
+    leaves the table of bricks in range, and the next build is right."""
+    pos = np.array([[0, 0, 0], [1, 1, 0.1], [0.2, 0.9, 1]], np.float32)
+    mem = 8 << 30  # one cache block
+
+    def build(k):
+        loader = svo.PlyLoader.from_arrays(pos, np.tile(np.arange(3, dtype=np.int32), (k, 1)))
+        return svo.VoxelOctree(svo.VoxelData(loader, 1024, mem, threads))
+
+    with pytest.raises(svo.SvoError) as e:
+        build(n)
+    assert e.value.code == svo.SVO_ERR_LIMIT
+    assert build(1).num_words() > 100_000
+
+
 @pytest.mark.parametrize("n_threads", [1, 24])
 def test_builds_side_by_side(svo, oracle, scenes, n_threads):
     """More builds, tables and mesh builds at a time than there are page-locked
