@@ -16,6 +16,18 @@
 // kHandleDirect bytes or more, which it would not keep for long, are the
 // driver's, for the pool maps memory more slowly: with a 1 GB table the first
 // trace of a 2048^3 terrain waited 3.2 ms for it, 2.3 ms with the driver's.
+//
+// A pool hands out freed memory again at once, so the device has to be done
+// with an octree before its memory goes back.  cudaDeviceSynchronize cannot be
+// that wait: it is refused while any stream of any thread is captured, and it
+// ends the capture.  cudaFree waits for all streams (also non-blocking ones: a
+// 20 ms kernel held it for 20 ms) and minds no capture of another thread in
+// thread-local or relaxed mode, so the wait is the cudaFree of 256 bytes taken
+// for it: 2 us where another small block keeps their 2 MB mapped, 58 where not
+// (a rebuilt and viewed 200x131x177 volume 169 us with the device's
+// synchronisation, 175 with this).
+// What cannot be waited for (in a global capture, where cudaFree is refused
+// too) is parked until the next octree is destroyed or memory is trimmed.
 #include <cstring>
 #include <mutex>
 #include <vector>
@@ -37,6 +49,8 @@ cudaStream_t g_streams[kMaxDevices] = {};
 constexpr int kMaxSlots = 16;
 std::vector<HostSlot *> g_free_slots[kMaxDevices];
 int g_slots[kMaxDevices] = {};
+std::vector<HandleMemory> g_parked[kMaxDevices];
+void *g_small[kMaxDevices] = {};  // keeps the block that wait_for_device's 256 bytes come from mapped
 
 cudaError_t pool_for_current_device(Pool which, cudaMemPool_t *out) {
     int dev = 0;
@@ -60,9 +74,26 @@ cudaError_t pool_for_current_device(Pool which, cudaMemPool_t *out) {
             return e;
         }
         slot = pool;
+        if (!g_small[dev] && cudaMalloc(&g_small[dev], 256) != cudaSuccess) {
+            g_small[dev] = nullptr;
+            cudaGetLastError();
+        }
     }
     *out = slot;
     return cudaSuccess;
+}
+
+// Waits for everything that the device runs, or is refused (see the top).
+cudaError_t wait_for_device() {
+    void *p = nullptr;
+    cudaError_t e = cudaMalloc(&p, 256);
+    if (e == cudaSuccess) e = cudaFree(p);
+    else if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        e = cudaDeviceSynchronize();
+    }
+    if (e != cudaSuccess) cudaGetLastError();  // a refusal is no later call's error
+    return e;
 }
 
 cudaError_t pool_alloc(Pool which, void **p, size_t bytes, cudaStream_t st) {
@@ -81,6 +112,30 @@ cudaError_t handle_alloc(void **p, size_t bytes, cudaStream_t st) {
 
 cudaError_t handle_free(void *p, size_t bytes, cudaStream_t st) {
     return bytes < kHandleDirect ? cudaFreeAsync(p, st) : cudaFree(p);
+}
+
+void handle_retire(const HandleMemory *blocks, int n) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return;
+    std::vector<HandleMemory> ready(blocks, blocks + n);
+    {
+        // what is parked before the wait may go after it
+        std::lock_guard<std::mutex> lk(g_pool_mtx);
+        ready.insert(ready.end(), g_parked[dev].begin(), g_parked[dev].end());
+        g_parked[dev].clear();
+    }
+    cudaStream_t st = nullptr;
+    const bool waited = library_stream(&st) == cudaSuccess && wait_for_device() == cudaSuccess;
+    std::vector<HandleMemory> left;
+    for (const HandleMemory &m : ready) {
+        if (!m.p) continue;
+        if (waited && handle_free(m.p, m.bytes, st) == cudaSuccess) continue;
+        if (waited) cudaGetLastError();  // refused since: a capture has begun
+        left.push_back(m);
+    }
+    if (left.empty()) return;
+    std::lock_guard<std::mutex> lk(g_pool_mtx);
+    g_parked[dev].insert(g_parked[dev].end(), left.begin(), left.end());
 }
 
 size_t words_bytes(uint64_t n) { return (size_t)(status_offset(n) + kStatusWords) * sizeof(uint32_t); }
@@ -210,6 +265,7 @@ extern "C" int svo_trim_memory(void) {
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return svo::cuda_fail(e, "cudaGetDevice");
     if (dev >= 0 && dev < svo::kMaxDevices) svo::host_slots_trim(dev);
+    svo::handle_retire(nullptr, 0);  // what is parked
     cudaMemPool_t pools[svo::kPools] = {};
     {
         std::lock_guard<std::mutex> lk(svo::g_pool_mtx);

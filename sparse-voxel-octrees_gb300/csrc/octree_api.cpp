@@ -499,16 +499,13 @@ int svo_octree_destroy(svo_octree *oct) {
         std::lock_guard<std::mutex> lock(oct->staging_mtx);
         host_drain(oct);
     }
-    // what the octree's own device still runs may use its memory: wait for
-    // it, after which the pool may hand the memory out again
+    // what the octree's own device still runs may use its memory
     int dev = oct->device;
     cudaGetDevice(&dev);
     if (dev != oct->device) cudaSetDevice(oct->device);
-    cudaStream_t st = nullptr;
-    cudaDeviceSynchronize();
-    library_stream(&st);
-    free_words(oct->d_words, oct->n_words, st);
-    if (oct->d_tab) handle_free(oct->d_tab, (size_t)oct->n_tab * sizeof(uint4), st);
+    const HandleMemory memory[2] = {{oct->d_words, words_bytes(oct->n_words)},
+                                    {oct->d_tab, (size_t)oct->n_tab * sizeof(uint4)}};
+    handle_retire(memory, 2);
     if (dev != oct->device) cudaSetDevice(dev);
     if (oct->stage_dev) cudaFree(oct->stage_dev);
     if (oct->copy_in) cudaStreamDestroy(oct->copy_in);

@@ -83,6 +83,15 @@ cudaError_t scratch_alloc(void **p, size_t bytes, cudaStream_t st);
 cudaError_t handle_alloc(void **p, size_t bytes, cudaStream_t st);
 cudaError_t handle_free(void *p, size_t bytes, cudaStream_t st);
 
+// The same for memory of the current device that its streams may still use:
+// waits for the device first, and keeps the memory aside where that is refused.
+struct HandleMemory {
+    void *p;
+    size_t bytes;
+};
+void handle_retire(const HandleMemory *blocks, int n);
+size_t words_bytes(uint64_t n);  // of alloc_words
+
 // An octree's words from that pool, with the handle's zeroed error word behind
 // them, at status_offset(n) words.
 constexpr uint64_t kStatusWords = 32;

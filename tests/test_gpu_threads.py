@@ -75,3 +75,67 @@ def test_host_calls_from_16_threads(svo, oracle, scenes):
             if ref["hit"][j] == 1:
                 assert word == int(ref["word"][j]) and np.float32(t) == ref["t"][j], (i, j)
     assert hits > N_THREADS * 500
+
+
+@pytest.mark.parametrize("mode,own_thread", [("thread_local", False), ("relaxed", False), ("relaxed", True)])
+def test_destroy_beside_a_capture(cuda, svo, scenes, mode, own_thread):
+    """An octree destroyed while another call is being captured: the capture
+    goes on, and the octree's memory goes back only once the device is idle."""
+    torch = cuda
+    tree = svo.VoxelOctree(svo.VoxelData(scenes.sphere_scene(64, 9, 3)))
+    other = svo.VoxelOctree(svo.VoxelData(scenes.sphere_scene(64, 9, 4)))
+    rays = torch.from_numpy(scenes.random_rays(4096, 5)).cuda()
+    out = {"t": torch.zeros(4096, device="cuda")}
+    tree.trace(rays, out=out)
+    torch.cuda.synchronize()
+    want = out["t"].clone()
+    assert bool(torch.isfinite(want).any())
+    busy, ended, idle = torch.cuda.Stream(), torch.cuda.Event(), []
+
+    def destroy():
+        other.close()
+        idle.append(ended.query())
+
+    graph = torch.cuda.CUDAGraph()
+    st = torch.cuda.Stream()
+    with torch.cuda.graph(graph, stream=st, capture_error_mode=mode):
+        tree.trace(rays, out=out, stream=st)
+        with torch.cuda.stream(busy):
+            torch.cuda._sleep(40_000_000)  # about 20 ms
+            ended.record(busy)
+        if own_thread:
+            destroy()
+        else:
+            t = threading.Thread(target=destroy)
+            t.start()
+            t.join()
+    assert idle == [True]
+    out["t"].zero_()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out["t"], want)
+
+
+def test_destroy_inside_a_global_capture(cuda, svo):
+    """Where no wait is allowed the memory is kept aside: no later octree gets
+    it, and svo_trim_memory returns it once the capture has ended."""
+    import ctypes
+    torch = cuda
+    rt = ctypes.CDLL("/usr/local/cuda/lib64/libcudart.so")
+    grid = torch.ones((256, 256, 256), dtype=torch.int32, device="cuda")
+    tree = svo.VoxelOctree(svo.VoxelData(grid))
+    held, size = tree.device_words_ptr(), 4 * tree.num_words()
+    torch.cuda.synchronize()
+    st = torch.cuda.Stream()
+    handle, graph = ctypes.c_void_p(st.cuda_stream), ctypes.c_void_p()
+    assert rt.cudaStreamBeginCapture(handle, 0) == 0
+    tree.close()
+    assert rt.cudaStreamEndCapture(handle, ctypes.byref(graph)) != 0  # as with any free in such a capture
+    rt.cudaGetLastError()
+    later = [svo.VoxelOctree(svo.VoxelData(grid)) for _ in range(2)]
+    at = [t.device_words_ptr() for t in later]
+    assert all(p + size <= held or held + size <= p for p in at)
+    before = torch.cuda.mem_get_info()[0]
+    svo.trim_memory()
+    assert torch.cuda.mem_get_info()[0] - before >= size
+    assert later[0].num_words() * 4 == size
