@@ -174,8 +174,9 @@ __global__ void __launch_bounds__(kTopThreads) k_table_top(WordOrder t) {
 // notes the list's length for the next level; no CTA waits for another.
 __global__ void __launch_bounds__(256) k_table_expand(WordOrder t, int L) {
     chain_begin();
-    // after an error the list may hold places that were never written
-    if (t.ctl[kCtlErr]) return;
+    // after an error the list may hold places that were never written (the
+    // whole CTA decides: another one of this launch may be setting the flag)
+    if (__syncthreads_or(t.ctl[kCtlErr] != 0)) return;
     __shared__ uint32_t base;
     const uint32_t begin = L > kTopLevels ? t.ctl[kCtlEnd + L - 1] : 0u, end = min(t.ctl[kCtlEnd + L], t.cap);
     for (uint32_t i0 = begin + blockIdx.x * blockDim.x; i0 < end; i0 += gridDim.x * blockDim.x) {

@@ -414,6 +414,41 @@ def test_table_orders(cuda, svo, oracle, scenes, kind):
     _assert_same(_device_trace(cuda, svo, tree, rays), ref)
 
 
+def _nodes(words):
+    """(word, level, child block, stride, internal children) of every node."""
+    out, level, L = [], [0], 0
+    while level:
+        below = []
+        for p in level:
+            d = int(words[p])
+            off = d >> 18
+            if d & 0x20000:
+                off = (off << 32) | int(words[p + 1])
+            k, stride = bin(d & 0xFF).count("1"), 2 if d & 0x10000 else 1
+            out.append((p, L, p + off, stride, k))
+            below += [p + off + j * stride for j in range(k)]
+        level, L = below, L + 1
+    return out
+
+
+@pytest.mark.parametrize("level,part", [(4, 1.0), (5, 0.002), (5, 0.5), (6, 0.01)])
+def test_table_refused_while_levels_are_expanded(cuda, svo, oracle, scenes, level, part):
+    """Bad nodes all over a level that many CTAs expand at the same time: the
+    table is refused, and again by a second build, and good octrees after it
+    have theirs."""
+    words, center = oracle.build_dense(scenes.random_grid((128, 128, 128), 0.3, 4))
+    nodes = [n for n in _nodes(words) if n[1] == level]
+    rng = np.random.default_rng(level)
+    bad = words.copy()
+    for p, _, _, _, _ in (nodes[i] for i in rng.choice(len(nodes), max(1, int(part * len(nodes))), replace=False)):
+        bad[p] = (int(bad[p]) & ~0xFF00) | 0x100 | 0xFE  # internal children that are not valid
+    for _ in range(3):
+        tree = svo.VoxelOctree.from_words(bad, center)
+        assert tree.table_size() == 0
+        good = svo.VoxelOctree.from_words(words, center)
+        assert good.table_size() == good.validate()[0]
+
+
 @pytest.mark.parametrize("n", [1, 33, 16384, 16385])
 def test_host_calls_around_the_in_place_limit(cuda, svo, oracle, scenes, n):
     """Waiting host calls of up to 16,384 rays are traced in page-locked memory
