@@ -244,24 +244,31 @@ __global__ void __launch_bounds__(kScanThreads) k_table_rank(WordOrder t, uint64
     if (!first && blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) report[kCtlWords - 1] = before + total;
 }
 
+// The entry of a child block's first internal child.  A far block's children
+// are consecutive entries only if the far words between them are no
+// descriptors.
+__device__ __forceinline__ uint32_t child_entry(const WordOrder &t, uint32_t n_top, uint32_t cb, uint32_t stride,
+                                                uint32_t k, uint32_t *err) {
+    if (!k) return 0u;
+    if (stride == 2)
+        for (uint32_t f = cb + 1; f < cb + 2 * k - 1; f += 2)
+            if ((t.bits[f >> 5] >> (f & 31)) & 1u) atomicOr(err, kErrOrder);
+    return n_top + rank_of(t, cb);
+}
+
 __global__ void __launch_bounds__(256) k_table_entries(WordOrder t, uint4 *__restrict__ tab, uint32_t *__restrict__ err) {
     const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t n_top = t.ctl[kCtlTop];
     if (i < n_top) {  // table_node has passed for every node here
         uint32_t cb, stride, k, first = t.top[2 * i + 1];
         table_node(t.words, t.n_words, t.top[2 * i], 0, cb, stride, k);
-        if (i >= t.ctl[kCtlInner]) first = k ? n_top + rank_of(t, cb) : 0u;
+        if (i >= t.ctl[kCtlInner]) first = child_entry(t, n_top, cb, stride, k, err);
         tab[i] = make_uint4(t.words[t.top[2 * i]], first, cb, 0u);
     }
     if (i >= t.n_words || !((t.bits[i >> 5] >> (i & 31)) & 1u)) return;
     uint32_t cb, stride, k;
     table_node(t.words, t.n_words, (uint32_t)i, 0, cb, stride, k);
-    // a far block's children are consecutive entries only if the far words
-    // between them are no descriptors
-    if (k && stride == 2)
-        for (uint32_t f = cb + 1; f < cb + 2 * k - 1; f += 2)
-            if ((t.bits[f >> 5] >> (f & 31)) & 1u) atomicOr(err, kErrOrder);
-    tab[n_top + rank_of(t, (uint32_t)i)] = make_uint4(t.words[i], k ? n_top + rank_of(t, cb) : 0u, cb, 0u);
+    tab[n_top + rank_of(t, (uint32_t)i)] = make_uint4(t.words[i], child_entry(t, n_top, cb, stride, k, err), cb, 0u);
 }
 
 struct Scratch {

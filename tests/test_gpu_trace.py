@@ -449,6 +449,33 @@ def test_table_refused_while_levels_are_expanded(cuda, svo, oracle, scenes, leve
         assert good.table_size() == good.validate()[0]
 
 
+@pytest.mark.parametrize("above", [1, 2, 3, 4, 6])
+def test_table_with_a_node_between_far_slots(cuda, svo, oracle, scenes, above):
+    """Two children of a far block with another node's child in the slot
+    between them, on the levels around the breadth-first top (level 3's
+    children are the first of the word order)."""
+    one = (1 << 18) | (0x80 << 8) | 0x80
+    words = [one] * above + [
+        (1 << 18) | (0xC0 << 8) | 0xC0,             # two children, N and M
+        (2 << 18) | 0x10000 | (0xC0 << 8) | 0xC0,   # N: A and B, a far block's two words apart
+        (2 << 18) | (0x80 << 8) | 0x80,             # M: C, the word between them
+        (3 << 18) | (0x80 << 8),                    # A: one voxel
+        (3 << 18) | (0xFF << 8),                    # C: eight
+        (10 << 18) | (0x40 << 8),                   # B: one
+        100] + [200 + k for k in range(8)] + [300]
+    words = np.array(words, np.uint32)
+    center = np.full(3, 0.5, np.float32)
+    rng = np.random.default_rng(above)
+    rays = scenes.random_rays(20_000, 29)
+    to = 2.0 - rng.random((20_000, 3), dtype=np.float32) * np.float32(2.0 ** -above) - rays[:, :3]
+    rays[:, 3:] = to / np.linalg.norm(to, axis=1, keepdims=True)
+    tree = svo.VoxelOctree.from_words(words, center)
+    assert tree.table_size() == above + 6
+    ref = oracle.raymarch(words, rays, threads=4)
+    assert set(np.unique(ref["word"])) >= {0, 100, 200, 207, 300}
+    _assert_same(_device_trace(cuda, svo, tree, rays), ref)
+
+
 @pytest.mark.parametrize("n", [1, 33, 16384, 16385])
 def test_host_calls_around_the_in_place_limit(cuda, svo, oracle, scenes, n):
     """Waiting host calls of up to 16,384 rays are traced in page-locked memory
