@@ -177,6 +177,7 @@ cudaError_t library_stream(cudaStream_t *out) {
 
 static void host_slot_free(HostSlot *s) {
     if (s->st) cudaStreamDestroy(s->st);
+    if (s->order) cudaEventDestroy(s->order);
     if (s->host) cudaFreeHost(s->host);
     delete s;
 }
@@ -194,13 +195,14 @@ HostSlot *host_slot_take() {
         if (g_slots[dev] >= kMaxSlots) return nullptr;
         ++g_slots[dev];
     }
-    HostSlot *s = new HostSlot{dev, nullptr, nullptr, nullptr};
+    HostSlot *s = new HostSlot{dev, nullptr, nullptr, nullptr, nullptr};
     void *h = nullptr, *d = nullptr;
     cudaError_t e = cudaHostAlloc(&h, kHostSlotBytes, cudaHostAllocMapped);
     s->host = (char *)h;
     if (e == cudaSuccess) e = cudaHostGetDevicePointer(&d, h, 0);
     s->dev = (char *)d;
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&s->st, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->order, cudaEventDisableTiming);
     if (e == cudaSuccess) return s;
     cudaGetLastError();  // the call takes the staged path instead
     host_slot_free(s);

@@ -309,6 +309,10 @@ static_assert(kSmallRays * 53 + 8 * 256 <= kHostSlotBytes, "a slot holds the ray
 // and one wait, no copies on the device.  Sets `done` unless no slot can be
 // had.  launch(d_rays, outputs, stream, status) enqueues the trace.  Called
 // without staging_mtx, with nothing pending on the handle.
+//
+// The call reports what earlier traces left in the handle's error word, so the
+// kernel, which reads it, follows the work of the default stream and those
+// that synchronise with it, as the staged path's blocking copy of the word does.
 template <typename Launch>
 static int trace_small(const float *rays, uint64_t n, const svo_trace_out &out, Launch launch, bool &done) {
     done = false;
@@ -335,6 +339,8 @@ static int trace_small(const float *rays, uint64_t n, const svo_trace_out &out, 
     uint32_t &status = *(uint32_t *)(s->host + o_status);
     status = 0;
     std::memcpy(s->host + o_rays, rays, n * 24);
+    SVO_CUDA_TRY(cudaEventRecord(s->order, cudaStreamLegacy));
+    SVO_CUDA_TRY(cudaStreamWaitEvent(s->st, s->order, 0));
     const int rc = launch((const float *)(s->dev + o_rays), o, s->st, (uint32_t *)(s->dev + o_status));
     const cudaError_t e = cudaStreamSynchronize(s->st);  // also after a failure: the slot goes back idle
     if (rc) return rc;

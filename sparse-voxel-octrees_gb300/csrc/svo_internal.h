@@ -111,6 +111,7 @@ struct HostSlot {
     int device;
     char *host, *dev;  // the same memory
     cudaStream_t st;
+    cudaEvent_t order;  // to put the stream behind another's work
 };
 HostSlot *host_slot_take();
 void host_slot_give(HostSlot *slot);

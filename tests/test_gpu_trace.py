@@ -512,6 +512,28 @@ def test_host_calls_around_the_in_place_limit(cuda, svo, oracle, scenes, n):
     assert not bad.trace_host(away)["hit"].any()
 
 
+@pytest.mark.parametrize("n", [1, 128, 16384, 16385])
+@pytest.mark.parametrize("image", [False, True])
+def test_host_calls_report_queued_traces(cuda, svo, n, image):
+    """A waiting host call of any size reports the bounds check of a trace that
+    the default stream still has to run, and no later call does."""
+    torch = cuda
+    bad = svo.VoxelOctree.from_words(np.array([(0x3FFF << 18) | 0xFFFF], np.uint32), (0.5, 0.5, 0.5))
+    down = torch.tensor([[1.5, 1.5, -1.0, 0.0, 0.0, 1.0]], device="cuda")
+    out = {"hit": torch.empty(1, dtype=torch.uint8, device="cuda")}
+    away = np.tile(np.array([[5.0, 5.0, 5.0, 0.6, 0.0, 0.8]], np.float32), (n, 1))
+    w = 128 if n % 128 == 0 else n
+    call = (lambda: bad.trace_image_host(away, w, n // w)) if image else (lambda: bad.trace_host(away))
+    assert not call()["hit"].any()  # the table is refused here, not below
+    for _ in range(3):
+        torch.cuda._sleep(20_000_000)  # about 10 ms
+        bad.trace(down, out=out)
+        with pytest.raises(svo.SvoError) as e:
+            call()
+        assert e.value.code == svo.SVO_ERR_DEVICE
+        assert not call()["hit"].any()
+
+
 @pytest.mark.parametrize("W,H", [(640, 256), (641, 257), (1024, 643)])
 def test_page_locked_host_calls_in_chunks(cuda, svo, oracle, scenes, W, H):
     """Page-locked arrays go through the host pipeline in chunks (from 163,841
