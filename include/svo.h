@@ -116,7 +116,10 @@ int svo_octree_table_size(svo_octree *oct, uint64_t *entries);
 /* Copies the words to host memory `dst` (n_words entries). */
 int svo_octree_copy_words(const svo_octree *oct, uint32_t *dst, uint64_t n_words);
 
-/* Device pointer to the resident words (valid until svo_octree_destroy). */
+/* Device pointer to the resident words (valid until svo_octree_destroy).  The
+ * words of svo_octree_load and svo_octree_from_words are one cudaMalloc
+ * allocation (cudaIpcGetMemHandle takes it); built octrees' are mostly pool
+ * memory of the library. */
 int svo_octree_device_words(const svo_octree *oct, const uint32_t **d_words);
 
 /* Replaces VoxelOctree::center(), VoxelOctree.hpp:55-57. */

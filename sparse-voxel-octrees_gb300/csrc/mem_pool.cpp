@@ -8,7 +8,8 @@
 // for the next build until svo_trim_memory() returns it.
 //
 // Octrees themselves (words and descriptor tables) live in a second pool that
-// keeps at most kHandleKeep of freed memory mapped, so that a program that
+// keeps at most kHandleKeep of freed memory mapped (the words of loaded octrees
+// and of those made from words are the driver's), so that a program that
 // replaces an octree every frame does not map and unmap it each time: a
 // rebuilt 200x131x177 volume spent 130 us freeing the octree before it and 100
 // allocating its own, of 385.  A pool holding more than that in live octrees
@@ -129,7 +130,7 @@ void handle_retire(const HandleMemory *blocks, int n) {
     std::vector<HandleMemory> left;
     for (const HandleMemory &m : ready) {
         if (!m.p) continue;
-        if (waited && handle_free(m.p, m.bytes, st) == cudaSuccess) continue;
+        if (waited && (m.plain ? cudaFree(m.p) : handle_free(m.p, m.bytes, st)) == cudaSuccess) continue;
         if (waited) cudaGetLastError();  // refused since: a capture has begun
         left.push_back(m);
     }
@@ -140,22 +141,24 @@ void handle_retire(const HandleMemory *blocks, int n) {
 
 size_t words_bytes(uint64_t n) { return (size_t)(status_offset(n) + kStatusWords) * sizeof(uint32_t); }
 
-cudaError_t alloc_words(uint32_t **words, uint64_t n, cudaStream_t st) {
+cudaError_t alloc_words(uint32_t **words, uint64_t n, cudaStream_t st, bool plain) {
     void *p = nullptr;
     const uint64_t at = status_offset(n);
-    cudaError_t e = handle_alloc(&p, words_bytes(n), st);
+    cudaError_t e = plain ? cudaMalloc(&p, words_bytes(n)) : handle_alloc(&p, words_bytes(n), st);
     if (e != cudaSuccess) return e;
     e = cudaMemsetAsync((uint32_t *)p + at, 0, kStatusWords * sizeof(uint32_t), st);
     if (e != cudaSuccess) {
-        handle_free(p, words_bytes(n), st);
+        free_words((uint32_t *)p, n, st, plain);
         return e;
     }
     *words = (uint32_t *)p;
     return cudaSuccess;
 }
 
-void free_words(uint32_t *words, uint64_t n, cudaStream_t st) {
-    if (words) handle_free(words, words_bytes(n), st);
+void free_words(uint32_t *words, uint64_t n, cudaStream_t st, bool plain) {
+    if (!words) return;
+    if (plain) cudaFree(words);
+    else handle_free(words, words_bytes(n), st);
 }
 
 cudaError_t library_stream(cudaStream_t *out) {

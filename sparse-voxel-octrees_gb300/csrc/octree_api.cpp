@@ -95,14 +95,16 @@ static int upload_words(const uint32_t *words, uint64_t n, const float center[3]
     uint32_t *d = nullptr;
     cudaStream_t st = nullptr;
     SVO_CUDA_TRY(library_stream(&st));
-    SVO_CUDA_TRY(alloc_words(&d, n, st));
+    SVO_CUDA_TRY(alloc_words(&d, n, st, true));
     cudaError_t e = cudaMemcpyAsync(d, words, n * sizeof(uint32_t), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) {
-        free_words(d, n, st);
+        free_words(d, n, st, true);
         return cuda_fail(e, "upload octree words");
     }
-    return make_handle(d, n, center, out);
+    const int rc = make_handle(d, n, center, out);
+    if (rc == SVO_OK) (*out)->plain_words = true;
+    return rc;
 }
 
 static int ensure_staging(svo_octree *oct, size_t dev_bytes) {
@@ -509,8 +511,8 @@ int svo_octree_destroy(svo_octree *oct) {
     int dev = oct->device;
     cudaGetDevice(&dev);
     if (dev != oct->device) cudaSetDevice(oct->device);
-    const HandleMemory memory[2] = {{oct->d_words, words_bytes(oct->n_words)},
-                                    {oct->d_tab, (size_t)oct->n_tab * sizeof(uint4)}};
+    const HandleMemory memory[2] = {{oct->d_words, words_bytes(oct->n_words), oct->plain_words},
+                                    {oct->d_tab, (size_t)oct->n_tab * sizeof(uint4), false}};
     handle_retire(memory, 2);
     if (dev != oct->device) cudaSetDevice(dev);
     if (oct->stage_dev) cudaFree(oct->stage_dev);

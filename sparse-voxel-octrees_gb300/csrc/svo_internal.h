@@ -19,6 +19,7 @@
 struct svo_octree {
     uint32_t *d_words = nullptr;  // resident octree words (HBM)
     uint64_t n_words = 0;
+    bool plain_words = false;  // from cudaMalloc, not the library's pool
     float center[3] = {0.0f, 0.0f, 0.0f};
     int device = 0;
     int levels = 0;  // descriptor levels, 0: not known
@@ -88,16 +89,19 @@ cudaError_t handle_free(void *p, size_t bytes, cudaStream_t st);
 struct HandleMemory {
     void *p;
     size_t bytes;
+    bool plain;  // from cudaMalloc
 };
 void handle_retire(const HandleMemory *blocks, int n);
 size_t words_bytes(uint64_t n);  // of alloc_words
 
 // An octree's words from that pool, with the handle's zeroed error word behind
-// them, at status_offset(n) words.
+// them, at status_offset(n) words.  plain: from cudaMalloc instead, for words
+// that were so before the pool: such memory can be shared with other processes
+// and devices.
 constexpr uint64_t kStatusWords = 32;
 inline uint64_t status_offset(uint64_t n_words) { return (n_words + 31) / 32 * 32; }
-cudaError_t alloc_words(uint32_t **words, uint64_t n, cudaStream_t st);
-void free_words(uint32_t *words, uint64_t n, cudaStream_t st);  // of alloc_words, or null
+cudaError_t alloc_words(uint32_t **words, uint64_t n, cudaStream_t st, bool plain = false);
+void free_words(uint32_t *words, uint64_t n, cudaStream_t st, bool plain = false);  // of alloc_words, or null
 
 // A non-blocking stream per device, shared by the library's own work.
 cudaError_t library_stream(cudaStream_t *out);

@@ -512,6 +512,23 @@ def test_host_calls_around_the_in_place_limit(cuda, svo, oracle, scenes, n):
     assert not bad.trace_host(away)["hit"].any()
 
 
+@pytest.mark.parametrize("side", [16, 256])
+def test_loaded_words_can_be_shared(cuda, svo, scenes, tmp_path, side):
+    """The words of loaded octrees are plain device memory, whose handle other
+    processes can open."""
+    import ctypes
+    rt = ctypes.CDLL("/usr/local/cuda/lib64/libcudart.so")
+    tree = svo.VoxelOctree(svo.VoxelData(scenes.sphere_scene(side, 9, 3)))
+    path = str(tmp_path / "t.oct")
+    tree.save(path)
+    for t in (svo.VoxelOctree(path), svo.VoxelOctree.from_words(tree.words(), tree.center())):
+        handle = ctypes.create_string_buffer(64)
+        assert rt.cudaIpcGetMemHandle(handle, ctypes.c_void_p(t.device_words_ptr())) == 0
+        assert any(handle.raw)
+        assert np.array_equal(t.words(), tree.words())
+        t.close()
+
+
 @pytest.mark.parametrize("n", [1, 128, 16384, 16385])
 @pytest.mark.parametrize("image", [False, True])
 def test_host_calls_report_queued_traces(cuda, svo, n, image):
