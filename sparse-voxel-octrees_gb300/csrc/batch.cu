@@ -356,9 +356,12 @@ __global__ void __launch_bounds__(kSlotThreads) k_trace_slots(BatchArgs a) {
 }
 
 // One image view, passed by value (svo_trace_image): an 8x4-pixel tile per
-// warp, in small CTAs that the hardware starts one after another, or (kQueue,
-// images of more than kImageQueue tile slots) a persistent grid whose warps
-// take the next tile from a counter.  An image is bound by instruction issue,
+// warp, in small CTAs that the hardware starts one after another, or (images of
+// more than kImageQueue tile slots) a persistent grid whose warps take the next
+// tile from a counter.  A call that is captured keeps the small CTAs: the
+// counter, which each call takes from the pool, would put allocation nodes into
+// the caller's graph, and such a graph has one instance at a time and is no
+// child of another.  An image is bound by instruction issue,
 // a small one by its longest ray's chain of steps.  The small CTAs save the
 // counter's reset and reads, but a CTA's slots wait for its slowest warp.
 // Counter / small CTAs (us): 256x256 over 128^3 27.7 / 25.3; 1080p images of a
@@ -477,7 +480,8 @@ int launch_trace_image(const svo_octree *oct, const float *d_rays, uint32_t widt
     J.tab = octree_table(oct, st);
     const uint64_t slots = (uint64_t)J.tiles_x * ((height + kImageTileH - 1) / kImageTileH) * 32;  // at most 2^35
     uint32_t *const to = status ? status : oct->d_status, *const carry = status ? oct->d_status : nullptr;
-    if (slots > kImageQueue) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (slots > kImageQueue && cudaStreamIsCapturing(st, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone) {
         void (*kern)(JobDev, uint64_t, unsigned long long *, uint32_t *, uint32_t *) =
             J.tab ? (ray_scale != 0.0f ? k_trace_image_queue<true, true> : k_trace_image_queue<true, false>)
                   : (ray_scale != 0.0f ? k_trace_image_queue<false, true> : k_trace_image_queue<false, false>);

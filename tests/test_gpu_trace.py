@@ -623,3 +623,43 @@ def test_large_sets_of_rays(cuda, svo, scenes):
             torch.cuda.synchronize()
             assert equal(image, want) and equal(linear, want)
     assert tree.device_status() == 0
+
+
+@pytest.mark.parametrize("W,H", [(640, 480), (2051, 2053)])
+def test_captured_images_allocate_nothing(cuda, svo, scenes, W, H):
+    """A captured image call is kernels alone, whatever its size: its graph can
+    be instantiated more than once."""
+    import ctypes
+    torch = cuda
+    rt = ctypes.CDLL("/usr/local/cuda/lib64/libcudart.so")
+    tree = svo.VoxelOctree(svo.VoxelData(scenes.sphere_scene(64, 9, 3)))
+    rays = scenes.gpu_camera_rays(scenes.orbit_cameras(1, 5, tree.center())[0], W, H)
+    want, t = torch.zeros(W * H, device="cuda"), torch.zeros(W * H, device="cuda")
+    tree.trace_image(rays, W, H, out={"t": want})
+    torch.cuda.synchronize()
+    st = torch.cuda.Stream()
+    stream, graph, n = ctypes.c_void_p(st.cuda_stream), ctypes.c_void_p(), ctypes.c_size_t()
+    assert rt.cudaStreamBeginCapture(stream, 0) == 0
+    tree.trace_image(rays, W, H, out={"t": t}, stream=st)
+    assert rt.cudaStreamEndCapture(stream, ctypes.byref(graph)) == 0
+    assert rt.cudaGraphGetNodes(graph, None, ctypes.byref(n)) == 0
+    nodes = (ctypes.c_void_p * n.value)()
+    assert rt.cudaGraphGetNodes(graph, nodes, ctypes.byref(n)) == 0
+    kinds = []
+    for node in nodes:
+        kind = ctypes.c_int(-1)
+        assert rt.cudaGraphNodeGetType(ctypes.c_void_p(node), ctypes.byref(kind)) == 0
+        kinds.append(kind.value)
+    assert kinds == [0]  # cudaGraphNodeTypeKernel
+    execs = [ctypes.c_void_p() for _ in range(2)]
+    for e in execs:
+        assert rt.cudaGraphInstantiate(ctypes.byref(e), graph, ctypes.c_ulonglong(0)) == 0
+    for e in execs:
+        t.zero_()
+        torch.cuda.synchronize()
+        assert rt.cudaGraphLaunch(e, stream) == 0
+        st.synchronize()
+        assert torch.equal(t.view(torch.int32), want.view(torch.int32))
+    for e in execs:
+        rt.cudaGraphExecDestroy(e)
+    rt.cudaGraphDestroy(graph)
