@@ -469,7 +469,7 @@ __device__ __forceinline__ void brick_place(const BrickPlaces &a, uint64_t p, ui
 // the cells read after the place.
 template <bool kDense>
 __global__ void __launch_bounds__(kBrickThreads, 6) k_place_brick16(GridGeom g, BrickPlaces at_of,
-                                                                 const uint32_t *__restrict__ bits,
+                                                                 const uint32_t *bits,
                                                                  uint32_t *__restrict__ words, uint64_t W,
                                                                  uint32_t *__restrict__ err) {
     chain_begin();
@@ -617,8 +617,8 @@ __global__ void __launch_bounds__(kBrickThreads, 6) k_place_brick16(GridGeom g, 
 // the place, the bits and the voxels read one after another.
 template <bool kDense>
 __global__ void __launch_bounds__(256) k_place_brick8(BrickPlaces at_of, uint64_t n_dense,
-                                                      const uint32_t *__restrict__ bits,
-                                                      const uint32_t *__restrict__ slot, uint32_t *__restrict__ words,
+                                                      const uint32_t *bits, const uint32_t *slot,
+                                                      uint32_t *__restrict__ words,
                                                       uint64_t W, uint32_t *__restrict__ err) {
     chain_begin();
     const unsigned FULL = 0xffffffffu;

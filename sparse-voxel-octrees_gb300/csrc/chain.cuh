@@ -9,6 +9,11 @@
 // and before any return, so a finished kernel means that those before it have
 // finished too.  Launched in the plain way such a kernel runs as any other.
 //
+// What the kernel before may write is not taken as const __restrict__ and not
+// read by __ldg: both let the compiler move the read over chain_begin() and
+// serve it from the non-coherent cache.  __ldg is for what was complete before
+// the chain began (a wait of the host or a plain launch lies between).
+//
 // chain_next() lets the next kernel's CTAs up earlier, beside this one's last.
 // It pays in a kernel of one wave that ends in a few long warps (a frame's
 // corners: 320x180 of a 1024^3 octree 59.8 -> 57.8 us).  In a build it costs.

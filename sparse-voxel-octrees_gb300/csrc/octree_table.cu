@@ -218,7 +218,7 @@ __global__ void __launch_bounds__(kScanThreads) k_table_tiles(WordOrder t, uint6
 
 // first: the tiles' scan, or null: this tile adds up those before it.  Reports
 // ctl to the host, and as its last word the bitmap's total.
-__global__ void __launch_bounds__(kScanThreads) k_table_rank(WordOrder t, uint64_t n, const uint32_t *__restrict__ first,
+__global__ void __launch_bounds__(kScanThreads) k_table_rank(WordOrder t, uint64_t n, const uint32_t *first,
                                                              uint32_t *__restrict__ report) {
     chain_begin();
     uint32_t before = 0, total;

@@ -388,7 +388,7 @@ __device__ __forceinline__ uint64_t tile_sum(const uint32_t *n, uint64_t i0, uin
     return s;
 }
 
-__global__ void __launch_bounds__(256) k_brick_tiles(const uint32_t *__restrict__ n, uint64_t cells,
+__global__ void __launch_bounds__(256) k_brick_tiles(const uint32_t *n, uint64_t cells,
                                                      uint64_t *__restrict__ tiles, uint32_t *__restrict__ largest) {
     chain_begin();
     uint32_t c[8], most = 0;
@@ -407,7 +407,7 @@ __global__ void __launch_bounds__(256) k_brick_tiles(const uint32_t *__restrict_
 // (packed as above), the largest brick and the error word, and the large
 // triangles' pairs.
 __global__ void __launch_bounds__(256) k_brick_layout(uint32_t *__restrict__ n, uint64_t cells,
-                                                      const uint64_t *__restrict__ tiles, uint32_t *__restrict__ bkey,
+                                                      const uint64_t *tiles, uint32_t *__restrict__ bkey,
                                                       uint32_t *__restrict__ bstart, const uint32_t *largest,
                                                       const uint32_t *err, const unsigned long long *wide_pairs,
                                                       uint64_t *__restrict__ report) {
@@ -463,7 +463,7 @@ __device__ __forceinline__ void put_pair(uint32_t *tri, uint32_t *cell, uint32_t
 constexpr int kBrickSortWarps = 4;
 
 template <bool kCells>
-__global__ void __launch_bounds__(kBrickSortWarps * 32) k_sort_bricks(uint32_t nb, const uint32_t *__restrict__ bstart,
+__global__ void __launch_bounds__(kBrickSortWarps * 32) k_sort_bricks(uint32_t nb, const uint32_t *bstart,
                                                                       uint32_t *tri, uint32_t *cell) {
     chain_begin();
     using Key = PairKey<kCells>;
@@ -495,7 +495,7 @@ __global__ void __launch_bounds__(kBrickSortWarps * 32) k_sort_bricks(uint32_t n
 
 // A CTA per brick of more: a bitonic sort in shared memory.
 template <bool kCells>
-__global__ void __launch_bounds__(256) k_sort_large(uint32_t nb, const uint32_t *__restrict__ bstart, uint32_t *tri,
+__global__ void __launch_bounds__(256) k_sort_large(uint32_t nb, const uint32_t *bstart, uint32_t *tri,
                                                     uint32_t *cell) {
     chain_begin();
     using Key = PairKey<kCells>;
