@@ -496,9 +496,10 @@ typedef struct svo_trace_config {
     int blocks_per_sm;   /* persistent grid = SM count x blocks_per_sm */
     int refill_idle;     /* a warp refills its idle lanes once this many (1..32) are idle; 0 = no
                             refill: a warp takes its next 32 slots once all its lanes finish.  With 0
-                            or 32, no table cache and a blocks_per_sm no lower than what fits, the
+                            or 32, no table cache, up to 2^25 slots and a blocks_per_sm no lower than
+                            what fits of CTAs of block_threads with the registers of reg_cap, the
                             hardware schedules a thread per slot, and block_threads, chunk and reg_cap
-                            have no effect */
+                            have no further effect */
     int steps_per_round; /* traversal steps between refill checks */
     int tile_w;          /* image tile width in pixels: 4, 8, 16 or 32 (tile = tile_w x 32/tile_w) */
     int chunk;           /* ray slots a warp takes from the work queue at once (multiple of 32) */

@@ -868,20 +868,24 @@ int svo_batch_autotune(svo_batch *b, svo_trace_config *best, float *best_ms, svo
     };
     // table cache depths: none; 64 entries (levels 0-1 hold at most 9 nodes,
     // level 2 at most 64 more); 256 entries (levels 0-2 hold at most 73)
-    // (without a cache, launches of a thread per slot do not depend on the CTA
-    // and chunk sizes)
+    // Up to kSlotsMost slots an uncached whole-warp schedule is a thread per slot
+    // whatever the CTA, the chunk and the registers (its blocks_per_sm is no lower
+    // than what fits), so each tile width is timed once.
+    const bool slots = b->total <= kSlotsMost;
     for (int cache : {0, 64, 256})
         for (int bt : {128, 256, 512})
             for (int tw : {4, 8, 16})
                 for (int chunk : {32, 128})
-                    if (cache || b->total > kSlotsMost || (bt == 256 && chunk == 32))
+                    if (cache || !slots || (bt == 256 && chunk == 32))
                         add(bt, 0, 1, tw, chunk, cache);  // whole-warp tiles, no refill
     // lane refill, default build (64 registers) or 48-register build
     for (int cap : {0, 48})
         for (int bt : {128, 256})
-            for (int refill : {8, 16, 32})
+            for (int refill : {8, 16, 32}) {
+                if (slots && refill == 32) continue;
                 for (int steps : {16, 64})
                     for (int tw : {4, 8}) add(bt, refill, steps, tw, 64, 0, cap);
+            }
     cudaEvent_t e0, e1;
     SVO_CUDA_TRY(cudaEventCreate(&e0));
     SVO_CUDA_TRY(cudaEventCreate(&e1));

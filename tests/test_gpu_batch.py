@@ -202,3 +202,14 @@ def test_batch_whole_warp_schedules(cuda, svo, scene, cfg):
         b.launch_graph()
         _check(torch, views, refs)
     assert b.status() == 0
+
+
+def test_autotune_times_a_schedule_once(cuda, svo, scene, tmp_path, monkeypatch):
+    """Refill of whole warps only (32) is no candidate beside none (0) where both
+    are a thread per slot."""
+    monkeypatch.setenv("SVO_AUTOTUNE_CACHE", str(tmp_path / "tune.jsonl"))
+    monkeypatch.setenv("SVO_AUTOTUNE_FORCE", "1")
+    views, _ = scene
+    for k in range(8):
+        cfg, ms = svo.Batch(views[k:]).autotune()
+        assert ms > 0 and cfg.refill_idle in (0, 8, 16)
