@@ -663,3 +663,28 @@ def test_captured_images_allocate_nothing(cuda, svo, scenes, W, H):
     for e in execs:
         rt.cudaGraphExecDestroy(e)
     rt.cudaGraphDestroy(graph)
+
+
+@pytest.mark.parametrize("side,step", [(448, 1), (512, 1), (768, 4)])
+def test_tables_of_large_octrees(cuda, svo, scenes, side, step):
+    """The table's forms by size: a tile scan of its own (from 67 M words), the
+    breadth-first form (from 134 M), and a node list longer than a quarter of
+    the words (mostly single-voxel nodes), which is left to that form."""
+    torch = cuda
+    grid = torch.zeros((side, side, side), dtype=torch.int32, device="cuda")
+    grid[::step, ::step, ::step] = 0x7F4F
+    tree = svo.VoxelOctree(svo.VoxelData(grid, 32 << 30))
+    del grid
+    edge, nodes = 2, 0
+    while edge < 2 * side:
+        nodes += -(-side // max(edge, step)) ** 3
+        edge *= 2
+    words = tree.num_words()
+    assert {448: 1 << 26 < words <= 1 << 27, 512: words > 1 << 27, 768: 1 << 24 < words < 4 * nodes}[side]
+    assert tree.table_size() == nodes
+    rays = scenes.random_rays(200_000, side)
+    tab = _device_trace(cuda, svo, tree, rays)
+    tree.set_table(False)
+    plain = _device_trace(cuda, svo, tree, rays)
+    _assert_same(tab, dict(plain, grey=plain["rgb"][:, 0]))
+    assert 0 < int((tab["hit"] == 1).sum()) < rays.shape[0]
