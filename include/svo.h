@@ -82,10 +82,15 @@ int svo_octree_from_words(const uint32_t *words, uint64_t n_words, const float c
 /* The builds keep their freed scratch memory in a per-device pool of the
  * library for the next build, and destroyed octrees up to 1 GiB of theirs in
  * another; this returns that memory to the driver (after a device
- * synchronisation). */
+ * synchronisation), with what octrees destroyed inside a global stream capture
+ * left behind. */
 int svo_trim_memory(void);
 
-/* Frees the handle and its device memory. */
+/* Frees the handle and its device memory once the device is idle.  Stream
+ * captures in relaxed mode, and in thread-local mode of other threads, go on; a
+ * global one, or a thread-local one of the calling thread, is ended, as by any
+ * cudaFree, and the memory is then freed by the next svo_octree_destroy or
+ * svo_trim_memory outside it. */
 int svo_octree_destroy(svo_octree *oct);
 
 /* Number of 32-bit words (VoxelOctree::_octreeSize, VoxelOctree.hpp:40). */

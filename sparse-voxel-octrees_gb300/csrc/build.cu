@@ -1264,7 +1264,10 @@ __global__ void __launch_bounds__(256) k_place_leaf_runs(uint64_t np, const uint
 // 6 launches and 172 us through bricks: 87 for the bits, 59 to place the
 // bricks, 26 for the five levels above.  Beyond kPyramidBits (a 4096^3 cube or
 // a thin grid in one) the arrays would grow with the cube and not with what it
-// holds, so the bricks are compacted and go through the sorted levels.
+// holds, so the bricks are compacted and go through the sorted levels.  The
+// line lies at the largest cubes measured (2048^3 grids, 1024^3 meshes, whose
+// table of brick counts it bounds too); a cube just past it has not been timed
+// in this form.
 constexpr int kPyramidBits = 21;
 constexpr uint32_t kTopCells = 4096, kTopPlaced = 512;  // going up, coming down
 constexpr int kPyramidMax = kPyramidBits / 3 + 1;  // levels, bricks included

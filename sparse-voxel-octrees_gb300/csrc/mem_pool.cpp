@@ -25,8 +25,7 @@
 // 20 ms kernel held it for 20 ms) and minds no capture of another thread in
 // thread-local or relaxed mode, so the wait is the cudaFree of 256 bytes taken
 // for it: 2 us where another small block keeps their 2 MB mapped, 58 where not
-// (a rebuilt and viewed 200x131x177 volume 169 us with the device's
-// synchronisation, 175 with this).
+// (a rebuilt and viewed 200x131x177 volume takes 165 to 175 us with either).
 // What cannot be waited for (in a global capture, where cudaFree is refused
 // too) is parked until the next octree is destroyed or memory is trimmed.
 #include <cstring>

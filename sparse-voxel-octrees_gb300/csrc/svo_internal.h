@@ -17,7 +17,7 @@
 
 // The opaque handle behind svo_octree*.
 struct svo_octree {
-    uint32_t *d_words = nullptr;  // resident octree words (HBM)
+    uint32_t *d_words = nullptr;  // resident octree words (HBM), the error word behind them
     uint64_t n_words = 0;
     bool plain_words = false;  // from cudaMalloc, not the library's pool
     float center[3] = {0.0f, 0.0f, 0.0f};
@@ -155,7 +155,7 @@ class Report {
 int cache_block_log2(int w, int h, int d, uint64_t mem, uint64_t cell_cost);
 
 // GPU build from a device-resident dense grid (build.cu).  On success the
-// caller owns *d_words (cudaFree).
+// caller owns *d_words (make_handle, or free_words).
 int build_dense_device(const uint32_t *d_grid, int w, int h, int d, int log_side, int log_block, cudaStream_t st,
                        uint32_t **d_words, uint64_t *n_words);
 
